@@ -338,24 +338,61 @@ __device__ __forceinline__ bool neutral_col(uint32_t q, uint32_t r) {
     return q < 4 && r < 4 && (q == r || (r == 0 && q == 2) || (r == 3 && q == 1));
 }
 
-// Step kinds recorded by the first traceback walk (4 bits each) so the second
-// walk replays from registers/local memory instead of re-reading the
-// traceback words: M with a match / mismatch / zero (editing-exempt) score,
-// I or D opening a gap run (walk order), I or D extending it.
+// Step kinds of a traceback walk: M with a match / mismatch / zero
+// (editing-exempt) score, I or D opening a gap run (walk order), I or D
+// extending it.
 enum : int { K_MM = 0, K_MX = 1, K_MZ = 2, K_IO = 3, K_IE = 4, K_DO = 5, K_DE = 6 };
-constexpr int REC_WORDS = 64;  // 512 recorded steps; longer walks re-walk
+constexpr int REC_RUNS = 64;  // recorded runs of equal steps; walks with more walk twice
 constexpr int RUNS_LOCAL = 16;  // CIGAR runs kept in the thread's own list
 
 __device__ __forceinline__ int kind_op(int k) { return k < 3 ? ESP_OP_M : (k < 5 ? ESP_OP_I : ESP_OP_D); }
 
+// The 32 bases ending at position q - 1 of a sequence, base q - 1 in bits
+// 1:0, q - 2 in bits 3:2, ...; zeros above the sequence's first base.
+// Reads no word past the one after the word that holds base q - 1.
+__device__ __forceinline__ uint64_t tail32(const uint8_t *__restrict__ arena, uint64_t pos, int q) {
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(arena);
+    const int q0 = q >= 32 ? q - 32 : 0;
+    const uint64_t p0 = pos + (uint64_t)q0, wi = p0 >> 4, wl = (pos + (uint64_t)(q - 1)) >> 4;
+    const uint32_t sh = (uint32_t)(p0 & 15) * 2;
+    const uint32_t a = __byte_perm(__ldg(w + wi), 0, 0x0123);
+    const uint32_t b = __byte_perm(__ldg(w + wi + 1), 0, 0x0123);
+    const uint32_t c = __byte_perm(__ldg(w + (wi + 2 <= wl + 1 ? wi + 2 : wl + 1)), 0, 0x0123);
+    const uint64_t v = ((uint64_t)__funnelshift_l(b, a, sh) << 32) | __funnelshift_l(c, b, sh);
+    return v >> (2 * (32 - (q - q0)));
+}
+
+// Bases between position q and the nearest N below it (q itself when there
+// is none): how far a run of matches ending at q - 1 may reach.
+__device__ __forceinline__ int n_free(const esp_n_interval *iv, uint32_t cnt, int q) {
+    int room = q;
+    for (uint32_t k = 0; k < cnt; k++)
+        if ((int)iv[k].start < q) room = min(room, q - min((int)iv[k].end, q));
+    return room;
+}
+
 // One traceback walk over the packed bits (extend.rs:884-930): state machine
 // H/E/F from (best_i, best_j), stopping at i <= 0, j <= 0, outside the row
-// window, or on an H START cell.  Word loads are cached and the word of the
-// next column is prefetched (most steps move one column left in the strip);
-// the read and window codes at the walk's position ride in shift registers
-// that move with it (reloaded 16 bases at a time), and each step's kind and
-// next state are chosen by selects, so that the lanes' walks, which take
-// different kinds of steps, do not split on branches.
+// window, or on an H START cell.
+//
+// A matching base in state H always steps along the diagonal, whatever the
+// traceback word says, so the walk takes a run of matches in one move from
+// the sequences alone and reads a word only at the other steps.  Why: with
+// match the largest substitution score, match > 0 and gap costs >= 0, take
+// an in-window cell (i, j) of equal bases whose predecessor (i-1, j-1) is in
+// the window too.  A path into E(i, j) that leaves row i-k in H, shifted one
+// column left, runs inside the window (row windows move right by 0 or 1
+// columns a row) and shows H(i-1, j-1) >= E(i, j) - match; the same for
+// F(i, j) and a path shifted up one row.  So the diagonal's value is >= E, F
+// and > 0, and diagonal wins ties: hsrc is diag.  On the matrix border (i = 1
+// or j = 1) E and F are at most match, and the same holds.  Only where the
+// predecessor lies outside the window (the left edge of a band clamped at
+// the window's end) is the word read for a match.  `skip` is K.match_skip.
+//
+// A read of a 2 % error rate so costs its ~4 mismatches and a 32-base
+// compare per 32 bases instead of ~175 dependent word loads and state steps;
+// measured on one GB300: 4,194,304 mixed pairs 49.8 -> 43.9 ms, one
+// extend_hint call 146 -> 109 us.
 template <int TBS>
 struct Walker {
     const Geo &g;
@@ -365,104 +402,66 @@ struct Walker {
     const Seq &win;
     const GotohConst &K;
     int i, j, state;
-    int cs, cclo;          // current strip and its first column
-    int pdelta, pmin;      // word index offset of (i-8, j-8) and the first j it exists for
-    int ck, nk;            // cached / prefetched word index
-    uint32_t cw, nw;
 
     __device__ Walker(const Geo &g_, const uint32_t *tb_, int sw_, const Seq &r_, const Seq &w_,
                       const GotohConst &K_, int bi, int bj)
-        : g(g_), tb(tb_), sw(sw_), read(r_), win(w_), K(K_), i(bi), j(bj), state(0), cs(-1),
-          cclo(0), pdelta(0), pmin(0x7fffffff), ck(-1), nk(-1), cw(0), nw(0) {}
+        : g(g_), tb(tb_), sw(sw_), read(r_), win(w_), K(K_), i(bi), j(bj), state(0) {}
 
-    // codes of read position i-1 and window position j-1 at bits 1:0 (N
-    // flag at bit 0 of rnb / wnb); rleft / wleft = positions below still
-    // in the register (< 0: reload)
-    uint32_t rv = 0, wv = 0, rnb = 0, wnb = 0;
-    int rleft = -1, wleft = -1;
-    __device__ __forceinline__ void rfill() {
-        const int q = i - 1, q0 = q >= 15 ? q - 15 : 0, k = q - q0;
-        rv = load16(read.arena, read.pos + (uint64_t)q0) >> (30 - 2 * k);
-        rnb = read.cnt ? nmask16(read.iv, read.cnt, q0) >> (31 - k) : 0u;
-        rleft = k;
-    }
-    __device__ __forceinline__ void wfill() {
-        const int q = j - 1, q0 = q >= 15 ? q - 15 : 0, k = q - q0;
-        wv = load16(win.arena, win.pos + (uint64_t)q0) >> (30 - 2 * k);
-        wnb = win.cnt ? nmask16(win.iv, win.cnt, q0) >> (31 - k) : 0u;
-        wleft = k;
-    }
-    __device__ __forceinline__ void idec() {
-        i--;
-        rv >>= 2;
-        rnb >>= 1;
-        rleft--;
-    }
-    __device__ __forceinline__ void jdec() {
-        j--;
-        wv >>= 2;
-        wnb >>= 1;
-        wleft--;
-    }
-
-    // Take one step; returns false when the walk stops.  `kind` is the step.
-    __device__ __forceinline__ bool step(int &kind) {
+    // Take a run of `len` matches (0..32) and then one step of `kind` (-1:
+    // none this time).  Returns false when the walk stops (with len = 0).
+    __device__ __forceinline__ bool next(int &len, int &kind) {
+        len = 0;
+        kind = -1;
         if (i <= 0 || j <= 0) return false;
         if (j < g.lo(i) || j > g.hi(i)) return false;
-        int s = (i - 1) >> 3, r = (i - 1) & 7;
-        if (s != cs) {
-            cs = s;
-            cclo = g.lo(s * STRIP + 1);
-            if (TBS == 32 && s > 0) {  // (i-8, j-8) lies in strip s-1, row r
-                const int pclo = g.lo((s - 1) * STRIP + 1);
-                pdelta = cclo - pclo - sw - 8;
-                pmin = pclo + 8;
+        uint32_t q = 4, rc = 4;  // base codes at the walk's position (state H)
+        if (state == 0) {
+            const uint64_t rv = tail32(read.arena, read.pos, i), wv = tail32(win.arena, win.pos, j);
+            uint64_t d = rv ^ wv;
+            d = (d | (d >> 1)) & 0x5555555555555555ull;
+            int room = min(min(i, j), 32), rn = i, wn = j;
+            if (read.cnt) rn = n_free(read.iv, read.cnt, i);
+            if (win.cnt) wn = n_free(win.iv, win.cnt, j);
+            room = min(room, min(rn, wn));
+            int run = min(room, d ? (__ffsll((long long)d) - 1) >> 1 : 32);
+            // every predecessor in the window: i - lo(i) - j grows upwards
+            // along the diagonal, so the lowest one decides
+            const int e = run == i || run == j ? run - 1 : run;
+            if (!K.match_skip || (e > 0 && j - e < g.lo(i - e))) run = 0;
+            if (run) {
+                len = run;
+                i -= run;
+                j -= run;
+                if (run == 32 || i <= 0 || j <= 0) return true;
+                if (j < g.lo(i)) return true;  // the next call stops there
+                rn -= run;
+                wn -= run;
             }
+            q = rn == 0 ? 4u : (uint32_t)(rv >> (2 * run)) & 3u;
+            rc = wn == 0 ? 4u : (uint32_t)(wv >> (2 * run)) & 3u;
         }
         // word indices fit 32 bits: a slot holds at most 4,096 strips of
         // 32,767 columns
-        const int idx = s * sw + (j - cclo);
-        uint32_t w;
-        if (idx == ck) {
-            w = cw;
-        } else if (idx == nk) {
-            w = nw;
-        } else {
-            w = tb[(size_t)(uint32_t)idx * TBS];
-        }
-        ck = idx;
-        cw = w;
-        if (j - 1 >= cclo) {  // prefetch the word one column left (same strip)
-            nk = idx - 1;
-            nw = tb[(size_t)(uint32_t)nk * TBS];
-        } else {
-            nk = -1;
-        }
-        // L2 prefetch of the word 8 diagonal steps ahead (the lane-interleaved
-        // global traceback of the thread kernels): the walk mostly runs
-        // along the diagonal, and the lines it reads have left L2 since the
-        // fill wrote them
-        if (TBS == 32 && s > 0 && j >= pmin) {
-            const uint32_t *pa = tb + (size_t)(uint32_t)(idx + pdelta) * TBS;
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(pa));
-        }
-        int sh = 2 * (7 - r);
-        uint32_t hsrc = (w >> sh) & 3u;
-        uint32_t eo = (w >> (16 + sh)) & 1u;
-        uint32_t fo = (w >> (17 + sh)) & 1u;
+        const int s = (i - 1) >> 3, r = (i - 1) & 7;
+        const uint32_t idx = (uint32_t)(s * sw + (j - g.lo(s * STRIP + 1)));
+        const uint32_t w = tb[(size_t)idx * TBS];
+        const int sh = 2 * (7 - r);
+        const uint32_t hsrc = (w >> sh) & 3u;
+        const uint32_t eo = (w >> (16 + sh)) & 1u;
+        const uint32_t fo = (w >> (17 + sh)) & 1u;
         // the step's source: the cell's H tag in state 0, else the gap it is in
         const uint32_t eff = state == 0 ? hsrc : (state == 1 ? 1u : 0u);
-        if (eff == 3u) return false;  // H_START
-        if (rleft < 0) rfill();
-        if (wleft < 0) wfill();
-        const uint32_t q = (rnb & 1u) ? 4u : (rv & 3u), rc = (wnb & 1u) ? 4u : (wv & 3u);
+        if (eff == 3u) {  // H_START: the walk ends after the run just taken
+            i = 0;
+            return len != 0;
+        }
         const int open = state == 0;
         const int kdiag = (int)((K.dkind >> (2 * (q * 5 + rc))) & 3u);
         const int kvert = open ? K_IO : K_IE, khor = open ? K_DO : K_DE;
         kind = eff == 2u ? kdiag : (eff == 1u ? kvert : khor);
         state = eff == 2u ? 0 : (eff == 1u ? (eo ? 0 : 1) : (fo ? 0 : 2));
-        if (eff != 0u) idec();
-        if (eff != 1u) jdec();
+        if (eff != 0u) i--;
+        if (eff != 1u) j--;
         return true;
     }
 };
@@ -485,45 +484,54 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
                           const uint32_t *tb, int sw, int m, int n, const Seq &read,
                           const Seq &win, const FillResult &F, esp_extension &o, uint32_t *cig,
                           uint32_t cap) {
-    const int dtab[7] = {K.match, (int)K.lut[1], 0, K.open_ext, K.ext, K.open_ext, K.ext};
-    // Walk 1 records each 8-step block of the walk: its steps' kinds (rec),
-    // the prefix sum before it (pst) and its largest prefix sum (bmx), so
-    // that the trim below finds its cut by blocks instead of re-walking.
-    uint32_t rec[REC_WORDS];
-    int pst[REC_WORDS], bmx[REC_WORDS];
-    // walk 1: number of steps N, total T and trail (the walk's steps up to
-    // and including its last non-positive prefix sum)
-    int N = 0, P = 0, trail = 0;
+    auto delta_of = [&](int kind) {  // score of one step
+        return kind < 3 ? (kind == K_MM ? K.match : (kind == K_MX ? (int)K.lut[1] : 0))
+                        : ((kind & 1) ? K.open_ext : K.ext);
+    };
+    // Walk 1 records the walk as runs of equal steps (len << 3 | kind) and
+    // finds its number of steps N, its total T and trail (its steps up to and
+    // including the last non-positive prefix sum).
+    uint32_t rec[REC_RUNS];
+    int n_rec = 0, N = 0, P = 0, trail = 0;
     {
         Walker<TBS> W(g, tb, sw, read, win, K, F.best_i, F.best_j);
-        int kind;
-        uint32_t acc = 0;  // the open block's kinds, entering at the top
-        int bm = INT_MIN, pb = 0;
-        while (W.step(kind)) {
-            P += dtab[kind];
-            bm = max(bm, P);
-            acc = (acc >> 4) | ((uint32_t)kind << 28);
-            N++;
-            if ((N & 7) == 0) {
-                if ((N >> 3) <= REC_WORDS) {
-                    rec[(N >> 3) - 1] = acc;
-                    pst[(N >> 3) - 1] = pb;
-                    bmx[(N >> 3) - 1] = bm;
+        uint32_t open = 0;  // the run being extended (0: none yet)
+        auto add = [&](int kind, int len) {
+            if (open && (int)(open & 7u) == kind) {
+                open += (uint32_t)len << 3;
+            } else {
+                if (open) {
+                    if (n_rec < REC_RUNS) rec[n_rec] = open;
+                    n_rec++;
                 }
-                bm = INT_MIN;
-                pb = P;
+                open = ((uint32_t)len << 3) | (uint32_t)kind;
             }
-            if (P <= 0) trail = N;
+        };
+        int len, kind;
+        while (W.next(len, kind)) {
+            if (len) {  // match > 0 here: the prefix sums of the run rise
+                if (P < 0) {
+                    const int k = min(len, -P / K.match);
+                    if (k) trail = N + k;
+                }
+                P += len * K.match;
+                N += len;
+                add(K_MM, len);
+            }
+            if (kind >= 0) {
+                P += delta_of(kind);
+                N++;
+                if (P <= 0) trail = N;
+                add(kind, 1);
+            }
         }
-        if ((N & 7) && (N >> 3) < REC_WORDS) {
-            rec[N >> 3] = acc >> (4 * (8 - (N & 7)));
-            pst[N >> 3] = pb;
-            bmx[N >> 3] = bm;
+        if (open) {
+            if (n_rec < REC_RUNS) rec[n_rec] = open;
+            n_rec++;
         }
     }
-    const bool replay = N <= REC_WORDS * 8;
     const int T = P;
-    uint32_t read_start, ref_start, read_end, ref_end;
+    uint32_t read_start = 0, ref_start = 0, read_end = 0, ref_end = 0;
     int score = 0;
     CigarOut co{cig, cap, false};
     uint32_t K_runs = 0;  // kept runs in walk order: rr, or from cig[2] when many
@@ -548,171 +556,92 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
         ref_start = (uint32_t)max(F.best_j, 0);
         read_end = read_start;
         ref_end = ref_start;
-    } else if (replay) {
+    } else {
         // With walk-order prefix sums P_t, the reference's forward lead is
         // N-1-u where u is the first index in [-1, N-2] with P_u >= T
-        // (P_-1 = 0): the first block whose largest prefix sum reaches T
-        // holds it (the last block always does, through P_N-1 = T, but
-        // only its steps up to N-2 count).  The kept steps are walk indices
-        // [trail, u] -- through N-1 when no u exists -- and lead + trail >=
-        // N (the degenerate keep-the-middle case, extend.rs:956-960) is
-        // exactly u < trail, or T <= 0.
-        int ue = N - 1, Pue = T;
-        bool degenerate = T <= 0;
-        if (!degenerate) {
-            const int nb = (N + 7) >> 3;
-            for (int b = 0; b < nb; b++) {
-                if (bmx[b] < T) continue;
-                int Pb = pst[b];
-                uint32_t w = rec[b];
-                const int tend = min(8 * b + 7, N - 2);
-                int t = 8 * b;
-                for (; t <= tend; t++, w >>= 4) {
-                    Pb += dtab[w & 15u];
-                    if (Pb >= T) break;
-                }
-                if (t <= tend) {
-                    ue = t;
-                    Pue = Pb;
-                    degenerate = t < trail;
-                }
-                break;
-            }
-        }
-        if (degenerate) {  // the middle step t* = N-1-N/2 alone
-            const int tstar = N - 1 - N / 2;
-            int i = F.best_i, j = F.best_j, op = 0, d = 0;
-            for (int t = 0; t <= tstar; t++) {
-                const int kind = (int)((rec[t >> 3] >> (4 * (t & 7))) & 15u);
-                op = kind_op(kind);
-                d = dtab[kind];
-                if (t == tstar) break;
-                if (op != ESP_OP_D) i--;
-                if (op != ESP_OP_I) j--;
-            }
-            read_end = (uint32_t)i;
-            ref_end = (uint32_t)j;
-            read_start = (uint32_t)(op != ESP_OP_D ? i - 1 : i);
-            ref_start = (uint32_t)(op != ESP_OP_I ? j - 1 : j);
-            score = d;
-            emit((1u << 4) | (uint32_t)op);
-            first_op = last_op = op;
-        } else {
-            // the cell the walk stood on before step `trail` and the prefix
-            // sum there, from the record
-            int tr_i = F.best_i, tr_j = F.best_j, ptrail = 0;
-            for (int t = 0; t < trail; t++) {
-                const int kind = (int)((rec[t >> 3] >> (4 * (t & 7))) & 15u);
-                const int op = kind_op(kind);
-                ptrail += dtab[kind];
-                if (op != ESP_OP_D) tr_i--;
-                if (op != ESP_OP_I) tr_j--;
-            }
-            // runs of steps [trail, ue] in walk order; the kept region ends
-            // (forward order) where the walk stood before step `trail`
-            read_end = (uint32_t)tr_i;
-            ref_end = (uint32_t)tr_j;
-            uint32_t w = rec[trail >> 3] >> (4 * (trail & 7));
-            last_op = kind_op((int)(w & 15u));
-            int cur_op = last_op;
-            uint32_t cur_len = 0, di = 0, dj = 0;
-            for (int t = trail; t <= ue; t++) {
-                if ((t & 7) == 0) w = rec[t >> 3];
-                const int op = kind_op((int)(w & 15u));
-                w >>= 4;
-                if (op != cur_op) {
-                    emit((cur_len << 4) | (uint32_t)cur_op);
-                    if (cur_op != ESP_OP_D) di += cur_len;
-                    if (cur_op != ESP_OP_I) dj += cur_len;
-                    cur_op = op;
-                    cur_len = 0;
-                }
-                cur_len++;
-            }
-            emit((cur_len << 4) | (uint32_t)cur_op);
-            if (cur_op != ESP_OP_D) di += cur_len;
-            if (cur_op != ESP_OP_I) dj += cur_len;
-            first_op = cur_op;
-            read_start = read_end - di;
-            ref_start = ref_end - dj;
-            score = Pue - ptrail;
-        }
-    } else {
-        // Walks longer than the record: walk 2 re-walks the traceback,
-        // finding u (as above) on the way.  Step t* (the middle step) is
-        // captured in case the degenerate case comes up.
-        bool degenerate = (T <= 0);  // u = -1
+        // (P_-1 = 0).  The kept steps are walk indices [trail, u] -- through
+        // N-1 when no u exists -- and lead + trail >= N (the degenerate
+        // keep-the-middle case, extend.rs:956-960) is exactly u < trail, or
+        // T <= 0: then step tstar alone is kept, captured on the way.  A run
+        // of equal steps crosses T at most once, and only rising.
+        bool degenerate = T <= 0, done = false;
         const int tstar = N - 1 - N / 2;
-        Walker<TBS> W(g, tb, sw, read, win, K, F.best_i, F.best_j);
         int i = F.best_i, j = F.best_j;
-        int pos_acc = 0;
-        bool found = false;
+        int t0 = 0, P0 = 0, ptrail = 0;
+        int ts_i = 0, ts_j = 0, ts_op = 0, ts_d = 0;
         int cur_op = -1;
         uint32_t cur_len = 0;
-        read_end = ref_end = read_start = ref_start = 0;
-        int ts_ib = 0, ts_jb = 0, ts_ia = 0, ts_ja = 0, ts_op = 0, ts_d = 0;
-        bool done = false;
-        for (int t = 0; t < N && !done; t++) {
-            int i_before = i, j_before = j;
-            int kind;
-            W.step(kind);
-            int op = kind_op(kind), d = dtab[kind];
-            if (op != ESP_OP_D) i--;
-            if (op != ESP_OP_I) j--;
-            if (t == tstar) {
-                ts_ib = i_before;
-                ts_jb = j_before;
-                ts_ia = i;
-                ts_ja = j;
+        auto take = [&](int kind, int len) {
+            const int op = kind_op(kind), d = delta_of(kind);
+            const int di = op != ESP_OP_D, dj = op != ESP_OP_I;
+            if (tstar >= t0 && tstar < t0 + len) {
+                ts_i = i - di * (tstar - t0);
+                ts_j = j - dj * (tstar - t0);
                 ts_op = op;
                 ts_d = d;
             }
-            pos_acc += d;
-            if (!degenerate && !found && t <= N - 2 && pos_acc >= T) {
-                found = true;
-                if (t < trail) degenerate = true;  // nothing emitted yet
-            }
-            if (degenerate) {
-                if (t >= tstar) done = true;
-                continue;
-            }
-            if (t >= trail) {
-                if (t == trail) {
-                    read_end = (uint32_t)i_before;
-                    ref_end = (uint32_t)j_before;
-                    last_op = op;
-                }
-                score += d;
-                if (op == cur_op) {
-                    cur_len++;
-                } else {
-                    if (cur_op >= 0) emit((cur_len << 4) | (uint32_t)cur_op);
-                    cur_op = op;
-                    cur_len = 1;
-                }
-                first_op = op;
-                if (found) {  // t == u_min: the kept region starts here
-                    read_start = (uint32_t)i;
-                    ref_start = (uint32_t)j;
+            int end = t0 + len - 1;
+            if (!degenerate && d > 0 && P0 + d * len >= T) {  // P0 < T here
+                const int u = t0 + (T - P0 + d - 1) / d - 1;
+                if (u <= N - 2) {
+                    end = u;
                     done = true;
+                    degenerate = u < trail;
                 }
+            }
+            if (!degenerate && end >= trail) {
+                const int a = max(t0, trail);
+                if (cur_op < 0) {  // the kept region's end (forward order)
+                    read_end = (uint32_t)(i - di * (a - t0));
+                    ref_end = (uint32_t)(j - dj * (a - t0));
+                    ptrail = P0 + d * (a - t0);
+                    last_op = op;
+                    cur_op = op;
+                }
+                if (op != cur_op) {
+                    emit((cur_len << 4) | (uint32_t)cur_op);
+                    cur_op = op;
+                    cur_len = 0;
+                }
+                cur_len += (uint32_t)(end - a + 1);
+            }
+            const int k = end - t0 + 1;
+            i -= di * k;
+            j -= dj * k;
+            P0 += d * k;
+            t0 += k;
+            if (degenerate) {  // run on to tstar (it may lie past this end)
+                i -= di * (len - k);
+                j -= dj * (len - k);
+                t0 += len - k;
+                done = t0 > tstar;
+            }
+        };
+        if (n_rec <= REC_RUNS) {
+            for (int k = 0; k < n_rec && !done; k++) take((int)(rec[k] & 7u), (int)(rec[k] >> 3));
+        } else {  // more runs than the record holds: walk again
+            Walker<TBS> W(g, tb, sw, read, win, K, F.best_i, F.best_j);
+            int len, kind;
+            while (!done && W.next(len, kind)) {
+                if (len) take(K_MM, len);
+                if (kind >= 0 && !done) take(kind, 1);
             }
         }
         if (degenerate) {
-            read_end = (uint32_t)ts_ib;
-            ref_end = (uint32_t)ts_jb;
-            read_start = (uint32_t)ts_ia;
-            ref_start = (uint32_t)ts_ja;
+            read_end = (uint32_t)ts_i;
+            ref_end = (uint32_t)ts_j;
+            read_start = (uint32_t)(ts_i - (ts_op != ESP_OP_D));
+            ref_start = (uint32_t)(ts_j - (ts_op != ESP_OP_I));
             score = ts_d;
             K_runs = 0;
             emit((1u << 4) | (uint32_t)ts_op);
             first_op = last_op = ts_op;
         } else {
-            if (cur_op >= 0) emit((cur_len << 4) | (uint32_t)cur_op);
-            if (!found) {  // lead = 0: kept through the last step
-                read_start = (uint32_t)i;
-                ref_start = (uint32_t)j;
-            }
+            emit((cur_len << 4) | (uint32_t)cur_op);
+            first_op = cur_op;
+            read_start = (uint32_t)i;
+            ref_start = (uint32_t)j;
+            score = P0 - ptrail;
         }
     }
     // reverse the kept runs into forward order (a long CIGAR's, in place)
@@ -880,6 +809,12 @@ __device__ __forceinline__ bool finish_pair(const GotohJob &job, const GotohCons
                                             PairSetup &S, const FillResult &F,
                                             const uint32_t *tb, bool queue = true) {
     esp_extension &o = S.o;
+    // A touched band escalates whatever its score: the second attempt writes
+    // the pair's record and CIGAR, so the first one's are not built.
+    if (job.mode == 1 && !S.full && F.trow != 0) {
+        if (queue) job.esc_list[atomicAdd(job.esc_count, 1u)] = pi;
+        return true;
+    }
     dp_finish<TBS>(K, lut, S.g, tb, S.sw, S.m, S.n, S.read, S.win, F, o, S.cig,
                    job.cigar_stride);
     if (F.trow) {
@@ -890,9 +825,9 @@ __device__ __forceinline__ bool finish_pair(const GotohJob &job, const GotohCons
     }
     bool esc = false;
     if (job.mode == 1 && !S.full) {
-        // escalate on a band-edge touch or < 85% of perfect
+        // escalate (on a band-edge touch, above, or) below 85% of perfect
         int perfect = S.m * K.match;
-        if (F.trow != 0 || o.score * 20 < perfect * 17) {
+        if (o.score * 20 < perfect * 17) {
             if (queue) job.esc_list[atomicAdd(job.esc_count, 1u)] = pi;
             o.escalated = 1;
             esc = true;
@@ -1634,6 +1569,8 @@ int make_gotoh_const(const esp_extend_params &p, GotohConst &k) {
     int smax = 0;
     for (int i = 0; i < 25; i++) smax = lut[i] > smax ? lut[i] : smax;
     k.max_m = smax > 0 ? 8191 / smax : 32767;
+    // a walk may take matches without reading the traceback (Walker::next)
+    k.match_skip = p.match_score > 0 && p.match_score == smax;
     // traceback kind of a diagonal step by read code * 5 + window code:
     // K_MM for equal ACGT codes, K_MZ for the edit-tolerated pair, K_MX
     // otherwise (a match and a tolerated pair exclude each other)
