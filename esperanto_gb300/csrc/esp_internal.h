@@ -14,8 +14,7 @@ namespace esp {
 // Device copy of the scoring constants (derived once per call from
 // esp_extend_params; see gotoh.cu for the scaled-key arithmetic).
 struct GotohConst {
-    int32_t oe1;        // 4*open_ext - 1  (E open key, low bits 01)
-    int32_t oe4;        // 4*open_ext      (F open key, low bits 10 after + Hp)
+    int32_t oe4;        // 4*open_ext      (gap-open key, low bits 10 after + Hp)
     int32_t ex4;        // 4*ext
     int32_t open_ext;   // -(gap_open + gap_ext)
     int32_t ext;        // -gap_ext
@@ -24,6 +23,7 @@ struct GotohConst {
     uint32_t lut4[5][2];  // per read code: bytes = 4*score vs ref codes 0..7 (4..7 = N)
     int8_t lut[25];       // SubstLut scores[read*5 + ref] (raw, for traceback deltas)
     int32_t max_m;        // longest read whose scores fit the int16 row buffer
+    int32_t smax;         // largest substitution score (>= 0): H <= read length * smax
     int32_t match_skip;   // match > 0 is the largest substitution score: matches step diagonally
     uint64_t dkind;       // traceback kind of a diagonal step (2 bits) by read code * 5 + ref code
 };

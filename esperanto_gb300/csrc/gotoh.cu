@@ -21,15 +21,21 @@
 // Scaled-key arithmetic (what makes the reference's tie cascade cheap):
 // every score is held as 4*v plus a 2-bit tag so that a plain integer max
 // performs both the value comparison and the reference's tie preference.
-//   H is held as Hp = 4H + 2.
-//   E key: max(Hp_up + 4*open_ext - 1, E4_up + 4*ext): low bit 1 <=> opened,
+//   H is held as Hp = 4H + 2, E as E1 = 4E + 1, F as F4 = 4F.
+//   Ho = Hp + 4*open_ext opens a gap from a cell, to the right and down: one
+//          add serves both.
+//   E key: max(E1_up + 4*ext, Ho_up): low bits 2 <=> opened, 1 <=> extended,
 //          and an open/extend tie resolves to "open" as `better` (strict >)
 //          does at extend.rs:731.
-//   F key: max(Hp_left + 4*open_ext, F4_left + 4*ext): bit 1 <=> opened.
-//   H key: max(4*diag + 2, 4E + 1, 4F + 0, 3): among equal values diag
-//          beats E beats F (the cascade order of extend.rs:764-777), and the
-//          START tag 3 wins whenever the maximum is 0 (the zero-floor rewrite
-//          of extend.rs:780-782).  hsrc = key & 3: 3 start, 2 diag, 1 E, 0 F.
+//   F key: max(F4_left + 4*ext, Ho_left): low bits 2 <=> opened, 0 <=>
+//          extended; formed as soon as the left cell is (kF), so that a row
+//          carries (Hp, kF) to the next column.
+//   H key: max(4*diag + 2, E1, F4, 3): among equal values diag beats E beats
+//          F (the cascade order of extend.rs:764-777), and the START tag 3
+//          wins whenever the maximum is 0 (the zero-floor rewrite of
+//          extend.rs:780-782).  hsrc = key & 3: 3 start, 2 diag, 1 E, 0 F.
+//   Flags: (kE ^ kF) & 3 has bit 0 clear <=> E opened and bit 1 set <=>
+//          exactly one of E, F opened.
 // Out-of-window cells present H = 0, E = F = NEG to their neighbours exactly
 // as the scalar kernel's margins do (extend.rs:718-759).
 #include <cuda_runtime.h>
@@ -43,7 +49,6 @@
 
 namespace esp {
 
-static constexpr int NEG4 = -32768;  // E/F sentinel in scaled units (int16 min)
 static constexpr int STRIP = 8;
 
 struct Geo {
@@ -77,7 +82,7 @@ struct Seq {
 template <bool WIDE>
 struct StripT {
     using RK = typename std::conditional<WIDE, long long, int>::type;
-    int Hl[STRIP], Fl[STRIP];
+    int Hl[STRIP], kF[STRIP];  // Hp of the column left of the next one; F key of the next one
     RK rk[STRIP];
     uint32_t l0[STRIP], l1[STRIP];
     int lo[STRIP], hi[STRIP];
@@ -98,10 +103,10 @@ __device__ __forceinline__ uint32_t and_u32(uint32_t a, uint32_t m) {
     return d;
 }
 
-// (a | b) & m in one LOP3
-__device__ __forceinline__ uint32_t or_and_u32(uint32_t a, uint32_t b, uint32_t m) {
+// (a ^ b) & m in one LOP3
+__device__ __forceinline__ uint32_t xor_and_u32(uint32_t a, uint32_t b, uint32_t m) {
     uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xA8;" : "=r"(d) : "r"(a), "r"(b), "r"(m));
+    asm("lop3.b32 %0, %1, %2, %3, 0x28;" : "=r"(d) : "r"(a), "r"(b), "r"(m));
     return d;
 }
 
@@ -109,6 +114,14 @@ __device__ __forceinline__ uint32_t and_or_u32(uint32_t a, uint32_t m, uint32_t 
     uint32_t d;
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(m), "r"(o));
     return d;
+}
+
+// What a cell outside its row's window (or the matrix) shows to its
+// neighbours: H = 0, and an E so low that opening from that H = 0 always
+// wins, as it does against the scalar kernel's NEG.
+__device__ __forceinline__ int absent_E(const GotohConst &K) { return K.oe4 + 1; }
+__device__ __forceinline__ uint32_t absent_HE(const GotohConst &K) {
+    return __byte_perm(2u, (uint32_t)absent_E(K), 0x5410);
 }
 
 // One column of one strip.  upH/upE enter as the row above the strip at
@@ -121,31 +134,31 @@ __device__ __forceinline__ uint32_t dp_column(StripT<WIDE> &S, const GotohConst 
                                               uint32_t sel, uint32_t cj, int &upH, int &upE,
                                               int diag) {
     uint32_t wa = 0, wb = 0;
-    int d = diag;
+    int d = diag, upHo = upH + K.oe4;
 #pragma unroll
     for (int r = 0; r < STRIP; r++) {
         int left = S.Hl[r];
-        int kE = max(upE + K.ex4, upH + K.oe1);
-        int kF = max(S.Fl[r] + K.ex4, left + K.oe4);
-        // kE = 0 or 1 and kF = 0 or 2 (mod 4): the two opened flags are
-        // (kE | kF) & 3 (one LOP3); the E tag is E4 + 1 and the key's tag
-        // key - Hp + 2 -- adds, which also issue on the FMA pipe, instead of
-        // logic ops on the saturated ALU pipe
-        int E4 = (int)and_u32((uint32_t)kE, ~3u);
+        int kE = max(upE + K.ex4, upHo);
+        int kF = S.kF[r];
+        int E1 = (int)and_or_u32((uint32_t)kE, ~3u, 1u);
         int F4 = (int)and_u32((uint32_t)kF, ~3u);
         int kd = max(d + prmt_sx(S.l0[r], S.l1[r], sel), 3);  // START tag 3 folded in
-        int key = max(max(kd, E4 + 1), F4);
+        int key = max(max(kd, E1), F4);
         int Hp = (int)and_or_u32((uint32_t)key, ~3u, 2u);
-        wa = mad_u32(wa, 4u, (uint32_t)(key - Hp + 2));
-        wb = mad_u32(wb, 4u, or_and_u32((uint32_t)kE, (uint32_t)kF, 3u));
+        int Ho = Hp + K.oe4;
+        // tags are accumulated as key - Hp = tag - 2 (adds and multiply-adds
+        // issue off the saturated ALU pipe); the 2s are put back at the end
+        wa = mad_u32(wa, 4u, (uint32_t)(key - Hp));
+        wb = mad_u32(wb, 4u, xor_and_u32((uint32_t)kE, (uint32_t)kF, 3u));
         typename StripT<WIDE>::RK rkey;
         if constexpr (WIDE)
             rkey = ((long long)Hp << 15) | (long long)cj;
         else
             rkey = (int)mad_u32((uint32_t)Hp, 32768u, cj);
+        kF = max(F4 + K.ex4, Ho);  // of the next column
         if (MASK) {
-            // An out-of-window cell shows H = 0, E = NEG to the row below and
-            // leaves its row's state alone: before the window that is still
+            // An out-of-window cell shows H = 0 and no E to the row below and
+            // leaves its own row's state alone: before the window that is still
             // the start state, after it Hl keeps H at the window's last
             // column (the strip's bookkeeping reads it; the cells of the row
             // below that follow are out of their window too, as hi(i+1) <=
@@ -154,24 +167,26 @@ __device__ __forceinline__ uint32_t dp_column(StripT<WIDE> &S, const GotohConst 
             if (in) {
                 S.rk[r] = max(S.rk[r], rkey);
                 S.Hl[r] = Hp;
-                S.Fl[r] = F4;
+                S.kF[r] = kF;
             }
-            upH = in ? Hp : 2;
-            upE = in ? E4 : NEG4;
+            upHo = in ? Ho : 2 + K.oe4;
+            upE = in ? E1 : absent_E(K);
         } else {
             S.rk[r] = max(S.rk[r], rkey);
             S.Hl[r] = Hp;
-            S.Fl[r] = F4;
-            upH = Hp;
-            upE = E4;
+            S.kF[r] = kF;
+            upHo = Ho;
+            upE = E1;
         }
         d = left;
     }
-    return __byte_perm(wa, wb, 0x5410);
+    upH = upHo - K.oe4;
+    return __byte_perm(wa + 0xAAAAu, wb, 0x5410);
 }
 
 struct FillResult {
     int bestHp, best_i, best_j;
+    int last_j;  // the best cell is row best_i's first cell of value bestHp in [best_j, last_j]
     int trow;
     bool tleft, tclamp;
 };
@@ -180,11 +195,11 @@ struct FillResult {
 // time.  CHECK = true (strip ramps) tests the row-buffer read (the row above
 // has a value only up to phi) and write (the strip's last row starts at
 // lo7) per column; the interior needs neither test.
-template <int MASK, bool CHECK, bool HASN>
+template <int MASK, bool CHECK, bool HASN, int STR>
 __device__ __forceinline__ void dp_cols(Strip &S, const GotohConst &K, int a, int b, int &diag,
                                         const Seq &win, uint32_t *rb, int plo, int phi, int lo7,
                                         uint32_t *tbp) {
-    uint32_t *rbr = rb + (size_t)(a - plo) * 32;
+    uint32_t *rbr = rb + (size_t)(a - plo) * STR;
     uint32_t cj = 32767u - (uint32_t)a;
     // Interior: the row above is read two columns ahead of its use (the
     // L2 round trip of a row-buffer line is longer than one column of
@@ -193,7 +208,7 @@ __device__ __forceinline__ void dp_cols(Strip &S, const GotohConst &K, int a, in
     uint32_t wn0 = 0, wn1 = 0;
     if (!CHECK) {
         wn0 = rbr[0];
-        if (a + 1 <= b) wn1 = rbr[32];
+        if (a + 1 <= b) wn1 = rbr[STR];
     }
     for (int j = a; j <= b;) {
         uint32_t cw = load16(win.arena, win.pos + (uint64_t)(j - 1));
@@ -205,7 +220,7 @@ __device__ __forceinline__ void dp_cols(Strip &S, const GotohConst &K, int a, in
             cw <<= 2;
             if (HASN) nm <<= 1;
             uint32_t sel = code * 0x1111u + 0x8880u;
-            int bH = 2, bE = NEG4;
+            int bH = 2, bE = absent_E(K);
             if (!CHECK || j <= phi) {
                 uint32_t w;
                 if (CHECK) {
@@ -213,7 +228,7 @@ __device__ __forceinline__ void dp_cols(Strip &S, const GotohConst &K, int a, in
                 } else {
                     w = wn0;
                     wn0 = wn1;
-                    if (j + 2 <= b) wn1 = rbr[64];
+                    if (j + 2 <= b) wn1 = rbr[2 * STR];
                 }
                 bH = (int)(w & 0xffffu);
                 bE = ((int)w) >> 16;
@@ -223,40 +238,41 @@ __device__ __forceinline__ void dp_cols(Strip &S, const GotohConst &K, int a, in
             diag = bH;
             uint32_t packed = __byte_perm((uint32_t)upH, (uint32_t)upE, 0x5410);
             if (CHECK) {
-                if (j >= lo7) rb[(size_t)(j - lo7) * 32] = packed;
+                if (j >= lo7) rb[(size_t)(j - lo7) * STR] = packed;
             } else {
-                rbr[(ptrdiff_t)(plo - lo7) * 32] = packed;  // row-buffer slot j - lo7
+                rbr[(ptrdiff_t)(plo - lo7) * STR] = packed;  // row-buffer slot j - lo7
             }
             *tbp = word;
-            tbp += 32;
-            rbr += 32;
+            tbp += STR;
+            rbr += STR;
             cj--;
         }
     }
 }
 
-// Fill the DP for one pair; traceback words land in tb (stride sw per strip).
+// Fill the DP for one pair; traceback words land in tb (sw words per strip, STR
+// words apart: the lanes of a warp interleave theirs).
 // The row buffer holds sw words: strip 0 reads row 0 (H = 0, E = NEG on every
 // column, extend.rs:664-681) from a prefilled copy, later strips read the last
 // row of the previous strip, which each strip rewrites in place (a slot is
 // always read at or before the column that overwrites it, since the strip's
 // window start lo7 never precedes the previous row's start plo).
-template <bool HASN>
+template <bool HASN, int STR>
 __device__ FillResult dp_fill(const GotohConst &K, const uint32_t *__restrict__ s_lut, int m,
                               int n, const Geo &g, const Seq &read, const Seq &win,
                               uint32_t *tb, int sw, uint32_t *rb) {
     FillResult R;
     R.bestHp = 2;
     R.best_i = 0;
-    R.best_j = 0;
+    R.best_j = R.last_j = 0;
     R.trow = 0;
     R.tleft = false;
     R.tclamp = false;
     int nstrips = (m + STRIP - 1) / STRIP;
     int plo = g.lo(1), phi = g.hi(min(STRIP, m));
     {
-        const uint32_t row0 = __byte_perm(2u, (uint32_t)NEG4, 0x5410);
-        for (int k = 0; k <= phi - plo; k++) rb[(size_t)k * 32] = row0;
+        const uint32_t row0 = absent_HE(K);
+        for (int k = 0; k <= phi - plo; k++) rb[(size_t)k * STR] = row0;
     }
     Strip S;
     for (int s = 0; s < nstrips; s++) {
@@ -267,7 +283,7 @@ __device__ FillResult dp_fill(const GotohConst &K, const uint32_t *__restrict__ 
             S.lo[r] = g.lo(i0 + r);
             S.hi[r] = g.hi(i0 + r);
             S.Hl[r] = 2;
-            S.Fl[r] = NEG4;
+            S.kF[r] = 2 + K.oe4;  // F opened from H = 0
             S.rk[r] = -1;
         }
         int clo = S.lo[0];
@@ -286,14 +302,14 @@ __device__ FillResult dp_fill(const GotohConst &K, const uint32_t *__restrict__ 
         }
         int diag = 2;
         if (clo - 1 >= plo && clo - 1 <= phi)
-            diag = (int)(rb[(size_t)(clo - 1 - plo) * 32] & 0xffffu);
-        uint32_t *tbp = tb + (size_t)s * sw * 32;
+            diag = (int)(rb[(size_t)(clo - 1 - plo) * STR] & 0xffffu);
+        uint32_t *tbp = tb + (size_t)s * sw * STR;
         int a_end = min(lo7, chi);
-        dp_cols<1, true, HASN>(S, K, clo, a_end, diag, win, rb, plo, phi, lo7, tbp);
+        dp_cols<1, true, HASN, STR>(S, K, clo, a_end, diag, win, rb, plo, phi, lo7, tbp);
         int b_beg = lo7 + 1, b_end = min(hi0 - 1, chi);
         if (b_beg <= b_end)
-            dp_cols<0, false, HASN>(S, K, b_beg, b_end, diag, win, rb, plo, phi, lo7,
-                                    tbp + (size_t)(b_beg - clo) * 32);
+            dp_cols<0, false, HASN, STR>(S, K, b_beg, b_end, diag, win, rb, plo, phi, lo7,
+                                    tbp + (size_t)(b_beg - clo) * STR);
         int c_beg = max(lo7 + 1, hi0);
         // the row windows again rather than kept live across the interior
 #pragma unroll
@@ -302,8 +318,8 @@ __device__ FillResult dp_fill(const GotohConst &K, const uint32_t *__restrict__ 
             S.hi[r] = g.hi(i0 + r);
         }
         if (c_beg <= chi)
-            dp_cols<1, true, HASN>(S, K, c_beg, chi, diag, win, rb, plo, phi, lo7,
-                                   tbp + (size_t)(c_beg - clo) * 32);
+            dp_cols<1, true, HASN, STR>(S, K, c_beg, chi, diag, win, rb, plo, phi, lo7,
+                                   tbp + (size_t)(c_beg - clo) * STR);
         // row bookkeeping in row order (extend.rs:795-827)
 #pragma unroll
         for (int r = 0; r < STRIP; r++) {
@@ -324,7 +340,7 @@ __device__ FillResult dp_fill(const GotohConst &K, const uint32_t *__restrict__ 
                 if (rowHp > R.bestHp) {
                     R.bestHp = rowHp;
                     R.best_i = i0 + r;
-                    R.best_j = argj;
+                    R.best_j = R.last_j = argj;
                 }
             }
         }
@@ -447,8 +463,8 @@ struct Walker {
         const uint32_t w = tb[(size_t)idx * TBS];
         const int sh = 2 * (7 - r);
         const uint32_t hsrc = (w >> sh) & 3u;
-        const uint32_t eo = (w >> (16 + sh)) & 1u;
-        const uint32_t fo = (w >> (17 + sh)) & 1u;
+        const uint32_t eo = ~(w >> (16 + sh)) & 1u;
+        const uint32_t fo = ((w >> (17 + sh)) & 1u) ^ eo;
         // the step's source: the cell's H tag in state 0, else the gap it is in
         const uint32_t eff = state == 0 ? hsrc : (state == 1 ? 1u : 0u);
         if (eff == 3u) {  // H_START: the walk ends after the run just taken
@@ -491,10 +507,20 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
     // Walk 1 records the walk as runs of equal steps (len << 3 | kind) and
     // finds its number of steps N, its total T and trail (its steps up to and
     // including the last non-positive prefix sum).
+    // When the best cell's column is known as a range, its columns are walked
+    // in order until one's total is the best score: a walk's total is its
+    // cell's H, and the first such cell is the best one.  (With mismatches
+    // scoring <= 0 it ends on a match: a cell that equals the best by any
+    // other step has an equal cell before it in row order.)
     uint32_t rec[REC_RUNS];
-    int n_rec = 0, N = 0, P = 0, trail = 0;
-    {
-        Walker<TBS> W(g, tb, sw, read, win, K, F.best_i, F.best_j);
+    int n_rec = 0, N = 0, P = 0, trail = 0, best_j = F.best_j;
+    const bool on_match = K.match_skip && K.lut[1] <= 0;
+    for (;; best_j++) {
+        if (on_match && best_j < F.last_j &&
+            read.code(F.best_i - 1) != win.code(best_j - 1))
+            continue;
+        n_rec = N = P = trail = 0;
+        Walker<TBS> W(g, tb, sw, read, win, K, F.best_i, best_j);
         uint32_t open = 0;  // the run being extended (0: none yet)
         auto add = [&](int kind, int len) {
             if (open && (int)(open & 7u) == kind) {
@@ -529,6 +555,7 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
             if (n_rec < REC_RUNS) rec[n_rec] = open;
             n_rec++;
         }
+        if (best_j >= F.last_j || 4 * P + 2 == F.bestHp) break;
     }
     const int T = P;
     uint32_t read_start = 0, ref_start = 0, read_end = 0, ref_end = 0;
@@ -553,7 +580,7 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
     int first_op = -1, last_op = -1;  // forward order first / last kept op
     if (N == 0) {
         read_start = (uint32_t)max(F.best_i, 0);
-        ref_start = (uint32_t)max(F.best_j, 0);
+        ref_start = (uint32_t)max(best_j, 0);
         read_end = read_start;
         ref_end = ref_start;
     } else {
@@ -566,7 +593,7 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
         // of equal steps crosses T at most once, and only rising.
         bool degenerate = T <= 0, done = false;
         const int tstar = N - 1 - N / 2;
-        int i = F.best_i, j = F.best_j;
+        int i = F.best_i, j = best_j;
         int t0 = 0, P0 = 0, ptrail = 0;
         int ts_i = 0, ts_j = 0, ts_op = 0, ts_d = 0;
         int cur_op = -1;
@@ -620,7 +647,7 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
         if (n_rec <= REC_RUNS) {
             for (int k = 0; k < n_rec && !done; k++) take((int)(rec[k] & 7u), (int)(rec[k] >> 3));
         } else {  // more runs than the record holds: walk again
-            Walker<TBS> W(g, tb, sw, read, win, K, F.best_i, F.best_j);
+            Walker<TBS> W(g, tb, sw, read, win, K, F.best_i, best_j);
             int len, kind;
             while (!done && W.next(len, kind)) {
                 if (len) take(K_MM, len);
@@ -842,8 +869,9 @@ __device__ void process_pair(const GotohJob &job, const GotohConst &K,
                              uint32_t pi, uint32_t *tb, uint32_t *rb) {
     PairSetup S;
     if (!setup_pair(job, K, pi, job.tb_words, job.rb_words, true, S)) return;
-    FillResult F = S.win.cnt ? dp_fill<true>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb)
-                             : dp_fill<false>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb);
+    FillResult F =
+        S.win.cnt ? dp_fill<true, 32>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb)
+                  : dp_fill<false, 32>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb);
     finish_pair<32>(job, K, lut, pi, S, F, tb);
 }
 
@@ -903,10 +931,10 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
                                 const PairSetup &P, uint32_t *tb, uint32_t *rb, int lane) {
     const int m = P.m, n = P.n, sw = P.sw;
     const Geo &g = P.g;
-    const uint32_t ABSENT = __byte_perm(2u, (uint32_t)NEG4, 0x5410);  // H = 0, E = NEG
+    const uint32_t ABSENT = absent_HE(K);
     FillResult R;
     R.bestHp = 2;
-    R.best_i = R.best_j = 0;
+    R.best_i = R.best_j = R.last_j = 0;
     R.trow = 0;
     R.tleft = R.tclamp = false;
     const int nstrips = (m + STRIP - 1) / STRIP;
@@ -921,7 +949,7 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
             S.lo[r] = g.lo(i0 + r);
             S.hi[r] = g.hi(i0 + r);
             S.Hl[r] = 2;
-            S.Fl[r] = NEG4;
+            S.kF[r] = 2 + K.oe4;  // F opened from H = 0
             S.rk[r] = -1;
         }
         const int clo = S.lo[0];
@@ -946,7 +974,7 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
         t1 = __reduce_max_sync(0xffffffffu, t1);
         // bottom row published at the end of a step: packed (int16) or H / E (int32)
         uint32_t pub = ABSENT;
-        int pubH = 2, pubE = NEG4;
+        int pubH = 2, pubE = absent_E(K);
         int diag = 2;           // H of the row above at the previous column
         if (lane == 0 && base && clo - 1 >= plo && clo - 1 <= phi)
             diag = WIDE ? (int)rb[2 * (clo - 1 - plo)] : (int)(rb[clo - 1 - plo] & 0xffffu);
@@ -965,7 +993,7 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
                 if (lane == 0) {
                     const bool have = base && j >= plo && j <= phi;
                     inH = have ? (int)rb[2 * (j - plo)] : 2;
-                    inE = have ? (int)rb[2 * (j - plo) + 1] : NEG4;
+                    inE = have ? (int)rb[2 * (j - plo) + 1] : absent_E(K);
                 }
             } else {
                 uint32_t in = __shfl_up_sync(0xffffffffu, pub, 1);
@@ -973,7 +1001,7 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
                 inH = (int)(in & 0xffffu);
                 inE = ((int)in) >> 16;
             }
-            int outH = 2, outE = NEG4;
+            int outH = 2, outE = absent_E(K);
             if (act && j >= clo && j <= chi) {
                 // window codes 16 at a time, each word loaded while the
                 // one before is in use: a load that a lane waits for stalls
@@ -1055,7 +1083,7 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
         if (mx > R.bestHp) {
             R.bestHp = mx;
             R.best_i = wi;
-            R.best_j = wj;
+            R.best_j = R.last_j = wj;
         }
         const uint32_t tm = __ballot_sync(0xffffffffu, trow != 0);
         if (R.trow == 0 && tm) {
@@ -1159,24 +1187,70 @@ cudaError_t launch_gotoh_wide(const GotohJob &job, const GotohConst &k, int warp
 // geometry and N-free windows share one thread: every register holds the
 // scaled key of pair A in its low half and of pair B in its high half, and
 // the half-word operations (add-max, 3-way max) evaluate both cells at once
-// with the arithmetic above (values stay inside int16: H <= 8191 by the
-// score-range rule, gap keys >= -16384 - 4*ext).  Substitution scores of
-// both cells come from one PRMT over the two rows' LUT words.  The traceback
-// words, row maxima and touches of each pair are exactly those of the
-// thread-per-pair kernel, and each pair's traceback is walked by the same
-// code (its words at stride 32, pair B's region after pair A's).
+// with the arithmetic above.  Keys carry a bias of BIAS2 a half, so that all
+// of them are positive and a plain 32-bit add or subtract of two packed
+// constants never carries across the halves (those adds may issue off the
+// saturated ALU pipe): H <= 8191 by the score-range rule and gap costs <=
+// 2,000 a side give keys in [384, 49,152] of an unsigned half.
+// Substitution scores of both cells come from one PRMT over the two rows'
+// LUT words.  Traceback words, row maxima and touches of each pair are
+// exactly those of the thread-per-pair kernel, and each pair's traceback is
+// walked by the same code (pair A's and B's words side by side, stride 64).
+//
+// A row's maximum is one max of keys H*S + (S - 1 - t), where t numbers the
+// strip's columns (in blocks of 2^g columns where S of them do not reach):
+// equal H keeps the first column, as the scalar kernel's strict > does, and
+// the column comes with the maximum.  S, a multiple of 4, is as large as the
+// read's highest score allows in 16 bits (H <= m * match: S = 216 for a
+// 150-base read), and the key is one multiply-add of Hp, off the ALU pipe;
+// keeping the column beside the maximum took three more ALU instructions.
+// Where g > 0 the walk picks the block's column (FillResult::last_j).
+//
+// Strip shapes: where a strip's row windows move right by one column a row
+// (a band away from the matrix edge) its two corners are unrolled as
+// triangles, 28 and 36 cells with no test; where they stand still (the whole
+// matrix, a band clamped at column 1 or n) that side has no corner at all;
+// a strip in which clamping begins or ends tests every cell.  A band of 33
+// columns so computes 272 cells a strip instead of 320, half of them masked.
+//
+// Bound by the ALU pipe (78 % busy in the fill, 13.5 ALU of 23.5 issued
+// instructions a row of two cells; 28.9 ALU before these keys and corners).
+// 4,194,304 mixed pairs: 43.9 -> 38.0 ms.
 // ---------------------------------------------------------------------------
 
-constexpr uint32_t NEG2 = 0xC000C000u;   // E/F sentinel (-16384) in both halves
-constexpr uint32_t VNEG2 = 0x80008000u;  // -32768: max against it is a plain add
+constexpr uint32_t BIAS2 = 0x40004000u;
 constexpr uint32_t KEEP2 = 0xFFFCFFFCu;
+constexpr int PAIR_BLOCK = 128;  // threads of a paired block (stride of the shared first-cell keys)
 
 struct Strip2 {
-    uint32_t Hl[STRIP], Fl[STRIP], rmax[STRIP];
+    uint32_t Hl[STRIP], kF[STRIP], rmax[STRIP];
     uint32_t la[STRIP], lb[STRIP];
-    uint32_t arg[STRIP];   // first column of the row maximum: pair A low half, B high
-    uint32_t lohi[STRIP];  // row window: first column low half, last column high half
 };
+
+struct Keys2 {
+    uint32_t oe;     // 4*(gap_open + gap_ext) in both halves (subtracted)
+    uint32_t ex;     // 4*ext in both halves (as 16-bit adds)
+    uint32_t h0;     // H = 0
+    uint32_t ho0;    // a gap opened from H = 0
+    uint32_t e0;     // the E an out-of-window cell shows
+    uint32_t ks;     // S / 4
+    uint32_t ck0;    // row-max key of Hp at the strip's first column: Hp * ks + ck0
+    int g;           // columns of a row-max key: blocks of 2^g
+};
+
+__device__ __forceinline__ Keys2 keys2_of(const GotohConst &K, int m, int sw) {
+    Keys2 c;
+    c.oe = (uint32_t)(-K.oe4) * 0x10001u;
+    c.ex = (uint32_t)(K.ex4 & 0xffff) * 0x10001u;
+    c.h0 = BIAS2 + 0x00020002u;
+    c.ho0 = c.h0 - c.oe;
+    c.e0 = c.ho0 - 0x00010001u;
+    c.ks = 16384u / (uint32_t)(m * K.smax + 1);
+    c.ck0 = (4u * c.ks - 1u) * 0x10001u - c.h0 * c.ks;
+    c.g = 0;
+    while ((uint32_t)(sw - 1) >> c.g >= 4u * c.ks) c.g++;
+    return c;
+}
 
 __device__ __forceinline__ uint32_t prmt(uint32_t lo, uint32_t hi, uint32_t sel) {
     uint32_t r;
@@ -1184,209 +1258,318 @@ __device__ __forceinline__ uint32_t prmt(uint32_t lo, uint32_t hi, uint32_t sel)
     return r;
 }
 
-// Row maximum and its first column for both lanes.  Hp and the running max
-// are in [0, 32766], so old + 0x8000 - Hp per half neither carries nor
-// borrows across halves and its bit 15 is set exactly when old >= Hp; PRMT's
-// sign-replicate mode spreads that bit into a keep mask per half.
-__device__ __forceinline__ void row_max2(uint32_t &rmax, uint32_t &arg, uint32_t Hp, uint32_t jj) {
-    uint32_t t = rmax + 0x80008000u - Hp;
-    uint32_t keep = prmt(t, 0u, 0xBB99u);
-    rmax = (rmax & keep) | (Hp & ~keep);
-    arg = (arg & keep) | (jj & ~keep);
-}
-
-template <int MASK>
-__device__ __forceinline__ void dp_column2(Strip2 &S, const uint32_t oe1, const uint32_t oe4,
-                                           const uint32_t ex4, int j, uint32_t sel, uint32_t &upH,
-                                           uint32_t &upE, uint32_t diag, uint32_t &wa,
-                                           uint32_t &wb) {
-    wa = 0;
-    wb = 0;
-    uint32_t d = diag;
-    const uint32_t jj = (uint32_t)j * 0x10001u;
+// Rows R0..R1 of one column, top to bottom.  Enters with the row above R0:
+// its Ho and E at this column and its Hp at the previous one (d); leaves with
+// row R1's Ho and E.  Returns the column's traceback words (pair A, pair B).
+template <int R0, int R1>
+__device__ __forceinline__ uint2 dp_rows2(Strip2 &S, const Keys2 &c, uint32_t sel, uint32_t ck,
+                                          uint32_t &upHo, uint32_t &upE, uint32_t d) {
+    uint32_t wa = 0, wb = 0;
 #pragma unroll
-    for (int r = 0; r < STRIP; r++) {
-        uint32_t left = S.Hl[r];
-        uint32_t kE = __viaddmax_s16x2(upE, ex4, __viaddmax_s16x2(upH, oe1, VNEG2));
-        uint32_t kF = __viaddmax_s16x2(S.Fl[r], ex4, __viaddmax_s16x2(left, oe4, VNEG2));
-        // tags by adds and flags by one LOP3 as in dp_column: every half's
-        // result is in [0, 3] (E4 + 1 cannot carry: E4's low bits are 0), so
-        // the packed 32-bit adds are exact per half
-        uint32_t E4 = and_u32(kE, KEEP2);
-        uint32_t F4 = and_u32(kF, KEEP2);
-        uint32_t kd = __viaddmax_s16x2(d, prmt(S.la[r], S.lb[r], sel), 0x00030003u);
-        uint32_t key = __vimax3_s16x2(kd, E4 + 0x00010001u, F4);
-        uint32_t Hp = and_or_u32(key, KEEP2, 0x00020002u);
-        wa = mad_u32(wa, 4u, key - Hp + 0x00020002u);
-        wb = mad_u32(wb, 4u, or_and_u32(kE, kF, 0x00030003u));
-        if (MASK) {  // out-of-window cells: as in dp_column
-            const int lo = (int)(S.lohi[r] & 0xffffu), hi = (int)(S.lohi[r] >> 16);
-            const bool in = (j >= lo) & (j <= hi);
-            if (in) {
-                row_max2(S.rmax[r], S.arg[r], Hp, jj);
-                S.Hl[r] = Hp;
-                S.Fl[r] = F4;
-            }
-            upH = in ? Hp : 0x00020002u;
-            upE = in ? E4 : NEG2;
-        } else {
-            row_max2(S.rmax[r], S.arg[r], Hp, jj);
-            S.Hl[r] = Hp;
-            S.Fl[r] = F4;
-            upH = Hp;
-            upE = E4;
-        }
+    for (int r = R0; r <= R1; r++) {
+        const uint32_t left = S.Hl[r], kF = S.kF[r];
+        const uint32_t kE = __viaddmax_u16x2(upE, c.ex, upHo);
+        upE = and_or_u32(kE, KEEP2, 0x00010001u);
+        const uint32_t F4 = and_u32(kF, KEEP2);
+        const uint32_t kd = __viaddmax_u16x2(d, prmt(S.la[r], S.lb[r], sel), BIAS2 + 0x00030003u);
+        const uint32_t key = __vimax3_u16x2(kd, upE, F4);
+        const uint32_t Hp = and_or_u32(key, KEEP2, 0x00020002u);
+        wa = mad_u32(wa, 4u, key - Hp);
+        wb = mad_u32(wb, 4u, xor_and_u32(kE, kF, 0x00030003u));
+        upHo = Hp - c.oe;
+        S.kF[r] = __viaddmax_u16x2(F4, c.ex, upHo);
+        S.rmax[r] = __vmaxu2(S.rmax[r], mad_u32(Hp, c.ks, ck));
+        S.Hl[r] = Hp;
         d = left;
     }
+    constexpr int SH = 2 * (STRIP - 1 - R1);
+    wa += 0xAAAAAAAAu & ((0x10001u << (2 * (R1 - R0 + 1))) - 0x10001u);  // tags, not tag - 2
+    wa <<= SH;
+    wb <<= SH;
+    return make_uint2(__byte_perm(wa, wb, 0x5410), __byte_perm(wa, wb, 0x7632));
 }
 
-// Columns [a, b] for both pairs; rb holds (H, E) of both pairs per column
-// (one uint2 per lane and column).
-template <int MASK, bool CHECK>
-__device__ __forceinline__ void dp_cols2(Strip2 &S, const uint32_t oe1, const uint32_t oe4,
-                                         const uint32_t ex4, int a, int b, uint32_t &diag,
-                                         const uint8_t *warena, uint64_t wposA, uint64_t wposB,
-                                         uint2 *rb, int plo,
-                                         int phi, int lo7, uint32_t *tbA, uint32_t *tbB) {
-    uint2 *rbr = rb + (size_t)(a - plo) * 32;
-    uint2 wn0 = make_uint2(0u, 0u), wn1 = make_uint2(0u, 0u);
-    if (!CHECK) {  // interior: the row above two columns ahead
-        wn0 = rbr[0];
-        if (a + 1 <= b) wn1 = rbr[32];
+// The same over all 8 rows with every cell tested against its row window
+// (clamping strips): as dp_column's MASK.  hf: the rows' first-cell keys
+// (stride PAIR_BLOCK).  Leaves the last row's Hp in botH.
+__device__ __forceinline__ uint2 dp_masked2(Strip2 &S, const Keys2 &c, const Geo &g, int i0, int j,
+                                            uint32_t sel, uint32_t ck, uint32_t upHo, uint32_t &upE, uint32_t d,
+                                            uint32_t &botH, uint32_t *hf) {
+    uint32_t wa = 0, wb = 0;
+#pragma unroll
+    for (int r = 0; r < STRIP; r++) {
+        const uint32_t left = S.Hl[r], kF = S.kF[r];
+        const uint32_t kE = __viaddmax_u16x2(upE, c.ex, upHo);
+        const uint32_t E1 = and_or_u32(kE, KEEP2, 0x00010001u);
+        const uint32_t F4 = and_u32(kF, KEEP2);
+        const uint32_t kd = __viaddmax_u16x2(d, prmt(S.la[r], S.lb[r], sel), BIAS2 + 0x00030003u);
+        const uint32_t key = __vimax3_u16x2(kd, E1, F4);
+        const uint32_t Hp = and_or_u32(key, KEEP2, 0x00020002u);
+        wa = mad_u32(wa, 4u, key - Hp + 0x00020002u);
+        wb = mad_u32(wb, 4u, xor_and_u32(kE, kF, 0x00030003u));
+        const int lo = g.lo(i0 + r);
+        const bool in = (j >= lo) & (j <= g.hi(i0 + r));
+        if (in) {
+            S.kF[r] = __viaddmax_u16x2(F4, c.ex, Hp - c.oe);
+            S.rmax[r] = __vmaxu2(S.rmax[r], mad_u32(Hp, c.ks, ck));
+            S.Hl[r] = Hp;
+        }
+        if (j == lo) hf[r * PAIR_BLOCK] = S.rmax[r];
+        upHo = in ? Hp - c.oe : c.ho0;
+        upE = in ? E1 : c.e0;
+        d = left;
     }
-    for (int j = a; j <= b;) {
-        uint32_t cwA = load16(warena, wposA + (uint64_t)(j - 1));
-        uint32_t cwB = load16(warena, wposB + (uint64_t)(j - 1));
-        int cnt = min(16, b - j + 1);
-#pragma unroll 1
-        for (int k = 0; k < cnt; k++, j++) {
-            uint32_t sel = (cwA >> 30) * 0x11u + (cwB >> 30) * 0x1100u + 0xC480u;
-            cwA <<= 2;
-            cwB <<= 2;
-            uint2 w = make_uint2(0x00020002u, NEG2);
-            if (CHECK) {
-                if (j <= phi) w = *rbr;
-            } else {
-                w = wn0;
-                wn0 = wn1;
-                if (j + 2 <= b) wn1 = rbr[64];
-            }
-            uint32_t upH = w.x, upE = w.y;
-            uint32_t wa, wb;
-            dp_column2<MASK>(S, oe1, oe4, ex4, j, sel, upH, upE, diag, wa, wb);
-            diag = w.x;
-            uint2 packed = make_uint2(upH, upE);
-            if (CHECK) {
-                if (j >= lo7) rb[(size_t)(j - lo7) * 32] = packed;
-            } else {
-                rbr[(ptrdiff_t)(plo - lo7) * 32] = packed;
-            }
-            // streaming stores: the traceback words make way in L2 for the
-            // row buffer (measured +1.8 % here; the one-pair kernel's own
-            // stores measured 0.8 % slower so)
-            __stcs(tbA, __byte_perm(wa, wb, 0x5410));
-            __stcs(tbB, __byte_perm(wa, wb, 0x7632));
-            tbA += 32;
-            tbB += 32;
-            rbr += 32;
+    botH = upHo + c.oe;
+    return make_uint2(__byte_perm(wa, wb, 0x5410), __byte_perm(wa, wb, 0x7632));
+}
+
+// The codes of both windows from column j on, 16 columns at a time.
+struct Codes2 {
+    uint32_t a, b;
+    int t;        // columns taken so far in this strip
+    uint32_t ck;  // ck0 of the column taken last
+    __device__ __forceinline__ void load(const uint8_t *arena, uint64_t wposA, uint64_t wposB, int j) {
+        a = load16(arena, wposA + (uint64_t)(j - 1));
+        b = load16(arena, wposB + (uint64_t)(j - 1));
+    }
+    // PRMT selector of this column's codes, then on to the next column
+    // (whose row-max keys are 1 lower every 2^g columns)
+    __device__ __forceinline__ uint32_t next(const Keys2 &c) {
+        const uint32_t sel = (a >> 30) * 0x11u + (b >> 30) * 0x1100u + 0xC480u;
+        a <<= 2;
+        b <<= 2;
+        ck = c.ck0 - (uint32_t)(t >> c.g) * 0x10001u;
+        t++;
+        return sel;
+    }
+};
+
+// Columns clo + K of a sloped strip's left corner: rows 0..K.
+template <int K>
+__device__ __forceinline__ void head2(Strip2 &S, const Keys2 &c, Codes2 &w, const uint2 *&rbr,
+                                      uint32_t &diag, uint2 *&tb, uint32_t *hf) {
+    if constexpr (K < STRIP - 1) {
+        const uint2 up = *rbr;
+        uint32_t upHo = up.x - c.oe, upE = up.y;
+        const uint32_t sel = w.next(c);
+        __stcs(tb, dp_rows2<0, K>(S, c, sel, w.ck, upHo, upE, diag));
+        hf[K * PAIR_BLOCK] = S.rmax[K];
+        diag = up.x;
+        rbr += 32;
+        tb += 32;
+        head2<K + 1>(S, c, w, rbr, diag, tb, hf);
+    }
+}
+
+// Columns hi0 + K of a sloped strip's right corner: rows K..7, the row above
+// out of its window; up to column hi0 + last.
+template <int K>
+__device__ __forceinline__ void tail2(Strip2 &S, const Keys2 &c, Codes2 &w, int last, uint32_t &diag,
+                                      uint2 *&rbw, uint2 *&tb) {
+    if constexpr (K < STRIP) {
+        if (K <= last) {
+            uint32_t upHo = c.ho0, upE = c.e0;
+            const uint32_t sel = w.next(c);
+            __stcs(tb, dp_rows2<K, STRIP - 1>(S, c, sel, w.ck, upHo, upE, diag));
+            diag = S.Hl[K];  // row K's last cell: the next column's diagonal
+            *rbw = make_uint2(upHo + c.oe, upE);
+            rbw += 32;
+            tb += 32;
+            tail2<K + 1>(S, c, w, last, diag, rbw, tb);
         }
     }
 }
+
+// The best cells so far of both pairs: H (thr: the largest row-max key of
+// that H), row, and the columns that hold the row's first cell of that H.
+struct Best2 {
+    uint32_t thr;
+    int h[2], i[2], j0[2], j1[2];
+};
 
 // Fill the DP of two pairs with identical geometry (shared g, m, n, sw).
+// hf: the keys of the strip's 8 first cells in shared memory (stride PAIR_BLOCK).
 __device__ void dp_fill2(const GotohConst &K, const uint32_t *__restrict__ s_lut, int m, int n,
                          const Geo &g, const Seq &readA, const Seq &readB, const uint8_t *warena,
-                         uint64_t wposA, uint64_t wposB, uint32_t *tbA, uint32_t *tbB, int sw, uint2 *rb,
+                         uint64_t wposA, uint64_t wposB, uint2 *tb0, int sw, uint2 *rb, uint32_t *hf,
                          FillResult &FA, FillResult &FB) {
-    const uint32_t oe1 = (uint32_t)(K.oe1 & 0xffff) * 0x10001u;
-    const uint32_t oe4 = (uint32_t)(K.oe4 & 0xffff) * 0x10001u;
-    const uint32_t ex4 = (uint32_t)(K.ex4 & 0xffff) * 0x10001u;
-    // the best cell so far of both pairs, packed like the row maxima: its
-    // scaled H, row and column (pair A low half, B high half); the first
-    // touching row of each pair with its left / clamped flags, and bit 15 of
-    // each half of open_halves while that pair has none (all in registers:
-    // FA and FB are the caller's memory)
-    uint32_t bestHp2 = 0x00020002u, bestI2 = 0u, bestJ2 = 0u;
+    const Keys2 c = keys2_of(K, m, sw);
+    const uint32_t ksc = 4u * c.ks;                  // S
+    const uint32_t inv_s = 0xffffffffu / ksc + 1u;  // key / S = mulhi(key, inv_s): key < 2^16, S <= 2^16
+    Best2 B;
+    B.thr = (ksc - 1u) * 0x10001u;
+#pragma unroll
+    for (int q = 0; q < 2; q++) B.h[q] = B.i[q] = B.j0[q] = B.j1[q] = 0;
+    // the first touching row of each pair with its left / clamped flags, and
+    // bit 15 of each half of open_halves while that pair has none
     uint32_t trow2 = 0u, tflags = 0u;  // touch rows (halves); left / clamped bits 0-1 (A), 2-3 (B)
     uint32_t open_halves = 0x80008000u;
-    int nstrips = (m + STRIP - 1) / STRIP;
-    int plo = g.lo(1), phi = g.hi(min(STRIP, m));
-    for (int k = 0; k <= phi - plo; k++) rb[(size_t)k * 32] = make_uint2(0x00020002u, NEG2);
     Strip2 S;
+    const int nstrips = (m + STRIP - 1) / STRIP;
+    int plo = g.lo(1), phi = g.hi(min(STRIP, m));
+    for (int k = 0; k <= phi - plo; k++) rb[(size_t)k * 32] = make_uint2(c.h0, c.e0);
     for (int s = 0; s < nstrips; s++) {
-        int i0 = s * STRIP + 1;
-        int nact = min(STRIP, m - i0 + 1);
+        const int i0 = s * STRIP + 1;
+        const int nact = min(STRIP, m - i0 + 1);
+        const uint32_t rwA = load16(readA.arena, readA.pos + (uint64_t)(i0 - 1));
+        const uint32_t rwB = load16(readA.arena, readB.pos + (uint64_t)(i0 - 1));  // one arena
+        const uint32_t rnA = readA.cnt ? nmask16(readA.iv, readA.cnt, i0 - 1) : 0u;
+        const uint32_t rnB = readB.cnt ? nmask16(readB.iv, readB.cnt, i0 - 1) : 0u;
 #pragma unroll
         for (int r = 0; r < STRIP; r++) {
-            S.lohi[r] = (uint32_t)g.lo(i0 + r) | ((uint32_t)g.hi(i0 + r) << 16);
-            S.Hl[r] = 0x00020002u;
-            S.Fl[r] = NEG2;
+            S.Hl[r] = c.h0;
+            S.kF[r] = c.ho0;
             S.rmax[r] = 0u;
-            S.arg[r] = 0u;
-        }
-        int clo = (int)(S.lohi[0] & 0xffffu);
-        int chi = g.hi(i0 + nact - 1);
-        int lo7 = (int)(S.lohi[STRIP - 1] & 0xffffu);
-        int hi0 = (int)(S.lohi[0] >> 16);
-        uint32_t rwA = load16(readA.arena, readA.pos + (uint64_t)(i0 - 1));
-        uint32_t rwB = load16(readA.arena, readB.pos + (uint64_t)(i0 - 1));  // one arena
-        uint32_t rnA = readA.cnt ? nmask16(readA.iv, readA.cnt, i0 - 1) : 0u;
-        uint32_t rnB = readB.cnt ? nmask16(readB.iv, readB.cnt, i0 - 1) : 0u;
-#pragma unroll
-        for (int r = 0; r < STRIP; r++) {
             uint32_t ca = (rwA >> (30 - 2 * r)) & 3u, cb = (rwB >> (30 - 2 * r)) & 3u;
             if ((rnA >> (31 - r)) & 1u) ca = 4;
             if ((rnB >> (31 - r)) & 1u) cb = 4;
             S.la[r] = s_lut[2 * ca];
             S.lb[r] = s_lut[2 * cb];
         }
-        uint32_t diag = 0x00020002u;
+        const int clo = g.lo(i0), lo7 = g.lo(i0 + STRIP - 1);
+        const int hi0 = g.hi(i0), chi = g.hi(i0 + nact - 1);
+        // windows move by 0 or 1 columns a row, so the ends tell the shape
+        const bool lslope = lo7 == clo + STRIP - 1 && hi0 >= lo7, lflat = lo7 == clo;
+        const bool rslope = chi == hi0 + nact - 1, rflat = chi == hi0;
+        uint32_t diag = c.h0;
         if (clo - 1 >= plo && clo - 1 <= phi) diag = rb[(size_t)(clo - 1 - plo) * 32].x;
-        uint32_t *ta = tbA + (size_t)s * sw * 32, *tbq = tbB + (size_t)s * sw * 32;
-        int a_end = min(lo7, chi);
-        dp_cols2<1, true>(S, oe1, oe4, ex4, clo, a_end, diag, warena, wposA, wposB, rb, plo, phi, lo7, ta,
-                          tbq);
-        int b_beg = lo7 + 1, b_end = min(hi0 - 1, chi);
-        if (b_beg <= b_end)
-            dp_cols2<0, false>(S, oe1, oe4, ex4, b_beg, b_end, diag, warena, wposA, wposB, rb, plo, phi,
-                               lo7, ta + (size_t)(b_beg - clo) * 32,
-                               tbq + (size_t)(b_beg - clo) * 32);
-        int c_beg = max(lo7 + 1, hi0);
-        // the row windows again rather than kept live across the interior
+        uint2 *tb = tb0 + (size_t)s * sw * 32;
+        const uint2 *rbr = rb + (size_t)(clo - plo) * 32;  // the row above at the next column
+        uint2 *rbw = rb;                                   // the last row from column lo7 on
+        Codes2 w;
+        w.t = 0;
+        if ((lslope | lflat) & (rslope | rflat)) {
+            int jb = clo;  // first column with all 8 rows
+            if (lslope) {
+                w.load(warena, wposA, wposB, clo);
+                head2<0>(S, c, w, rbr, diag, tb, hf);
+                jb = lo7;
+            }
+            // interior: all 8 rows in their windows, the row above present;
+            // its words are read two columns ahead of their use (the L2
+            // round trip is longer than one column of arithmetic).  A slot
+            // is rewritten only at or after the column that reads it.
+            const int je = rslope ? hi0 - 1 : min(hi0, phi);
+            uint2 up0 = make_uint2(c.h0, c.e0), up1 = up0;
+            if (jb <= je) up0 = rbr[0];
+            if (jb + 1 <= je) up1 = rbr[32];
+            for (int j = jb; j <= je;) {
+                w.load(warena, wposA, wposB, j);
+                const int cnt = min(16, je - j + 1);
+#pragma unroll 1
+                for (int k = 0; k < cnt; k++, j++) {
+                    const uint2 up = up0;
+                    up0 = up1;
+                    if (j + 2 <= je) up1 = rbr[64];
+                    uint32_t upHo = up.x - c.oe, upE = up.y;
+                    const uint32_t sel = w.next(c);
+                    __stcs(tb, dp_rows2<0, STRIP - 1>(S, c, sel, w.ck, upHo, upE, diag));
+                    *rbw = make_uint2(upHo + c.oe, upE);
+                    diag = up.x;
+                    if (j == jb) {  // the first cells of the rows that begin here
+                        if (lflat) {
 #pragma unroll
-        for (int r = 0; r < STRIP; r++)
-            S.lohi[r] = (uint32_t)g.lo(i0 + r) | ((uint32_t)g.hi(i0 + r) << 16);
-        if (c_beg <= chi)
-            dp_cols2<1, true>(S, oe1, oe4, ex4, c_beg, chi, diag, warena, wposA, wposB, rb, plo, phi, lo7,
-                              ta + (size_t)(c_beg - clo) * 32, tbq + (size_t)(c_beg - clo) * 32);
-        // row bookkeeping in row order (extend.rs:795-827).  The best cell:
-        // a strictly larger row maximum replaces it, both pairs at once with
-        // the keep mask of the row maximum (row_max2)
+                            for (int r = 0; r < STRIP - 1; r++) hf[r * PAIR_BLOCK] = S.rmax[r];
+                        }
+                        hf[(STRIP - 1) * PAIR_BLOCK] = S.rmax[STRIP - 1];
+                    }
+                    rbr += 32;
+                    rbw += 32;
+                    tb += 32;
+                }
+            }
+            const bool first = jb > je;  // no interior column: rows begin in the one below
+            if (rslope | (hi0 > phi)) {
+                w.load(warena, wposA, wposB, je + 1);
+                // the first row's last column: the row above has a cell there
+                // only where its window did not move
+                const uint2 up = hi0 <= phi ? *rbr : make_uint2(c.h0, c.e0);
+                uint32_t upHo = up.x - c.oe, upE = up.y;
+                const uint32_t sel = w.next(c);
+                __stcs(tb, dp_rows2<0, STRIP - 1>(S, c, sel, w.ck, upHo, upE, diag));
+                *rbw = make_uint2(upHo + c.oe, upE);
+                diag = S.Hl[0];
+                rbw += 32;
+                tb += 32;
+                if (first) {
 #pragma unroll
-        for (int r = 0; r < STRIP; r++) {
-            if (r < nact) {
-                const uint32_t keep = prmt(bestHp2 + 0x80008000u - S.rmax[r], 0u, 0xBB99u);
-                bestHp2 = (bestHp2 & keep) | (S.rmax[r] & ~keep);
-                bestI2 = (bestI2 & keep) | ((uint32_t)(i0 + r) * 0x10001u & ~keep);
-                bestJ2 = (bestJ2 & keep) | (S.arg[r] & ~keep);
+                    for (int r = 0; r < STRIP; r++)
+                        if (lflat | (r == STRIP - 1)) hf[r * PAIR_BLOCK] = S.rmax[r];
+                }
+                if (rslope) tail2<1>(S, c, w, nact - 1, diag, rbw, tb);
+            }
+        } else {
+            // clamping begins or ends inside the strip
+            for (int j = clo; j <= chi;) {
+                w.load(warena, wposA, wposB, j);
+                const int cnt = min(16, chi - j + 1);
+#pragma unroll 1
+                for (int k = 0; k < cnt; k++, j++) {
+                    const uint2 up = j <= phi ? *rbr : make_uint2(c.h0, c.e0);
+                    uint32_t upE = up.y, botH;
+                    const uint32_t sel = w.next(c);
+                    __stcs(tb, dp_masked2(S, c, g, i0, j, sel, w.ck, up.x - c.oe, upE, diag, botH, hf));
+                    diag = up.x;
+                    if (j >= lo7) {
+                        *rbw = make_uint2(botH, upE);
+                        rbw += 32;
+                    }
+                    rbr += 32;
+                    tb += 32;
+                }
             }
         }
-        // the first touching row, per pair, until both pairs have one.  A
-        // touch needs a zero half in arg ^ lo (left edge) or, when hi < n, in
-        // rmax ^ Hl (right edge); (x - 0x10001) & ~x has bit 15 of a half set
-        // for every zero half (and may set it in the half above one), so a
-        // strip whose rows have none for a pair still without a touch skips
+        // row bookkeeping (extend.rs:795-827); rows past the read do not count
+        if (nact < STRIP) {
+#pragma unroll
+            for (int r = 1; r < STRIP; r++)
+                if (r >= nact) S.rmax[r] = 0u;
+        }
+        // the best cell: a strictly larger row maximum, in row order, replaces it
+        uint32_t smax = __vimax3_u16x2(S.rmax[0], S.rmax[1], S.rmax[2]);
+        smax = __vimax3_u16x2(smax, S.rmax[3], S.rmax[4]);
+        smax = __vimax3_u16x2(smax, S.rmax[5], __vmaxu2(S.rmax[6], S.rmax[7]));
+        if (__vmaxu2(B.thr, smax) != B.thr) {
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const uint32_t v = (smax >> (16 * q)) & 0xffffu;
+                if (v > ((B.thr >> (16 * q)) & 0xffffu)) {
+                    const uint32_t h = __umulhi(v, inv_s), base = h * ksc;
+                    int row = 0;
+                    uint32_t key = 0;
+#pragma unroll
+                    for (int r = STRIP - 1; r >= 0; r--) {
+                        const uint32_t x = (S.rmax[r] >> (16 * q)) & 0xffffu;
+                        if (x >= base) {
+                            row = i0 + r;
+                            key = x;
+                        }
+                    }
+                    const int j0 = clo + (int)((base + ksc - 1u - key) << c.g);
+                    B.h[q] = (int)h;
+                    B.i[q] = row;
+                    B.j0[q] = max(j0, g.lo(row));
+                    B.j1[q] = min(j0 + (1 << c.g) - 1, g.hi(row));
+                    B.thr = (B.thr & (0xffff0000u >> (16 * q))) | ((base + ksc - 1u) << (16 * q));
+                }
+            }
+        }
+        // the first touching row, per pair, until both pairs have one: the
+        // row's maximum is its first cell's key (left edge) or, when hi < n,
+        // no larger than a key of its last cell's H (right edge).  (x - 0x10001) & ~x has bit 15 of a half
+        // set for every zero half (and may set it in the half above one), so
+        // a strip whose rows have none for a pair still without a touch skips
         // the exact per-row tests
         uint32_t zero_halves = 0u;
         if (open_halves) {
 #pragma unroll
             for (int r = 0; r < STRIP; r++) {
                 if (r < nact) {
-                    const uint32_t lo_r = (uint32_t)g.lo(i0 + r);
-                    const uint32_t zl = S.arg[r] ^ (lo_r * 0x10001u);
+                    const uint32_t zl = S.rmax[r] ^ hf[r * PAIR_BLOCK];
                     zero_halves |= (zl - 0x00010001u) & ~zl;
                     if (g.hi(i0 + r) < n) {
-                        const uint32_t zr = S.rmax[r] ^ S.Hl[r];
+                        const uint32_t u = mad_u32(S.Hl[r], c.ks, c.ck0);
+                        const uint32_t zr = __vmaxu2(S.rmax[r], u) ^ u;
                         zero_halves |= (zr - 0x00010001u) & ~zr;
                     }
                 }
@@ -1397,19 +1580,20 @@ __device__ void dp_fill2(const GotohConst &K, const uint32_t *__restrict__ s_lut
             for (int r = 0; r < STRIP; r++) {
                 if (r < nact) {
                     const int lo = g.lo(i0 + r), hi = g.hi(i0 + r);
+                    const uint32_t first = hf[r * PAIR_BLOCK];
+                    const uint32_t last = mad_u32(S.Hl[r], c.ks, c.ck0);
 #pragma unroll
                     for (int q = 0; q < 2; q++) {
                         const uint32_t bit = 0x8000u << (16 * q);
                         if (open_halves & bit) {
-                            const int argj = (int)((S.arg[r] >> (16 * q)) & 0xffffu);
-                            const bool tr = (((S.rmax[r] ^ S.Hl[r]) >> (16 * q)) & 0xffffu) == 0;
-                            if (argj == lo) {
+                            const bool tl = (((S.rmax[r] ^ first) >> (16 * q)) & 0xffffu) == 0;
+                            const bool tr = ((S.rmax[r] >> (16 * q)) & 0xffffu) <= ((last >> (16 * q)) & 0xffffu);
+                            if (tl) {
                                 trow2 |= (uint32_t)(i0 + r) << (16 * q);
                                 tflags |= (1u | (lo <= 1 ? 2u : 0u)) << (2 * q);
                                 open_halves &= ~bit;
                             } else if (hi < n && tr) {
                                 trow2 |= (uint32_t)(i0 + r) << (16 * q);
-                                tflags |= (hi >= n ? 2u : 0u) << (2 * q);
                                 open_halves &= ~bit;
                             }
                         }
@@ -1420,52 +1604,51 @@ __device__ void dp_fill2(const GotohConst &K, const uint32_t *__restrict__ s_lut
         plo = lo7;
         phi = g.hi(i0 + STRIP - 1);
     }
-    FA.bestHp = (int)(bestHp2 & 0xffffu);
-    FA.best_i = (int)(bestI2 & 0xffffu);
-    FA.best_j = (int)(bestJ2 & 0xffffu);
-    FB.bestHp = (int)(bestHp2 >> 16);
-    FB.best_i = (int)(bestI2 >> 16);
-    FB.best_j = (int)(bestJ2 >> 16);
-    FA.trow = (int)(trow2 & 0xffffu);
-    FA.tleft = tflags & 1u;
-    FA.tclamp = (tflags >> 1) & 1u;
-    FB.trow = (int)(trow2 >> 16);
-    FB.tleft = (tflags >> 2) & 1u;
-    FB.tclamp = (tflags >> 3) & 1u;
+    auto put = [&](FillResult &F, int q) {
+        F.bestHp = 4 * B.h[q] + 2;
+        F.best_i = B.i[q];
+        F.best_j = B.j0[q];
+        F.last_j = B.j1[q];
+        F.trow = (int)((trow2 >> (16 * q)) & 0xffffu);
+        F.tleft = (tflags >> (2 * q)) & 1u;
+        F.tclamp = (tflags >> (2 * q + 1)) & 1u;
+    };
+    put(FA, 0);
+    put(FB, 1);
 }
 
 // Out-of-line fill, finish and lone-pair paths of the paired kernel: one
 // copy of each in the kernel's code, and their registers are not reserved
 // across one another.
 __device__ __noinline__ void fill2_call(const GotohConst &K, const uint32_t *__restrict__ s_lut,
-                                        const PairSetup &A, const PairSetup &B, uint32_t *tbA,
-                                        uint32_t *tbB, uint32_t *rb, FillResult &FA,
-                                        FillResult &FB) {
-    dp_fill2(K, s_lut, A.m, A.n, A.g, A.read, B.read, A.win.arena, A.win.pos, B.win.pos, tbA,
-             tbB, A.sw, reinterpret_cast<uint2 *>(rb), FA, FB);
+                                        const PairSetup &A, const PairSetup &B, uint32_t *tb,
+                                        uint32_t *rb, uint32_t *hf, FillResult &FA, FillResult &FB) {
+    dp_fill2(K, s_lut, A.m, A.n, A.g, A.read, B.read, A.win.arena, A.win.pos, B.win.pos,
+             reinterpret_cast<uint2 *>(tb), A.sw, reinterpret_cast<uint2 *>(rb), hf, FA, FB);
 }
 
 __device__ __noinline__ void finish_call(const GotohJob &job, const GotohConst &K,
                                          const int8_t *__restrict__ lut, uint32_t pi,
                                          PairSetup &S, const FillResult &F, const uint32_t *tb) {
-    finish_pair<32>(job, K, lut, pi, S, F, tb);
+    finish_pair<64>(job, K, lut, pi, S, F, tb);
 }
 
 // A pair without a partner of its geometry: the paired fill with itself in
-// both lanes (the second lane's traceback lands in the slot's unused half),
-// or, when its window has N (the paired fill takes N in reads only), the
-// one-pair fill with its row buffer in that unused half (tb_words >=
-// rb_words: a pair's traceback holds at least one strip of row-buffer width).
+// both lanes, or, when its window has N (the paired fill takes N in reads
+// only), the one-pair fill with its row buffer in the words of the second
+// pair (tb_words >= rb_words: a pair's traceback holds at least one strip of
+// row-buffer width; the lane's own words, as the other lanes' fills run
+// beside it).
 __device__ __noinline__ void lone_call(const GotohJob &job, const GotohConst &K,
                                        const uint32_t *__restrict__ s_lut,
-                                       const int8_t *__restrict__ lut, uint32_t pi,
-                                       PairSetup &S, uint32_t *tb, uint32_t *tbB, uint32_t *rb) {
+                                       const int8_t *__restrict__ lut, uint32_t pi, PairSetup &S,
+                                       uint32_t *tb, uint32_t *rb, uint32_t *hf) {
     FillResult F, F2;
     if (S.win.cnt)
-        F = dp_fill<true>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, tbB);
+        F = dp_fill<true, 64>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, tb + 1);
     else
-        fill2_call(K, s_lut, S, S, tb, tbB, rb, F, F2);
-    finish_pair<32>(job, K, lut, pi, S, F, tb);
+        fill2_call(K, s_lut, S, S, tb, rb, hf, F, F2);
+    finish_call(job, K, lut, pi, S, F, tb);
 }
 
 // Work item (a, b): both pairs in one thread when their geometry matches and
@@ -1476,8 +1659,8 @@ constexpr uint32_t NO_PAIR = 0xffffffffu;
 
 __device__ void process_item2(const GotohJob &job, const GotohConst &K,
                               const uint32_t *__restrict__ s_lut, const int8_t *__restrict__ lut,
-                              uint32_t pa, uint32_t pb, uint32_t *tb, uint32_t *rb) {
-    uint32_t *tbB = tb + job.tb_words * 32;  // second half of the thread's slot
+                              uint32_t pa, uint32_t pb, uint32_t *tb, uint32_t *rb,
+                              uint32_t *hf) {
     bool both;
     FillResult FA, FB;
     {
@@ -1487,10 +1670,10 @@ __device__ void process_item2(const GotohJob &job, const GotohConst &K,
         both = ra && rb_ && A.m == B.m && A.n == B.n && A.full == B.full &&
                A.g.off == B.g.off && A.g.half == B.g.half && A.win.cnt == 0 && B.win.cnt == 0;
         if (both) {
-            fill2_call(K, s_lut, A, B, tb, tbB, rb, FA, FB);
+            fill2_call(K, s_lut, A, B, tb, rb, hf, FA, FB);
         } else {
-            if (ra) lone_call(job, K, s_lut, lut, pa, A, tb, tbB, rb);
-            if (rb_) lone_call(job, K, s_lut, lut, pb, B, tb, tbB, rb);
+            if (ra) lone_call(job, K, s_lut, lut, pa, A, tb, rb, hf);
+            if (rb_) lone_call(job, K, s_lut, lut, pb, B, tb, rb, hf);
         }
     }
     if (both) {
@@ -1498,7 +1681,7 @@ __device__ void process_item2(const GotohJob &job, const GotohConst &K,
         setup_pair(job, K, pa, job.tb_words, job.rb_words, false, A);
         finish_call(job, K, lut, pa, A, FA, tb);
         setup_pair(job, K, pb, job.tb_words, job.rb_words, false, B);
-        finish_call(job, K, lut, pb, B, FB, tbB);
+        finish_call(job, K, lut, pb, B, FB, tb + 1);
     }
 }
 
@@ -1507,9 +1690,10 @@ __device__ void process_item2(const GotohJob &job, const GotohConst &K,
 // geometry key.  Scratch per warp: 2 x tb_words and 2 x rb_words words per
 // lane.
 template <int MINB>
-__global__ void __launch_bounds__(128, MINB) gotoh2_kernel(GotohJob job, GotohConst K) {
+__global__ void __launch_bounds__(PAIR_BLOCK, MINB) gotoh2_kernel(GotohJob job, GotohConst K) {
     __shared__ uint32_t s_lut[10];
     __shared__ int8_t s_lut25[32];
+    __shared__ uint32_t s_first[STRIP * PAIR_BLOCK];
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int k = 0; k < 10; k++) s_lut[k] = K.lut4[k >> 1][k & 1];
@@ -1519,7 +1703,7 @@ __global__ void __launch_bounds__(128, MINB) gotoh2_kernel(GotohJob job, GotohCo
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const uint64_t warp_slot = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t *tb = job.tb + warp_slot * (2 * job.tb_words) * 32 + lane;
+    uint32_t *tb = job.tb + warp_slot * (2 * job.tb_words) * 32 + 2 * lane;
     uint32_t *rb = job.rb + warp_slot * (2 * job.rb_words) * 32 + 2 * lane;
     uint64_t b0 = 0, b1 = job.list_count ? (uint64_t)(*job.list_count) : job.n_pairs;
     if (job.range) {  // one length class of the binned list
@@ -1537,7 +1721,7 @@ __global__ void __launch_bounds__(128, MINB) gotoh2_kernel(GotohJob job, GotohCo
             uint64_t x = b0 + 2 * k, y = x + 1;
             uint32_t pa = job.list ? job.list[x] : (uint32_t)x;
             uint32_t pb = y < b1 ? (job.list ? job.list[y] : (uint32_t)y) : NO_PAIR;
-            process_item2(job, K, s_lut, s_lut25, pa, pb, tb, rb);
+            process_item2(job, K, s_lut, s_lut25, pa, pb, tb, rb, s_first + threadIdx.x);
         }
     }
 }
@@ -1552,7 +1736,6 @@ int make_gotoh_const(const esp_extend_params &p, GotohConst &k) {
         return ESP_EDOMAIN;
     k.open_ext = -(p.gap_open + p.gap_ext);
     k.ext = -p.gap_ext;
-    k.oe1 = 4 * k.open_ext - 1;
     k.oe4 = 4 * k.open_ext;
     k.ex4 = 4 * k.ext;
     k.match = p.match_score;
@@ -1569,6 +1752,7 @@ int make_gotoh_const(const esp_extend_params &p, GotohConst &k) {
     int smax = 0;
     for (int i = 0; i < 25; i++) smax = lut[i] > smax ? lut[i] : smax;
     k.max_m = smax > 0 ? 8191 / smax : 32767;
+    k.smax = smax;
     // a walk may take matches without reading the traceback (Walker::next)
     k.match_skip = p.match_score > 0 && p.match_score == smax;
     // traceback kind of a diagonal step by read code * 5 + window code:
