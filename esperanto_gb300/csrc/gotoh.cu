@@ -40,7 +40,7 @@
 // as the scalar kernel's margins do (extend.rs:718-759).
 #include <cuda_runtime.h>
 
-#include <climits>
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -195,11 +195,11 @@ struct FillResult {
 // time.  CHECK = true (strip ramps) tests the row-buffer read (the row above
 // has a value only up to phi) and write (the strip's last row starts at
 // lo7) per column; the interior needs neither test.
-template <int MASK, bool CHECK, bool HASN, int STR>
+template <int MASK, bool CHECK, bool HASN>
 __device__ __forceinline__ void dp_cols(Strip &S, const GotohConst &K, int a, int b, int &diag,
                                         const Seq &win, uint32_t *rb, int plo, int phi, int lo7,
                                         uint32_t *tbp) {
-    uint32_t *rbr = rb + (size_t)(a - plo) * STR;
+    uint32_t *rbr = rb + (size_t)(a - plo) * 32;
     uint32_t cj = 32767u - (uint32_t)a;
     // Interior: the row above is read two columns ahead of its use (the
     // L2 round trip of a row-buffer line is longer than one column of
@@ -208,7 +208,7 @@ __device__ __forceinline__ void dp_cols(Strip &S, const GotohConst &K, int a, in
     uint32_t wn0 = 0, wn1 = 0;
     if (!CHECK) {
         wn0 = rbr[0];
-        if (a + 1 <= b) wn1 = rbr[STR];
+        if (a + 1 <= b) wn1 = rbr[32];
     }
     for (int j = a; j <= b;) {
         uint32_t cw = load16(win.arena, win.pos + (uint64_t)(j - 1));
@@ -228,7 +228,7 @@ __device__ __forceinline__ void dp_cols(Strip &S, const GotohConst &K, int a, in
                 } else {
                     w = wn0;
                     wn0 = wn1;
-                    if (j + 2 <= b) wn1 = rbr[2 * STR];
+                    if (j + 2 <= b) wn1 = rbr[64];
                 }
                 bH = (int)(w & 0xffffu);
                 bE = ((int)w) >> 16;
@@ -238,26 +238,26 @@ __device__ __forceinline__ void dp_cols(Strip &S, const GotohConst &K, int a, in
             diag = bH;
             uint32_t packed = __byte_perm((uint32_t)upH, (uint32_t)upE, 0x5410);
             if (CHECK) {
-                if (j >= lo7) rb[(size_t)(j - lo7) * STR] = packed;
+                if (j >= lo7) rb[(size_t)(j - lo7) * 32] = packed;
             } else {
-                rbr[(ptrdiff_t)(plo - lo7) * STR] = packed;  // row-buffer slot j - lo7
+                rbr[(ptrdiff_t)(plo - lo7) * 32] = packed;  // row-buffer slot j - lo7
             }
             *tbp = word;
-            tbp += STR;
-            rbr += STR;
+            tbp += 32;
+            rbr += 32;
             cj--;
         }
     }
 }
 
-// Fill the DP for one pair; traceback words land in tb (sw words per strip, STR
+// Fill the DP for one pair; traceback words land in tb (sw words per strip, 32
 // words apart: the lanes of a warp interleave theirs).
 // The row buffer holds sw words: strip 0 reads row 0 (H = 0, E = NEG on every
 // column, extend.rs:664-681) from a prefilled copy, later strips read the last
 // row of the previous strip, which each strip rewrites in place (a slot is
 // always read at or before the column that overwrites it, since the strip's
 // window start lo7 never precedes the previous row's start plo).
-template <bool HASN, int STR>
+template <bool HASN>
 __device__ FillResult dp_fill(const GotohConst &K, const uint32_t *__restrict__ s_lut, int m,
                               int n, const Geo &g, const Seq &read, const Seq &win,
                               uint32_t *tb, int sw, uint32_t *rb) {
@@ -272,7 +272,7 @@ __device__ FillResult dp_fill(const GotohConst &K, const uint32_t *__restrict__ 
     int plo = g.lo(1), phi = g.hi(min(STRIP, m));
     {
         const uint32_t row0 = absent_HE(K);
-        for (int k = 0; k <= phi - plo; k++) rb[(size_t)k * STR] = row0;
+        for (int k = 0; k <= phi - plo; k++) rb[(size_t)k * 32] = row0;
     }
     Strip S;
     for (int s = 0; s < nstrips; s++) {
@@ -302,14 +302,14 @@ __device__ FillResult dp_fill(const GotohConst &K, const uint32_t *__restrict__ 
         }
         int diag = 2;
         if (clo - 1 >= plo && clo - 1 <= phi)
-            diag = (int)(rb[(size_t)(clo - 1 - plo) * STR] & 0xffffu);
-        uint32_t *tbp = tb + (size_t)s * sw * STR;
+            diag = (int)(rb[(size_t)(clo - 1 - plo) * 32] & 0xffffu);
+        uint32_t *tbp = tb + (size_t)s * sw * 32;
         int a_end = min(lo7, chi);
-        dp_cols<1, true, HASN, STR>(S, K, clo, a_end, diag, win, rb, plo, phi, lo7, tbp);
+        dp_cols<1, true, HASN>(S, K, clo, a_end, diag, win, rb, plo, phi, lo7, tbp);
         int b_beg = lo7 + 1, b_end = min(hi0 - 1, chi);
         if (b_beg <= b_end)
-            dp_cols<0, false, HASN, STR>(S, K, b_beg, b_end, diag, win, rb, plo, phi, lo7,
-                                    tbp + (size_t)(b_beg - clo) * STR);
+            dp_cols<0, false, HASN>(S, K, b_beg, b_end, diag, win, rb, plo, phi, lo7,
+                                    tbp + (size_t)(b_beg - clo) * 32);
         int c_beg = max(lo7 + 1, hi0);
         // the row windows again rather than kept live across the interior
 #pragma unroll
@@ -318,8 +318,8 @@ __device__ FillResult dp_fill(const GotohConst &K, const uint32_t *__restrict__ 
             S.hi[r] = g.hi(i0 + r);
         }
         if (c_beg <= chi)
-            dp_cols<1, true, HASN, STR>(S, K, c_beg, chi, diag, win, rb, plo, phi, lo7,
-                                   tbp + (size_t)(c_beg - clo) * STR);
+            dp_cols<1, true, HASN>(S, K, c_beg, chi, diag, win, rb, plo, phi, lo7,
+                                   tbp + (size_t)(c_beg - clo) * 32);
         // row bookkeeping in row order (extend.rs:795-827)
 #pragma unroll
         for (int r = 0; r < STRIP; r++) {
@@ -387,6 +387,20 @@ __device__ __forceinline__ int n_free(const esp_n_interval *iv, uint32_t cnt, in
     return room;
 }
 
+// Where a fill left the traceback word of (strip s, column j): sw words a
+// strip from its first column on, STR words apart (the lanes of a warp
+// interleave theirs; 1: a warp's own pair).
+template <int STR>
+struct StripTb {
+    const uint32_t *tb;
+    int sw;
+    __device__ __forceinline__ uint32_t word(const Geo &g, int s, int j) const {
+        // word indices fit 32 bits: a slot holds at most 4,096 strips of
+        // 32,767 columns
+        return tb[(size_t)(uint32_t)(s * sw + (j - g.lo(s * STRIP + 1))) * STR];
+    }
+};
+
 // One traceback walk over the packed bits (extend.rs:884-930): state machine
 // H/E/F from (best_i, best_j), stopping at i <= 0, j <= 0, outside the row
 // window, or on an H START cell.
@@ -407,37 +421,46 @@ __device__ __forceinline__ int n_free(const esp_n_interval *iv, uint32_t cnt, in
 //
 // A read of a 2 % error rate so costs its ~4 mismatches and a 32-base
 // compare per 32 bases instead of ~175 dependent word loads and state steps;
-// measured on one GB300: 4,194,304 mixed pairs 49.8 -> 43.9 ms, one
+// measured when it came: 4,194,304 mixed pairs 49.8 -> 43.9 ms, one
 // extend_hint call 146 -> 109 us.
-template <int TBS>
+template <class TB>
 struct Walker {
     const Geo &g;
-    const uint32_t *tb;
-    int sw;
+    const TB &tb;
     const Seq &read;
     const Seq &win;
     const GotohConst &K;
     int i, j, state;
+    bool over = false;  // on an H START cell
+    // the bases from (i, j) down, at bits 1:0 up, and how many are left
+    uint64_t rv = 0, wv = 0;
+    int rl = 0, wl = 0;
 
-    __device__ Walker(const Geo &g_, const uint32_t *tb_, int sw_, const Seq &r_, const Seq &w_,
+    __device__ Walker(const Geo &g_, const TB &tb_, const Seq &r_, const Seq &w_,
                       const GotohConst &K_, int bi, int bj)
-        : g(g_), tb(tb_), sw(sw_), read(r_), win(w_), K(K_), i(bi), j(bj), state(0) {}
+        : g(g_), tb(tb_), read(r_), win(w_), K(K_), i(bi), j(bj), state(0) {}
 
     // Take a run of `len` matches (0..32) and then one step of `kind` (-1:
     // none this time).  Returns false when the walk stops (with len = 0).
     __device__ __forceinline__ bool next(int &len, int &kind) {
         len = 0;
         kind = -1;
-        if (i <= 0 || j <= 0) return false;
+        if (over || i <= 0 || j <= 0) return false;
         if (j < g.lo(i) || j > g.hi(i)) return false;
         uint32_t q = 4, rc = 4;  // base codes at the walk's position (state H)
         if (state == 0) {
-            const uint64_t rv = tail32(read.arena, read.pos, i), wv = tail32(win.arena, win.pos, j);
+            if (rl <= 0 || wl <= 0) {
+                rv = tail32(read.arena, read.pos, i);
+                wv = tail32(win.arena, win.pos, j);
+                rl = min(i, 32);
+                wl = min(j, 32);
+            }
             uint64_t d = rv ^ wv;
             d = (d | (d >> 1)) & 0x5555555555555555ull;
-            int room = min(min(i, j), 32), rn = i, wn = j;
+            int room = min(rl, wl), rn = i, wn = j;
             if (read.cnt) rn = n_free(read.iv, read.cnt, i);
             if (win.cnt) wn = n_free(win.iv, win.cnt, j);
+            const int known = room;
             room = min(room, min(rn, wn));
             int run = min(room, d ? (__ffsll((long long)d) - 1) >> 1 : 32);
             // every predecessor in the window: i - lo(i) - j grows upwards
@@ -448,19 +471,20 @@ struct Walker {
                 len = run;
                 i -= run;
                 j -= run;
-                if (run == 32 || i <= 0 || j <= 0) return true;
+                rl -= run;
+                wl -= run;
+                if (run == known || i <= 0 || j <= 0) return true;
                 if (j < g.lo(i)) return true;  // the next call stops there
+                rv >>= 2 * run;
+                wv >>= 2 * run;
                 rn -= run;
                 wn -= run;
             }
-            q = rn == 0 ? 4u : (uint32_t)(rv >> (2 * run)) & 3u;
-            rc = wn == 0 ? 4u : (uint32_t)(wv >> (2 * run)) & 3u;
+            q = rn == 0 ? 4u : (uint32_t)rv & 3u;
+            rc = wn == 0 ? 4u : (uint32_t)wv & 3u;
         }
-        // word indices fit 32 bits: a slot holds at most 4,096 strips of
-        // 32,767 columns
         const int s = (i - 1) >> 3, r = (i - 1) & 7;
-        const uint32_t idx = (uint32_t)(s * sw + (j - g.lo(s * STRIP + 1)));
-        const uint32_t w = tb[(size_t)idx * TBS];
+        const uint32_t w = tb.word(g, s, j);
         const int sh = 2 * (7 - r);
         const uint32_t hsrc = (w >> sh) & 3u;
         const uint32_t eo = ~(w >> (16 + sh)) & 1u;
@@ -468,7 +492,7 @@ struct Walker {
         // the step's source: the cell's H tag in state 0, else the gap it is in
         const uint32_t eff = state == 0 ? hsrc : (state == 1 ? 1u : 0u);
         if (eff == 3u) {  // H_START: the walk ends after the run just taken
-            i = 0;
+            over = true;
             return len != 0;
         }
         const int open = state == 0;
@@ -476,51 +500,119 @@ struct Walker {
         const int kvert = open ? K_IO : K_IE, khor = open ? K_DO : K_DE;
         kind = eff == 2u ? kdiag : (eff == 1u ? kvert : khor);
         state = eff == 2u ? 0 : (eff == 1u ? (eo ? 0 : 1) : (fo ? 0 : 2));
-        if (eff != 0u) i--;
-        if (eff != 1u) j--;
+        if (eff != 0u) {
+            i--;
+            rv >>= 2;
+            rl--;
+        }
+        if (eff != 1u) {
+            j--;
+            wv >>= 2;
+            wl--;
+        }
         return true;
     }
 };
 
-struct CigarOut {
-    uint32_t *p;
-    uint32_t cap;
+// Score of one traceback step.
+__device__ __forceinline__ int delta_of(const GotohConst &K, int kind) {
+    return kind < 3 ? (kind == K_MM ? K.match : (kind == K_MX ? (int)K.lut[1] : 0))
+                    : ((kind & 1) ? K.open_ext : K.ext);
+}
+
+// The kept part of an alignment: its CIGAR runs in walk order, ends and score.
+// Runs go to the thread's local list, so short CIGARs are written once, in
+// final order, with no global read-back, and need only their final length in
+// capacity; a long CIGAR moves the list to its slots cig[2..] (and needs them:
+// it is reversed there in place).
+struct Kept {
+    uint32_t rr[RUNS_LOCAL];
+    uint32_t runs;
+    uint32_t read_start, ref_start, read_end, ref_end;
+    int score;
+    int first_op, last_op;  // forward order
     bool overflow;
-    __device__ __forceinline__ void put(uint32_t idx, uint32_t v) {
-        if (idx < cap) p[idx] = v;
-        else overflow = true;
+    __device__ __forceinline__ void emit(uint32_t v, uint32_t *cig, uint32_t cap) {
+        if (runs < RUNS_LOCAL) {
+            rr[runs] = v;
+        } else {
+            if (2 + runs < cap) {
+                if (runs == RUNS_LOCAL)
+                    for (int k = 0; k < RUNS_LOCAL; k++) cig[2 + k] = rr[k];
+                cig[2 + runs] = v;
+            } else {
+                overflow = true;
+            }
+        }
+        runs++;
     }
 };
 
-// Traceback, end trimming, rebuild and neutral flanks (extend.rs:864-1068).
-// TBS: word stride of the traceback (32 for the lane-interleaved scratch of
-// the thread-per-pair kernel, 1 for the warp-per-pair kernel's own scratch).
-template <int TBS>
-__device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, const Geo &g,
-                          const uint32_t *tb, int sw, int m, int n, const Seq &read,
-                          const Seq &win, const FillResult &F, esp_extension &o, uint32_t *cig,
-                          uint32_t cap) {
-    auto delta_of = [&](int kind) {  // score of one step
-        return kind < 3 ? (kind == K_MM ? K.match : (kind == K_MX ? (int)K.lut[1] : 0))
-                        : ((kind & 1) ? K.open_ext : K.ext);
-    };
-    // Walk 1 records the walk as runs of equal steps (len << 3 | kind) and
-    // finds its number of steps N, its total T and trail (its steps up to and
-    // including the last non-positive prefix sum).
-    // When the best cell's column is known as a range, its columns are walked
-    // in order until one's total is the best score: a walk's total is its
-    // cell's H, and the first such cell is the best one.  (With mismatches
-    // scoring <= 0 it ends on a match: a cell that equals the best by any
-    // other step has an equal cell before it in row order.)
+// Walk the traceback from (F.best_i, j) and keep all of it.  Returns whether
+// that is the alignment: its total is the best score T and the end trim
+// (extend.rs:931-968) takes nothing off, i.e. the walk-order prefix sums stay
+// positive and reach T with the last step only.  (They do for an optimal
+// local alignment; the general rule is walk_trimmed.)
+template <class TB>
+__device__ __forceinline__ bool walk_whole(const GotohConst &K, const Geo &g, const TB &tb,
+                                           const Seq &read, const Seq &win, int bi, int bj, int T,
+                                           Kept &k, uint32_t *cig, uint32_t cap) {
+    Walker<TB> W(g, tb, read, win, K, bi, bj);
+    int P = 0, cur_op = ESP_OP_M, last_op = -1, len, kind;
+    uint32_t cur_len = 0;
+    bool whole = true;
+    k.runs = 0;
+    k.overflow = false;
+    // no early way out: the lanes of a warp leave the loop together
+    while (W.next(len, kind)) {
+        const int op = kind < 0 ? ESP_OP_M : kind_op(kind);
+        if (len) {
+            whole = whole && P + (len - 1) * K.match < T;
+            P += len * K.match;
+            if (cur_op != ESP_OP_M) {
+                k.emit((cur_len << 4) | (uint32_t)cur_op, cig, cap);
+                cur_op = ESP_OP_M;
+                cur_len = 0;
+            }
+            cur_len += (uint32_t)len;
+            if (last_op < 0) last_op = ESP_OP_M;
+        }
+        if (kind >= 0) {
+            whole = whole && P < T;
+            P += delta_of(K, kind);
+            whole = whole && P > 0;
+            if (op != cur_op) {
+                if (cur_len) k.emit((cur_len << 4) | (uint32_t)cur_op, cig, cap);
+                cur_op = op;
+                cur_len = 0;
+            }
+            cur_len++;
+            if (last_op < 0) last_op = op;
+        }
+    }
+    whole = whole && P == T && cur_len != 0;
+    if (whole) k.emit((cur_len << 4) | (uint32_t)cur_op, cig, cap);
+    k.first_op = cur_op;
+    k.last_op = last_op;
+    k.read_start = (uint32_t)W.i;
+    k.ref_start = (uint32_t)W.j;
+    k.read_end = (uint32_t)bi;
+    k.ref_end = (uint32_t)bj;
+    k.score = P;
+    return whole;
+}
+
+// The same with the end trim: walk 1 records the walk as runs of equal steps
+// (len << 3 | kind) and finds its number of steps N, its total T and trail
+// (its steps up to and including the last non-positive prefix sum).
+template <class TB>
+__device__ __noinline__ void walk_trimmed(const GotohConst &K, const Geo &g, const TB &tb,
+                                          const Seq &read, const Seq &win, int best_i, int best_j,
+                                          Kept &kept, uint32_t *cig, uint32_t cap) {
     uint32_t rec[REC_RUNS];
-    int n_rec = 0, N = 0, P = 0, trail = 0, best_j = F.best_j;
-    const bool on_match = K.match_skip && K.lut[1] <= 0;
-    for (;; best_j++) {
-        if (on_match && best_j < F.last_j &&
-            read.code(F.best_i - 1) != win.code(best_j - 1))
-            continue;
-        n_rec = N = P = trail = 0;
-        Walker<TBS> W(g, tb, sw, read, win, K, F.best_i, best_j);
+    int n_rec = 0, N = 0, P = 0, trail = 0;
+    {
+        Walker<TB> W(g, tb, read, win, K, best_i, best_j);
         uint32_t open = 0;  // the run being extended (0: none yet)
         auto add = [&](int kind, int len) {
             if (open && (int)(open & 7u) == kind) {
@@ -545,7 +637,7 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
                 add(K_MM, len);
             }
             if (kind >= 0) {
-                P += delta_of(kind);
+                P += delta_of(K, kind);
                 N++;
                 if (P <= 0) trail = N;
                 add(kind, 1);
@@ -555,34 +647,17 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
             if (n_rec < REC_RUNS) rec[n_rec] = open;
             n_rec++;
         }
-        if (best_j >= F.last_j || 4 * P + 2 == F.bestHp) break;
     }
     const int T = P;
-    uint32_t read_start = 0, ref_start = 0, read_end = 0, ref_end = 0;
-    int score = 0;
-    CigarOut co{cig, cap, false};
-    uint32_t K_runs = 0;  // kept runs in walk order: rr, or from cig[2] when many
-    uint32_t rr[RUNS_LOCAL];
-    // A run goes to the thread's local list, so short CIGARs are written
-    // once, in final order, with no global read-back, and need only their
-    // final length in capacity; a long CIGAR moves the list to its slots
-    // cig[2..] (and needs them: it is reversed there in place).
-    auto emit = [&](uint32_t v) {
-        if (K_runs < RUNS_LOCAL) {
-            rr[K_runs] = v;
-        } else {
-            if (K_runs == RUNS_LOCAL)
-                for (int k = 0; k < RUNS_LOCAL; k++) co.put(2 + k, rr[k]);
-            co.put(2 + K_runs, v);
-        }
-        K_runs++;
-    };
-    int first_op = -1, last_op = -1;  // forward order first / last kept op
+    kept.runs = 0;
+    kept.overflow = false;
+    kept.first_op = kept.last_op = -1;
+    kept.score = 0;
     if (N == 0) {
-        read_start = (uint32_t)max(F.best_i, 0);
-        ref_start = (uint32_t)max(best_j, 0);
-        read_end = read_start;
-        ref_end = ref_start;
+        kept.read_start = (uint32_t)max(best_i, 0);
+        kept.ref_start = (uint32_t)max(best_j, 0);
+        kept.read_end = kept.read_start;
+        kept.ref_end = kept.ref_start;
     } else {
         // With walk-order prefix sums P_t, the reference's forward lead is
         // N-1-u where u is the first index in [-1, N-2] with P_u >= T
@@ -593,13 +668,13 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
         // of equal steps crosses T at most once, and only rising.
         bool degenerate = T <= 0, done = false;
         const int tstar = N - 1 - N / 2;
-        int i = F.best_i, j = best_j;
+        int i = best_i, j = best_j;
         int t0 = 0, P0 = 0, ptrail = 0;
         int ts_i = 0, ts_j = 0, ts_op = 0, ts_d = 0;
         int cur_op = -1;
         uint32_t cur_len = 0;
         auto take = [&](int kind, int len) {
-            const int op = kind_op(kind), d = delta_of(kind);
+            const int op = kind_op(kind), d = delta_of(K, kind);
             const int di = op != ESP_OP_D, dj = op != ESP_OP_I;
             if (tstar >= t0 && tstar < t0 + len) {
                 ts_i = i - di * (tstar - t0);
@@ -619,14 +694,14 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
             if (!degenerate && end >= trail) {
                 const int a = max(t0, trail);
                 if (cur_op < 0) {  // the kept region's end (forward order)
-                    read_end = (uint32_t)(i - di * (a - t0));
-                    ref_end = (uint32_t)(j - dj * (a - t0));
+                    kept.read_end = (uint32_t)(i - di * (a - t0));
+                    kept.ref_end = (uint32_t)(j - dj * (a - t0));
                     ptrail = P0 + d * (a - t0);
-                    last_op = op;
+                    kept.last_op = op;
                     cur_op = op;
                 }
                 if (op != cur_op) {
-                    emit((cur_len << 4) | (uint32_t)cur_op);
+                    kept.emit((cur_len << 4) | (uint32_t)cur_op, cig, cap);
                     cur_op = op;
                     cur_len = 0;
                 }
@@ -647,7 +722,7 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
         if (n_rec <= REC_RUNS) {
             for (int k = 0; k < n_rec && !done; k++) take((int)(rec[k] & 7u), (int)(rec[k] >> 3));
         } else {  // more runs than the record holds: walk again
-            Walker<TBS> W(g, tb, sw, read, win, K, F.best_i, best_j);
+            Walker<TB> W(g, tb, read, win, K, best_i, best_j);
             int len, kind;
             while (!done && W.next(len, kind)) {
                 if (len) take(K_MM, len);
@@ -655,24 +730,64 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
             }
         }
         if (degenerate) {
-            read_end = (uint32_t)ts_i;
-            ref_end = (uint32_t)ts_j;
-            read_start = (uint32_t)(ts_i - (ts_op != ESP_OP_D));
-            ref_start = (uint32_t)(ts_j - (ts_op != ESP_OP_I));
-            score = ts_d;
-            K_runs = 0;
-            emit((1u << 4) | (uint32_t)ts_op);
-            first_op = last_op = ts_op;
+            kept.read_end = (uint32_t)ts_i;
+            kept.ref_end = (uint32_t)ts_j;
+            kept.read_start = (uint32_t)(ts_i - (ts_op != ESP_OP_D));
+            kept.ref_start = (uint32_t)(ts_j - (ts_op != ESP_OP_I));
+            kept.score = ts_d;
+            kept.runs = 0;
+            kept.emit((1u << 4) | (uint32_t)ts_op, cig, cap);
+            kept.first_op = kept.last_op = ts_op;
         } else {
-            emit((cur_len << 4) | (uint32_t)cur_op);
-            first_op = cur_op;
-            read_start = (uint32_t)i;
-            ref_start = (uint32_t)j;
-            score = P0 - ptrail;
+            kept.emit((cur_len << 4) | (uint32_t)cur_op, cig, cap);
+            kept.first_op = cur_op;
+            kept.read_start = (uint32_t)i;
+            kept.ref_start = (uint32_t)j;
+            kept.score = P0 - ptrail;
         }
     }
+}
+
+// Traceback, end trimming, rebuild and neutral flanks (extend.rs:864-1068).
+template <class TB>
+__device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, const Geo &g,
+                          const TB &tb, int m, int n, const Seq &read, const Seq &win,
+                          const FillResult &F, esp_extension &o, uint32_t *cig, uint32_t cap) {
+    // When the best cell's column is known as a range, its columns are walked
+    // in order until one's total is the best score: a walk's total is its
+    // cell's H, and the first such cell is the best one.  (With mismatches
+    // scoring <= 0 it ends on a match: a cell that equals the best by any
+    // other step has an equal cell before it in row order.)
+    Kept kept;
+    const int T = (F.bestHp - 2) >> 2;
+    bool done = false;
+    int bj = F.best_j;
+    if (T > 0) {
+        const bool on_match = K.match_skip && K.lut[1] <= 0;
+        do {
+            while (on_match && bj < F.last_j && read.code(F.best_i - 1) != win.code(bj - 1)) bj++;
+            done = walk_whole(K, g, tb, read, win, F.best_i, bj, T, kept, cig, cap);
+        } while (!done && ++bj <= F.last_j);
+        bj = min(bj, F.last_j);
+    }
+    if (!done) {
+        // a trimmed alignment: the first column whose walk's total is T
+        for (int j = F.best_j; j < F.last_j; j++) {
+            Walker<TB> W(g, tb, read, win, K, F.best_i, j);
+            int P = 0, len, kind;
+            while (W.next(len, kind)) P += len * K.match + (kind >= 0 ? delta_of(K, kind) : 0);
+            bj = j;
+            if (P == T) break;
+            bj = F.last_j;
+        }
+        walk_trimmed(K, g, tb, read, win, F.best_i, bj, kept, cig, cap);
+    }
+    uint32_t read_start = kept.read_start, ref_start = kept.ref_start;
+    uint32_t read_end = kept.read_end;
+    const uint32_t ref_end = kept.ref_end, K_runs = kept.runs;
+    const int score = kept.score, first_op = kept.first_op, last_op = kept.last_op;
     // reverse the kept runs into forward order (a long CIGAR's, in place)
-    if (!co.overflow && K_runs > RUNS_LOCAL) {
+    if (!kept.overflow && K_runs > RUNS_LOCAL) {
         for (uint32_t a = 0, b = K_runs ? K_runs - 1 : 0; a < b; a++, b--) {
             uint32_t t = cig[2 + a];
             cig[2 + a] = cig[2 + b];
@@ -708,7 +823,7 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
     if (nr > 0 && last_op != ESP_OP_M) total++;
     if (read_start > 0) total++;
     if (read_end < (uint32_t)m) total++;
-    if (!co.overflow && total <= cap) {
+    if (!kept.overflow && total <= cap) {
         uint32_t w = 0;
         int prev = -1;
         auto push = [&](uint32_t op, uint32_t len) {
@@ -722,7 +837,7 @@ __device__ void dp_finish(const GotohConst &K, const int8_t *__restrict__ lut, c
         if (read_start > 0) push(ESP_OP_S, read_start);
         if (nl > 0) push(ESP_OP_M, nl);
         for (uint32_t k = 0; k < K_runs; k++) {
-            uint32_t v = K_runs <= RUNS_LOCAL ? rr[K_runs - 1 - k] : cig[2 + k];
+            uint32_t v = K_runs <= RUNS_LOCAL ? kept.rr[K_runs - 1 - k] : cig[2 + k];
             push(v & 15u, v >> 4);
         }
         if (nr > 0) push(ESP_OP_M, nr);
@@ -830,11 +945,11 @@ __device__ __forceinline__ bool setup_pair(const GotohJob &job, const GotohConst
 // then the result record.  Returns whether attempt 1 escalates; the pair is
 // appended to the escalation list when `queue` (the wide kernel runs its
 // second attempt itself).
-template <int TBS>
+template <class TB>
 __device__ __forceinline__ bool finish_pair(const GotohJob &job, const GotohConst &K,
                                             const int8_t *__restrict__ lut, uint32_t pi,
-                                            PairSetup &S, const FillResult &F,
-                                            const uint32_t *tb, bool queue = true) {
+                                            PairSetup &S, const FillResult &F, const TB &tb,
+                                            bool queue = true) {
     esp_extension &o = S.o;
     // A touched band escalates whatever its score: the second attempt writes
     // the pair's record and CIGAR, so the first one's are not built.
@@ -842,7 +957,7 @@ __device__ __forceinline__ bool finish_pair(const GotohJob &job, const GotohCons
         if (queue) job.esc_list[atomicAdd(job.esc_count, 1u)] = pi;
         return true;
     }
-    dp_finish<TBS>(K, lut, S.g, tb, S.sw, S.m, S.n, S.read, S.win, F, o, S.cig,
+    dp_finish(K, lut, S.g, tb, S.m, S.n, S.read, S.win, F, o, S.cig,
                    job.cigar_stride);
     if (F.trow) {
         o.touched = 1;
@@ -870,9 +985,9 @@ __device__ void process_pair(const GotohJob &job, const GotohConst &K,
     PairSetup S;
     if (!setup_pair(job, K, pi, job.tb_words, job.rb_words, true, S)) return;
     FillResult F =
-        S.win.cnt ? dp_fill<true, 32>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb)
-                  : dp_fill<false, 32>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb);
-    finish_pair<32>(job, K, lut, pi, S, F, tb);
+        S.win.cnt ? dp_fill<true>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb)
+                  : dp_fill<false>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb);
+    finish_pair(job, K, lut, pi, S, F, StripTb<32>{tb, S.sw});
 }
 
 template <int MINB>
@@ -1118,7 +1233,7 @@ __global__ void __launch_bounds__(128) gotoh_warp_kernel(GotohJob job, GotohCons
         if (!setup_pair(job, K, pi, job.tb_words, job.rb_words, lane == 0, S)) continue;
         FillResult F = warp_fill<false>(K, s_lut, S, tb, rb, lane);
         __syncwarp();  // traceback words of every lane are visible to lane 0
-        if (lane == 0) finish_pair<1>(job, K, s_lut25, pi, S, F, tb);
+        if (lane == 0) finish_pair(job, K, s_lut25, pi, S, F, StripTb<1>{tb, S.sw});
         __syncwarp();
     }
 }
@@ -1159,7 +1274,7 @@ __global__ void __launch_bounds__(128) gotoh_wide_kernel(GotohJob job, GotohCons
         FillResult F = warp_fill<true>(K, s_lut, S, tb, rb, lane);
         __syncwarp();
         int esc = 0;
-        if (lane == 0) esc = finish_pair<1>(job, K, s_lut25, pi, S, F, tb, false) ? 1 : 0;
+        if (lane == 0) esc = finish_pair(job, K, s_lut25, pi, S, F, StripTb<1>{tb, S.sw}, false) ? 1 : 0;
         esc = __shfl_sync(0xffffffffu, esc, 0);
         __syncwarp();
         if (!esc) continue;
@@ -1168,7 +1283,7 @@ __global__ void __launch_bounds__(128) gotoh_wide_kernel(GotohJob job, GotohCons
         if (!setup_pair(j2, K, pi, job.tb_words, job.rb_words, lane == 0, S)) continue;
         F = warp_fill<true>(K, s_lut, S, tb, rb, lane);
         __syncwarp();
-        if (lane == 0) finish_pair<1>(j2, K, s_lut25, pi, S, F, tb, false);
+        if (lane == 0) finish_pair(j2, K, s_lut25, pi, S, F, StripTb<1>{tb, S.sw}, false);
         __syncwarp();
     }
 }
@@ -1215,7 +1330,8 @@ cudaError_t launch_gotoh_wide(const GotohJob &job, const GotohConst &k, int warp
 //
 // Bound by the ALU pipe (78 % busy in the fill, 13.5 ALU of 23.5 issued
 // instructions a row of two cells; 28.9 ALU before these keys and corners).
-// 4,194,304 mixed pairs: 43.9 -> 38.0 ms.
+// 4,194,304 mixed pairs: 43.9 -> 33.4 ms (38.0 without the two-column interior,
+// its read-ahead and the one-pass walk).
 // ---------------------------------------------------------------------------
 
 constexpr uint32_t BIAS2 = 0x40004000u;
@@ -1236,6 +1352,7 @@ struct Keys2 {
     uint32_t ks;     // S / 4
     uint32_t ck0;    // row-max key of Hp at the strip's first column: Hp * ks + ck0
     int g;           // columns of a row-max key: blocks of 2^g
+    uint32_t miss;   // 4 * (score against N) in both halves
 };
 
 __device__ __forceinline__ Keys2 keys2_of(const GotohConst &K, int m, int sw) {
@@ -1247,6 +1364,7 @@ __device__ __forceinline__ Keys2 keys2_of(const GotohConst &K, int m, int sw) {
     c.e0 = c.ho0 - 0x00010001u;
     c.ks = 16384u / (uint32_t)(m * K.smax + 1);
     c.ck0 = (4u * c.ks - 1u) * 0x10001u - c.h0 * c.ks;
+    c.miss = (uint32_t)(4 * K.lut[4] & 0xffff) * 0x10001u;
     c.g = 0;
     while ((uint32_t)(sw - 1) >> c.g >= 4u * c.ks) c.g++;
     return c;
@@ -1258,29 +1376,43 @@ __device__ __forceinline__ uint32_t prmt(uint32_t lo, uint32_t hi, uint32_t sel)
     return r;
 }
 
+// One column as the rows see it.
+struct Col2 {
+    uint32_t sel;  // PRMT selector of both windows' codes
+    uint32_t ck;   // row-max key of Hp: Hp * ks + ck
+    uint32_t nkeep, nfill;  // N in a window: its half's score is nfill's
+};
+
+template <bool HASN>
+__device__ __forceinline__ uint32_t sub2(uint32_t la, uint32_t lb, const Col2 &col) {
+    const uint32_t x = prmt(la, lb, col.sel);
+    return HASN ? and_or_u32(x, col.nkeep, col.nfill) : x;
+}
+
 // Rows R0..R1 of one column, top to bottom.  Enters with the row above R0:
 // its Ho and E at this column and its Hp at the previous one (d); leaves with
 // row R1's Ho and E.  Returns the column's traceback words (pair A, pair B).
-template <int R0, int R1>
-__device__ __forceinline__ uint2 dp_rows2(Strip2 &S, const Keys2 &c, uint32_t sel, uint32_t ck,
+template <int R0, int R1, bool HASN>
+__device__ __forceinline__ uint2 dp_rows2(Strip2 &S, const Keys2 &c, const Col2 &col,
                                           uint32_t &upHo, uint32_t &upE, uint32_t d) {
     uint32_t wa = 0, wb = 0;
+    uint32_t kd = __viaddmax_u16x2(d, sub2<HASN>(S.la[R0], S.lb[R0], col), BIAS2 + 0x00030003u);
 #pragma unroll
     for (int r = R0; r <= R1; r++) {
-        const uint32_t left = S.Hl[r], kF = S.kF[r];
-        const uint32_t kE = __viaddmax_u16x2(upE, c.ex, upHo);
+        const uint32_t kE = __viaddmax_u16x2(upE, c.ex, upHo), kF = S.kF[r];
         upE = and_or_u32(kE, KEEP2, 0x00010001u);
         const uint32_t F4 = and_u32(kF, KEEP2);
-        const uint32_t kd = __viaddmax_u16x2(d, prmt(S.la[r], S.lb[r], sel), BIAS2 + 0x00030003u);
         const uint32_t key = __vimax3_u16x2(kd, upE, F4);
+        if (r < R1)  // the next row's diagonal, before this row's H is replaced
+            kd = __viaddmax_u16x2(S.Hl[r], sub2<HASN>(S.la[r + 1], S.lb[r + 1], col),
+                                  BIAS2 + 0x00030003u);
         const uint32_t Hp = and_or_u32(key, KEEP2, 0x00020002u);
+        S.Hl[r] = Hp;
         wa = mad_u32(wa, 4u, key - Hp);
         wb = mad_u32(wb, 4u, xor_and_u32(kE, kF, 0x00030003u));
         upHo = Hp - c.oe;
         S.kF[r] = __viaddmax_u16x2(F4, c.ex, upHo);
-        S.rmax[r] = __vmaxu2(S.rmax[r], mad_u32(Hp, c.ks, ck));
-        S.Hl[r] = Hp;
-        d = left;
+        S.rmax[r] = __vmaxu2(S.rmax[r], mad_u32(Hp, c.ks, col.ck));
     }
     constexpr int SH = 2 * (STRIP - 1 - R1);
     wa += 0xAAAAAAAAu & ((0x10001u << (2 * (R1 - R0 + 1))) - 0x10001u);  // tags, not tag - 2
@@ -1292,8 +1424,9 @@ __device__ __forceinline__ uint2 dp_rows2(Strip2 &S, const Keys2 &c, uint32_t se
 // The same over all 8 rows with every cell tested against its row window
 // (clamping strips): as dp_column's MASK.  hf: the rows' first-cell keys
 // (stride PAIR_BLOCK).  Leaves the last row's Hp in botH.
+template <bool HASN>
 __device__ __forceinline__ uint2 dp_masked2(Strip2 &S, const Keys2 &c, const Geo &g, int i0, int j,
-                                            uint32_t sel, uint32_t ck, uint32_t upHo, uint32_t &upE, uint32_t d,
+                                            const Col2 &col, uint32_t upHo, uint32_t &upE, uint32_t d,
                                             uint32_t &botH, uint32_t *hf) {
     uint32_t wa = 0, wb = 0;
 #pragma unroll
@@ -1302,7 +1435,7 @@ __device__ __forceinline__ uint2 dp_masked2(Strip2 &S, const Keys2 &c, const Geo
         const uint32_t kE = __viaddmax_u16x2(upE, c.ex, upHo);
         const uint32_t E1 = and_or_u32(kE, KEEP2, 0x00010001u);
         const uint32_t F4 = and_u32(kF, KEEP2);
-        const uint32_t kd = __viaddmax_u16x2(d, prmt(S.la[r], S.lb[r], sel), BIAS2 + 0x00030003u);
+        const uint32_t kd = __viaddmax_u16x2(d, sub2<HASN>(S.la[r], S.lb[r], col), BIAS2 + 0x00030003u);
         const uint32_t key = __vimax3_u16x2(kd, E1, F4);
         const uint32_t Hp = and_or_u32(key, KEEP2, 0x00020002u);
         wa = mad_u32(wa, 4u, key - Hp + 0x00020002u);
@@ -1311,7 +1444,7 @@ __device__ __forceinline__ uint2 dp_masked2(Strip2 &S, const Keys2 &c, const Geo
         const bool in = (j >= lo) & (j <= g.hi(i0 + r));
         if (in) {
             S.kF[r] = __viaddmax_u16x2(F4, c.ex, Hp - c.oe);
-            S.rmax[r] = __vmaxu2(S.rmax[r], mad_u32(Hp, c.ks, ck));
+            S.rmax[r] = __vmaxu2(S.rmax[r], mad_u32(Hp, c.ks, col.ck));
             S.Hl[r] = Hp;
         }
         if (j == lo) hf[r * PAIR_BLOCK] = S.rmax[r];
@@ -1324,58 +1457,96 @@ __device__ __forceinline__ uint2 dp_masked2(Strip2 &S, const Keys2 &c, const Geo
 }
 
 // The codes of both windows from column j on, 16 columns at a time.
+template <bool HASN>
 struct Codes2 {
-    uint32_t a, b;
-    int t;        // columns taken so far in this strip
-    uint32_t ck;  // ck0 of the column taken last
-    __device__ __forceinline__ void load(const uint8_t *arena, uint64_t wposA, uint64_t wposB, int j) {
-        a = load16(arena, wposA + (uint64_t)(j - 1));
-        b = load16(arena, wposB + (uint64_t)(j - 1));
+    const Seq &wa, &wb;
+    uint32_t a, b, na, nb;
+    int t;  // columns taken so far in this strip
+    __device__ __forceinline__ void load(int j) {
+        a = load16(wa.arena, wa.pos + (uint64_t)(j - 1));
+        b = load16(wa.arena, wb.pos + (uint64_t)(j - 1));  // one arena
+        if (HASN) {
+            na = wa.cnt ? nmask16(wa.iv, wa.cnt, j - 1) : 0u;
+            nb = wb.cnt ? nmask16(wb.iv, wb.cnt, j - 1) : 0u;
+        }
     }
-    // PRMT selector of this column's codes, then on to the next column
-    // (whose row-max keys are 1 lower every 2^g columns)
-    __device__ __forceinline__ uint32_t next(const Keys2 &c) {
-        const uint32_t sel = (a >> 30) * 0x11u + (b >> 30) * 0x1100u + 0xC480u;
+    // This column, then on to the next one (whose row-max keys are 1 lower
+    // every 2^g columns)
+    __device__ __forceinline__ Col2 next(const Keys2 &c) {
+        Col2 col;
+        col.sel = (a >> 30) * 0x11u + (b >> 30) * 0x1100u + 0xC480u;
         a <<= 2;
         b <<= 2;
-        ck = c.ck0 - (uint32_t)(t >> c.g) * 0x10001u;
+        col.ck = c.ck0 - (uint32_t)(t >> c.g) * 0x10001u;
         t++;
-        return sel;
+        if (HASN) {
+            col.nkeep = (na >> 31 ? 0u : 0xffffu) | (nb >> 31 ? 0u : 0xffff0000u);
+            col.nfill = c.miss & ~col.nkeep;
+            na <<= 1;
+            nb <<= 1;
+        }
+        return col;
+    }
+};
+
+// The words of the row above at the next AHEAD columns, read ahead of their
+// use: a column's arithmetic is ~200 cycles of dependent steps, an L2 round
+// trip several times that when few warps share the scheduler.  A slot is
+// rewritten only at or after the column that reads it.
+constexpr int AHEAD = 4;
+struct Above2 {
+    uint2 q[AHEAD];
+    const uint2 *p;  // the row above at the next column
+    int left;        // columns of it from there on
+    __device__ __forceinline__ uint2 at(int k, uint2 absent) const {
+        return k < left ? p[k * 32] : absent;
+    }
+    __device__ __forceinline__ void start(const uint2 *p_, int left_, uint2 absent) {
+        p = p_;
+        left = left_;
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++) q[k] = at(k, absent);
+    }
+    __device__ __forceinline__ uint2 next(uint2 absent) {
+        const uint2 up = q[0];
+#pragma unroll
+        for (int k = 0; k + 1 < AHEAD; k++) q[k] = q[k + 1];
+        q[AHEAD - 1] = at(AHEAD, absent);
+        p += 32;
+        left--;
+        return up;
     }
 };
 
 // Columns clo + K of a sloped strip's left corner: rows 0..K.
-template <int K>
-__device__ __forceinline__ void head2(Strip2 &S, const Keys2 &c, Codes2 &w, const uint2 *&rbr,
-                                      uint32_t &diag, uint2 *&tb, uint32_t *hf) {
+template <int K, bool HASN>
+__device__ __forceinline__ void head2(Strip2 &S, const Keys2 &c, Codes2<HASN> &w, Above2 &ab,
+                                      uint2 absent, uint32_t &diag, uint2 *&tb, uint32_t *hf) {
     if constexpr (K < STRIP - 1) {
-        const uint2 up = *rbr;
+        const uint2 up = ab.next(absent);
         uint32_t upHo = up.x - c.oe, upE = up.y;
-        const uint32_t sel = w.next(c);
-        __stcs(tb, dp_rows2<0, K>(S, c, sel, w.ck, upHo, upE, diag));
+        __stcs(tb, dp_rows2<0, K, HASN>(S, c, w.next(c), upHo, upE, diag));
         hf[K * PAIR_BLOCK] = S.rmax[K];
         diag = up.x;
-        rbr += 32;
         tb += 32;
-        head2<K + 1>(S, c, w, rbr, diag, tb, hf);
+        head2<K + 1, HASN>(S, c, w, ab, absent, diag, tb, hf);
     }
 }
 
 // Columns hi0 + K of a sloped strip's right corner: rows K..7, the row above
 // out of its window; up to column hi0 + last.
-template <int K>
-__device__ __forceinline__ void tail2(Strip2 &S, const Keys2 &c, Codes2 &w, int last, uint32_t &diag,
+template <int K, bool HASN>
+__device__ __forceinline__ void tail2(Strip2 &S, const Keys2 &c, Codes2<HASN> &w, int last, uint32_t &diag,
                                       uint2 *&rbw, uint2 *&tb) {
     if constexpr (K < STRIP) {
         if (K <= last) {
             uint32_t upHo = c.ho0, upE = c.e0;
-            const uint32_t sel = w.next(c);
-            __stcs(tb, dp_rows2<K, STRIP - 1>(S, c, sel, w.ck, upHo, upE, diag));
+            __stcs(tb, dp_rows2<K, STRIP - 1, HASN>(S, c, w.next(c), upHo, upE, diag));
             diag = S.Hl[K];  // row K's last cell: the next column's diagonal
             *rbw = make_uint2(upHo + c.oe, upE);
             rbw += 32;
             tb += 32;
-            tail2<K + 1>(S, c, w, last, diag, rbw, tb);
+            tail2<K + 1, HASN>(S, c, w, last, diag, rbw, tb);
         }
     }
 }
@@ -1387,12 +1558,16 @@ struct Best2 {
     int h[2], i[2], j0[2], j1[2];
 };
 
-// Fill the DP of two pairs with identical geometry (shared g, m, n, sw).
-// hf: the keys of the strip's 8 first cells in shared memory (stride PAIR_BLOCK).
-__device__ void dp_fill2(const GotohConst &K, const uint32_t *__restrict__ s_lut, int m, int n,
-                         const Geo &g, const Seq &readA, const Seq &readB, const uint8_t *warena,
-                         uint64_t wposA, uint64_t wposB, uint2 *tb0, int sw, uint2 *rb, uint32_t *hf,
-                         FillResult &FA, FillResult &FB) {
+// Fill the DP of two pairs with identical geometry (A's).  tb0, rb: the
+// lane's traceback words and row buffer, 32 word pairs apart; hf: the keys of
+// the strip's 8 first cells in shared memory (stride PAIR_BLOCK).
+template <bool HASN>
+__device__ void dp_fill2(const GotohConst &K, const uint32_t *__restrict__ s_lut,
+                         const PairSetup &A, const PairSetup &B2, uint2 *tb0, uint2 *rb,
+                         uint32_t *hf, FillResult &FA, FillResult &FB) {
+    const int m = A.m, n = A.n, sw = A.sw;
+    const Geo g = A.g;
+    const Seq readA = A.read, readB = B2.read;
     const Keys2 c = keys2_of(K, m, sw);
     const uint32_t ksc = 4u * c.ks;                  // S
     const uint32_t inv_s = 0xffffffffu / ksc + 1u;  // key / S = mulhi(key, inv_s): key < 2^16, S <= 2^16
@@ -1436,79 +1611,78 @@ __device__ void dp_fill2(const GotohConst &K, const uint32_t *__restrict__ s_lut
         uint2 *tb = tb0 + (size_t)s * sw * 32;
         const uint2 *rbr = rb + (size_t)(clo - plo) * 32;  // the row above at the next column
         uint2 *rbw = rb;                                   // the last row from column lo7 on
-        Codes2 w;
+        Codes2<HASN> w{A.win, B2.win};
         w.t = 0;
         if ((lslope | lflat) & (rslope | rflat)) {
             int jb = clo;  // first column with all 8 rows
+            const uint2 absent = make_uint2(c.h0, c.e0);
+            Above2 ab;
+            ab.start(rbr, phi - clo + 1, absent);
+            w.load(clo);
             if (lslope) {
-                w.load(warena, wposA, wposB, clo);
-                head2<0>(S, c, w, rbr, diag, tb, hf);
+                head2<0, HASN>(S, c, w, ab, absent, diag, tb, hf);
                 jb = lo7;
             }
-            // interior: all 8 rows in their windows, the row above present;
-            // its words are read two columns ahead of their use (the L2
-            // round trip is longer than one column of arithmetic).  A slot
-            // is rewritten only at or after the column that reads it.
-            const int je = rslope ? hi0 - 1 : min(hi0, phi);
-            uint2 up0 = make_uint2(c.h0, c.e0), up1 = up0;
-            if (jb <= je) up0 = rbr[0];
-            if (jb + 1 <= je) up1 = rbr[32];
-            for (int j = jb; j <= je;) {
-                w.load(warena, wposA, wposB, j);
-                const int cnt = min(16, je - j + 1);
+            // interior: all 8 rows in their windows, up to the first row's
+            // last column, where the row above is out of its window if that
+            // moved.  Two columns a turn: more of them, or a copy of the
+            // column for the odd one, do not fit the instruction cache
+            // beside the corners and the finish (four: no-instruction stalls
+            // 0.1 -> 3.1 an issue, 5.7 -> 6.8 ms for 1,048,576 pairs).
+            bool begins = true;  // rows begin in the next column
+            for (int j = jb; j <= hi0;) {
+                w.load(j);
+                const int stop = min(j + 16, hi0 + 1);
 #pragma unroll 1
-                for (int k = 0; k < cnt; k++, j++) {
-                    const uint2 up = up0;
-                    up0 = up1;
-                    if (j + 2 <= je) up1 = rbr[64];
-                    uint32_t upHo = up.x - c.oe, upE = up.y;
-                    const uint32_t sel = w.next(c);
-                    __stcs(tb, dp_rows2<0, STRIP - 1>(S, c, sel, w.ck, upHo, upE, diag));
+                while (j < stop) {
+                    const uint2 n0 = ab.at(AHEAD, absent), n1 = ab.at(AHEAD + 1, absent);
+                    uint32_t upHo = ab.q[0].x - c.oe, upE = ab.q[0].y;
+                    __stcs(tb, dp_rows2<0, STRIP - 1, HASN>(S, c, w.next(c), upHo, upE, diag));
                     *rbw = make_uint2(upHo + c.oe, upE);
-                    diag = up.x;
-                    if (j == jb) {  // the first cells of the rows that begin here
-                        if (lflat) {
+                    diag = ab.q[0].x;
+                    if (begins) {  // their first cells
 #pragma unroll
-                            for (int r = 0; r < STRIP - 1; r++) hf[r * PAIR_BLOCK] = S.rmax[r];
-                        }
-                        hf[(STRIP - 1) * PAIR_BLOCK] = S.rmax[STRIP - 1];
+                        for (int r = 0; r < STRIP; r++)
+                            if (lflat | (r == STRIP - 1)) hf[r * PAIR_BLOCK] = S.rmax[r];
+                        begins = false;
                     }
-                    rbr += 32;
+                    if (++j < stop) {
+                        upHo = ab.q[1].x - c.oe;
+                        upE = ab.q[1].y;
+                        __stcs(tb + 32,
+                               dp_rows2<0, STRIP - 1, HASN>(S, c, w.next(c), upHo, upE, diag));
+                        rbw[32] = make_uint2(upHo + c.oe, upE);
+                        diag = ab.q[1].x;
+                        j++;
+                        rbw += 32;
+                        tb += 32;
+                    }
+                    ab.q[0] = ab.q[2];
+                    ab.q[1] = ab.q[3];
+                    ab.q[2] = n0;
+                    ab.q[3] = n1;
+                    ab.p += 64;
+                    ab.left -= 2;
                     rbw += 32;
                     tb += 32;
                 }
             }
-            const bool first = jb > je;  // no interior column: rows begin in the one below
-            if (rslope | (hi0 > phi)) {
-                w.load(warena, wposA, wposB, je + 1);
-                // the first row's last column: the row above has a cell there
-                // only where its window did not move
-                const uint2 up = hi0 <= phi ? *rbr : make_uint2(c.h0, c.e0);
-                uint32_t upHo = up.x - c.oe, upE = up.y;
-                const uint32_t sel = w.next(c);
-                __stcs(tb, dp_rows2<0, STRIP - 1>(S, c, sel, w.ck, upHo, upE, diag));
-                *rbw = make_uint2(upHo + c.oe, upE);
+            if (rslope && nact > 1) {
+                w.load(hi0 + 1);
                 diag = S.Hl[0];
-                rbw += 32;
-                tb += 32;
-                if (first) {
-#pragma unroll
-                    for (int r = 0; r < STRIP; r++)
-                        if (lflat | (r == STRIP - 1)) hf[r * PAIR_BLOCK] = S.rmax[r];
-                }
-                if (rslope) tail2<1>(S, c, w, nact - 1, diag, rbw, tb);
+                tail2<1, HASN>(S, c, w, nact - 1, diag, rbw, tb);
             }
         } else {
             // clamping begins or ends inside the strip
             for (int j = clo; j <= chi;) {
-                w.load(warena, wposA, wposB, j);
+                w.load(j);
                 const int cnt = min(16, chi - j + 1);
 #pragma unroll 1
                 for (int k = 0; k < cnt; k++, j++) {
                     const uint2 up = j <= phi ? *rbr : make_uint2(c.h0, c.e0);
                     uint32_t upE = up.y, botH;
-                    const uint32_t sel = w.next(c);
-                    __stcs(tb, dp_masked2(S, c, g, i0, j, sel, w.ck, up.x - c.oe, upE, diag, botH, hf));
+                    __stcs(tb, dp_masked2<HASN>(S, c, g, i0, j, w.next(c), up.x - c.oe, upE, diag, botH,
+                                                 hf));
                     diag = up.x;
                     if (j >= lo7) {
                         *rbw = make_uint2(botH, upE);
@@ -1617,71 +1791,78 @@ __device__ void dp_fill2(const GotohConst &K, const uint32_t *__restrict__ s_lut
     put(FB, 1);
 }
 
-// Out-of-line fill, finish and lone-pair paths of the paired kernel: one
-// copy of each in the kernel's code, and their registers are not reserved
-// across one another.
+// Out-of-line fill, set-up and finish of the paired kernel: one copy of each in
+// the kernel's code (the instruction cache holds the fill and little more),
+// and their registers are not reserved across one another.
+template <bool HASN>
 __device__ __noinline__ void fill2_call(const GotohConst &K, const uint32_t *__restrict__ s_lut,
                                         const PairSetup &A, const PairSetup &B, uint32_t *tb,
                                         uint32_t *rb, uint32_t *hf, FillResult &FA, FillResult &FB) {
-    dp_fill2(K, s_lut, A.m, A.n, A.g, A.read, B.read, A.win.arena, A.win.pos, B.win.pos,
-             reinterpret_cast<uint2 *>(tb), A.sw, reinterpret_cast<uint2 *>(rb), hf, FA, FB);
+    dp_fill2<HASN>(K, s_lut, A, B, reinterpret_cast<uint2 *>(tb), reinterpret_cast<uint2 *>(rb), hf,
+                   FA, FB);
 }
 
 __device__ __noinline__ void finish_call(const GotohJob &job, const GotohConst &K,
                                          const int8_t *__restrict__ lut, uint32_t pi,
                                          PairSetup &S, const FillResult &F, const uint32_t *tb) {
-    finish_pair<64>(job, K, lut, pi, S, F, tb);
+    finish_pair(job, K, lut, pi, S, F, StripTb<64>{tb, S.sw});
 }
 
-// A pair without a partner of its geometry: the paired fill with itself in
-// both lanes, or, when its window has N (the paired fill takes N in reads
-// only), the one-pair fill with its row buffer in the words of the second
-// pair (tb_words >= rb_words: a pair's traceback holds at least one strip of
-// row-buffer width; the lane's own words, as the other lanes' fills run
-// beside it).
-__device__ __noinline__ void lone_call(const GotohJob &job, const GotohConst &K,
-                                       const uint32_t *__restrict__ s_lut,
-                                       const int8_t *__restrict__ lut, uint32_t pi, PairSetup &S,
-                                       uint32_t *tb, uint32_t *rb, uint32_t *hf) {
-    FillResult F, F2;
-    if (S.win.cnt)
-        F = dp_fill<true, 64>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, tb + 1);
-    else
-        fill2_call(K, s_lut, S, S, tb, rb, hf, F, F2);
-    finish_call(job, K, lut, pi, S, F, tb);
+__device__ __noinline__ bool setup_call(const GotohJob &job, const GotohConst &K, uint32_t pi,
+                                        bool write, PairSetup &S) {
+    return setup_pair(job, K, pi, job.tb_words, job.rb_words, write, S);
 }
 
-// Work item (a, b): both pairs in one thread when their geometry matches and
-// their windows carry no N; otherwise one after the other (b = NONE: a alone).
-// The descriptors are resolved again after the fill rather than kept live
-// across it.
+// Work item (p[0], p[1]) of every lane (NO_PAIR: none): both pairs in one
+// fill when their geometry matches; a pair without a partner of its geometry
+// fills both halves, in the same pass over the lanes (lanes that took turns
+// doubled a warp's time), and a second pass takes the other pair of a
+// mismatched item.  N in a window costs one more instruction a row, so a warp
+// that holds one runs that fill for all its lanes.  The descriptors are
+// resolved again for the finish rather than kept live across the fill.
 constexpr uint32_t NO_PAIR = 0xffffffffu;
 
 __device__ void process_item2(const GotohJob &job, const GotohConst &K,
                               const uint32_t *__restrict__ s_lut, const int8_t *__restrict__ lut,
-                              uint32_t pa, uint32_t pb, uint32_t *tb, uint32_t *rb,
-                              uint32_t *hf) {
-    bool both;
-    FillResult FA, FB;
-    {
-        PairSetup A, B;
-        const bool ra = setup_pair(job, K, pa, job.tb_words, job.rb_words, true, A);
-        const bool rb_ = pb != NO_PAIR && setup_pair(job, K, pb, job.tb_words, job.rb_words, true, B);
-        both = ra && rb_ && A.m == B.m && A.n == B.n && A.full == B.full &&
-               A.g.off == B.g.off && A.g.half == B.g.half && A.win.cnt == 0 && B.win.cnt == 0;
-        if (both) {
-            fill2_call(K, s_lut, A, B, tb, rb, hf, FA, FB);
-        } else {
-            if (ra) lone_call(job, K, s_lut, lut, pa, A, tb, rb, hf);
-            if (rb_) lone_call(job, K, s_lut, lut, pb, B, tb, rb, hf);
+                              const uint32_t (&p)[2], uint32_t *tb, uint32_t *rb, uint32_t *hf) {
+    int todo = 0;  // bit q: pair q has a DP
+    bool together = false;
+    for (int pass = 0; pass < 2; pass++) {
+        FillResult F[2];
+        int now = 0;  // pairs of this pass
+        {
+            PairSetup A, B;
+            if (pass == 0) {
+                const bool a = p[0] != NO_PAIR && setup_call(job, K, p[0], true, A);
+                const bool b = p[1] != NO_PAIR && setup_call(job, K, p[1], true, B);
+                todo = (a ? 1 : 0) | (b ? 2 : 0);
+                together = todo == 3 && A.m == B.m && A.n == B.n && A.full == B.full &&
+                           A.g.off == B.g.off && A.g.half == B.g.half;
+                now = together ? 3 : (todo == 3 ? 1 : todo);
+                if (now == 1) B = A;
+                if (now == 2) A = B;
+            } else {
+                now = todo == 3 && !together ? 2 : 0;
+                if (!__any_sync(0xffffffffu, now != 0)) break;
+                if (now) {
+                    setup_call(job, K, p[1], false, A);
+                    B = A;
+                }
+            }
+            const bool n = __any_sync(0xffffffffu, now && (A.win.cnt || B.win.cnt));
+            if (now) {
+                if (n) fill2_call<true>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
+                else fill2_call<false>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
+            }
         }
-    }
-    if (both) {
-        PairSetup A, B;
-        setup_pair(job, K, pa, job.tb_words, job.rb_words, false, A);
-        finish_call(job, K, lut, pa, A, FA, tb);
-        setup_pair(job, K, pb, job.tb_words, job.rb_words, false, B);
-        finish_call(job, K, lut, pb, B, FB, tb + 1);
+#pragma unroll 1
+        for (int q = 0; q < 2; q++) {
+            if (now >> q & 1) {
+                PairSetup S;
+                setup_call(job, K, p[q], false, S);
+                finish_call(job, K, lut, p[q], S, F[q], tb + q);
+            }
+        }
     }
 }
 
@@ -1717,12 +1898,13 @@ __global__ void __launch_bounds__(PAIR_BLOCK, MINB) gotoh2_kernel(GotohJob job, 
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= total) break;
         uint64_t k = base + lane;
+        uint32_t p[2] = {NO_PAIR, NO_PAIR};
         if (k < total) {
-            uint64_t x = b0 + 2 * k, y = x + 1;
-            uint32_t pa = job.list ? job.list[x] : (uint32_t)x;
-            uint32_t pb = y < b1 ? (job.list ? job.list[y] : (uint32_t)y) : NO_PAIR;
-            process_item2(job, K, s_lut, s_lut25, pa, pb, tb, rb, s_first + threadIdx.x);
+            const uint64_t x = b0 + 2 * k, y = x + 1;
+            p[0] = job.list ? job.list[x] : (uint32_t)x;
+            if (y < b1) p[1] = job.list ? job.list[y] : (uint32_t)y;
         }
+        process_item2(job, K, s_lut, s_lut25, p, tb, rb, s_first + threadIdx.x);
     }
 }
 
