@@ -14,8 +14,9 @@
 #include "esp_host.h"
 
 // Kernel variant of a handle that was neither set nor tuned: the
-// ESP_GOTOH_VARIANT environment variable (0..3), else 1 -- and then band
-// batches of 2^20 pairs and more take the paired kernel (band_variant).
+// ESP_GOTOH_VARIANT environment variable (0..3), else 1 -- and then batches of
+// 2^18 pairs and more take the paired kernel (band_variant), smaller binned
+// ones the mixed kernel (mixed_by_size).
 static int default_variant(bool *by_size = nullptr) {
     const char *v = getenv("ESP_GOTOH_VARIANT");
     const bool env = v && v[0] >= '0' && v[0] < '0' + esp::kGotohVariants && !v[1];
@@ -28,24 +29,20 @@ static void resolve_variant(esp_handle *h) {
 }
 
 // Variant of an untuned band batch of n pairs: the handle's, except that a
-// handle left at the default runs batches of 2^20 pairs and more on the
-// paired kernel (the mixed-length workload: 1,054 vs ~900 GCUPS at 2^20
-// pairs, 1,148 vs 930 at 2^22; at 2^18 the one-pair kernel wins, 738 vs
-// 397).  esp_batch_autotune measures instead of assuming.
+// handle left at the default runs batches of 2^18 pairs and more on the paired
+// kernel (262,144 pairs of 150 x 214 in 1.51 ms against 2.44 with one pair per
+// thread, mixed 3.52 / 4.63; 600,000 mixed 4.94 / 8.16).  esp_batch_autotune
+// measures instead of assuming.
 static int band_variant(esp_handle *h, uint64_t n) {
     resolve_variant(h);
-    if (h->variant_by_size && h->binning && n >= (1u << 20)) return 3;
+    if (h->variant_by_size && h->binning && n >= (1u << 18)) return 3;
     return h->variant;
 }
 
-// Kernel variant of a hint-mode batch of n pairs.  Hint batches repeat one
-// geometry when their windows are cut the same way (the splice flanks: read
-// segment vs segment + 30 bases at offset 0), so from 2^20 pairs on they run
-// the paired kernel (measured: the 69M-pair splice flank batch 1,063 vs 974
-// GCUPS); smaller ones cannot fill the GPU with two-pair items (a 65,536-pair
-// batch 3.94 vs 3.14 ms, the serve loop's requests 16.0 vs 22.5 M pairs/s
-// peak) and run one pair per thread.  ESP_GOTOH_HINT_VARIANT (0..3)
-// overrides.
+// Kernel variant of a hint-mode batch of n pairs: from 2^18 pairs on the
+// paired kernel (262,144 pairs of 150 x 214 in 3.75 ms against 7.89 with one pair
+// per thread, mixed 8.76 / 13.3), below it, where the mixed kernel does not apply,
+// the handle's one-pair variant.  ESP_GOTOH_HINT_VARIANT (0..3) overrides.
 static int hint_variant(esp_handle *h, uint64_t n) {
     if (h->hint_variant < -1) {
         const char *v = getenv("ESP_GOTOH_HINT_VARIANT");
@@ -53,7 +50,7 @@ static int hint_variant(esp_handle *h, uint64_t n) {
             (v && v[0] >= '0' && v[0] < '0' + esp::kGotohVariants && !v[1]) ? v[0] - '0' : -1;
     }
     if (h->hint_variant >= 0) return h->hint_variant;
-    if (h->binning && n >= (1u << 20)) return 3;
+    if (h->binning && n >= (1u << 18)) return 3;
     resolve_variant(h);
     return esp::gotoh_paired(h->variant) ? h->variant - 2 : h->variant;
 }
@@ -70,6 +67,22 @@ static bool band_paired(esp_handle *h, uint64_t n) {
     return esp::gotoh_paired(band_variant(h, n));
 }
 
+// Whether a batch of n pairs runs the mixed kernel: a handle whose kernel was
+// neither set nor tuned, below 2^18 pairs.  Measured against one pair per thread
+// (the earlier choice) and two, in ms: 4,096 mixed pairs 0.54 / 1.84 / 2.21,
+// 65,536 mixed 1.49 / 3.46 / 2.98, 131,072 mixed 2.60 / 3.62 / 2.96; 4,096 of 150
+// x 214 0.25 / 0.35 / 0.40, 65,536 0.85 / 0.81 / 0.80, 131,072 0.92 / 1.44 / 0.90;
+// extend_hint over 65,536 mixed pairs 3.18 / 7.27 / 6.57.  At 262,144 pairs two
+// per thread are even (1.51 of 1.55 and 3.52 of 3.15 ms), at 600,000 ahead
+// (4.94 of 5.60).
+static bool mixed_by_size(esp_handle *h, int mode, uint64_t n) {
+    resolve_variant(h);
+    if (!h->binning || n <= 32 || n >= (1u << 18) || h->autotune_ms) return false;
+    if (mode == ESP_MODE_BAND) return h->variant_by_size && !h->tuned;
+    hint_variant(h, n);  // reads ESP_GOTOH_HINT_VARIANT
+    return h->hint_variant < 0 && h->variant_by_size;
+}
+
 // How one batch of n_pairs uses DP scratch: which kernel runs, with how
 // many warps, and the traceback / row-buffer bytes they need (the choices
 // enqueue_batch makes; the serve loop charges launches with it).
@@ -78,6 +91,12 @@ struct DpPlan {
     int var = 1;             // thread-kernel variant
     bool per_class = false;  // one launch per length class of the binned list
     bool paired = false;     // a two-pairs-per-thread variant is among the launches
+    bool mixed = false;      // the mixed kernel
+    bool all_groups = false; // ... with every item in groups of at least 1 << min_lg lanes
+    int min_lg = 2;
+    uint64_t gtw = 0, grw = 0;    // its groups' word pairs per lane / per group
+    uint64_t wtb = 0, wrb = 0;    // its words per warp
+    float threads = 0;            // threads of its full grid
     uint64_t warps = 0;
     uint64_t tbw = 0, rbw = 0;  // words per thread (warp kernel: per warp)
     uint64_t tb_bytes = 0, rb_bytes = 0;
@@ -101,6 +120,44 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
         warps = std::min(warps, std::max<uint64_t>(1, h->scratch_budget / per_warp_bytes));
         P.warps = (warps + 3) / 4 * 4;  // whole blocks: every launched warp owns its scratch
         P.tb_bytes = P.warps * per_warp_bytes;
+        return P;
+    }
+    if (mixed_by_size(h, mode, n_pairs)) {
+        if (!h->mixed_bps) h->mixed_bps = esp::gotoh_mixed_blocks_per_sm();
+        const uint64_t resident = (uint64_t)h->num_sms * h->mixed_bps * 4;  // warps
+        const uint64_t items = (n_pairs + 1) / 2;
+        P.mixed = P.paired = true;
+        P.threads = (float)(resident * 32);
+        // bin_plan's x for pairs of one cost, the least it can be: below its
+        // line all items are the costliest, and all go to groups
+        const double x = P.threads * 0.305 / (0.4 * (double)items);
+        P.all_groups = x * 0.4 > 0.75;
+        if (P.all_groups) P.min_lg = x < 5 ? 2 : (x < 11 ? 3 : (x < 60 ? 4 : 5));
+        auto size = [&](int lg) {
+            P.min_lg = lg;
+            P.gtw = P.grw = 0;
+            for (const Limits *L : {&L1, &L2}) {
+                if (L == &L2 && mode != ESP_MODE_HINT) continue;
+                P.gtw = std::max(P.gtw, esp::group_steps(L->max_m, L->max_n, L->rb_words, lg));
+                P.grw = std::max<uint64_t>(P.grw, L->max_n + 1ull);
+            }
+            P.wtb = 64 * P.gtw;
+            P.wrb = 2 * P.grw * (32u >> lg);
+            if (!P.all_groups) {
+                P.wtb = std::max(P.wtb, 64 * P.tbw);
+                P.wrb = std::max(P.wrb, 64 * P.rbw);
+            }
+            const uint64_t groups = 32u >> lg;
+            const uint64_t want = std::min(resident, P.all_groups ? (items + groups - 1) / groups : items);
+            P.warps = std::min(want, std::max<uint64_t>(1, h->scratch_budget / ((P.wtb + P.wrb) * 4)));
+            P.warps = (P.warps + 3) / 4 * 4;  // whole blocks: every launched warp owns its scratch
+            return P.warps >= want;
+        };
+        // more lanes an item need less scratch for as many items in flight
+        int lg = P.min_lg;
+        while (!size(lg) && P.all_groups && lg < 5) lg++;
+        P.tb_bytes = P.warps * P.wtb * 4;
+        P.rb_bytes = P.warps * P.wrb * 4;
         return P;
     }
     // scratch slots: one warp per 32 pairs up to the resident limit, bounded
@@ -269,6 +326,20 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
     CK(h, cudaMemsetAsync(h->d_ctr, 0, 256, st));
     const uint32_t *order = nullptr;
     const uint32_t *list_len = nullptr;  // device word: length of a padded list
+    auto plan_for = [&](int attempt) {
+        return esp::BinPlan{h->d_ctr + 40 + 4 * attempt, h->d_ctr + 36 + 2 * attempt, P.min_lg,
+                            P.all_groups, P.threads};
+    };
+    auto launch_dp = [&](esp::GotohJob &j, int attempt) {
+        if (!P.mixed) return esp::launch_gotoh(j, K, (int)warps, 128, st, var);
+        j.group_plan = h->d_ctr + 36 + 2 * attempt;
+        j.group_queue = h->d_ctr + 32 + 2 * attempt;
+        j.group_tb_words = P.gtw;
+        j.group_rb_words = P.grw;
+        j.warp_tb_words = P.wtb;
+        j.warp_rb_words = P.wrb;
+        return esp::launch_gotoh_mixed(j, K, (int)warps, st);
+    };
     if (h->binning && n_pairs > 32) {
         // the paired kernels want each geometry bin at an even list offset
         const uint64_t slots = n_pairs + (paired ? esp::bin_pad_slots(n_pairs) : 0);
@@ -276,10 +347,12 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
             return rc;
         if ((rc = grow_device(h, (void **)&h->d_order, &h->d_order_cap, slots * sizeof(uint32_t))) != ESP_OK)
             return rc;
+        const esp::BinPlan bp = plan_for(0);
         CK(h, esp::launch_binning(d_pairs, n_pairs, mode == ESP_MODE_HINT ? 1 : 0, h->d_hist,
                                   h->d_order, h->num_sms, st, h->d_ctr + 29,
-                                  per_class ? h->d_ctr + 24 : nullptr, paired));
-        h->launches += 5 + (per_class ? 1 : 0);  // kernels; the memsets are not counted
+                                  per_class ? h->d_ctr + 24 : nullptr, paired, nullptr, nullptr,
+                                  P.mixed ? &bp : nullptr));
+        h->launches += 5 + (per_class || P.mixed ? 1 : 0);  // kernels; the memsets are not counted
         order = h->d_order;
         if (paired) list_len = h->d_ctr + 29;
     }
@@ -347,7 +420,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
             h->launches++;
         }
     } else {
-        CK(h, esp::launch_gotoh(job, K, (int)warps, 128, st, var));
+        CK(h, launch_dp(job, 0));
         h->launches++;
     }
     if (mode == ESP_MODE_HINT) {
@@ -361,13 +434,15 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
         j2.list_count = h->d_ctr + 4;
         j2.queue = h->d_ctr + 2;
         if (order) {
+            const esp::BinPlan bp = plan_for(1);
             CK(h, esp::launch_binning(d_pairs, n_pairs, 2, h->d_hist, h->d_order, h->num_sms, st,
-                                      h->d_ctr + 31, nullptr, paired, h->d_esc, h->d_ctr + 4));
-            h->launches += 5;
+                                      h->d_ctr + 31, nullptr, paired, h->d_esc, h->d_ctr + 4,
+                                      P.mixed ? &bp : nullptr));
+            h->launches += 5 + (P.mixed ? 1 : 0);
             j2.list = h->d_order;
             j2.list_count = paired ? h->d_ctr + 31 : h->d_ctr + 4;
         }
-        CK(h, esp::launch_gotoh(j2, K, (int)warps, 128, st, var));
+        CK(h, launch_dp(j2, 1));
         h->launches++;
     }
     return launch_wide(job);
@@ -380,7 +455,8 @@ int reserve_lists(esp_handle *h, uint64_t max_pairs) {
     if ((rc = grow_device(h, (void **)&h->d_esc, &h->d_esc_cap, max_pairs * 4)) != ESP_OK) return rc;
     if ((rc = grow_device(h, (void **)&h->d_hist, &h->d_hist_cap, esp::bin_scratch_bytes())) != ESP_OK)
         return rc;
-    return grow_device(h, (void **)&h->d_order, &h->d_order_cap, max_pairs * 4);
+    return grow_device(h, (void **)&h->d_order, &h->d_order_cap,
+                       (max_pairs + esp::bin_pad_slots(max_pairs)) * 4);
 }
 
 extern "C" {
@@ -599,9 +675,11 @@ static void merge(ScanOut &into, const ScanOut &s) {
     into.L1.tb_words = std::max(into.L1.tb_words, s.L1.tb_words);
     into.L1.rb_words = std::max(into.L1.rb_words, s.L1.rb_words);
     into.L1.max_m = std::max(into.L1.max_m, s.L1.max_m);
+    into.L1.max_n = std::max(into.L1.max_n, s.L1.max_n);
     into.L2.tb_words = std::max(into.L2.tb_words, s.L2.tb_words);
     into.L2.rb_words = std::max(into.L2.rb_words, s.L2.rb_words);
     into.L2.max_m = std::max(into.L2.max_m, s.L2.max_m);
+    into.L2.max_n = std::max(into.L2.max_n, s.L2.max_n);
     into.arena_end = std::max(into.arena_end, s.arena_end);
 }
 

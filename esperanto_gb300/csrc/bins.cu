@@ -63,15 +63,50 @@ __device__ __forceinline__ void agg_add(uint32_t *ctr, uint32_t key, uint32_t *s
     if (slot) *slot = base + rank;
 }
 
+// Cells a pair's DP computes, near enough to weigh one pair against another.
+__device__ __forceinline__ uint32_t cost_of(const esp_pair &P, int mode) {
+    const uint32_t n = P.win_len;
+    const bool full = mode == 0 ? P.band_half < 0 : (mode == 2 || n <= 30);
+    const uint64_t band = 2ull * (mode == 0 ? (uint32_t)P.band_half : 30u) + 1;
+    const uint64_t w = full || band > n ? n : band;
+    const uint64_t c = w * P.read_len;
+    return c < 0xffffffffull ? (uint32_t)c : 0xffffffffu;
+}
+
+// stats (optional, zeroed): the sum of the pairs' costs, the largest cost and
+// the longest read.
+struct BinStats {
+    unsigned long long cost;
+    uint32_t max_cost, max_m;
+};
+
 __global__ void bin_hist(const esp_pair *__restrict__ pairs, uint64_t n, BinInput in, int mode,
-                         uint32_t *__restrict__ hist) {
+                         uint32_t *__restrict__ hist, BinStats *__restrict__ stats) {
     const uint64_t cnt = in.size(n);
+    unsigned long long cost = 0;
+    uint32_t max_cost = 0, max_m = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t pi = in.at(i);
         if (pi >= n) continue;  // never index past the batch
-        uint32_t key = geometry_key(pairs[pi], mode);
-        agg_add(hist, NBINS - 1 - key, nullptr);  // descending cost order
+        const esp_pair P = pairs[pi];
+        agg_add(hist, NBINS - 1 - geometry_key(P, mode), nullptr);  // descending cost order
+        if (stats) {
+            const uint32_t c = cost_of(P, mode);
+            cost += c;
+            max_cost = max(max_cost, c);
+            max_m = max(max_m, P.read_len);
+        }
+    }
+    if (stats) {
+        for (int o = 16; o; o >>= 1) cost += __shfl_down_sync(0xffffffffu, cost, o);
+        max_cost = __reduce_max_sync(0xffffffffu, max_cost);
+        max_m = __reduce_max_sync(0xffffffffu, max_m);
+        if ((threadIdx.x & 31) == 0 && max_cost) {
+            atomicAdd(&stats->cost, cost);
+            atomicMax(&stats->max_cost, max_cost);
+            atomicMax(&stats->max_m, max_m);
+        }
     }
 }
 
@@ -235,10 +270,45 @@ __global__ void class_bounds(const uint32_t *__restrict__ hist, const uint32_t *
     }
 }
 
+// The mixed kernel's plan from the batch's costs (in cells; an item is two
+// pairs): {list entries its groups run, log2 of a group's lanes}.
+//
+// A thread takes ~25 ns a row of 8 x 2 cells when its warp has the scheduler
+// to itself (52 cycles, measured), the full chip 1.9 T cells/s: an item
+// finishes with the rest of the batch when its cost is the mean cost times
+// items / 23,700 (0.305 x the 77,824 resident threads).  Batches whose costliest
+// item takes more than three quarters of that give the items above it to
+// groups: 65,536 pairs of 150 x 214 (0.72 of it) take 0.80 ms by threads and 0.93
+// in groups of 4; 65,536 mixed pairs (3.3 times it) 2.98 ms by threads, 1.49 split.
+// Lanes of a group from how far the costliest item is above it (the fastest of
+// 4, 8, 16 and 32 lanes at 4,096 to 200,000 pairs of one shape and mixed).
+__global__ void bin_plan(const uint32_t *__restrict__ hist, const uint32_t *__restrict__ total,
+                         const BinStats *__restrict__ stats, int mode, int min_lg, bool all,
+                         float threads, uint32_t *__restrict__ plan) {
+    if (threadIdx.x != 0) return;
+    const float even = (float)stats->cost / (threads * 0.305f);  // of one pair of the item
+    const float top = 2.0f * (float)stats->max_cost;
+    const float x = even > 0.0f ? top / (0.4f * even) : 0.0f;
+    const int lg = x < 5.0f ? 2 : (x < 11.0f ? 3 : (x < 60.0f ? 4 : 5));
+    uint32_t split = 0;
+    if (all) {
+        split = *total;
+    } else if (top > 0.75f * even) {
+        // items of w columns a row and more: the list's order.  extend_hint's
+        // first attempt has one width, its list goes by window length.
+        const uint32_t cap = (1u << KEY_BITS) - 1;
+        const float w = 0.375f * even / (float)max(stats->max_m, 1u);
+        if (mode == 1) split = *total;
+        else split = w < 1.0f ? *total : hist[NBINS - 1 - ((min((uint32_t)w, cap - 1u) << KEY_BITS) | cap)];
+    }
+    plan[0] = split;
+    plan[1] = (uint32_t)max(lg, min_lg);
+}
+
 cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t *hist,
                            uint32_t *order, int num_sms, cudaStream_t st, uint32_t *total,
                            uint32_t *bounds, bool pad, const uint32_t *list,
-                           const uint32_t *list_count) {
+                           const uint32_t *list_count, const BinPlan *plan) {
     const BinInput in{list, list_count};
     cudaError_t e = cudaMemsetAsync(hist, 0, bin_scratch_bytes(), st);
     if (e == cudaSuccess && pad)
@@ -247,13 +317,17 @@ cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t
     int grid = num_sms * 4;
     uint64_t need = (n + 255) / 256;
     if ((uint64_t)grid > need) grid = (int)(need ? need : 1);
-    bin_hist<<<grid, 256, 0, st>>>(pairs, n, in, mode, hist);
+    BinStats *stats = plan ? reinterpret_cast<BinStats *>(plan->stats) : nullptr;
+    bin_hist<<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, stats);
     if (pad) bin_scan_up<true><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     else bin_scan_up<false><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     bin_scan_top<<<1, 1024, 0, st>>>(hist + NBINS, total);
     if (pad) bin_scan_down<true><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     else bin_scan_down<false><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     if (bounds) class_bounds<<<1, 32, 0, st>>>(hist, total, bounds);
+    if (plan)
+        bin_plan<<<1, 32, 0, st>>>(hist, total, stats, mode, plan->min_lg, plan->all, plan->threads,
+                                   plan->plan);
     bin_scatter<<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, order);
     return cudaGetLastError();
 }

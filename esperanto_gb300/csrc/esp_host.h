@@ -26,6 +26,7 @@ struct esp_handle {
     uint64_t launches = 0;
     int gotoh_bps[esp::kGotohVariants] = {};  // resident DP blocks per SM (queried once)
     int variant = -1;   // DP kernel variant; -1 = ESP_GOTOH_VARIANT env or default
+    int mixed_bps = 0;             // resident blocks of the mixed kernel per SM (queried once)
     bool variant_by_size = false;  // default variant: large band batches run paired
     int hint_variant = -2;  // variant of hint-mode batches: >= 0 forced (ESP_GOTOH_HINT_VARIANT),
                             // -1 by batch size (abi.cu hint_variant), -2 = env not read yet
@@ -58,7 +59,9 @@ struct esp_handle {
     // d_ctr (256 B): u64 queues at [0..1] (attempt 1), [2..3] (attempt 2),
     // u32 esc count at [4], u64 class queues at [8..15], class bounds at
     // [24..28], binned list length at [29], wide-list count at [30], binned
-    // escalation list length at [31]
+    // escalation list length at [31]; the mixed kernel's group queues at
+    // [32..33] and [34..35] (second attempt), plans at [36..37] and [38..39],
+    // batch costs at [40..43] and [44..47]
     uint32_t *d_ctr = nullptr;
     int tune[esp::kLengthClasses] = {-1, -1, -1, -1};  // DP variant per length class (autotuned)
     bool tuned = false;
@@ -169,8 +172,8 @@ inline void encode_seq(const uint8_t *s, size_t len, uint8_t *arena, uint64_t po
 
 
 struct Limits {
-    uint64_t tb_words = 1, rb_words = 1;
-    uint32_t max_m = 0;
+    uint64_t tb_words = 1, rb_words = 1;  // rb_words: columns a strip
+    uint32_t max_m = 0, max_n = 0;
 };
 
 // The handle's host worker pool (up to 16 threads with the caller).
@@ -188,6 +191,7 @@ inline void add_limits(Limits &L, uint32_t m, uint32_t n, int32_t half) {
     L.tb_words = std::max(L.tb_words, tb);
     L.rb_words = std::max(L.rb_words, rb);
     L.max_m = std::max(L.max_m, m);
+    L.max_n = std::max(L.max_n, n);
 }
 
 

@@ -63,6 +63,12 @@ struct GotohJob {
     uint32_t *wide_list;
     uint32_t *wide_count;
     int wide;
+    // mixed kernel: device {list entries run by groups, log2 of a group's
+    // lanes}, their queue, and the scratch of a warp
+    const uint32_t *group_plan;
+    uint32_t *group_queue;
+    uint64_t group_tb_words, group_rb_words;  // word pairs per lane / per group
+    uint64_t warp_tb_words, warp_rb_words;    // words per warp (both sections)
 };
 
 // Launch the persistent DP kernel with `warps` warps total.
@@ -89,6 +95,18 @@ cudaError_t launch_gotoh_wide(const GotohJob &job, const GotohConst &k, int warp
 // traceback scratch (job.tb), job.rb unused.  Same results as launch_gotoh.
 cudaError_t launch_gotoh_warp(const GotohJob &job, const GotohConst &k, int warps,
                               cudaStream_t st);
+
+// Mixed kernel over a padded binned list (job.list, job.list_count): the
+// entries before job.group_plan[0] run in groups of 4..32 lanes per two pairs,
+// the rest two pairs per thread.  Each warp owns warp_tb_words words of job.tb
+// and warp_rb_words of job.rb, each the larger of what its sections need: 64 *
+// group_tb_words (>= group_steps of the pairs) or 64 * tb_words; 2 *
+// group_rb_words (> the pairs' windows) per group or 64 * rb_words.  Same results
+// as launch_gotoh.
+cudaError_t launch_gotoh_mixed(const GotohJob &job, const GotohConst &k, int warps,
+                               cudaStream_t st);
+uint64_t group_steps(uint64_t m, uint64_t n, uint64_t sw, int lg);
+int gotoh_mixed_blocks_per_sm();
 
 // Resident blocks per SM of the DP kernel at `block` threads.
 int gotoh_blocks_per_sm(int block, int variant);
@@ -164,10 +182,19 @@ cudaError_t launch_count_cells(const esp_pair *pairs, const esp_extension *out, 
 // mode: 0 band, 1 extend_hint's first attempt, 2 its full-matrix attempt.
 // list / list_count (device, optional): bin only the pairs list[0 ..
 // *list_count), n bounding the count (extend_hint's escalations).
+// plan (optional): also weigh the pairs and plan the mixed kernel (one launch
+// more).
+struct BinPlan {
+    uint32_t *stats;  // 4 zeroed device words, 8-byte aligned
+    uint32_t *plan;   // 2 device words: GotohJob::group_plan
+    int min_lg;       // fewest lanes (log2) the scratch was sized for
+    bool all;         // the whole list goes to groups
+    float threads;    // resident threads of the launch's full grid
+};
 cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t *hist,
                            uint32_t *order, int num_sms, cudaStream_t st, uint32_t *total,
                            uint32_t *bounds, bool pad, const uint32_t *list = nullptr,
-                           const uint32_t *list_count = nullptr);
+                           const uint32_t *list_count = nullptr, const BinPlan *plan = nullptr);
 // Spare slots a padded list may add to n pairs (the list holds n + this).
 uint64_t bin_pad_slots(uint64_t n);
 constexpr int kLengthClasses = 4;

@@ -1470,21 +1470,30 @@ struct Codes2 {
             nb = wb.cnt ? nmask16(wb.iv, wb.cnt, j - 1) : 0u;
         }
     }
-    // This column, then on to the next one (whose row-max keys are 1 lower
-    // every 2^g columns)
-    __device__ __forceinline__ Col2 next(const Keys2 &c) {
+    __device__ __forceinline__ Col2 here(const Keys2 &c) const {
         Col2 col;
         col.sel = (a >> 30) * 0x11u + (b >> 30) * 0x1100u + 0xC480u;
-        a <<= 2;
-        b <<= 2;
         col.ck = c.ck0 - (uint32_t)(t >> c.g) * 0x10001u;
-        t++;
         if (HASN) {
             col.nkeep = (na >> 31 ? 0u : 0xffffu) | (nb >> 31 ? 0u : 0xffff0000u);
             col.nfill = c.miss & ~col.nkeep;
+        }
+        return col;
+    }
+    // ... and on to the next column (whose row-max keys are 1 lower every 2^g
+    // columns)
+    __device__ __forceinline__ void step() {
+        a <<= 2;
+        b <<= 2;
+        t++;
+        if (HASN) {
             na <<= 1;
             nb <<= 1;
         }
+    }
+    __device__ __forceinline__ Col2 next(const Keys2 &c) {
+        const Col2 col = here(c);
+        step();
         return col;
     }
 };
@@ -1866,16 +1875,38 @@ __device__ void process_item2(const GotohJob &job, const GotohConst &K,
     }
 }
 
-// Persistent paired kernel: work item k of the (class range of the) list is
-// positions 2k and 2k + 1; neighbours in the binned list share their
-// geometry key.  Scratch per warp: 2 x tb_words and 2 x rb_words words per
-// lane.
+// Work items of two list entries each, positions b0 + 2k and b0 + 2k + 1 below
+// b1; neighbours in the binned list share their geometry key.
+__device__ __forceinline__ void paired_section(const GotohJob &job, const GotohConst &K,
+                                               const uint32_t *__restrict__ s_lut,
+                                               const int8_t *__restrict__ lut, uint64_t b0,
+                                               uint64_t b1, uint32_t *tb, uint32_t *rb, int lane,
+                                               uint32_t *hf) {
+    const uint64_t total = (b1 - b0 + 1) / 2;
+    for (;;) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd((unsigned long long *)job.queue, 32ull);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= total) break;
+        const uint64_t k = base + lane;
+        uint32_t p[2] = {NO_PAIR, NO_PAIR};
+        if (k < total) {
+            const uint64_t x = b0 + 2 * k, y = x + 1;
+            p[0] = job.list ? job.list[x] : (uint32_t)x;
+            if (y < b1) p[1] = job.list ? job.list[y] : (uint32_t)y;
+        }
+        process_item2(job, K, s_lut, lut, p, tb, rb, hf);
+    }
+}
+
+// Persistent paired kernel over the (class range of the) list.  Scratch per
+// warp: 2 x tb_words and 2 x rb_words words per lane.
 template <int MINB>
 __global__ void __launch_bounds__(PAIR_BLOCK, MINB) gotoh2_kernel(GotohJob job, GotohConst K) {
     __shared__ uint32_t s_lut[10];
     __shared__ int8_t s_lut25[32];
     __shared__ uint32_t s_first[STRIP * PAIR_BLOCK];
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0) {  // static indices keep the parameter block out of local memory
 #pragma unroll
         for (int k = 0; k < 10; k++) s_lut[k] = K.lut4[k >> 1][k & 1];
 #pragma unroll
@@ -1891,21 +1922,480 @@ __global__ void __launch_bounds__(PAIR_BLOCK, MINB) gotoh2_kernel(GotohJob job, 
         b0 = job.range[0];
         b1 = job.range[1] > job.range[0] ? job.range[1] : b0;
     }
-    const uint64_t total = (b1 - b0 + 1) / 2;
+    paired_section(job, K, s_lut, s_lut25, b0, b1, tb, rb, lane, s_first + threadIdx.x);
+}
+
+// ---------------------------------------------------------------------------
+// Group kernel: G lanes (4, 8, 16 or 32) share a work item of one or two
+// pairs.  Lane g of a group fills strips g, g + G, g + 2G, ... one after the
+// other; all lanes step together, a strip one column behind the strip above
+// it, whose bottom row (H, E) arrives by a warp shuffle one step after it
+// was produced.  Strip s (lane g = s mod G, pass p = s / G) meets column j at
+// time j + g + p*R; R is the smallest shift that lets every lane finish a
+// strip before its next one begins.  Where R = G the last lane's bottom row
+// reaches lane 0 by the same shuffle; otherwise it crosses passes through a
+// row buffer of one word pair per column.
+//
+// Why: a thread that owns whole pairs needs the time of its largest pair
+// whatever the batch's size (a 300 x 556 window: 5 ms), and with two pairs a
+// thread the chip holds 155,648 pairs before it is full.  A group of G lanes
+// takes 1/G of that time and holds 1/G of the pairs, so small and middling
+// batches fill the chip; small groups waste fewer steps at a pair's ends,
+// large ones finish it sooner (group_lanes in abi.cu chooses).
+//
+// Cells, keys and packing are the paired kernel's.  A row is computed only
+// inside its window by predicates: `act` has a bit per row whose window holds
+// the column.  A row below one that is outside its window takes the E that an
+// absent cell gives; rows not yet begun or already ended keep their state.
+// Steps in which every lane has all 8 rows inside skip the predicates.
+// Traceback words of a step lie side by side (one 256-byte line a warp), at
+// the step's time; the walks of the group's two pairs run on its first lanes.
+// ---------------------------------------------------------------------------
+
+// The traceback of a group's item: words of (strip, column) at their time.
+struct GroupTb {
+    const uint32_t *tb;  // the warp's region, already at the pair's word of an entry
+    int lg, first, R, t0;  // log2 G, the group's first lane, pass shift, time of step 0
+    __device__ __forceinline__ uint32_t word(const Geo &, int s, int j) const {
+        const int gl = s & ((1 << lg) - 1), t = j + gl + (s >> lg) * R - t0;
+        return tb[((size_t)(uint32_t)t * 32 + (uint32_t)(first + gl)) * 2];
+    }
+};
+
+// One column of a strip, as dp_rows2 over all rows.  MASK: only the rows of
+// `act` are inside their windows.  Selects, not branches: the rows' dependent
+// steps overlap only within one basic block.
+template <bool MASK, bool HASN>
+__device__ __forceinline__ uint2 group_rows(Strip2 &S, const Keys2 &c, const Col2 &col,
+                                            uint32_t act, uint32_t &upHo, uint32_t &upE,
+                                            uint32_t d) {
+    uint32_t wa = 0, wb = 0;
+    uint32_t kd = __viaddmax_u16x2(d, sub2<HASN>(S.la[0], S.lb[0], col), BIAS2 + 0x00030003u);
+#pragma unroll
+    for (int r = 0; r < STRIP; r++) {
+        const uint32_t kF = S.kF[r];
+        uint32_t kE = __viaddmax_u16x2(upE, c.ex, upHo);
+        if (MASK && r > 0) kE = (act & (1u << (r - 1))) ? kE : c.ho0;
+        upE = and_or_u32(kE, KEEP2, 0x00010001u);
+        const uint32_t F4 = and_u32(kF, KEEP2);
+        const uint32_t key = __vimax3_u16x2(kd, upE, F4);
+        if (r < STRIP - 1)
+            kd = __viaddmax_u16x2(S.Hl[r], sub2<HASN>(S.la[r + 1], S.lb[r + 1], col),
+                                  BIAS2 + 0x00030003u);
+        const uint32_t Hp = and_or_u32(key, KEEP2, 0x00020002u);
+        wa = mad_u32(wa, 4u, key - Hp);
+        wb = mad_u32(wb, 4u, xor_and_u32(kE, kF, 0x00030003u));
+        upHo = Hp - c.oe;
+        const uint32_t nF = __viaddmax_u16x2(F4, c.ex, upHo);
+        const uint32_t nr = __vmaxu2(S.rmax[r], mad_u32(Hp, c.ks, col.ck));
+        const bool in = !MASK || (act & (1u << r));
+        S.Hl[r] = in ? Hp : S.Hl[r];
+        S.kF[r] = in ? nF : S.kF[r];
+        S.rmax[r] = in ? nr : S.rmax[r];
+    }
+    wa += 0xAAAAAAAAu;  // tags, not tag - 2
+    return make_uint2(__byte_perm(wa, wb, 0x5410), __byte_perm(wa, wb, 0x7632));
+}
+
+// What a lane knows of its pairs from the strips it has done: the best cell
+// (thr, h, i, j0, j1 as in Best2) and the first touching row << 2 | clamped <<
+// 1 | left (all ones: none) of each pair.  In shared memory (word w of thread
+// t at w * GROUP_BLOCK + t): it is touched once a strip, and the fill needs
+// the registers.
+constexpr int GROUP_BLOCK = 128;
+constexpr int TRACK_WORDS = 11;
+enum : int { TR_THR = 0, TR_H = 1, TR_I = 3, TR_J0 = 5, TR_J1 = 7, TR_TOUCH = 9 };
+
+// A strip's rows are done (extend.rs:795-827), as at the end of a strip in
+// dp_fill2.  first: the keys of the rows' first cells (stride GROUP_BLOCK).
+__device__ __forceinline__ void end_strip2(uint32_t *track, Strip2 &S, const Keys2 &c,
+                                           const uint32_t *first, const Geo &g, int n, int i0,
+                                           int nact, int clo) {
+    const uint32_t ksc = 4u * c.ks;
+    if (nact < STRIP) {  // rows past the read do not count
+#pragma unroll
+        for (int r = 1; r < STRIP; r++)
+            if (r >= nact) S.rmax[r] = 0u;
+    }
+    uint32_t smax = __vimax3_u16x2(S.rmax[0], S.rmax[1], S.rmax[2]);
+    smax = __vimax3_u16x2(smax, S.rmax[3], S.rmax[4]);
+    smax = __vimax3_u16x2(smax, S.rmax[5], __vmaxu2(S.rmax[6], S.rmax[7]));
+    uint32_t thr = track[TR_THR * GROUP_BLOCK];
+    if (__vmaxu2(thr, smax) != thr) {
+        const uint32_t inv_s = 0xffffffffu / ksc + 1u;  // key / S = mulhi(key, inv_s)
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const uint32_t v = (smax >> (16 * q)) & 0xffffu;
+            if (v > ((thr >> (16 * q)) & 0xffffu)) {
+                const uint32_t h = __umulhi(v, inv_s), base = h * ksc;
+                int row = 0;
+                uint32_t key = 0;
+#pragma unroll
+                for (int r = STRIP - 1; r >= 0; r--) {
+                    const uint32_t x = (S.rmax[r] >> (16 * q)) & 0xffffu;
+                    if (x >= base) {
+                        row = i0 + r;
+                        key = x;
+                    }
+                }
+                const int j0 = clo + (int)((base + ksc - 1u - key) << c.g);
+                track[(TR_H + q) * GROUP_BLOCK] = h;
+                track[(TR_I + q) * GROUP_BLOCK] = (uint32_t)row;
+                track[(TR_J0 + q) * GROUP_BLOCK] = (uint32_t)max(j0, g.lo(row));
+                track[(TR_J1 + q) * GROUP_BLOCK] = (uint32_t)min(j0 + (1 << c.g) - 1, g.hi(row));
+                thr = (thr & (0xffff0000u >> (16 * q))) | ((base + ksc - 1u) << (16 * q));
+            }
+        }
+        track[TR_THR * GROUP_BLOCK] = thr;
+    }
+    uint32_t touch[2] = {track[TR_TOUCH * GROUP_BLOCK], track[(TR_TOUCH + 1) * GROUP_BLOCK]};
+    if ((touch[0] == ~0u) | (touch[1] == ~0u)) {
+        uint32_t zero_halves = 0u;  // as in dp_fill2: no zero half, no touch
+#pragma unroll
+        for (int r = 0; r < STRIP; r++) {
+            const uint32_t u = mad_u32(S.Hl[r], c.ks, c.ck0);
+            const uint32_t zl = S.rmax[r] ^ first[r * GROUP_BLOCK], zr = __vmaxu2(S.rmax[r], u) ^ u;
+            zero_halves |= ((zl - 0x00010001u) & ~zl) | ((zr - 0x00010001u) & ~zr);
+        }
+        if (zero_halves & 0x80008000u) {
+#pragma unroll
+            for (int r = 0; r < STRIP; r++) {
+                if (r < nact) {
+                    const int lo = g.lo(i0 + r), hi = g.hi(i0 + r);
+                    const uint32_t u = mad_u32(S.Hl[r], c.ks, c.ck0), f = first[r * GROUP_BLOCK];
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        const uint32_t x = (S.rmax[r] >> (16 * q)) & 0xffffu;
+                        if (touch[q] == ~0u) {
+                            if (x == ((f >> (16 * q)) & 0xffffu))
+                                touch[q] = ((uint32_t)(i0 + r) << 2) | (lo <= 1 ? 3u : 1u);
+                            else if (hi < n && x <= ((u >> (16 * q)) & 0xffffu))
+                                touch[q] = (uint32_t)(i0 + r) << 2;
+                        }
+                    }
+                }
+            }
+            track[TR_TOUCH * GROUP_BLOCK] = touch[0];
+            track[(TR_TOUCH + 1) * GROUP_BLOCK] = touch[1];
+        }
+    }
+}
+
+// Pass shift of an item: lanes g of the group take the strips in turn.
+__device__ __forceinline__ int group_shift(const Geo &g, int m, int nstrips, int lg, int gl) {
+    const int G = 1 << lg;
+    int r = 0;
+    for (int s = gl; s + G < nstrips; s += G)  // chi(s) - clo(s + G) + 1
+        r = max(r, g.hi(min((s + 1) * STRIP, m)) - g.lo((s + G) * STRIP + 1) + 1);
+    for (int x = 1; x < G; x <<= 1) r = max(r, __shfl_xor_sync(0xffffffffu, r, x));
+    // a buffered pass runs two columns behind its writes (read ahead)
+    return r <= G ? G : max(r, G + 4);
+}
+
+// *p = v (shared memory) when x is not 0, as one predicated store: a branch a
+// row cost as much as the row.
+__device__ __forceinline__ void put_if(uint32_t *p, uint32_t v, uint32_t x) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.shared.u32 [%0], %1;\n\t}" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(p)),
+                 "r"(v), "r"(x)
+                 : "memory");
+}
+
+// Fill the DP of every group's item (two pairs of one geometry, or one pair
+// in both halves; nstrips = 0: none).  tb: the warp's traceback region, a
+// word pair per step and lane; rb: the group's row buffer, a word pair per
+// column 1..n; first, track: the thread's words in shared memory.
+// Every lane of a group returns its item's results.
+template <bool HASN>
+__device__ __noinline__ void group_fill(const GotohConst &K, const uint32_t *__restrict__ s_lut,
+                                        const PairSetup &A, const PairSetup &B, int nstrips, int R,
+                                        int steps, uint2 *tb, uint2 *rb, int lane,
+                                        int lg, uint32_t *first, uint32_t *track, FillResult &FA,
+                                        FillResult &FB) {
+    constexpr uint32_t ALL = 0xffffffffu;
+    const int G = 1 << lg, gl = lane & (G - 1);
+    const int src = (lane & ~(G - 1)) + ((gl - 1) & (G - 1));
+    const int m = A.m, n = A.n;
+    const Geo g = A.g;
+    const Keys2 c = keys2_of(K, m, A.sw);
+    const bool ring = R == G;
+    const int nh = n - g.half, h1 = g.half + 1;  // c(i) clamped at n / at 1 (Geo)
+    track[TR_THR * GROUP_BLOCK] = (4u * c.ks - 1u) * 0x10001u;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        track[(TR_H + q) * GROUP_BLOCK] = track[(TR_I + q) * GROUP_BLOCK] = 0u;
+        track[(TR_J0 + q) * GROUP_BLOCK] = track[(TR_J1 + q) * GROUP_BLOCK] = 0u;
+        track[(TR_TOUCH + q) * GROUP_BLOCK] = ~0u;
+    }
+    Strip2 S;
+    uint32_t pubH = c.h0, pubE = c.e0, raw = c.h0, diag = c.h0;
+    uint2 u0 = make_uint2(c.h0, c.e0), u1 = u0;
+    Codes2<HASN> w{A.win, B.win};
+    int s = gl - G, j = 0, clo = 1 << 30, chi = -1, phi = -1;
+    int r0 = 0;        // off + i0: row r's window begins at j = r0 + r - half
+    uint32_t was = 0;  // rows inside their windows one column before
+    bool turn = nstrips > 0;  // the lane goes on to its next strip
+    bool open = false;        // the lane has a strip, waiting, running or just ended
+    for (int t = 0;; t++) {
+        if (turn) {
+            if (open) {
+                const int i0 = s * STRIP + 1;
+                end_strip2(track, S, c, first, g, n, i0, min(STRIP, m - i0 + 1), clo);
+            }
+            open = false;
+            turn = false;
+            s += G;
+            if (s < nstrips) {
+                const int i0 = s * STRIP + 1;
+                clo = g.lo(i0);
+                chi = g.hi(min(i0 + STRIP - 1, m));
+                phi = s ? g.hi(i0 - 1) : -1;
+                r0 = g.off + i0;
+                j = t + g.lo(1) - gl - (s >> lg) * R;
+                w.load(clo);
+                w.t = 0;
+                const uint32_t rwA = load16(A.read.arena, A.read.pos + (uint64_t)(i0 - 1));
+                const uint32_t rwB = load16(A.read.arena, B.read.pos + (uint64_t)(i0 - 1));
+                const uint32_t rnA = A.read.cnt ? nmask16(A.read.iv, A.read.cnt, i0 - 1) : 0u;
+                const uint32_t rnB = B.read.cnt ? nmask16(B.read.iv, B.read.cnt, i0 - 1) : 0u;
+#pragma unroll
+                for (int r = 0; r < STRIP; r++) {
+                    uint32_t ca = (rwA >> (30 - 2 * r)) & 3u, cb = (rwB >> (30 - 2 * r)) & 3u;
+                    if ((rnA >> (31 - r)) & 1u) ca = 4;
+                    if ((rnB >> (31 - r)) & 1u) cb = 4;
+                    S.la[r] = s_lut[2 * ca];
+                    S.lb[r] = s_lut[2 * cb];
+                    S.Hl[r] = c.h0;
+                    S.kF[r] = c.ho0;
+                    S.rmax[r] = 0u;
+                }
+                was = 0;
+                open = true;
+            } else {
+                clo = 1 << 30;
+                chi = -1;
+            }
+        }
+        if (t >= steps) break;
+        const bool active = j >= clo && j <= chi;
+        // the bottom row of the strip above at this column
+        uint32_t upH = __shfl_sync(ALL, pubH, src), upE = __shfl_sync(ALL, pubE, src);
+        if (!ring && gl == 0 && active && s) {
+            if (j == clo) {
+                if (clo > 1) raw = rb[clo - 1].x;
+                u0 = rb[clo];
+                if (clo + 1 <= phi) u1 = rb[clo + 1];
+            }
+            upH = u0.x;
+            upE = u0.y;
+            u0 = u1;
+            if (j + 2 <= phi) u1 = rb[j + 2];
+        }
+        if (j == clo)  // the row above's last column left of this strip's
+            diag = s && clo - 1 >= g.lo(s * STRIP) && clo - 1 <= phi ? raw : c.h0;
+        raw = upH;
+        upH = j > phi ? c.h0 : upH;
+        upE = j > phi ? c.e0 : upE;
+        // rows inside their windows: lo(r) <= j <= hi(r) (Geo), a run of rows
+        const int x = j - r0;
+        const int rb_ = j >= nh ? STRIP - 1 : min(STRIP - 1, x + g.half);
+        const int ra = j <= h1 ? 0 : max(0, x - g.half);
+        const uint32_t act = active ? ((2u << rb_) - (1u << ra)) & 0xffu : 0u;
+        const uint32_t begin = act & ~was;
+        was = act;
+        uint32_t upHo = upH - c.oe;
+        const Col2 col = w.here(c);
+        uint2 words;
+        // a lane without a strip may compute what it likes
+        if (__all_sync(ALL, !open || act == 0xffu))
+            words = group_rows<false, HASN>(S, c, col, act, upHo, upE, diag);
+        else
+            words = group_rows<true, HASN>(S, c, col, act, upHo, upE, diag);
+#pragma unroll
+        for (int r = 0; r < STRIP; r++)  // rows that met their first column
+            put_if(first + r * GROUP_BLOCK, S.rmax[r], begin & (1u << r));
+        pubH = upHo + c.oe;
+        pubE = upE;
+        diag = upH;
+        if (active) {
+            __stcs(tb + (size_t)t * 32 + lane, words);
+            if (!ring && gl == G - 1) rb[j] = make_uint2(pubH, pubE);
+            turn = j == chi && s + G < nstrips;
+            w.step();
+        }
+        j++;
+        // new codes for all lanes at once, 16 columns after the last ones or
+        // sooner
+        if ((t & 15) == 15 && j > clo && j <= chi) w.load(j);
+        __syncwarp();
+    }
+    // the lanes' last strips, all at once
+    if (open) {
+        const int i0 = s * STRIP + 1;
+        end_strip2(track, S, c, first, g, n, i0, min(STRIP, m - i0 + 1), clo);
+    }
+    // merge the lanes: the largest H, its first row; the first touching row
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        uint32_t key = (track[(TR_H + q) * GROUP_BLOCK] << 16) |
+                       (0xffffu - track[(TR_I + q) * GROUP_BLOCK]);
+        uint32_t j0 = track[(TR_J0 + q) * GROUP_BLOCK], j1 = track[(TR_J1 + q) * GROUP_BLOCK];
+        uint32_t touch = track[(TR_TOUCH + q) * GROUP_BLOCK];
+        for (int x = 1; x < G; x <<= 1) {
+            const uint32_t ok = __shfl_xor_sync(ALL, key, x), ot = __shfl_xor_sync(ALL, touch, x);
+            const uint32_t o0 = __shfl_xor_sync(ALL, j0, x), o1 = __shfl_xor_sync(ALL, j1, x);
+            touch = min(touch, ot);
+            if (ok > key) {
+                key = ok;
+                j0 = o0;
+                j1 = o1;
+            }
+        }
+        FillResult &F = q ? FB : FA;
+        F.bestHp = 4 * (int)(key >> 16) + 2;
+        F.best_i = key >> 16 ? (int)(0xffffu - (key & 0xffffu)) : 0;
+        F.best_j = (int)j0;
+        F.last_j = (int)j1;
+        F.trow = touch == ~0u ? 0 : (int)(touch >> 2);
+        F.tleft = touch != ~0u && (touch & 1u);
+        F.tclamp = touch != ~0u && (touch & 2u);
+    }
+}
+
+// Upper bound of the steps of an item of at most m rows, n columns and sw
+// columns a strip.
+uint64_t group_steps(uint64_t m, uint64_t n, uint64_t sw, int lg) {
+    const uint64_t G = 1ull << lg, strips = (m + STRIP - 1) / STRIP, passes = (strips + G - 1) / G;
+    return n + G + (passes ? passes - 1 : 0) * std::max<uint64_t>(sw, G + 4);
+}
+
+// A pair's set-up; the group section checks its own scratch.
+__device__ __noinline__ bool setup_group(const GotohJob &job, const GotohConst &K, uint32_t pi,
+                                         bool write, PairSetup &S) {
+    return setup_pair(job, K, pi, ~0ull, ~0ull, write, S);
+}
+
+// Items 0 .. items - 1 of the (padded, binned) list in groups of 1 << lg
+// lanes; item k is positions 2k and 2k + 1.  A warp takes 32 >> lg items at a
+// time.  Scratch: the warp's traceback region (group_tb_words word pairs per
+// lane) and row buffers (group_rb_words word pairs per group).
+__device__ void group_section(const GotohJob &job, const GotohConst &K,
+                              const uint32_t *__restrict__ s_lut, const int8_t *__restrict__ lut,
+                              uint64_t items, int lg, uint2 *tb, uint2 *rb0, int lane,
+                              uint32_t *first, uint32_t *track) {
+    const int G = 1 << lg, groups = 32 >> lg, gl = lane & (G - 1), grp = lane >> lg;
+    uint2 *rb = rb0 + (uint64_t)grp * job.group_rb_words;
+    const uint64_t total = items;
     for (;;) {
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd((unsigned long long *)job.queue, 32ull);
+        if (lane == 0)
+            base = atomicAdd((unsigned long long *)job.group_queue, (unsigned long long)groups);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= total) break;
-        uint64_t k = base + lane;
+        const uint64_t k = base + grp;
         uint32_t p[2] = {NO_PAIR, NO_PAIR};
         if (k < total) {
-            const uint64_t x = b0 + 2 * k, y = x + 1;
-            p[0] = job.list ? job.list[x] : (uint32_t)x;
-            if (y < b1) p[1] = job.list ? job.list[y] : (uint32_t)y;
+            p[0] = job.list[2 * k];
+            p[1] = job.list[2 * k + 1];
         }
-        process_item2(job, K, s_lut, s_lut25, p, tb, rb, s_first + threadIdx.x);
+        // both pairs at once when their geometry matches, else one by one
+        int need = 0;  // bit q: pair q has a DP; bit 2: together
+        {
+            PairSetup A, B;
+            const bool a = p[0] != NO_PAIR && setup_group(job, K, p[0], gl == 0, A);
+            const bool b = p[1] != NO_PAIR && setup_group(job, K, p[1], gl == 0, B);
+            need = (a ? 1 : 0) | (b ? 2 : 0);
+            if (a && b && A.m == B.m && A.n == B.n && A.g.off == B.g.off && A.g.half == B.g.half)
+                need = 4;
+        }
+        for (int round = 0; round < 2; round++) {
+            // this round's first pair: the only one, or both
+            const bool on = round == 0 ? need != 0 : need == 3;
+            if (!__any_sync(0xffffffffu, on)) break;
+            const int q = round == 0 ? (need == 2 ? 1 : 0) : 1;
+            PairSetup A, B;
+            int nstrips = 0, R = G, steps = -1;
+            A.m = A.n = A.sw = 1;
+            A.g = Geo{0, 1, 1};
+            A.win.cnt = 0;
+            if (on) {
+                setup_group(job, K, p[q], false, A);
+                nstrips = (A.m + STRIP - 1) / STRIP;
+            }
+            R = group_shift(A.g, A.m, nstrips, lg, gl);
+            bool fits = on;
+            if (on) {
+                const int l = nstrips - 1;
+                steps = A.g.hi(A.m) + (l & (G - 1)) + (l >> lg) * R - A.g.lo(1) + 1;
+                if ((uint64_t)steps > job.group_tb_words || (uint64_t)A.n >= job.group_rb_words) {
+                    // scratch sized too small by the host: refuse, never overrun
+                    fits = false;
+                    nstrips = 0;
+                    steps = -1;
+                    for (int x = 0; x < 2; x++)
+                        if (gl == 0 && (need == 4 || x == q)) {
+                            if (setup_group(job, K, p[x], false, B)) {
+                                B.o.status = ESP_EINVAL;
+                                job.out[p[x]] = B.o;
+                            }
+                        }
+                }
+            }
+            B = A;
+            if (need == 4 && fits) setup_group(job, K, p[1], false, B);
+            const int all_steps = __reduce_max_sync(0xffffffffu, steps);
+            FillResult FA, FB;
+            if (__any_sync(0xffffffffu, nstrips > 0 && (A.win.cnt != 0 || B.win.cnt != 0)))
+                group_fill<true>(K, s_lut, A, B, nstrips, R, all_steps, tb, rb, lane, lg, first, track, FA,
+                                  FB);
+            else
+                group_fill<false>(K, s_lut, A, B, nstrips, R, all_steps, tb, rb, lane, lg, first, track, FA,
+                                  FB);
+            __syncwarp();  // traceback words of every lane are visible to the walks
+            if (fits && gl < (need == 4 ? 2 : 1)) {
+                const int gfirst = lane & ~(G - 1);
+                PairSetup &S = gl ? B : A;
+                const GroupTb view{reinterpret_cast<const uint32_t *>(tb) + gl, lg, gfirst, R, A.g.lo(1)};
+                finish_pair(job, K, lut, p[gl ? 1 : q], S, gl ? FB : FA, view);
+            }
+            __syncwarp();
+        }
     }
+}
+
+// Small and middling batches of the binned list: its costly front in groups
+// (job.group_plan: list entries, log2 of a group's lanes), the rest two pairs
+// per thread.  A thread's pair takes as long as it takes, so the items that
+// would outlast the rest of the batch are the ones given to groups, and the
+// others keep the paired kernel's higher throughput (bin_plan, bins.cu).
+__global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob job, GotohConst K) {
+    static_assert(GROUP_BLOCK == PAIR_BLOCK, "one shared array serves both sections");
+    __shared__ uint32_t s_lut[10];
+    __shared__ int8_t s_lut25[32];
+    __shared__ uint32_t s_words[(STRIP + TRACK_WORDS) * GROUP_BLOCK];
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < 10; k++) s_lut[k] = K.lut4[k >> 1][k & 1];
+#pragma unroll
+        for (int k = 0; k < 25; k++) s_lut25[k] = K.lut[k];
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const uint64_t warp_slot = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint32_t *tb = job.tb + warp_slot * job.warp_tb_words;
+    uint32_t *rb = job.rb + warp_slot * job.warp_rb_words;
+    const uint64_t split = job.group_plan[0];
+    group_section(job, K, s_lut, s_lut25, split / 2, (int)job.group_plan[1],
+                  reinterpret_cast<uint2 *>(tb), reinterpret_cast<uint2 *>(rb), lane,
+                  s_words + threadIdx.x, s_words + STRIP * GROUP_BLOCK + threadIdx.x);
+    paired_section(job, K, s_lut, s_lut25, split, *job.list_count, tb + 2 * lane, rb + 2 * lane, lane,
+                   s_words + threadIdx.x);
+}
+
+cudaError_t launch_gotoh_mixed(const GotohJob &job, const GotohConst &k, int warps,
+                               cudaStream_t st) {
+    gotoh_mixed_kernel<<<(warps + 3) / 4, GROUP_BLOCK, 0, st>>>(job, k);
+    return cudaGetLastError();
 }
 
 int make_gotoh_const(const esp_extend_params &p, GotohConst &k) {
@@ -1983,6 +2473,13 @@ int gotoh_blocks_per_sm(int block, int variant) {
     default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, gotoh_kernel<4>, block, 0);
     }
     if (e != cudaSuccess) return 1;
+    return nb > 0 ? nb : 1;
+}
+
+int gotoh_mixed_blocks_per_sm() {
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, gotoh_mixed_kernel, GROUP_BLOCK, 0) != cudaSuccess)
+        return 1;
     return nb > 0 ? nb : 1;
 }
 

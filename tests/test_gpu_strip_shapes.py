@@ -6,10 +6,11 @@ column, and of blocks of columns (long reads on the paired kernel); best
 columns that tie inside such a block; traceback walks whose matches run off
 the left edge of a clamped band; gap costs of 0.  Pairs with a partner of
 their geometry, without one, and with N in the window share every batch, so
-that the paired kernel's three ways of filling a pair run side by side.
+that the paired kernel's ways of filling a pair run side by side.
 Every record, touch and CIGAR equals the oracle's."""
 import random
 
+import numpy as np
 import pytest
 
 import oracle as O
@@ -60,33 +61,44 @@ def _batch(rng, shapes):
     return cases
 
 
-def _check(cases, params, variant):
+def _check(cases, params, variant, copies=1, mode=B.MODE_BAND):
+    """variant None: what the batch's size selects; copies: the batch holds the
+    cases so often."""
     buf = ExtendBuffer()
     buf.set_warp_max(0)
-    buf.set_kernel_variant(variant)
+    if variant is not None:
+        buf.set_kernel_variant(variant)
     arena, pairs, iv = B.pack_ascii_pairs([c[0] for c in cases], [c[1] for c in cases],
                                           [c[2][0] if c[2] else 0 for c in cases],
                                           [c[2][1] if c[2] else -1 for c in cases])
     stride = max(2 * (len(c[0]) + len(c[1])) + 8 for c in cases)
-    out, cig = B.extend_batch_host(pairs, arena, iv, params, B.MODE_BAND, stride, buf=buf)
+    n = len(cases)
+    out, cig = B.extend_batch_host(np.tile(pairs, copies), arena, iv, params, mode, stride, buf=buf)
     op = O.Params(params.match_score, params.mismatch, params.gap_open, params.gap_ext,
                   edit_dir=int(params.edit_dir))
     for k, (read, win, band) in enumerate(cases):
-        e, t = O.run_dispatch(read, win, op, band=band)
+        if mode == B.MODE_HINT:
+            e, t = O.extend_hint(read, win, op, offset=band[0] if band else 0), None
+        else:
+            e, t = O.run_dispatch(read, win, op, band=band)
         o = out[k]
         got = (int(o["score"]), int(o["read_start"]), int(o["read_end"]), int(o["ref_start"]),
                tuple(B.cigar_of(cig[k], int(o["n_ops"]))))
         touch = O.Touch(bool(o["touched"]), int(o["touch_row"]), bool(o["touch_left"]),
                         bool(o["touch_clamped"]))
-        assert int(o["status"]) == 0 and got == e.key() and touch == t, (len(read), len(win), band)
+        assert int(o["status"]) == 0 and got == e.key(), (len(read), len(win), band)
+        assert t is None or touch == t, (len(read), len(win), band)
+        ops = int(o["n_ops"])
+        for c in range(1, copies):
+            assert out[k + c * n] == o and (cig[k + c * n][:ops] == cig[k][:ops]).all(), (k, c)
 
 
-@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+@pytest.mark.parametrize("variant", [0, 1, 2, 3, None])
 @pytest.mark.parametrize("rows", [(1, 7, 8, 9), (15, 16, 17), (63, 64, 65)])
 def test_strip_shapes(rows, variant):
-    rng = random.Random(rows[0] * 10 + variant)
+    rng = random.Random(rows[0] * 10 + (variant or 0))
     shapes = [(m, m + 2 * f, b) for m in rows for f in (1, 8, 16) for b in _bands(m, m + 2 * f)]
-    _check(_batch(rng, shapes), ExtendParams(edit_dir=variant % 3), variant)
+    _check(_batch(rng, shapes), ExtendParams(edit_dir=(variant or 1) % 3), variant)
 
 
 @pytest.mark.parametrize("params", [ExtendParams(2, -4, 0, 0), ExtendParams(1, 1, 2, 1),
@@ -95,7 +107,7 @@ def test_strip_shapes(rows, variant):
 def test_score_ranges(params):
     rng = random.Random(7)
     shapes = [(m, m + 24, b) for m in (9, 24, 40) for b in _bands(m, m + 24)]
-    for variant in (1, 3):
+    for variant in (1, 3, None):
         _check(_batch(rng, shapes), params, variant)
 
 
@@ -111,4 +123,16 @@ def test_row_maximum_blocks(m, band):
         win = _seq(rng, m + 2 * flank, letters)
         for _ in range(3):
             cases.append((_read_of(rng, win, flank, m), win, band))
-    _check(cases, ExtendParams(), 3)
+    for variant in (3, None):
+        _check(cases * 6, ExtendParams(), variant)
+
+
+@pytest.mark.parametrize("mode", [B.MODE_BAND, B.MODE_HINT])
+@pytest.mark.parametrize("copies", [12, 50, 130, 330, 800, 2200])
+def test_groups_by_batch_size(copies, mode):
+    """The mixed kernel's groups of 32, 16, 8 and 4 lanes, a batch whose costly
+    pairs alone go to groups, and one that the paired kernel takes."""
+    rng = random.Random(copies)
+    shapes = [(m, m + 2 * f, b) for m in (9, 41) for f in (4, 10) for b in _bands(m, m + 2 * f)]
+    shapes = rng.sample(shapes, 40) + [(150, 182, (16, 16)), (96, 352, (128, 128)), (70, 130, None)]
+    _check(_batch(rng, shapes), ExtendParams(), None, copies, mode)
