@@ -1826,9 +1826,12 @@ __device__ __noinline__ bool setup_call(const GotohJob &job, const GotohConst &K
 // fill when their geometry matches; a pair without a partner of its geometry
 // fills both halves, in the same pass over the lanes (lanes that took turns
 // doubled a warp's time), and a second pass takes the other pair of a
-// mismatched item.  N in a window costs one more instruction a row, so a warp
-// that holds one runs that fill for all its lanes.  The descriptors are
-// resolved again for the finish rather than kept live across the fill.
+// mismatched item.  N in a window costs one more instruction a row; a batch
+// that has N runs at all runs that fill for all its pairs, as the two fills do
+// not fit the instruction cache together (1,000,003 mixed pairs, N in 0.5 % of
+// the windows: 12.3 ms with the fill chosen per warp, 10.1 so).  The
+// descriptors are resolved again for the finish rather than kept live across
+// the fill.
 constexpr uint32_t NO_PAIR = 0xffffffffu;
 
 __device__ void process_item2(const GotohJob &job, const GotohConst &K,
@@ -1858,9 +1861,8 @@ __device__ void process_item2(const GotohJob &job, const GotohConst &K,
                     B = A;
                 }
             }
-            const bool n = __any_sync(0xffffffffu, now && (A.win.cnt || B.win.cnt));
             if (now) {
-                if (n) fill2_call<true>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
+                if (job.n_iv_count) fill2_call<true>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
                 else fill2_call<false>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
             }
         }
@@ -2345,7 +2347,7 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
             if (need == 4 && fits) setup_group(job, K, p[1], false, B);
             const int all_steps = __reduce_max_sync(0xffffffffu, steps);
             FillResult FA, FB;
-            if (__any_sync(0xffffffffu, nstrips > 0 && (A.win.cnt != 0 || B.win.cnt != 0)))
+            if (job.n_iv_count)  // as in process_item2
                 group_fill<true>(K, s_lut, A, B, nstrips, R, all_steps, tb, rb, lane, lg, first, track, FA,
                                   FB);
             else
