@@ -1025,28 +1025,275 @@ __global__ void __launch_bounds__(128, MINB) gotoh_kernel(GotohJob job, GotohCon
 
 // ---------------------------------------------------------------------------
 // Warp-per-pair DP (the per-call drop-in and small batches).  One pair's
-// strips are spread over the lanes of a warp (lane s owns rows 8s+1..8s+8 of
-// the current 32-strip pass) and swept as a wavefront: at step t lane s
-// evaluates column j = t - s, receiving the bottom row (H, E) of lane s-1 at
-// the same column by a warp shuffle (lane s-1 produced it one step earlier)
-// and keeping the previous step's value as its diagonal.  Idle or
-// out-of-window lanes publish H = 0, E = NEG -- what the thread-per-pair
-// kernel's row buffer presents outside the previous strip's window -- so
-// every cell, traceback word, row maximum and touch is the same as there.
-// A pass of 32 strips hands its last row to the next pass through the row
-// buffer.  Lane 0 then walks the traceback.  Scratch is the warp's own
-// (word stride 1).
+// strips are taken in turn by the lanes of a warp (lane g has strips g, g + 32,
+// ...) and swept as a wavefront, two columns a step: at step t lane g, in pass
+// p, evaluates columns j and j + 1, j = base + 2 * (t - g - p * R), receiving the
+// strip above's bottom row (H, E packed as int16 halves) at both by warp
+// shuffles, one step after lane g - 1 produced it.  R, the steps from a lane's
+// strip to its next one, is 32 where every lane is done with a strip by then
+// (a band: lane 31's row reaches lane 0 by the same shuffle); else it is larger
+// and the row crosses passes through a row buffer.  Lane 0 then walks the
+// traceback.
+//
+// A lone warp is bound by latency: a row's five dependent steps (22 cycles)
+// times the rows and columns on the wavefront's path.  Two columns a step let
+// their rows overlap (column j + 1 follows one row behind column j), windows
+// are applied by selects (a branch a row ends the overlap), and a third pass of
+// strips no longer waits for the second.  Measured against one column a step,
+// a pass at a time: one extend_hint call of 150 x 214 111 -> 104 us, with its
+// second attempt 197 -> 172; 1,000 mixed pairs in bands 0.38 -> 0.295 ms, 2,000
+// 0.54 ms.  Strips of 2 or 4 rows (more lanes at work in a band) were slower:
+// 122 and 257 us, since a step's shuffles, windows and vote cost as before.
 // ---------------------------------------------------------------------------
 
-// WIDE = false: H and E of a row cross lanes and passes packed as int16
-// halves of one word (the int16 domain); WIDE = true: as two int32 words
-// (the row buffer then holds 2 words per column).
-template <bool WIDE>
+// One column of a strip for the int16 domain's warp kernel; `act` has a bit
+// per row whose window holds the column (MASK), as in dp_column otherwise.
+template <bool MASK>
+__device__ __forceinline__ uint32_t warp_column(Strip &S, const GotohConst &K, uint32_t sel,
+                                                int cj, uint32_t act, int upHo, int upE, int diag,
+                                                uint32_t &bottom) {
+    uint32_t wa = 0, wb = 0;
+    int kd = __viaddmax_s32(diag, prmt_sx(S.l0[0], S.l1[0], sel), 3);
+    int Hp = 2;
+#pragma unroll
+    for (int r = 0; r < STRIP; r++) {
+        int kE = __viaddmax_s32(upE, K.ex4, upHo);
+        if (MASK && r > 0) kE = (act & (1u << (r - 1))) ? kE : K.oe4 + 2;
+        const int kF = S.kF[r];
+        upE = (int)and_or_u32((uint32_t)kE, ~3u, 1u);
+        const int F4 = (int)and_u32((uint32_t)kF, ~3u);
+        const int key = __vimax3_s32(kd, upE, F4);
+        if (r < STRIP - 1)
+            kd = __viaddmax_s32(S.Hl[r], prmt_sx(S.l0[r + 1], S.l1[r + 1], sel), 3);
+        Hp = (int)and_or_u32((uint32_t)key, ~3u, 2u);
+        wa = mad_u32(wa, 4u, (uint32_t)(key - Hp));
+        wb = mad_u32(wb, 4u, xor_and_u32((uint32_t)kE, (uint32_t)kF, 3u));
+        upHo = Hp + K.oe4;
+        const int nF = __viaddmax_s32(F4, K.ex4, upHo);
+        const int nr = max(S.rk[r], (int)mad_u32((uint32_t)Hp, 32768u, (uint32_t)cj));
+        const bool in = !MASK || (act & (1u << r));
+        S.Hl[r] = in ? Hp : S.Hl[r];
+        S.kF[r] = in ? nF : S.kF[r];
+        S.rk[r] = in ? nr : S.rk[r];
+    }
+    bottom = __byte_perm((uint32_t)Hp, (uint32_t)upE, 0x5410);
+    return __byte_perm(wa + 0xAAAAu, wb, 0x5410);
+}
+
+// R of a pair, and its number of steps.
+__device__ __forceinline__ int warp_shift(const Geo &g, int m, int nstrips, int lane, int &steps) {
+    const int base = g.lo(1);
+    int r = 0;
+    for (int s = lane; s + 32 < nstrips; s += 32)
+        r = max(r, ((g.hi(min((s + 1) * STRIP, m)) - base) >> 1) -
+                       ((g.lo((s + 32) * STRIP + 1) - base) >> 1) + 1);
+    r = __reduce_max_sync(0xffffffffu, r);
+    const int R = r <= 32 ? 32 : max(r, 36);  // a buffered pass runs behind its writes
+    const int l = nstrips - 1;
+    steps = ((g.hi(m) - base) >> 1) + (l & 31) + (l >> 5) * R + 1;
+    return R;
+}
+
 __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict__ s_lut,
+                                const PairSetup &P, uint32_t *tb, uint32_t *rb, int lane) {
+    constexpr uint32_t ALL = 0xffffffffu;
+    const int m = P.m, n = P.n;
+    const Geo g = P.g;
+    const uint32_t ABSENT = absent_HE(K);
+    const int base = g.lo(1), nstrips = (m + STRIP - 1) / STRIP;
+    int steps;
+    const int R = warp_shift(g, m, nstrips, lane, steps);
+    const bool ring = R == 32;
+    int bHp = 2, bi = 0, bj = 0, trow = 0;  // of this lane's strips
+    bool tleft = false, tclamp = false;
+    Strip S;
+    int s = lane - 32, j = 0, clo = 1 << 30, chi = -1, plo = 0, phi = -1, lo7 = 0;
+    uint32_t pub0 = ABSENT, pub1 = ABSENT, last = ABSENT;
+    uint2 u0 = make_uint2(ABSENT, ABSENT), u1 = u0;
+    uint32_t cw = 0, cn = 0;
+    bool turn = true, open = false;
+    auto codes = [&](int c) {
+        cw = load16(P.win.arena, P.win.pos + (uint64_t)(c - 1));
+        cn = P.win.cnt ? nmask16(P.win.iv, P.win.cnt, c - 1) : 0u;
+    };
+    // bottom row of the pass before, from the row buffer
+    auto above = [&](int c) { return c >= plo && c <= phi ? rb[c - plo] : ABSENT; };
+    for (int t = 0;; t++) {
+        if (turn) {
+            if (open) {  // row bookkeeping in row order (extend.rs:795-827)
+                const int i0 = s * STRIP + 1;
+#pragma unroll
+                for (int r = 0; r < STRIP; r++) {
+                    const int i = i0 + r;
+                    if (i <= m) {
+                        const int rowHp = S.rk[r] >> 15, argj = 32767 - (S.rk[r] & 32767);
+                        if (trow == 0) {
+                            if (argj == g.lo(i)) {
+                                trow = i;
+                                tleft = true;
+                                tclamp = argj <= 1;
+                            } else if (g.hi(i) < n && S.Hl[r] == rowHp) {
+                                trow = i;
+                            }
+                        }
+                        if (rowHp > bHp) {
+                            bHp = rowHp;
+                            bi = i;
+                            bj = argj;
+                        }
+                    }
+                }
+            }
+            turn = false;
+            s += 32;
+            open = s < nstrips;
+            clo = 1 << 30;
+            chi = -1;
+            if (open) {
+                const int i0 = s * STRIP + 1;
+                clo = g.lo(i0);
+                chi = g.hi(min(i0 + STRIP - 1, m));
+                plo = s ? g.lo(i0 - 1) : 0;
+                phi = s ? g.hi(i0 - 1) : -1;
+                lo7 = g.lo(i0 + STRIP - 1);
+                j = base + 2 * (t - lane - (s >> 5) * R);
+                const uint32_t rw = load16(P.read.arena, P.read.pos + (uint64_t)(i0 - 1));
+                const uint32_t rn = P.read.cnt ? nmask16(P.read.iv, P.read.cnt, i0 - 1) : 0u;
+#pragma unroll
+                for (int r = 0; r < STRIP; r++) {
+                    uint32_t c = (rw >> (30 - 2 * r)) & 3u;
+                    if ((rn >> (31 - r)) & 1u) c = 4;
+                    S.l0[r] = s_lut[2 * c];
+                    S.l1[r] = s_lut[2 * c + 1];
+                    S.Hl[r] = 2;
+                    S.kF[r] = 2 + K.oe4;  // F opened from H = 0
+                    S.rk[r] = -1;
+                }
+                codes(base + (clo - base & ~1));
+            }
+        }
+        if (t >= steps) break;
+        const bool active = j + 1 >= clo && j <= chi;
+        uint32_t w0 = __shfl_sync(ALL, pub0, (lane - 1) & 31);
+        uint32_t w1 = __shfl_sync(ALL, pub1, (lane - 1) & 31);
+        if (!ring && lane == 0 && s >= 32 && active) {
+            if (j <= clo) {  // the strip's first step
+                last = above(j - 1);
+                u0 = make_uint2(above(j), above(j + 1));
+                u1 = make_uint2(above(j + 2), above(j + 3));
+            }
+            w0 = u0.x;
+            w1 = u0.y;
+            u0 = u1;
+            u1 = make_uint2(above(j + 4), above(j + 5));
+        }
+        // the row above: its cell at j - 1, j (diagonals) and j, j + 1
+        const uint32_t d0 = j - 1 >= plo && j - 1 <= phi ? last : ABSENT;
+        const uint32_t d1 = j >= plo && j <= phi ? w0 : ABSENT;
+        const uint32_t a0 = j <= phi ? w0 : ABSENT, a1 = j + 1 <= phi ? w1 : ABSENT;
+        last = w1;
+        // rows inside their windows: lo(r) <= j <= hi(r) (Geo), a run of rows
+        auto rows_at = [&](int c) {
+            const int x = c - g.off - s * STRIP - 1;
+            const int rl = c >= n - g.half ? STRIP - 1 : min(STRIP - 1, x + g.half);
+            const int rf = c <= g.half + 1 ? 0 : max(0, x - g.half);
+            return c >= clo && c <= chi ? ((2u << rl) - (1u << rf)) & 0xffu : 0u;
+        };
+        const uint32_t act0 = rows_at(j), act1 = rows_at(j + 1);
+        const uint32_t code0 = (cw >> 30) | ((cn >> 29) & 4u);
+        const uint32_t code1 = ((cw >> 28) & 3u) | ((cn >> 28) & 4u);
+        const uint32_t sel0 = code0 * 0x1111u + 0x8880u, sel1 = code1 * 0x1111u + 0x8880u;
+        const int h0 = (int)(a0 & 0xffffu) + K.oe4, e0 = (int)a0 >> 16;
+        const int h1 = (int)(a1 & 0xffffu) + K.oe4, e1 = (int)a1 >> 16;
+        uint32_t word0, word1;
+        // a lane without a strip may compute what it likes
+        if (__all_sync(ALL, !open || (act0 & act1) == 0xffu)) {
+            word0 = warp_column<false>(S, K, sel0, 32767 - j, 0xffu, h0, e0, (int)(d0 & 0xffffu),
+                                         pub0);
+            word1 = warp_column<false>(S, K, sel1, 32766 - j, 0xffu, h1, e1, (int)(d1 & 0xffffu),
+                                         pub1);
+        } else {
+            word0 = warp_column<true>(S, K, sel0, 32767 - j, act0, h0, e0, (int)(d0 & 0xffffu),
+                                        pub0);
+            word1 = warp_column<true>(S, K, sel1, 32766 - j, act1, h1, e1, (int)(d1 & 0xffffu),
+                                        pub1);
+        }
+        if (active) {
+            uint32_t *w = tb + (size_t)s * P.sw;
+            if (act0) w[j - clo] = word0;
+            if (act1) w[j + 1 - clo] = word1;
+            if (!ring && lane == 31 && s + 1 < nstrips) {  // a full strip: its last row
+                if (act0 & 0x80u) rb[j - lo7] = pub0;
+                if (act1 & 0x80u) rb[j + 1 - lo7] = pub1;
+            }
+            turn = j + 1 >= chi;
+            cw <<= 4;
+            cn <<= 2;
+        }
+        j += 2;
+        // new codes for all lanes at once, 16 columns after the last or sooner
+        if ((t & 7) == 7 && j > clo && j <= chi) codes(j);
+        __syncwarp();
+    }
+    // merge the lanes in row order: the largest H, its first row; the first
+    // touching row
+    FillResult F;
+    const uint32_t key = ((uint32_t)bHp << 16) | (0xffffu - (uint32_t)bi);
+    const uint32_t top = __reduce_max_sync(ALL, key);
+    const int wl = __ffs(__ballot_sync(ALL, key == top)) - 1;
+    F.bestHp = __shfl_sync(ALL, bHp, wl);
+    F.best_i = __shfl_sync(ALL, bi, wl);
+    F.best_j = F.last_j = __shfl_sync(ALL, bj, wl);
+    const uint32_t row = __reduce_min_sync(ALL, trow ? (uint32_t)trow : 0xffffffffu);
+    const int tl = __ffs(__ballot_sync(ALL, (uint32_t)trow == row)) - 1;
+    F.trow = row == 0xffffffffu ? 0 : (int)row;
+    F.tleft = F.trow && __shfl_sync(ALL, (int)tleft, tl & 31) != 0;
+    F.tclamp = F.trow && __shfl_sync(ALL, (int)tclamp, tl & 31) != 0;
+    return F;
+}
+
+__global__ void __launch_bounds__(128) gotoh_warp_kernel(GotohJob job, GotohConst K) {
+    __shared__ uint32_t s_lut[10];
+    __shared__ int8_t s_lut25[32];
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < 10; k++) s_lut[k] = K.lut4[k >> 1][k & 1];
+#pragma unroll
+        for (int k = 0; k < 25; k++) s_lut25[k] = K.lut[k];
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const uint64_t warp_slot = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    uint32_t *tb = job.tb + warp_slot * (job.tb_words + job.rb_words);
+    uint32_t *rb = tb + job.tb_words;
+    const uint64_t total = job.list_count ? (uint64_t)(*job.list_count) : job.n_pairs;
+    for (uint64_t k = warp_slot; k < total; k += n_warps) {
+        const uint32_t pi = job.list ? job.list[k] : (uint32_t)k;
+        PairSetup S;
+        if (!setup_pair(job, K, pi, job.tb_words, job.rb_words, lane == 0, S)) continue;
+        FillResult F = warp_fill(K, s_lut, S, tb, rb, lane);
+        __syncwarp();  // traceback words of every lane are visible to lane 0
+        if (lane == 0) finish_pair(job, K, s_lut25, pi, S, F, StripTb<1>{tb, S.sw});
+        __syncwarp();
+    }
+}
+
+cudaError_t launch_gotoh_warp(const GotohJob &job, const GotohConst &k, int warps,
+                              cudaStream_t st) {
+    int grid = (warps + 3) / 4;
+    gotoh_warp_kernel<<<grid, 128, 0, st>>>(job, k);
+    return cudaGetLastError();
+}
+
+// Pairs outside the int16 domain: passes of 32 strips (lane s owns rows
+// 8s+1..8s+8 of the pass) swept one column a step, H and E of a strip's bottom
+// row crossing lanes and passes as two int32 words (the row buffer holds 2
+// words per column); lanes outside their windows publish H = 0 and no E.
+__device__ FillResult wide_fill(const GotohConst &K, const uint32_t *__restrict__ s_lut,
                                 const PairSetup &P, uint32_t *tb, uint32_t *rb, int lane) {
     const int m = P.m, n = P.n, sw = P.sw;
     const Geo &g = P.g;
-    const uint32_t ABSENT = absent_HE(K);
     FillResult R;
     R.bestHp = 2;
     R.best_i = R.best_j = R.last_j = 0;
@@ -1058,7 +1305,7 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
         const bool act = s < nstrips;
         const int i0 = s * STRIP + 1;
         const int nact = act ? min(STRIP, m - i0 + 1) : 0;
-        StripT<WIDE> S;
+        StripT<true> S;
 #pragma unroll
         for (int r = 0; r < STRIP; r++) {
             S.lo[r] = g.lo(i0 + r);
@@ -1087,12 +1334,11 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
         int t0 = act ? clo + lane : 0x7fffffff, t1 = act ? chi + lane : -1;
         t0 = __reduce_min_sync(0xffffffffu, t0);
         t1 = __reduce_max_sync(0xffffffffu, t1);
-        // bottom row published at the end of a step: packed (int16) or H / E (int32)
-        uint32_t pub = ABSENT;
+        // bottom row published at the end of a step
         int pubH = 2, pubE = absent_E(K);
         int diag = 2;           // H of the row above at the previous column
         if (lane == 0 && base && clo - 1 >= plo && clo - 1 <= phi)
-            diag = WIDE ? (int)rb[2 * (clo - 1 - plo)] : (int)(rb[clo - 1 - plo] & 0xffffu);
+            diag = (int)rb[2 * (clo - 1 - plo)];
         uint32_t *tbs = tb + (size_t)s * sw;
         const bool handoff = lane == 31 && s + 1 < nstrips;
         int cw_at = -1000000;  // first window position of the cached code word
@@ -1101,20 +1347,12 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
         uint32_t nx = 0, nxn = 0;
         for (int t = t0; t <= t1; t++) {
             const int j = t - lane;
-            int inH, inE;
-            if (WIDE) {
-                inH = __shfl_up_sync(0xffffffffu, pubH, 1);
-                inE = __shfl_up_sync(0xffffffffu, pubE, 1);
-                if (lane == 0) {
-                    const bool have = base && j >= plo && j <= phi;
-                    inH = have ? (int)rb[2 * (j - plo)] : 2;
-                    inE = have ? (int)rb[2 * (j - plo) + 1] : absent_E(K);
-                }
-            } else {
-                uint32_t in = __shfl_up_sync(0xffffffffu, pub, 1);
-                if (lane == 0) in = (base && j >= plo && j <= phi) ? rb[j - plo] : ABSENT;
-                inH = (int)(in & 0xffffu);
-                inE = ((int)in) >> 16;
+            int inH = __shfl_up_sync(0xffffffffu, pubH, 1);
+            int inE = __shfl_up_sync(0xffffffffu, pubE, 1);
+            if (lane == 0) {
+                const bool have = base && j >= plo && j <= phi;
+                inH = have ? (int)rb[2 * (j - plo)] : 2;
+                inE = have ? (int)rb[2 * (j - plo) + 1] : absent_E(K);
             }
             int outH = 2, outE = absent_E(K);
             if (act && j >= clo && j <= chi) {
@@ -1141,27 +1379,19 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
                 uint32_t code = ((cn >> (31 - sh)) & 1u) ? 4u : ((cw >> (30 - 2 * sh)) & 3u);
                 uint32_t sel = code * 0x1111u + 0x8880u;
                 int upH = inH, upE = inE;
-                uint32_t word = dp_column<1, WIDE>(S, K, j, sel, 32767u - (uint32_t)j, upH, upE,
+                uint32_t word = dp_column<1, true>(S, K, j, sel, 32767u - (uint32_t)j, upH, upE,
                                                    diag);
                 tbs[j - clo] = word;
                 outH = upH;
                 outE = upE;
                 if (handoff && j >= lo7) {
-                    if (WIDE) {
-                        rb[2 * (j - lo7)] = (uint32_t)upH;
-                        rb[2 * (j - lo7) + 1] = (uint32_t)upE;
-                    } else {
-                        rb[j - lo7] = __byte_perm((uint32_t)upH, (uint32_t)upE, 0x5410);
-                    }
+                    rb[2 * (j - lo7)] = (uint32_t)upH;
+                    rb[2 * (j - lo7) + 1] = (uint32_t)upE;
                 }
             }
             diag = inH;
-            if (WIDE) {
-                pubH = outH;
-                pubE = outE;
-            } else {
-                pub = __byte_perm((uint32_t)outH, (uint32_t)outE, 0x5410);
-            }
+            pubH = outH;
+            pubE = outE;
         }
         __syncwarp();
         // this lane's rows, in row order (extend.rs:795-827)
@@ -1211,40 +1441,6 @@ __device__ FillResult warp_fill(const GotohConst &K, const uint32_t *__restrict_
     return R;
 }
 
-__global__ void __launch_bounds__(128) gotoh_warp_kernel(GotohJob job, GotohConst K) {
-    __shared__ uint32_t s_lut[10];
-    __shared__ int8_t s_lut25[32];
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < 10; k++) s_lut[k] = K.lut4[k >> 1][k & 1];
-#pragma unroll
-        for (int k = 0; k < 25; k++) s_lut25[k] = K.lut[k];
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp_slot = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    uint32_t *tb = job.tb + warp_slot * (job.tb_words + job.rb_words);
-    uint32_t *rb = tb + job.tb_words;
-    const uint64_t total = job.list_count ? (uint64_t)(*job.list_count) : job.n_pairs;
-    for (uint64_t k = warp_slot; k < total; k += n_warps) {
-        const uint32_t pi = job.list ? job.list[k] : (uint32_t)k;
-        PairSetup S;
-        if (!setup_pair(job, K, pi, job.tb_words, job.rb_words, lane == 0, S)) continue;
-        FillResult F = warp_fill<false>(K, s_lut, S, tb, rb, lane);
-        __syncwarp();  // traceback words of every lane are visible to lane 0
-        if (lane == 0) finish_pair(job, K, s_lut25, pi, S, F, StripTb<1>{tb, S.sw});
-        __syncwarp();
-    }
-}
-
-cudaError_t launch_gotoh_warp(const GotohJob &job, const GotohConst &k, int warps,
-                              cudaStream_t st) {
-    int grid = (warps + 3) / 4;
-    gotoh_warp_kernel<<<grid, 128, 0, st>>>(job, k);
-    return cudaGetLastError();
-}
-
 // Pairs outside the int16 domain (reads longer than GotohConst::max_m), one
 // warp per pair with int32 H / E / F and 64-bit row-max keys, otherwise the
 // warp-per-pair fill and the same traceback: the same cells, words, maxima,
@@ -1271,7 +1467,7 @@ __global__ void __launch_bounds__(128) gotoh_wide_kernel(GotohJob job, GotohCons
         const uint32_t pi = job.list[k];
         PairSetup S;
         if (!setup_pair(job, K, pi, job.tb_words, job.rb_words, lane == 0, S)) continue;
-        FillResult F = warp_fill<true>(K, s_lut, S, tb, rb, lane);
+        FillResult F = wide_fill(K, s_lut, S, tb, rb, lane);
         __syncwarp();
         int esc = 0;
         if (lane == 0) esc = finish_pair(job, K, s_lut25, pi, S, F, StripTb<1>{tb, S.sw}, false) ? 1 : 0;
@@ -1281,7 +1477,7 @@ __global__ void __launch_bounds__(128) gotoh_wide_kernel(GotohJob job, GotohCons
         GotohJob j2 = job;
         j2.mode = 2;
         if (!setup_pair(j2, K, pi, job.tb_words, job.rb_words, lane == 0, S)) continue;
-        F = warp_fill<true>(K, s_lut, S, tb, rb, lane);
+        F = wide_fill(K, s_lut, S, tb, rb, lane);
         __syncwarp();
         if (lane == 0) finish_pair(j2, K, s_lut25, pi, S, F, StripTb<1>{tb, S.sw}, false);
         __syncwarp();
