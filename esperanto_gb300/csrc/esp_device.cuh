@@ -22,6 +22,12 @@ __device__ __forceinline__ uint32_t load16(const uint8_t *__restrict__ arena, ui
     return __funnelshift_l(b, a, sh);
 }
 
+__device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;  // integer multiply-add: issues on the FMA pipe, off the saturated ALU pipe
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+
 // 2-bit code of one base.
 __device__ __forceinline__ uint32_t load1(const uint8_t *__restrict__ arena, uint64_t p) {
     uint8_t byte = __ldg(arena + (p >> 2));

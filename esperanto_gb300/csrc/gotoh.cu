@@ -89,12 +89,6 @@ struct StripT {
 };
 using Strip = StripT<false>;
 
-__device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;  // integer multiply-add: issues on the FMA pipe, off the saturated ALU pipe
-    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
 // a & m and (a & m) | o as opaque logic ops, so that the compiler keeps the
 // differences below as adds instead of folding them back into logic.
 __device__ __forceinline__ uint32_t and_u32(uint32_t a, uint32_t m) {
