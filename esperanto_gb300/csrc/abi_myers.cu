@@ -247,7 +247,12 @@ int esp_batch_myers_host(esp_handle *h, int mode, const esp_myers_pair *pairs,
         for (auto &e : ev) cudaEventDestroy(e);
     };
     // inputs, chunk by chunk: the pairs and the arena prefix the chunk reads
-    // (the last chunk also gets the zero tail that 64-bit code loads read)
+    // (the last chunk also gets the zero tail that 64-bit code loads read).
+    // A copy of pageable memory holds the caller until it is staged, so each
+    // chunk is launched as soon as its own inputs are sent and the results
+    // are fetched after the last (262,144 pairs of 150 x 200 at this entry 0.89 ->
+    // 0.59 ms, 1,048,576 2.10 -> 1.29; touching the result's pages from several
+    // threads meanwhile gained nothing).
     if (n_iv_count)
         CK(h, cudaMemcpyAsync((void *)div, n_iv, n_iv_count * sizeof(esp_n_interval),
                               cudaMemcpyHostToDevice, cs));
@@ -263,17 +268,18 @@ int esp_batch_myers_host(esp_handle *h, int mode, const esp_myers_pair *pairs,
         }
         if (c + 1 == C) CK(h, cudaMemsetAsync(da + arena_bytes, 0, 16, cs));
         CK(h, cudaEventRecord(ev[c], cs));
-    }
-    for (uint64_t c = 0; c < C; c++) {
-        const uint64_t a = bounds[c], n = bounds[c + 1] - a;
         CK(h, cudaStreamWaitEvent(st, ev[c], 0));
         rc = esp_batch_myers_device(h, mode, dp + a, n, mx, da, arena_bytes, div, n_iv_count,
                                     dout + a, st);
         if (rc != ESP_OK) {
+            cudaStreamSynchronize(cs);  // no copy of the caller's arrays stays in flight
             release();
             return rc;
         }
         CK(h, cudaEventRecord(ev[C + c], st));
+    }
+    for (uint64_t c = 0; c < C; c++) {
+        const uint64_t a = bounds[c], n = bounds[c + 1] - a;
         CK(h, cudaStreamWaitEvent(cs, ev[C + c], 0));
         CK(h, cudaMemcpyAsync(out + a, dout + a, n * sizeof(esp_myers_result), cudaMemcpyDeviceToHost, cs));
     }
