@@ -70,8 +70,8 @@ static bool band_paired(esp_handle *h, uint64_t n) {
 // Whether a batch of n pairs runs the mixed kernel: a handle whose kernel was
 // neither set nor tuned, below 2^18 pairs.  Measured against one pair per thread
 // (the earlier choice) and two, in ms: 4,096 mixed pairs 0.54 / 1.84 / 2.21,
-// 65,536 mixed 1.49 / 3.46 / 2.98, 131,072 mixed 2.60 / 3.62 / 2.96; 4,096 of 150
-// x 214 0.25 / 0.35 / 0.40, 65,536 0.85 / 0.81 / 0.80, 131,072 0.92 / 1.44 / 0.90;
+// 65,536 mixed 1.43 / 3.46 / 2.98, 131,072 mixed 2.60 / 3.62 / 2.96; 4,096 of 150
+// x 214 0.25 / 0.35 / 0.40, 65,536 0.58 / 0.81 / 0.58, 131,072 0.91 / 1.44 / 0.90;
 // extend_hint over 65,536 mixed pairs 3.18 / 7.27 / 6.57.  At 262,144 pairs two
 // per thread are even (1.51 of 1.55 and 3.52 of 3.15 ms), at 600,000 ahead
 // (4.94 of 5.60).
@@ -131,7 +131,7 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
         // bin_plan's x for pairs of one cost, the least it can be: below its
         // line all items are the costliest, and all go to groups
         const double x = P.threads * 0.305 / (0.4 * (double)items);
-        P.all_groups = x * 0.4 > 0.75;
+        P.all_groups = x * 0.4 > 1.1;
         if (P.all_groups) P.min_lg = x < 5 ? 2 : (x < 11 ? 3 : (x < 60 ? 4 : 5));
         auto size = [&](int lg) {
             P.min_lg = lg;
@@ -374,6 +374,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
     job.tb_words = tbw;
     job.rb = h->d_rb;
     job.rb_words = rbw;
+    job.sms = h->num_sms;
     job.queue = h->d_ctr;
     job.esc_list = h->d_esc;
     job.esc_count = h->d_ctr + 4;

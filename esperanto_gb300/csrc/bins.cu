@@ -277,9 +277,10 @@ __global__ void class_bounds(const uint32_t *__restrict__ hist, const uint32_t *
 // to itself (52 cycles, measured), the full chip 1.9 T cells/s: an item
 // finishes with the rest of the batch when its cost is the mean cost times
 // items / 23,700 (0.305 x the 77,824 resident threads).  Batches whose costliest
-// item takes more than three quarters of that give the items above it to
-// groups: 65,536 pairs of 150 x 214 (0.72 of it) take 0.80 ms by threads and 0.93
-// in groups of 4; 65,536 mixed pairs (3.3 times it) 2.98 ms by threads, 1.49 split.
+// item takes more than 1.1 times that give the items above half of it to
+// groups: 45,000 pairs of 150 x 214 (1.05 of it) take 0.56 ms by threads and 0.75
+// in groups of 4; 65,536 mixed pairs (3.3 times it) 2.98 ms by threads, 1.43 split.
+// A line at 1.5 or 2 costs 200,000 mixed pairs 4.0 ms, not 2.76.
 // Lanes of a group from how far the costliest item is above it (the fastest of
 // 4, 8, 16 and 32 lanes at 4,096 to 200,000 pairs of one shape and mixed).
 __global__ void bin_plan(const uint32_t *__restrict__ hist, const uint32_t *__restrict__ total,
@@ -293,11 +294,11 @@ __global__ void bin_plan(const uint32_t *__restrict__ hist, const uint32_t *__re
     uint32_t split = 0;
     if (all) {
         split = *total;
-    } else if (top > 0.75f * even) {
+    } else if (top > 1.1f * even) {
         // items of w columns a row and more: the list's order.  extend_hint's
         // first attempt has one width, its list goes by window length.
         const uint32_t cap = (1u << KEY_BITS) - 1;
-        const float w = 0.375f * even / (float)max(stats->max_m, 1u);
+        const float w = 0.55f * even / (float)max(stats->max_m, 1u);
         if (mode == 1) split = *total;
         else split = w < 1.0f ? *total : hist[NBINS - 1 - ((min((uint32_t)w, cap - 1u) << KEY_BITS) | cap)];
     }

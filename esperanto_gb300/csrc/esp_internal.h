@@ -56,6 +56,7 @@ struct GotohJob {
     uint32_t *rb;               // row-buffer scratch: slots * rb_words * 32 words
     uint64_t rb_words;
     uint32_t *queue;            // device work counter (zeroed before launch)
+    int sms;                    // SMs of the device (0: unknown)
     // Pairs outside the int16 domain (read longer than GotohConst::max_m):
     // the int16 kernels append them to wide_list (count in *wide_count) and
     // leave them to the wide kernel, which sets `wide` and runs them in
