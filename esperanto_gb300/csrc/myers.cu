@@ -5,7 +5,7 @@
 // bit-vector of NW 32-bit limbs held in registers; the pattern-equality
 // table Peq[limb][text code] lives in shared memory with a thread-private
 // column per lane (conflict-free: limb w of code c of thread t is at
-// (w * 4 + c) * MY_BLOCK + t).  Each text column advances the whole
+// (w * 4 + c) * blockDim + t).  Each text column advances the whole
 // bit-vector as one wide word: the match-propagation addition ripples its
 // carry across limbs in a single add.cc/addc chain and the horizontal deltas
 // shift across limbs through funnel shifts.  This is the ripple-carry form of
@@ -100,8 +100,7 @@ __device__ __forceinline__ void add_chain<8>(uint32_t (&s)[8], const uint32_t (&
           "r"(b[6]), "r"(b[7]));
 }
 
-constexpr int MY_BLOCK = 256;
-constexpr int MY_STEP = 2;  // columns unrolled
+constexpr int MY_BLOCK = 256, MY_SMALL = 128;  // threads a block, ordered and not
 
 // 16 text codes of one window in processing order: the code of the first
 // column in bits 31:30, its N flag in bit 31 of `n`.
@@ -234,10 +233,12 @@ __device__ __forceinline__ uint32_t virtual_bits(int off, int w) {
 // counts a column.  Columns go 16 a chunk, after the text's first n % 16 (all
 // lanes take that partial chunk together), so that a full chunk has constant
 // shifts and no N test, and its best column is the least of score * 16 +
-// column, one operation each.  1,048,576 reads of 150 bases in texts of 200:
-// 0.747 -> 0.696 ms.  Shifts as products with 2 (the multiply pipe) took
-// fewer ALU operations and as long: their high halves stall the dispatch.
-template <int NW, bool GLOB>
+// column, one operation each; a column's Peq row is read a column ahead.
+// 1,048,576 reads of 150 bases in texts of 200: 0.747 -> 0.687 ms; 12,000 of 200
+// in 260 (few warps, latency) 37.6 -> 33.5 us.  Shifts as products with 2 (the
+// multiply pipe) took fewer ALU operations and as long: their high halves
+// stall the dispatch.
+template <int NW, bool GLOB, int BLOCK>
 __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict__ peq) {
     const esp_myers_pair P = job.pairs[k];
     const int m = (int)P.read_len;
@@ -253,7 +254,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
         return;
     }
     const esp_n_interval *iv = job.n_iv + P.n_first;
-    uint32_t *col = peq + threadIdx.x;  // limb w of code c at (w * 4 + c) * MY_BLOCK
+    uint32_t *col = peq + threadIdx.x;  // limb w of code c at (w * 4 + c) * BLOCK
     const int off = NW * 32 - m;  // virtual rows below the pattern
     uint32_t pv[NW], mv[NW];
 #pragma unroll
@@ -267,7 +268,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
         const uint32_t virt = virtual_bits(off, w);
 #pragma unroll
         for (int q = 0; q < 4; q++)
-            col[(w * 4 + q) * MY_BLOCK] = (rev ? __brev(rows[q]) : rows[q]) | (GLOB ? 0u : virt);
+            col[(w * 4 + q) * BLOCK] = (rev ? __brev(rows[q]) : rows[q]) | (GLOB ? 0u : virt);
         pv[w] = ~virt;  // pattern rows start with vertical delta +1 (D[i][0] = i)
         mv[w] = 0u;
     }
@@ -276,29 +277,37 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
     uint32_t best_at = 0;
     const esp_n_interval *tiv = iv + P.n_read;
     const char *rows = reinterpret_cast<const char *>(col);
-    constexpr uint32_t ROW = MY_BLOCK * 4;  // bytes, a power of two
+    constexpr uint32_t ROW = BLOCK * 4;  // bytes, a power of two
     uint32_t done = 0;
     for (uint32_t cnt = n & 15; done < n; done += cnt, cnt = 16) {
         if (cnt == 0) continue;
         CodeWin win = text_codes(job, P, tiv, rev, rev ? n - done - cnt : done, (int)cnt);
         int least = INT_MAX;
         if (cnt == 16 && win.n >> 16 == 0) {
+            constexpr int STEP = 2;  // columns unrolled
+            uint32_t next[NW];  // the next column's Peq row, read a column ahead
+            const uint32_t *pe = reinterpret_cast<const uint32_t *>(rows + (win.c >> 30) * ROW);
+#pragma unroll
+            for (int w = 0; w < NW; w++) next[w] = pe[w * 4 * BLOCK];
 #pragma unroll 1
-            for (int g = 0; g < 16; g += MY_STEP) {
+            for (int g = 0; g < 16; g += STEP) {
 #pragma unroll
-                for (int x = 0; x < MY_STEP; x++) {
-                    const uint32_t r = ((win.c >> (30 - 2 * x)) & 3u) * ROW;
-                    const uint32_t *pe = reinterpret_cast<const uint32_t *>(rows + r);
+                for (int x = 0; x < STEP; x++) {
                     uint32_t eq[NW], up, down;
+                    const uint32_t r = ((win.c >> (28 - 2 * x)) & 3u) * ROW;  // 0 after the last
+                    pe = reinterpret_cast<const uint32_t *>(rows + r);
 #pragma unroll
-                    for (int w = 0; w < NW; w++) eq[w] = pe[w * 4 * MY_BLOCK];
+                    for (int w = 0; w < NW; w++) {
+                        eq[w] = next[w];
+                        next[w] = pe[w * 4 * BLOCK];
+                    }
                     myers_column<NW, GLOB>(eq, pv, mv, up, down);
                     key = (int)mad_u32(up, (uint32_t)KEY, (uint32_t)key);
                     key = (int)mad_u32(down, (uint32_t)-KEY, (uint32_t)key);
                     if (!GLOB) least = __viaddmin_s32(key, x, least);
                 }
-                win.c <<= 2 * MY_STEP;
-                if (!GLOB) key += MY_STEP;
+                win.c <<= 2 * STEP;
+                if (!GLOB) key += STEP;
             }
             if (!GLOB) key -= 16;
         } else {  // a partial step, or N in the text: it matches virtual rows only
@@ -311,7 +320,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
                     for (int w = 0; w < NW; w++) eq[w] = GLOB ? 0u : virtual_bits(off, w);
                 } else {
 #pragma unroll
-                    for (int w = 0; w < NW; w++) eq[w] = pe[w * 4 * MY_BLOCK];
+                    for (int w = 0; w < NW; w++) eq[w] = pe[w * 4 * BLOCK];
                 }
                 win.c <<= 2;
                 win.n <<= 1;
@@ -337,7 +346,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
 
 template <int NW, bool GLOB>
 __device__ __noinline__ void myers_call(const MyersJob &job, uint32_t k, uint32_t *peq) {
-    myers_pair<NW, GLOB>(job, k, peq);
+    myers_pair<NW, GLOB, MY_BLOCK>(job, k, peq);
 }
 
 // The limbs of the warp's longest read, 1..NW, choose its pairs' code.
@@ -352,72 +361,87 @@ __device__ __forceinline__ int limbs_of(uint32_t m) {
     return m ? (int)min((m - 1) / 32 + 1, (uint32_t)NW) : 0;
 }
 
-// `per` pairs a block (launch_myers), its warps given them in the order of
-// their limbs: a warp's time is that of its longest read, and without the
-// order nearly every warp of a ragged batch has one near the longest, and all
-// ran the limbs of the batch's longest.  Reads of 20 to 256 bases, best start: 100,003
-// pairs 0.248 -> 0.162 ms, 300,000 0.64 -> 0.45 (blocks of 128: 0.188 for 100,003).
-// Two columns unrolled: with 4 or 8 the code of several limb counts does not
-// fit the instruction cache (0.174 and 0.21 ms; one count alone 1 % faster).
+// A block's warps are given its pairs in the order of their limbs: a warp's time
+// is that of its longest read, and in the batch's order nearly every warp of a
+// ragged batch has one near the longest, and all run the limbs of the batch's longest.
+// Reads of 20 to 256 bases, best start: 100,003 pairs 0.248 -> 0.160 ms, 300,000
+// 0.64 -> 0.42 (100,003 in blocks of 128: 0.188).  Two columns unrolled: with 4 or 8
+// the code of several limb counts does not fit the instruction cache (0.174 and
+// 0.21 ms).  A block whose reads all have NW limbs keeps the batch's order.
 template <int NW, bool GLOB>
-__global__ void __launch_bounds__(MY_BLOCK) myers_kernel(MyersJob job, uint32_t per) {
+__global__ void __launch_bounds__(MY_BLOCK)
+    myers_ordered_kernel(const __grid_constant__ MyersJob job) {
     extern __shared__ uint32_t smem[];
-    constexpr int WARPS = MY_BLOCK / 32, CLASSES = NW + 1;
-    __shared__ uint32_t s_first[CLASSES * WARPS];  // pairs of (class, warp), then those before
+    __shared__ uint32_t s_first[(NW + 1) * MY_BLOCK / 32];  // pairs of (class, warp), then those before
     __shared__ uint16_t s_order[MY_BLOCK];
-    const uint64_t base = (uint64_t)blockIdx.x * per;
+    constexpr int WARPS = MY_BLOCK / 32, ENTRIES = (NW + 1) * WARPS;
+    const uint64_t base = (uint64_t)blockIdx.x * MY_BLOCK;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int limbs = 0;
-    if (threadIdx.x < per && base + threadIdx.x < job.n_pairs)
-        limbs = limbs_of<NW>(job.pairs[base + threadIdx.x].read_len);
-    uint32_t mine = 0;
+    uint64_t k = base + threadIdx.x;
+    bool have = k < job.n_pairs;
+    int limbs = have ? limbs_of<NW>(job.pairs[k].read_len) : 0;
+    if (!__syncthreads_and(!have || limbs == NW)) {
+        uint32_t mine = 0;
 #pragma unroll
-    for (int c = 0; c < CLASSES; c++) {
-        const uint32_t b = __ballot_sync(0xffffffffu, limbs == c);
-        if (limbs == c) mine = b;
-        if (lane == 0) s_first[c * WARPS + warp] = (uint32_t)__popc(b);
-    }
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t before = 0;
-        for (int e = 0; e < CLASSES * WARPS; e += 32) {
-            const uint32_t v = e + lane < CLASSES * WARPS ? s_first[e + lane] : 0u;
-            uint32_t x = v;
-            for (int d = 1; d < 32; d *= 2) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-                if (lane >= d) x += y;
-            }
-            if (e + lane < CLASSES * WARPS) s_first[e + lane] = before + x - v;
-            before += __shfl_sync(0xffffffffu, x, 31);
+        for (int c = 0; c <= NW; c++) {
+            const uint32_t b = __ballot_sync(0xffffffffu, limbs == c);
+            if (limbs == c) mine = b;
+            if (lane == 0) s_first[c * WARPS + warp] = (uint32_t)__popc(b);
         }
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t before = 0;
+            for (int e = 0; e < ENTRIES; e += 32) {
+                const uint32_t v = e + lane < ENTRIES ? s_first[e + lane] : 0u;
+                uint32_t x = v;
+                for (int d = 1; d < 32; d *= 2) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+                    if (lane >= d) x += y;
+                }
+                if (e + lane < ENTRIES) s_first[e + lane] = before + x - v;
+                before += __shfl_sync(0xffffffffu, x, 31);
+            }
+        }
+        __syncthreads();
+        s_order[s_first[limbs * WARPS + warp] + __popc(mine & ((1u << lane) - 1u))] =
+            (uint16_t)threadIdx.x;
+        __syncthreads();
+        k = base + s_order[threadIdx.x];
+        have = k < job.n_pairs;
+        limbs = have ? limbs_of<NW>(job.pairs[k].read_len) : 0;
     }
-    __syncthreads();
-    s_order[s_first[limbs * WARPS + warp] + __popc(mine & ((1u << lane) - 1u))] =
-        (uint16_t)threadIdx.x;
-    __syncthreads();
-    const uint32_t o = s_order[threadIdx.x];
-    const uint64_t k = base + o;
-    const bool have = o < per && k < job.n_pairs;
-    limbs = have ? limbs_of<NW>(job.pairs[k].read_len) : 1;
     limbs = max(1, __reduce_max_sync(0xffffffffu, limbs));
     if (have) myers_limbs<NW, GLOB>(job, (uint32_t)k, smem, limbs);
 }
 
+// A thread a pair, in the batch's order.
+template <int NW, bool GLOB>
+__global__ void __launch_bounds__(MY_SMALL) myers_kernel(const __grid_constant__ MyersJob job) {
+    extern __shared__ uint32_t smem[];
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < job.n_pairs) myers_pair<NW, GLOB, MY_SMALL>(job, (uint32_t)k, smem);
+}
+
+template <int NW, bool GLOB>
+static void launch_limbs(const MyersJob &job, bool ordered, cudaStream_t st) {
+    const int block = ordered ? MY_BLOCK : MY_SMALL;
+    const size_t smem = (size_t)4 * NW * block * sizeof(uint32_t);
+    const unsigned grid = (unsigned)((job.n_pairs + block - 1) / block);
+    if (ordered) myers_ordered_kernel<NW, GLOB><<<grid, block, smem, st>>>(job);
+    else myers_kernel<NW, GLOB><<<grid, block, smem, st>>>(job);
+}
+
 cudaError_t launch_myers(const MyersJob &job, int nw, int num_sms, cudaStream_t st) {
     if (job.n_pairs == 0) return cudaSuccess;
-    const size_t smem = (size_t)4 * nw * MY_BLOCK * sizeof(uint32_t);
-    // two blocks for every SM before any takes more pairs: 2,000 ragged pairs
-    // 0.056 ms, in blocks of 256 0.072
-    const uint64_t share = (job.n_pairs + 2 * num_sms - 1) / (2 * num_sms);
-    const uint32_t per = (uint32_t)std::min<uint64_t>(MY_BLOCK, (share + 31) / 32 * 32);
-    const unsigned grid = (unsigned)((job.n_pairs + per - 1) / per);
+    // up to two warps a scheduler a launch lasts as long as its longest pair in
+    // any order, and ordering costs 2 us: 12,000 reads of 60 bases 10.9 us, ordered
+    // 12.5; 60,000 of 40 to 120 bases 51 us, ordered 41
+    const bool ordered = job.n_pairs > (uint64_t)num_sms * 256;
     switch (nw) {
-#define ESP_MY_CASE(W)                                                   \
-    case W:                                                              \
-        if (job.flags & MYF_GLOBAL)                                      \
-            myers_kernel<W, true><<<grid, MY_BLOCK, smem, st>>>(job, per);  \
-        else                                                             \
-            myers_kernel<W, false><<<grid, MY_BLOCK, smem, st>>>(job, per); \
+#define ESP_MY_CASE(W)                                                           \
+    case W:                                                                      \
+        if (job.flags & MYF_GLOBAL) launch_limbs<W, true>(job, ordered, st);     \
+        else launch_limbs<W, false>(job, ordered, st);                           \
         break;
         ESP_MY_CASE(1) ESP_MY_CASE(2) ESP_MY_CASE(3) ESP_MY_CASE(4)
         ESP_MY_CASE(5) ESP_MY_CASE(6) ESP_MY_CASE(7) ESP_MY_CASE(8)

@@ -1,6 +1,6 @@
 """The Myers kernel where its launch and its loops branch (myers.cu): batches
-that give a block 32 to 256 pairs, whole or short in the last one, ordered by
-limb count; reads of every limb count with one row to either side, empty reads
+in their own order and (from 256 pairs an SM on) ordered by limb count within a
+block, the last block whole or short; reads of every limb count with one row to either side, empty reads
 among them; texts of every length modulo 16, empty, shorter than 16, and with N
 runs in partial and full chunks.  Every distance and position equals the
 oracle's."""
