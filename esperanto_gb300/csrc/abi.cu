@@ -855,7 +855,7 @@ int esp_batch_extend_device(esp_handle *h, int mode, const esp_pair *pairs, uint
         (uint64_t)params->mismatch, (uint64_t)params->gap_open, (uint64_t)params->gap_ext,
         (uint64_t)params->edit_dir, (uint64_t)(uintptr_t)out, (uint64_t)(uintptr_t)cigar,
         cigar_stride, (uint64_t)(uintptr_t)st, (uint64_t)h->warp_max, (uint64_t)h->variant,
-        (uint64_t)h->binning, (uint64_t)h->tuned};
+        (uint64_t)h->binning, (uint64_t)h->tuned, (uint64_t)h->variant_by_size};
     for (int s = 0; s < esp::kLengthClasses; s++) key.push_back((uint64_t)(int64_t)h->tune[s]);
     key.push_back(h->buf_gen);
     if (h->graph_exec && key == h->graph_key) {

@@ -317,7 +317,7 @@ int esp_server_create(esp_genome *g, const esp_extend_params *params,
     if (!c.max_read_len) c.max_read_len = 300;
     if (!c.max_win_len) c.max_win_len = c.max_read_len + 128;
     if (!c.mem_budget_bytes) c.mem_budget_bytes = 16ull << 30;
-    // a launch stays on the one-pair kernel (below the paired kernel's size)
+    // a launch's lists and scratch stay within what the slots were planned for
     if (c.max_reads >= (1u << 20) || c.n_streams > 64) {
         delete s;
         return ESP_EINVAL;

@@ -97,13 +97,14 @@ class ExtendBuffer:
 
     def set_warp_max(self, warp_max: int):
         """Batches of at most warp_max pairs (and every per-call entry) run
-        one warp per pair, larger ones one thread per pair; same results."""
+        one warp per pair, larger ones in groups of lanes or per thread; same
+        results."""
         self.check(self._L.esp_set_warp_max(self._h, int(warp_max)))
 
     def set_kernel_variant(self, variant: int):
-        """Thread-per-pair kernel variant: 0 / 1 one pair per thread (3 / 4
-        blocks per SM), 2 / 3 two pairs of one band geometry per thread
-        (band mode), -1 the default; same results."""
+        """Thread kernel variant: 0 / 1 one pair per thread (3 / 4 blocks per
+        SM), 2 / 3 two pairs of one band geometry per thread (band mode), -1
+        the ESP_GOTOH_VARIANT variable, else by size; same results."""
         self.check(self._L.esp_set_kernel_variant(self._h, int(variant)))
 
     def stream_ptr(self) -> int:

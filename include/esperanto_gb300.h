@@ -88,17 +88,19 @@ typedef struct {
 int esp_create(esp_handle **out, int device);
 /* Kernel choice (no counterpart in the reference): batches of at most
  * `warp_max` pairs -- every per-call entry point included -- run one warp per
- * pair (a wavefront over the pair's strips); larger batches run one thread
- * per pair in the persistent length-binned kernel.  Both give identical
- * results.  Default 2048, or the ESP_WARP_MAX environment variable. */
+ * pair (a wavefront over the pair's strips); larger batches run persistent
+ * length-binned kernels (groups of lanes per two pairs, two pairs or one pair
+ * per thread).  All give identical results.  Default 2048, or the ESP_WARP_MAX environment variable. */
 int esp_set_warp_max(esp_handle *h, long warp_max);
 /* Kernel variant of the thread-per-pair batches (no counterpart in the
  * reference): 0 = one pair per thread at 3 resident blocks per SM, 1 = at 4
  * blocks, 2 / 3 = two pairs of identical band geometry per thread (16x2 SIMD
  * lanes) at 3 / 4 blocks; -1 = the ESP_GOTOH_VARIANT environment variable,
- * else by size: variant 3 for batches of 2^20 pairs and more, 1 below.
+ * else by size: variant 3 for batches of 2^18 pairs and more; below, two pairs
+ * per thread with the costly pairs in groups of 4 to 32 lanes.
  * Applies to band-mode batches and clears a previous autotuning.  Hint-mode
- * batches choose by size the same way (ESP_GOTOH_HINT_VARIANT overrides).
+ * batches choose by size the same way (ESP_GOTOH_HINT_VARIANT overrides;
+ * below 2^18 pairs a variant set here runs as its one-pair counterpart).
  * All variants give identical results. */
 int esp_set_kernel_variant(esp_handle *h, int variant);
 int esp_destroy(esp_handle *h);
