@@ -50,13 +50,12 @@ MYERS_OPS_PER_CELL = 10.0 / 32.0
 # and the Myers batch (1,048,576 pairs, one launch); the mixed-length batch
 # per DP cell, captured on a
 # 524,288-pair case of the same distribution and scaled by cells.
-TRAFFIC_BYTES = {0: 51.8e6 + 348.4e6, 1: 125.5e6 + 9.3e6}
+TRAFFIC_BYTES = {0: 29.8e6 + 358.9e6, 1: 125.4e6 + 8.4e6}
 # keyed by (workload, SIMD lanes): one pair per thread, two pairs per thread
 TRAFFIC_PER_CELL = {(2, 1): (2713001472 + 6431804160) / 7716062109,
-                    (2, 2): (35225117184 + 60432276480) / 61820954081}
-TRAFFIC_SOURCE = {0: "profiles/gotoh_kernel_banded150x214_65536pairs.md",
-                  1: "profiles/myers_kernel_150x200_1048576pairs.md",
-                  2: "profiles/gotoh_kernel_traffic_mixedlength.md (scaled by cells)"}
+                    (2, 2): (3486293760 + 7249786624) / 7716062109}
+TRAFFIC_SOURCE = {c: "profiles/dp_and_myers_kernels_traffic_and_pipes.md" +
+                     (" (scaled by cells)" if c == 2 else "") for c in range(3)}
 DEFAULT_PAIRS = {0: 65536, 1: 1048576, 2: 4194304, 3: 524288}
 SEEDS = {0: 1, 1: 2, 2: 3, 3: 4}
 
@@ -201,7 +200,8 @@ class GotohWorkload(Workload):
             chosen = list(variants)
         else:  # the handle's default: by size unless ESP_GOTOH_VARIANT is set
             forced = os.environ.get("ESP_GOTOH_VARIANT")
-            chosen = [int(forced) if forced else (3 if n >= (1 << 20) else 1)]
+            # above the warp-per-pair size every default kernel is 16x2
+            chosen = [int(forced) if forced else (3 if n > 2048 else 1)]
         # variants 2 / 3 compute two pairs per thread in 16-bit SIMD halves
         self.lanes = 2 if any(v >= 2 for v in chosen) else 1
         if self.lanes == 2:
@@ -434,9 +434,9 @@ class SpliceWorkload(Workload):
         self.input_mb = (garena.nbytes + rarena.nbytes) / 1e6
         self.n_cands = len(cands)
         # the flank DPs (22 extend_hint pairs per candidate) run as one hint
-        # batch: on the 16x2 paired kernel from 2^20 pairs unless overridden
+        # batch: on the 16x2 kernels above 2,048 pairs unless overridden
         forced = os.environ.get("ESP_GOTOH_HINT_VARIANT")
-        paired = int(forced) >= 2 if forced else 22 * len(cands) >= (1 << 20)
+        paired = int(forced) >= 2 if forced else 22 * len(cands) > 2048
         self.lanes = 2 if paired else 1
         if paired:
             self.dtype = "int16x2"
@@ -506,12 +506,12 @@ def serve_phase(args, device=0, clocked=True):
            "load": res, "load_seconds": args.serve_seconds, "setup_s": setup_s,
            "clocks": clocks}
     if clocked:
-        peak_ops, _ = int_peak(device, 1)
+        peak_ops, _ = int_peak(device, 2)
         out["roofline"] = {"bound": "int_alu",
                            "achieved": peak_gcups * 1e9 * OPS_PER_CELL / 1e12,
                            "peak": peak_ops / 1e12, "unit": "Tops/s",
                            "frac": peak_gcups * 1e9 * OPS_PER_CELL / peak_ops,
-                           "note": "saturated serve throughput (one pair per thread kernel)"}
+                           "note": "saturated serve throughput (16x2 kernels)"}
     if not args.no_cpu_baseline:
         out["cpu_baseline"] = serve_cpu_baseline(garena, contigs, pool[0])
     return out
