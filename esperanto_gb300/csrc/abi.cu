@@ -770,14 +770,11 @@ int esp_batch_extend_host(esp_handle *h, int mode, const esp_pair *pairs, uint64
     std::vector<cudaEvent_t> ev(2 * C);
     for (auto &e : ev) CK(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     // inputs, chunk by chunk: the pairs and the arena prefix the chunk reads
-    // (the last chunk also gets the zero tail that 64-bit code loads read).
-    // A copy of pageable memory holds the caller until it is staged, so each
-    // chunk is launched as soon as its own inputs are sent and the results
-    // are fetched after the last.
+    // (the last chunk also gets the zero tail that 64-bit code loads read)
     if (n_iv_count)
         CK(h, cudaMemcpyAsync(div, n_iv, n_iv_count * sizeof(esp_n_interval), cudaMemcpyHostToDevice, cs));
     uint64_t copied = 0;  // arena bytes already sent
-    for (uint64_t c = 0; c < C; c++) {
+    auto send = [&](uint64_t c) -> int {
         const uint64_t a = bounds[c], n = bounds[c + 1] - a;
         CK(h, cudaMemcpyAsync(dp + a, pairs + a, n * sizeof(esp_pair), cudaMemcpyHostToDevice, cs));
         uint64_t need = c + 1 == C ? arena_bytes
@@ -788,23 +785,31 @@ int esp_batch_extend_host(esp_handle *h, int mode, const esp_pair *pairs, uint64
         }
         if (c + 1 == C) CK(h, cudaMemsetAsync(da + arena_bytes, 0, 16, cs));
         CK(h, cudaEventRecord(ev[c], cs));
+        return ESP_OK;
+    };
+    auto launch = [&](uint64_t c) -> int {
+        const uint64_t a = bounds[c], n = bounds[c + 1] - a;
         CK(h, cudaStreamWaitEvent(st, ev[c], 0));
-        rc = enqueue_batch(h, mode, dp + a, n, da, arena_bytes, div, n_iv_count, K, L1, L2,
-                           dout + a, dcig + a * cigar_stride, cigar_stride, st);
-        if (rc != ESP_OK) {
-            cudaStreamSynchronize(cs);  // no copy of the caller's arrays stays in flight
-            for (auto &e : ev) cudaEventDestroy(e);
-            return rc;
-        }
+        const int r = enqueue_batch(h, mode, dp + a, n, da, arena_bytes, div, n_iv_count, K, L1, L2,
+                                    dout + a, dcig + a * cigar_stride, cigar_stride, st);
+        if (r != ESP_OK) return r;
         CK(h, cudaEventRecord(ev[C + c], st));
-    }
-    for (uint64_t c = 0; c < C; c++) {
+        return ESP_OK;
+    };
+    auto fetch = [&](uint64_t c) -> int {
         const uint64_t a = bounds[c], n = bounds[c + 1] - a;
         CK(h, cudaStreamWaitEvent(cs, ev[C + c], 0));
         CK(h, cudaMemcpyAsync(out + a, dout + a, n * sizeof(esp_extension), cudaMemcpyDeviceToHost, cs));
         if (cigar && cigar_stride)
             CK(h, cudaMemcpyAsync(cigar + a * cigar_stride, dcig + a * cigar_stride,
                                   n * (size_t)cigar_stride * 4, cudaMemcpyDeviceToHost, cs));
+        return ESP_OK;
+    };
+    rc = run_chunks(C, pageable(pairs) || pageable(arena), send, launch, fetch);
+    if (rc != ESP_OK) {
+        cudaStreamSynchronize(cs);  // no copy of the caller's arrays stays in flight
+        for (auto &e : ev) cudaEventDestroy(e);
+        return rc;
     }
     CK(h, cudaStreamSynchronize(cs));
     CK(h, cudaStreamSynchronize(st));

@@ -247,17 +247,12 @@ int esp_batch_myers_host(esp_handle *h, int mode, const esp_myers_pair *pairs,
         for (auto &e : ev) cudaEventDestroy(e);
     };
     // inputs, chunk by chunk: the pairs and the arena prefix the chunk reads
-    // (the last chunk also gets the zero tail that 64-bit code loads read).
-    // A copy of pageable memory holds the caller until it is staged, so each
-    // chunk is launched as soon as its own inputs are sent and the results
-    // are fetched after the last (262,144 pairs of 150 x 200 at this entry 0.89 ->
-    // 0.59 ms, 1,048,576 2.10 -> 1.29; touching the result's pages from several
-    // threads meanwhile gained nothing).
+    // (the last chunk also gets the zero tail that 64-bit code loads read)
     if (n_iv_count)
         CK(h, cudaMemcpyAsync((void *)div, n_iv, n_iv_count * sizeof(esp_n_interval),
                               cudaMemcpyHostToDevice, cs));
     uint64_t copied = 0;  // arena bytes already sent
-    for (uint64_t c = 0; c < C; c++) {
+    auto send = [&](uint64_t c) -> int {
         const uint64_t a = bounds[c], n = bounds[c + 1] - a;
         CK(h, cudaMemcpyAsync(dp + a, pairs + a, n * sizeof(esp_myers_pair), cudaMemcpyHostToDevice, cs));
         uint64_t need = c + 1 == C ? arena_bytes
@@ -268,20 +263,28 @@ int esp_batch_myers_host(esp_handle *h, int mode, const esp_myers_pair *pairs,
         }
         if (c + 1 == C) CK(h, cudaMemsetAsync(da + arena_bytes, 0, 16, cs));
         CK(h, cudaEventRecord(ev[c], cs));
+        return ESP_OK;
+    };
+    auto launch = [&](uint64_t c) -> int {
+        const uint64_t a = bounds[c], n = bounds[c + 1] - a;
         CK(h, cudaStreamWaitEvent(st, ev[c], 0));
-        rc = esp_batch_myers_device(h, mode, dp + a, n, mx, da, arena_bytes, div, n_iv_count,
-                                    dout + a, st);
-        if (rc != ESP_OK) {
-            cudaStreamSynchronize(cs);  // no copy of the caller's arrays stays in flight
-            release();
-            return rc;
-        }
+        const int r = esp_batch_myers_device(h, mode, dp + a, n, mx, da, arena_bytes, div,
+                                             n_iv_count, dout + a, st);
+        if (r != ESP_OK) return r;
         CK(h, cudaEventRecord(ev[C + c], st));
-    }
-    for (uint64_t c = 0; c < C; c++) {
+        return ESP_OK;
+    };
+    auto fetch = [&](uint64_t c) -> int {
         const uint64_t a = bounds[c], n = bounds[c + 1] - a;
         CK(h, cudaStreamWaitEvent(cs, ev[C + c], 0));
         CK(h, cudaMemcpyAsync(out + a, dout + a, n * sizeof(esp_myers_result), cudaMemcpyDeviceToHost, cs));
+        return ESP_OK;
+    };
+    rc = run_chunks(C, pageable(pairs) || pageable(arena), send, launch, fetch);
+    if (rc != ESP_OK) {
+        cudaStreamSynchronize(cs);  // no copy of the caller's arrays stays in flight
+        release();
+        return rc;
     }
     CK(h, cudaStreamSynchronize(cs));
     CK(h, cudaStreamSynchronize(st));

@@ -185,6 +185,37 @@ inline HostPool &host_pool(esp_handle *h) {
     return *h->pool;
 }
 
+// Whether an asynchronous copy from host array p holds the caller until it is
+// staged (memory that is not page-locked).
+inline bool pageable(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();  // an unknown pointer: an ordinary host array
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// The order of a host batch's C chunks.  Copies of page-locked arrays are all
+// queued first.  Copies of other arrays hold the caller until they are staged,
+// so each chunk is launched once its own inputs are sent, and the results are
+// fetched after the last: 262,144 Myers pairs of 150 x 200 at the entry 0.89 ->
+// 0.59 ms, 1,048,576 2.10 -> 1.29.  (Touching the result's pages from several
+// threads meanwhile gained nothing.)
+template <class Send, class Launch, class Fetch>
+inline int run_chunks(uint64_t C, bool staged, Send send, Launch launch, Fetch fetch) {
+    int rc = ESP_OK;
+    for (uint64_t c = 0; c < C && rc == ESP_OK; c++) {
+        rc = send(c);
+        if (staged && rc == ESP_OK) rc = launch(c);
+    }
+    for (uint64_t c = 0; c < C && rc == ESP_OK; c++) {
+        if (!staged) rc = launch(c);
+        if (rc == ESP_OK) rc = fetch(c);
+    }
+    return rc;
+}
+
 inline void add_limits(Limits &L, uint32_t m, uint32_t n, int32_t half) {
     uint64_t tb, rb;
     esp::gotoh_scratch_words(m, n, half, tb, rb);
