@@ -5,7 +5,7 @@
 // bit-vector of NW 32-bit limbs held in registers; the pattern-equality
 // table Peq[limb][text code] lives in shared memory with a thread-private
 // column per lane (conflict-free: limb w of code c of thread t is at
-// (w * 4 + c) * blockDim + t).  Each text column advances the whole
+// (w * 4 + c) * MY_BLOCK + t).  Each text column advances the whole
 // bit-vector as one wide word: the match-propagation addition ripples its
 // carry across limbs in a single add.cc/addc chain and the horizontal deltas
 // shift across limbs through funnel shifts.  This is the ripple-carry form of
@@ -100,7 +100,7 @@ __device__ __forceinline__ void add_chain<8>(uint32_t (&s)[8], const uint32_t (&
           "r"(b[6]), "r"(b[7]));
 }
 
-constexpr int MY_BLOCK = 256, MY_SMALL = 128;  // threads a block, ordered and not
+constexpr int MY_BLOCK = 128;
 
 // 16 text codes of one window in processing order: the code of the first
 // column in bits 31:30, its N flag in bit 31 of `n`.
@@ -238,7 +238,7 @@ __device__ __forceinline__ uint32_t virtual_bits(int off, int w) {
 // in 260 (few warps, latency) 37.6 -> 33.5 us.  Shifts as products with 2 (the
 // multiply pipe) took fewer ALU operations and as long: their high halves
 // stall the dispatch.
-template <int NW, bool GLOB, int BLOCK>
+template <int NW, bool GLOB>
 __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict__ peq) {
     const esp_myers_pair P = job.pairs[k];
     const int m = (int)P.read_len;
@@ -254,7 +254,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
         return;
     }
     const esp_n_interval *iv = job.n_iv + P.n_first;
-    uint32_t *col = peq + threadIdx.x;  // limb w of code c at (w * 4 + c) * BLOCK
+    uint32_t *col = peq + threadIdx.x;  // limb w of code c at (w * 4 + c) * MY_BLOCK
     const int off = NW * 32 - m;  // virtual rows below the pattern
     uint32_t pv[NW], mv[NW];
 #pragma unroll
@@ -268,7 +268,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
         const uint32_t virt = virtual_bits(off, w);
 #pragma unroll
         for (int q = 0; q < 4; q++)
-            col[(w * 4 + q) * BLOCK] = (rev ? __brev(rows[q]) : rows[q]) | (GLOB ? 0u : virt);
+            col[(w * 4 + q) * MY_BLOCK] = (rev ? __brev(rows[q]) : rows[q]) | (GLOB ? 0u : virt);
         pv[w] = ~virt;  // pattern rows start with vertical delta +1 (D[i][0] = i)
         mv[w] = 0u;
     }
@@ -277,7 +277,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
     uint32_t best_at = 0;
     const esp_n_interval *tiv = iv + P.n_read;
     const char *rows = reinterpret_cast<const char *>(col);
-    constexpr uint32_t ROW = BLOCK * 4;  // bytes, a power of two
+    constexpr uint32_t ROW = MY_BLOCK * 4;  // bytes, a power of two
     uint32_t done = 0;
     for (uint32_t cnt = n & 15; done < n; done += cnt, cnt = 16) {
         if (cnt == 0) continue;
@@ -288,7 +288,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
             uint32_t next[NW];  // the next column's Peq row, read a column ahead
             const uint32_t *pe = reinterpret_cast<const uint32_t *>(rows + (win.c >> 30) * ROW);
 #pragma unroll
-            for (int w = 0; w < NW; w++) next[w] = pe[w * 4 * BLOCK];
+            for (int w = 0; w < NW; w++) next[w] = pe[w * 4 * MY_BLOCK];
 #pragma unroll 1
             for (int g = 0; g < 16; g += STEP) {
 #pragma unroll
@@ -299,7 +299,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
 #pragma unroll
                     for (int w = 0; w < NW; w++) {
                         eq[w] = next[w];
-                        next[w] = pe[w * 4 * BLOCK];
+                        next[w] = pe[w * 4 * MY_BLOCK];
                     }
                     myers_column<NW, GLOB>(eq, pv, mv, up, down);
                     key = (int)mad_u32(up, (uint32_t)KEY, (uint32_t)key);
@@ -320,7 +320,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
                     for (int w = 0; w < NW; w++) eq[w] = GLOB ? 0u : virtual_bits(off, w);
                 } else {
 #pragma unroll
-                    for (int w = 0; w < NW; w++) eq[w] = pe[w * 4 * BLOCK];
+                    for (int w = 0; w < NW; w++) eq[w] = pe[w * 4 * MY_BLOCK];
                 }
                 win.c <<= 2;
                 win.n <<= 1;
@@ -346,7 +346,7 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict
 
 template <int NW, bool GLOB>
 __device__ __noinline__ void myers_call(const MyersJob &job, uint32_t k, uint32_t *peq) {
-    myers_pair<NW, GLOB, MY_BLOCK>(job, k, peq);
+    myers_pair<NW, GLOB>(job, k, peq);
 }
 
 // The limbs of the warp's longest read, 1..NW, choose its pairs' code.
@@ -364,10 +364,12 @@ __device__ __forceinline__ int limbs_of(uint32_t m) {
 // A block's warps are given its pairs in the order of their limbs: a warp's time
 // is that of its longest read, and in the batch's order nearly every warp of a
 // ragged batch has one near the longest, and all run the limbs of the batch's longest.
-// Reads of 20 to 256 bases, best start: 100,003 pairs 0.248 -> 0.160 ms, 300,000
-// 0.64 -> 0.42 (100,003 in blocks of 128: 0.188).  Two columns unrolled: with 4 or 8
-// the code of several limb counts does not fit the instruction cache (0.174 and
-// 0.21 ms).  A block whose reads all have NW limbs keeps the batch's order.
+// Reads of 20 to 256 bases: 100,003 pairs, best start, 0.248 -> 0.168 ms; 262,144, best end,
+// 0.48 -> 0.34, 400,000 0.72 -> 0.56.  Blocks of 256 order better (400,000 in 0.51)
+// but fill the SMs unevenly: 131,072 reads of 150 bases took 107 us, in these 95,
+// before 101.  Two columns unrolled: with 4 or 8 the code of several limb counts
+// does not fit the instruction cache (a quarter slower).  A block whose reads all
+// have NW limbs keeps the batch's order.
 template <int NW, bool GLOB>
 __global__ void __launch_bounds__(MY_BLOCK)
     myers_ordered_kernel(const __grid_constant__ MyersJob job) {
@@ -416,19 +418,18 @@ __global__ void __launch_bounds__(MY_BLOCK)
 
 // A thread a pair, in the batch's order.
 template <int NW, bool GLOB>
-__global__ void __launch_bounds__(MY_SMALL) myers_kernel(const __grid_constant__ MyersJob job) {
+__global__ void __launch_bounds__(MY_BLOCK) myers_kernel(const __grid_constant__ MyersJob job) {
     extern __shared__ uint32_t smem[];
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < job.n_pairs) myers_pair<NW, GLOB, MY_SMALL>(job, (uint32_t)k, smem);
+    if (k < job.n_pairs) myers_pair<NW, GLOB>(job, (uint32_t)k, smem);
 }
 
 template <int NW, bool GLOB>
 static void launch_limbs(const MyersJob &job, bool ordered, cudaStream_t st) {
-    const int block = ordered ? MY_BLOCK : MY_SMALL;
-    const size_t smem = (size_t)4 * NW * block * sizeof(uint32_t);
-    const unsigned grid = (unsigned)((job.n_pairs + block - 1) / block);
-    if (ordered) myers_ordered_kernel<NW, GLOB><<<grid, block, smem, st>>>(job);
-    else myers_kernel<NW, GLOB><<<grid, block, smem, st>>>(job);
+    const size_t smem = (size_t)4 * NW * MY_BLOCK * sizeof(uint32_t);
+    const unsigned grid = (unsigned)((job.n_pairs + MY_BLOCK - 1) / MY_BLOCK);
+    if (ordered) myers_ordered_kernel<NW, GLOB><<<grid, MY_BLOCK, smem, st>>>(job);
+    else myers_kernel<NW, GLOB><<<grid, MY_BLOCK, smem, st>>>(job);
 }
 
 cudaError_t launch_myers(const MyersJob &job, int nw, int num_sms, cudaStream_t st) {
