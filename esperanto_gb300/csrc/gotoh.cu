@@ -890,13 +890,16 @@ __device__ __forceinline__ bool setup_pair(const GotohJob &job, const GotohConst
     }
     Geo g;
     bool full;
+    // an offset past either end of the longest sequences puts every row's
+    // centre on column 1 or n, however far past: sums with it stay in 32 bits
+    const int offset = min(max(P.band_offset, -65536), 65536);
     if (job.mode == 0) {
         full = P.band_half < 0;
-        g.off = full ? 0 : P.band_offset;
+        g.off = full ? 0 : offset;
         g.half = full ? n : P.band_half;
     } else if (job.mode == 1) {
         full = 30 >= n;  // INITIAL_BAND >= window: full matrix, accepted directly
-        g.off = full ? 0 : P.band_offset;
+        g.off = full ? 0 : offset;
         g.half = full ? n : 30;
     } else {
         full = true;
