@@ -83,6 +83,35 @@ static bool mixed_by_size(esp_handle *h, int mode, uint64_t n) {
     return h->hint_variant < 0 && h->variant_by_size;
 }
 
+// Resident blocks per SM of the kernels, queried once per handle.
+static int mixed_blocks(esp_handle *h) {
+    if (h->mixed_bps == 0) h->mixed_bps = esp::gotoh_mixed_blocks_per_sm();
+    return h->mixed_bps;
+}
+
+static int gotoh_blocks(esp_handle *h, int v) {
+    if (h->gotoh_bps[v] == 0) h->gotoh_bps[v] = esp::gotoh_blocks_per_sm(128, v);
+    return h->gotoh_bps[v];
+}
+
+static long warp_max(esp_handle *h) {
+    if (h->warp_max < 0) {
+        const char *v = getenv("ESP_WARP_MAX");
+        h->warp_max = v ? atol(v) : 2048;
+    }
+    return h->warp_max;
+}
+
+// Reads and queries all that plan_dp keeps in the handle, whatever the sizes to
+// come: later plans on it only read, so several threads may ask for them.
+void settle_kernel_choices(esp_handle *h) {
+    warp_max(h);
+    resolve_variant(h);
+    hint_variant(h, 1);
+    mixed_blocks(h);
+    for (int v = 0; v < esp::kGotohVariants; v++) gotoh_blocks(h, v);
+}
+
 // How one batch of n_pairs uses DP scratch: which kernel runs, with how
 // many warps, and the traceback / row-buffer bytes they need (the choices
 // enqueue_batch makes; the serve loop charges launches with it).
@@ -105,13 +134,9 @@ struct DpPlan {
 static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L1,
                       const Limits &L2) {
     DpPlan P;
-    if (h->warp_max < 0) {
-        const char *v = getenv("ESP_WARP_MAX");
-        h->warp_max = v ? atol(v) : 2048;
-    }
     P.tbw = std::max(L1.tb_words, mode == ESP_MODE_HINT ? L2.tb_words : 0);
     P.rbw = std::max(L1.rb_words, mode == ESP_MODE_HINT ? L2.rb_words : 0);
-    if (n_pairs <= (uint64_t)h->warp_max) {
+    if (n_pairs <= (uint64_t)warp_max(h)) {
         // Few pairs: one warp per pair (the wavefront kernel), so a lone
         // pair is not latency-bound on a single thread.
         P.warp_kernel = true;
@@ -123,8 +148,7 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
         return P;
     }
     if (mixed_by_size(h, mode, n_pairs)) {
-        if (!h->mixed_bps) h->mixed_bps = esp::gotoh_mixed_blocks_per_sm();
-        const uint64_t resident = (uint64_t)h->num_sms * h->mixed_bps * 4;  // warps
+        const uint64_t resident = (uint64_t)h->num_sms * mixed_blocks(h) * 4;  // warps
         const uint64_t items = (n_pairs + 1) / 2;
         P.mixed = P.paired = true;
         P.threads = (float)(resident * 32);
@@ -185,8 +209,7 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
         if (P.per_class)
             for (int s = 0; s < esp::kLengthClasses; s++) used |= h->autotune_ms || h->tune[s] == v;
         if (!used) continue;
-        if (h->gotoh_bps[v] == 0) h->gotoh_bps[v] = esp::gotoh_blocks_per_sm(128, v);
-        max_bps = std::max(max_bps, h->gotoh_bps[v]);
+        max_bps = std::max(max_bps, gotoh_blocks(h, v));
         P.paired |= esp::gotoh_paired(v);
     }
     P.var = var;

@@ -248,6 +248,8 @@ struct esp_genome {
     std::vector<esp_n_interval> h_iv;  // host copy (serve-loop window clipping)
 };
 
+// Settles what plans keep in the handle, so that later sizing only reads it.
+void settle_kernel_choices(esp_handle *h);
 // Bytes of traceback and row-buffer scratch one enqueue_batch of n_pairs
 // uses on this handle (the kernel, warps and words it would choose; abi.cu).
 void dp_scratch_bytes(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L1,

@@ -368,14 +368,9 @@ int esp_server_create(esp_genome *g, const esp_extend_params *params,
         esp_server_destroy(s);
         return rc;
     }
-    // the slot handles' kernel choices are settled here, once, so that the
-    // scheduler's scratch sizing (slot 0's handle, from any thread) only
-    // reads them afterwards
-    for (Slot &sl : s->slots) {
-        uint64_t tb, rb;
-        launch_scratch(sl.h, c.max_reads, c.max_read_len, c.max_win_len, tb, rb);
-        launch_scratch(sl.h, 1, c.max_read_len, c.max_win_len, tb, rb);
-    }
+    // the scheduler's scratch sizing (slot 0's handle) runs on any thread
+    // beside launches on that handle: from here on both only read it
+    for (Slot &sl : s->slots) settle_kernel_choices(sl.h);
     esp_handle *h0 = s->slots[0].h;
     s->sched = serve::Scheduler(
         c.mem_budget_bytes, c.max_reads, kMinLaunch, [h0](uint64_t n, uint32_t m, uint32_t w) {
