@@ -7,9 +7,9 @@
 // and a request larger than max_batch runs over several.  Every launch is
 // charged the DP scratch it needs (traceback words dominate) from one shared
 // pool of the memory budget: when the pool cannot hold the launch, it is cut
-// to the longest prefix whose scratch fits the largest free block, and when
-// not even min_batch reads fit, the head request waits until a running
-// launch returns its scratch.
+// to a prefix whose scratch fits the largest free block, and when not even
+// min_batch reads fit, the head request waits until a running launch returns
+// its scratch.
 #pragma once
 
 #include <algorithm>
@@ -202,9 +202,14 @@ class Scheduler {
     const ScratchPool &pool() const { return pool_; }
 
   private:
-    // Cut L to the longest prefix whose scratch fits the largest free block
-    // and carve it; false when that prefix is shorter than min_batch reads
-    // (or than L itself, when L is shorter).
+    // Cut L to the prefix that a search by halving finds to fit the largest
+    // free block -- the longest one where need() rises with the reads -- and
+    // carve it; false when that prefix is shorter than min_batch reads (or than
+    // L itself, when L is shorter).  need() may fall where a larger launch runs
+    // another kernel or more lanes an item; then the cut may be shorter than it
+    // had to be.  As need(n) <= need(min_batch) for n below min_batch, it is
+    // never shorter than min_batch where that fits, so an admitted request
+    // alone on an idle pool always goes on.
     bool fit_prefix(Launch &L) {
         const uint64_t F = pool_.largest_free();
         uint64_t lo = 0, hi = L.n;
@@ -215,7 +220,7 @@ class Scheduler {
         }
         if (lo == 0 || lo < std::min(L.n, min_batch_)) return false;
         truncate(L, lo);
-        shape(L);  // a shorter prefix needs at most need(lo) <= F
+        shape(L);  // of smaller reads than L had: possibly more than F, then not carved
         return pool_.alloc(L.bytes, L.off);
     }
     void shape(Launch &L) const {
