@@ -65,11 +65,14 @@ struct GotohJob {
     uint32_t *wide_count;
     int wide;
     // mixed kernel: device {list entries run by groups, log2 of a group's
-    // lanes}, their queue, and the scratch of a warp
+    // lanes}, their queue, and the scratch of a warp: of the first
+    // thread_warps warps, which alone run pairs per thread, and of the others
     const uint32_t *group_plan;
     uint32_t *group_queue;
     uint64_t group_tb_words, group_rb_words;  // word pairs per lane / per group
-    uint64_t warp_tb_words, warp_rb_words;    // words per warp (both sections)
+    uint64_t thread_warps;
+    uint64_t warp_tb_words, warp_rb_words;    // words of a warp below thread_warps
+    uint64_t group_warp_tb, group_warp_rb;    // words of a later warp (groups only)
 };
 
 // Launch the persistent DP kernel with `warps` warps total.
@@ -99,11 +102,10 @@ cudaError_t launch_gotoh_warp(const GotohJob &job, const GotohConst &k, int warp
 
 // Mixed kernel over a padded binned list (job.list, job.list_count): the
 // entries before job.group_plan[0] run in groups of 4..32 lanes per two pairs,
-// the rest two pairs per thread.  Each warp owns warp_tb_words words of job.tb
-// and warp_rb_words of job.rb, each the larger of what its sections need: 64 *
-// group_tb_words (>= group_steps of the pairs) or 64 * tb_words; 2 *
-// group_rb_words (> the pairs' windows) per group or 64 * rb_words.  Same results
-// as launch_gotoh.
+// the rest two pairs per thread.  Each warp owns words of job.tb and job.rb: 64 *
+// group_tb_words (>= group_steps of the pairs) and 2 * group_rb_words (> the
+// pairs' windows) per group, and where it runs pairs per thread as well at least
+// 64 * tb_words and 64 * rb_words.  Same results as launch_gotoh.
 cudaError_t launch_gotoh_mixed(const GotohJob &job, const GotohConst &k, int warps,
                                cudaStream_t st);
 uint64_t group_steps(uint64_t m, uint64_t n, uint64_t sw, int lg);

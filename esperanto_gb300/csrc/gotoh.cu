@@ -2150,7 +2150,7 @@ __global__ void __launch_bounds__(PAIR_BLOCK, MINB) gotoh2_kernel(GotohJob job, 
 // thread the chip holds 155,648 pairs before it is full.  A group of G lanes
 // takes 1/G of that time and holds 1/G of the pairs, so small and middling
 // batches fill the chip; small groups waste fewer steps at a pair's ends,
-// large ones finish it sooner (group_lanes in abi.cu chooses).
+// large ones finish it sooner (plan_dp in abi.cu and bin_plan in bins.cu choose).
 //
 // Cells, keys and packing are the paired kernel's.  A row is computed only
 // inside its window by predicates: `act` has a bit per row whose window holds
@@ -2576,7 +2576,10 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
 // (job.group_plan: list entries, log2 of a group's lanes), the rest two pairs
 // per thread.  A thread's pair takes as long as it takes, so the items that
 // would outlast the rest of the batch are the ones given to groups, and the
-// others keep the paired kernel's higher throughput (bin_plan, bins.cu).
+// others keep the paired kernel's higher throughput (bin_plan, bins.cu).  Two
+// pairs a lane take several times a group's scratch, so only as many warps as
+// have work of that kind own that much (65,536 reads of at most 300 x 428: 6.2
+// GB, 10.1 with all warps the same).
 __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob job, GotohConst K) {
     static_assert(GROUP_BLOCK == PAIR_BLOCK, "one shared array serves both sections");
     __shared__ uint32_t s_lut[10];
@@ -2591,15 +2594,17 @@ __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob jo
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const uint64_t warp_slot = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t *tb = job.tb + warp_slot * job.warp_tb_words;
-    uint32_t *rb = job.rb + warp_slot * job.warp_rb_words;
+    const uint64_t before = min(warp_slot, job.thread_warps), later = warp_slot - before;
+    uint32_t *tb = job.tb + before * job.warp_tb_words + later * job.group_warp_tb;
+    uint32_t *rb = job.rb + before * job.warp_rb_words + later * job.group_warp_rb;
     const uint64_t split = job.group_plan[0];
     stagger((split << job.group_plan[1]) / 64 + (*job.list_count - split + 63) / 64, job.sms);
     group_section(job, K, s_lut, s_lut25, split / 2, (int)job.group_plan[1],
                   reinterpret_cast<uint2 *>(tb), reinterpret_cast<uint2 *>(rb), lane,
                   s_words + threadIdx.x, s_words + STRIP * GROUP_BLOCK + threadIdx.x);
-    paired_section(job, K, s_lut, s_lut25, split, *job.list_count, tb + 2 * lane, rb + 2 * lane, lane,
-                   s_words + threadIdx.x);
+    if (warp_slot < job.thread_warps)
+        paired_section(job, K, s_lut, s_lut25, split, *job.list_count, tb + 2 * lane, rb + 2 * lane,
+                       lane, s_words + threadIdx.x);
 }
 
 cudaError_t launch_gotoh_mixed(const GotohJob &job, const GotohConst &k, int warps,
