@@ -124,9 +124,8 @@ struct DpPlan {
     bool all_groups = false; // ... with every item in groups of at least 1 << min_lg lanes
     int min_lg = 2;
     uint64_t gtw = 0, grw = 0;    // its groups' word pairs per lane / per group
-    uint64_t gwt = 0, gwr = 0;    // words of a warp that runs groups only
-    uint64_t wtb = 0, wrb = 0;    // words of one that runs pairs per thread too
-    uint64_t thread_warps = 0;    // how many of those
+    uint64_t gwt = 0, gwr = 0;    // its words per warp for groups
+    uint64_t thread_slots = 0;    // warps that may run two pairs per thread
     float threads = 0;            // threads of its full grid
     uint64_t warps = 0;
     uint64_t tbw = 0, rbw = 0;  // words per thread (warp kernel: per warp)
@@ -169,28 +168,25 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
             }
             P.gwt = 64 * P.gtw;
             P.gwr = 2 * P.grw * (32u >> lg);
-            P.wtb = std::max(P.gwt, 64 * P.tbw);
-            P.wrb = std::max(P.gwr, 64 * P.rbw);
             const uint64_t groups = 32u >> lg;
             const uint64_t want = std::min(resident, P.all_groups ? (items + groups - 1) / groups : items);
-            const uint64_t per_thread = (P.wtb + P.wrb) * 4, per_group = (P.gwt + P.gwr) * 4;
+            const uint64_t per_thread = 256 * (P.tbw + P.rbw), per_group = (P.gwt + P.gwr) * 4;
             uint64_t left = h->scratch_budget;
             // an eighth for the pairs that a bin of odd size leaves alone
-            P.thread_warps = P.all_groups ? 0 : std::min(want, (items + items / 8 + 31) / 32);
-            if (P.thread_warps) {
-                P.thread_warps = std::min(P.thread_warps, std::max<uint64_t>(1, left / per_thread));
-                left -= std::min(left, P.thread_warps * per_thread);
+            P.thread_slots = P.all_groups ? 0 : std::min(want, (items + items / 8 + 31) / 32);
+            if (P.thread_slots) {
+                P.thread_slots = std::min(P.thread_slots, std::max<uint64_t>(1, left / (per_thread + per_group)));
+                left -= std::min(left, P.thread_slots * per_thread);
             }
-            P.warps = P.thread_warps + std::min(want - P.thread_warps, left / per_group);
-            // whole blocks, one at least: every launched warp owns its scratch
-            P.warps = (std::max<uint64_t>(P.warps, 1) + 3) / 4 * 4;
+            P.warps = std::min(want, std::max<uint64_t>(1, left / per_group));
+            P.warps = (P.warps + 3) / 4 * 4;  // whole blocks: every launched warp owns its scratch
             return P.warps >= want;
         };
         // more lanes an item need less scratch for as many items in flight
         int lg = P.min_lg;
         while (!size(lg) && P.all_groups && lg < 5) lg++;
-        P.tb_bytes = (P.thread_warps * P.wtb + (P.warps - P.thread_warps) * P.gwt) * 4;
-        P.rb_bytes = (P.thread_warps * P.wrb + (P.warps - P.thread_warps) * P.gwr) * 4;
+        P.tb_bytes = (P.warps * P.gwt + P.thread_slots * 64 * P.tbw) * 4;
+        P.rb_bytes = (P.warps * P.gwr + P.thread_slots * 64 * P.rbw) * 4;
         return P;
     }
     // scratch slots: one warp per 32 pairs up to the resident limit, bounded
@@ -368,9 +364,10 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
         j.group_queue = h->d_ctr + 32 + 2 * attempt;
         j.group_tb_words = P.gtw;
         j.group_rb_words = P.grw;
-        j.thread_warps = P.thread_warps;
-        j.warp_tb_words = P.wtb;
-        j.warp_rb_words = P.wrb;
+        j.thread_slots = P.thread_slots;
+        j.thread_slot = h->d_ctr + 48 + attempt;
+        j.thread_tb = h->d_tb + P.warps * P.gwt;
+        j.thread_rb = h->d_rb + P.warps * P.gwr;
         j.group_warp_tb = P.gwt;
         j.group_warp_rb = P.gwr;
         return esp::launch_gotoh_mixed(j, K, (int)warps, st);

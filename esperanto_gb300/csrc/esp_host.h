@@ -61,7 +61,7 @@ struct esp_handle {
     // [24..28], binned list length at [29], wide-list count at [30], binned
     // escalation list length at [31]; the mixed kernel's group queues at
     // [32..33] and [34..35] (second attempt), plans at [36..37] and [38..39],
-    // batch costs at [40..43] and [44..47]
+    // batch costs at [40..43] and [44..47], its slots given out at [48] and [49]
     uint32_t *d_ctr = nullptr;
     int tune[esp::kLengthClasses] = {-1, -1, -1, -1};  // DP variant per length class (autotuned)
     bool tuned = false;

@@ -65,14 +65,15 @@ struct GotohJob {
     uint32_t *wide_count;
     int wide;
     // mixed kernel: device {list entries run by groups, log2 of a group's
-    // lanes}, their queue, and the scratch of a warp: of the first
-    // thread_warps warps, which alone run pairs per thread, and of the others
+    // lanes}, the groups' queue, a warp's scratch for groups, and that for
+    // pairs per thread: thread_slots times 64 * tb_words and 64 * rb_words
+    // words, given out by a device count (zeroed)
     const uint32_t *group_plan;
-    uint32_t *group_queue;
+    uint32_t *group_queue, *thread_slot;
     uint64_t group_tb_words, group_rb_words;  // word pairs per lane / per group
-    uint64_t thread_warps;
-    uint64_t warp_tb_words, warp_rb_words;    // words of a warp below thread_warps
-    uint64_t group_warp_tb, group_warp_rb;    // words of a later warp (groups only)
+    uint64_t group_warp_tb, group_warp_rb;    // words per warp
+    uint64_t thread_slots;
+    uint32_t *thread_tb, *thread_rb;
 };
 
 // Launch the persistent DP kernel with `warps` warps total.
@@ -102,10 +103,9 @@ cudaError_t launch_gotoh_warp(const GotohJob &job, const GotohConst &k, int warp
 
 // Mixed kernel over a padded binned list (job.list, job.list_count): the
 // entries before job.group_plan[0] run in groups of 4..32 lanes per two pairs,
-// the rest two pairs per thread.  Each warp owns words of job.tb and job.rb: 64 *
-// group_tb_words (>= group_steps of the pairs) and 2 * group_rb_words (> the
-// pairs' windows) per group, and where it runs pairs per thread as well at least
-// 64 * tb_words and 64 * rb_words.  Same results as launch_gotoh.
+// the rest two pairs per thread.  A warp's
+// scratch for groups: 64 * group_tb_words (>= group_steps of the pairs) and 2 *
+// group_rb_words (> the pairs' windows) per group.  Same results as launch_gotoh.
 cudaError_t launch_gotoh_mixed(const GotohJob &job, const GotohConst &k, int warps,
                                cudaStream_t st);
 uint64_t group_steps(uint64_t m, uint64_t n, uint64_t sw, int lg);

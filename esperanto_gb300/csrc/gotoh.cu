@@ -2577,9 +2577,11 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
 // per thread.  A thread's pair takes as long as it takes, so the items that
 // would outlast the rest of the batch are the ones given to groups, and the
 // others keep the paired kernel's higher throughput (bin_plan, bins.cu).  Two
-// pairs a lane take several times a group's scratch, so only as many warps as
-// have work of that kind own that much (65,536 reads of at most 300 x 428: 6.2
-// GB, 10.1 with all warps the same).
+// pairs a lane take several times a group's scratch, so there is only as much of
+// that as chunks of such work (65,536 reads of at most 300 x 428: 7.5 GB, 10.1
+// with as much for every warp), for the warps that come to it first: kept for
+// certain warps, the chip waits for those (80,000 whole windows of 50 to 250
+// rows 2.73 ms, so 3.16).
 __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob job, GotohConst K) {
     static_assert(GROUP_BLOCK == PAIR_BLOCK, "one shared array serves both sections");
     __shared__ uint32_t s_lut[10];
@@ -2594,17 +2596,22 @@ __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob jo
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const uint64_t warp_slot = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t before = min(warp_slot, job.thread_warps), later = warp_slot - before;
-    uint32_t *tb = job.tb + before * job.warp_tb_words + later * job.group_warp_tb;
-    uint32_t *rb = job.rb + before * job.warp_rb_words + later * job.group_warp_rb;
+    const uint32_t total = *job.list_count;
     const uint64_t split = job.group_plan[0];
-    stagger((split << job.group_plan[1]) / 64 + (*job.list_count - split + 63) / 64, job.sms);
+    stagger((split << job.group_plan[1]) / 64 + (total - split + 63) / 64, job.sms);
     group_section(job, K, s_lut, s_lut25, split / 2, (int)job.group_plan[1],
-                  reinterpret_cast<uint2 *>(tb), reinterpret_cast<uint2 *>(rb), lane,
+                  reinterpret_cast<uint2 *>(job.tb + warp_slot * job.group_warp_tb),
+                  reinterpret_cast<uint2 *>(job.rb + warp_slot * job.group_warp_rb), lane,
                   s_words + threadIdx.x, s_words + STRIP * GROUP_BLOCK + threadIdx.x);
-    if (warp_slot < job.thread_warps)
-        paired_section(job, K, s_lut, s_lut25, split, *job.list_count, tb + 2 * lane, rb + 2 * lane,
-                       lane, s_words + threadIdx.x);
+    if (split >= total) return;
+    uint32_t slot = 0;
+    if (lane == 0) slot = atomicAdd(job.thread_slot, 1u);
+    slot = __shfl_sync(0xffffffffu, slot, 0);
+    if (slot < job.thread_slots)
+        paired_section(job, K, s_lut, s_lut25, split, total,
+                       job.thread_tb + (uint64_t)slot * 64 * job.tb_words + 2 * lane,
+                       job.thread_rb + (uint64_t)slot * 64 * job.rb_words + 2 * lane, lane,
+                       s_words + threadIdx.x);
 }
 
 cudaError_t launch_gotoh_mixed(const GotohJob &job, const GotohConst &k, int warps,

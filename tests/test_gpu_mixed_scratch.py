@@ -1,6 +1,6 @@
-"""The mixed kernel's scratch: warps that run pairs per thread own more of it
-than those that run groups only.  Batches that use both kinds, under budgets
-that leave one block, a few warps of either kind, or all; every record and
+"""The mixed kernel's scratch: a warp's own for groups, and slots for pairs per
+thread that warps take as they come.  Batches that use both, under budgets
+that leave one block, a few warps and slots, or all; every record and
 CIGAR equals that of the same pairs by the one-pair kernel."""
 import numpy as np
 import pytest
@@ -34,9 +34,9 @@ def test_budgets(budget, mode, monkeypatch):
 def test_scratch_of_a_middling_batch():
     """65,536 extend_hint pairs of 150 x 214: 1.04 MB a warp with two pairs a
     lane (19 strips x 214 columns x 64 words), 0.28 MB with groups of 4.  1,152
-    warps of the first kind (32 items a warp, an eighth more for lone pairs)
-    and the rest of the 2,432 resident ones: 1.6 GB; 2.5 GB if all were of the
-    first kind."""
+    slots of the first kind (32 items a warp, an eighth more for lone pairs)
+    and groups in all 2,432 resident warps: 1.9 GB; 2.5 GB if every warp had the
+    first."""
     arena, pairs = W.synth_gotoh(1, 65536, 0)
     buf = ExtendBuffer()
     free = torch.cuda.mem_get_info()[0]
