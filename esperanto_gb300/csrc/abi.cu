@@ -125,7 +125,9 @@ struct DpPlan {
     int min_lg = 2;
     uint64_t gtw = 0, grw = 0;    // its groups' word pairs per lane / per group
     uint64_t gwt = 0, gwr = 0;    // its words per warp for groups
-    uint64_t thread_slots = 0;    // warps that may run two pairs per thread
+    uint64_t wtb = 0, wrb = 0;    // ... for pairs per thread too
+    uint32_t thread_warps = 0;    // warps of a unit with the latter (0: all warps of the launch)
+    uint32_t max_warps = 0;       // warps of a unit
     float threads = 0;            // threads of its full grid
     uint64_t warps = 0;
     uint64_t tbw = 0, rbw = 0;  // words per thread (warp kernel: per warp)
@@ -168,25 +170,39 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
             }
             P.gwt = 64 * P.gtw;
             P.gwr = 2 * P.grw * (32u >> lg);
+            P.wtb = P.all_groups ? P.gwt : std::max(P.gwt, 64 * P.tbw);
+            P.wrb = P.all_groups ? P.gwr : std::max(P.gwr, 64 * P.rbw);
             const uint64_t groups = 32u >> lg;
             const uint64_t want = std::min(resident, P.all_groups ? (items + groups - 1) / groups : items);
-            const uint64_t per_thread = 256 * (P.tbw + P.rbw), per_group = (P.gwt + P.gwr) * 4;
-            uint64_t left = h->scratch_budget;
-            // an eighth for the pairs that a bin of odd size leaves alone
-            P.thread_slots = P.all_groups ? 0 : std::min(want, (items + items / 8 + 31) / 32);
-            if (P.thread_slots) {
-                P.thread_slots = std::min(P.thread_slots, std::max<uint64_t>(1, left / (per_thread + per_group)));
-                left -= std::min(left, P.thread_slots * per_thread);
-            }
-            P.warps = std::min(want, std::max<uint64_t>(1, left / per_group));
+            P.warps = std::min(want, std::max<uint64_t>(1, h->scratch_budget / ((P.wtb + P.wrb) * 4)));
             P.warps = (P.warps + 3) / 4 * 4;  // whole blocks: every launched warp owns its scratch
             return P.warps >= want;
         };
         // more lanes an item need less scratch for as many items in flight
         int lg = P.min_lg;
         while (!size(lg) && P.all_groups && lg < 5) lg++;
-        P.tb_bytes = (P.warps * P.gwt + P.thread_slots * 64 * P.tbw) * 4;
-        P.rb_bytes = (P.warps * P.gwr + P.thread_slots * 64 * P.rbw) * 4;
+        P.tb_bytes = P.warps * P.wtb * 4;
+        P.rb_bytes = P.warps * P.wrb * 4;
+        // Where that is more than the budget (of a serving launch: half of the
+        // pool, so that two overlap), only as many warps with the words for pairs
+        // per thread as have such work, 32 items each and an eighth more for the
+        // pairs that a bin of odd size leaves alone.  Not always: the others
+        // cannot take over such work (45,000 extend_hint pairs of 50 to 150 bases
+        // 1.14 ms, so 1.24; but 65,536 mixed pairs, whose 13 GB do not fit 8 GiB,
+        // 1.59 -> 1.42).
+        const uint64_t units = 4ull * h->num_sms, most = resident / units;
+        const uint64_t busy = std::min(most, ((items + items / 8) / 32 + units - 1) / units);
+        const uint64_t tb = units * (busy * P.wtb + (most - busy) * P.gwt) * 4;
+        const uint64_t rb = units * (busy * P.wrb + (most - busy) * P.gwr) * 4;
+        const uint64_t ample = h->scratch_external ? h->scratch_budget / 2 : h->scratch_budget;
+        if (!P.all_groups && busy < most && resident * (P.wtb + P.wrb) * 4 > ample &&
+            tb + rb <= h->scratch_budget) {
+            P.thread_warps = (uint32_t)busy;
+            P.max_warps = (uint32_t)most;
+            P.warps = resident;
+            P.tb_bytes = tb;
+            P.rb_bytes = rb;
+        }
         return P;
     }
     // scratch slots: one warp per 32 pairs up to the resident limit, bounded
@@ -351,7 +367,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
     if (mode == ESP_MODE_HINT &&
         (rc = grow_device(h, (void **)&h->d_esc, &h->d_esc_cap, n_pairs * sizeof(uint32_t))) != ESP_OK)
         return rc;
-    CK(h, cudaMemsetAsync(h->d_ctr, 0, 256, st));
+    CK(h, cudaMemsetAsync(h->d_ctr, 0, 4 * (esp::kCounters + (P.mixed ? 8 * h->num_sms : 0)), st));
     const uint32_t *order = nullptr;
     const uint32_t *list_len = nullptr;  // device word: length of a padded list
     auto plan_for = [&](int attempt) {
@@ -364,12 +380,14 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
         j.group_queue = h->d_ctr + 32 + 2 * attempt;
         j.group_tb_words = P.gtw;
         j.group_rb_words = P.grw;
-        j.thread_slots = P.thread_slots;
-        j.thread_slot = h->d_ctr + 48 + attempt;
-        j.thread_tb = h->d_tb + P.warps * P.gwt;
-        j.thread_rb = h->d_rb + P.warps * P.gwr;
-        j.group_warp_tb = P.gwt;
+        j.warp_tb_words = P.wtb;
+        j.warp_rb_words = P.wrb;
+        j.thread_warps = P.thread_warps;
+        j.max_warps = P.max_warps;
         j.group_warp_rb = P.gwr;
+        j.unit_tb_words = P.tb_bytes / (16 * h->num_sms);
+        j.unit_rb_words = P.rb_bytes / (16 * h->num_sms);
+        j.unit_warps = h->d_ctr + esp::kCounters + attempt * 4 * h->num_sms;
         return esp::launch_gotoh_mixed(j, K, (int)warps, st);
     };
     if (h->binning && n_pairs > 32) {
@@ -509,7 +527,8 @@ int esp_create(esp_handle **out, int device) {
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_ctr, 256);
+    if (e == cudaSuccess)
+        e = cudaMalloc((void **)&h->d_ctr, 4 * (esp::kCounters + 8 * (size_t)h->num_sms));
     if (e != cudaSuccess) {
         delete h;
         return ESP_ECUDA;

@@ -65,16 +65,20 @@ struct GotohJob {
     uint32_t *wide_count;
     int wide;
     // mixed kernel: device {list entries run by groups, log2 of a group's
-    // lanes}, the groups' queue, a warp's scratch for groups, and that for
-    // pairs per thread: thread_slots times 64 * tb_words and 64 * rb_words
-    // words, given out by a device count (zeroed)
+    // lanes}, the groups' queue, and a warp's scratch, which both sections use
     const uint32_t *group_plan;
-    uint32_t *group_queue, *thread_slot;
+    uint32_t *group_queue;
     uint64_t group_tb_words, group_rb_words;  // word pairs per lane / per group
-    uint64_t group_warp_tb, group_warp_rb;    // words per warp
-    uint64_t thread_slots;
-    uint32_t *thread_tb, *thread_rb;
+    uint64_t warp_tb_words, warp_rb_words;    // words per warp
+    // thread_warps > 0: scratch by units, the warps of one place of a block on
+    // one SM, unit_*_words each: warp_*_words for the first thread_warps of
+    // them, 64 * group_tb_words and group_warp_rb for the others up to max_warps
+    uint32_t thread_warps, max_warps;
+    uint64_t unit_tb_words, unit_rb_words, group_warp_rb;
+    uint32_t *unit_warps;  // 4 * sms device counts (zeroed)
 };
+
+constexpr int kCounters = 64;  // words of a handle's counters (esp_handle::d_ctr) before the units'
 
 // Launch the persistent DP kernel with `warps` warps total.
 // variant 0: one pair per thread, 3 resident 128-thread blocks per SM (168
@@ -103,9 +107,10 @@ cudaError_t launch_gotoh_warp(const GotohJob &job, const GotohConst &k, int warp
 
 // Mixed kernel over a padded binned list (job.list, job.list_count): the
 // entries before job.group_plan[0] run in groups of 4..32 lanes per two pairs,
-// the rest two pairs per thread.  A warp's
-// scratch for groups: 64 * group_tb_words (>= group_steps of the pairs) and 2 *
-// group_rb_words (> the pairs' windows) per group.  Same results as launch_gotoh.
+// the rest two pairs per thread.  A warp's scratch holds 64 * group_tb_words
+// words (>= group_steps of the pairs) and 2 * group_rb_words (> the pairs'
+// windows) per group, and where it runs pairs per thread 64 * tb_words and 64 *
+// rb_words.  Same results as launch_gotoh.
 cudaError_t launch_gotoh_mixed(const GotohJob &job, const GotohConst &k, int warps,
                                cudaStream_t st);
 uint64_t group_steps(uint64_t m, uint64_t n, uint64_t sw, int lg);

@@ -2484,6 +2484,16 @@ __device__ __noinline__ bool setup_group(const GotohJob &job, const GotohConst &
     return setup_pair(job, K, pi, ~0ull, ~0ull, write, S);
 }
 
+// Out of line as in the paired kernel: inlined, the walk shared registers with all
+// that the kernel keeps, and any change there moved extend_hint over 60,000 pairs
+// between 1.58 and 1.72 ms (so 1.47), over 45,000 of 50 to 150 bases between 1.14 and
+// 1.24 (1.11).
+__device__ __noinline__ void finish_group(const GotohJob &job, const GotohConst &K,
+                                          const int8_t *__restrict__ lut, uint32_t pi, PairSetup &S,
+                                          const FillResult &F, const GroupTb &tb) {
+    finish_pair(job, K, lut, pi, S, F, tb);
+}
+
 // Items 0 .. items - 1 of the (padded, binned) list in groups of 1 << lg
 // lanes; item k is positions 2k and 2k + 1.  A warp takes 32 >> lg items at a
 // time.  Scratch: the warp's traceback region (group_tb_words word pairs per
@@ -2565,7 +2575,7 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
                 const int gfirst = lane & ~(G - 1);
                 PairSetup &S = gl ? B : A;
                 const GroupTb view{reinterpret_cast<const uint32_t *>(tb) + gl, lg, gfirst, R, A.g.lo(1)};
-                finish_pair(job, K, lut, p[gl ? 1 : q], S, gl ? FB : FA, view);
+                finish_group(job, K, lut, p[gl ? 1 : q], S, gl ? FB : FA, view);
             }
             __syncwarp();
         }
@@ -2576,12 +2586,15 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
 // (job.group_plan: list entries, log2 of a group's lanes), the rest two pairs
 // per thread.  A thread's pair takes as long as it takes, so the items that
 // would outlast the rest of the batch are the ones given to groups, and the
-// others keep the paired kernel's higher throughput (bin_plan, bins.cu).  Two
-// pairs a lane take several times a group's scratch, so there is only as much of
-// that as chunks of such work (65,536 reads of at most 300 x 428: 7.5 GB, 10.1
-// with as much for every warp), for the warps that come to it first: kept for
-// certain warps, the chip waits for those (80,000 whole windows of 50 to 250
-// rows 2.73 ms, so 3.16).
+// others keep the paired kernel's higher throughput (bin_plan, bins.cu).
+//
+// Two pairs a lane take several times a group's scratch.  With job.thread_warps
+// set only that many of the warps an SM starts in one of a block's four places
+// own it, the first to come, and the others as much as groups take (65,536 reads
+// of at most 300 x 428: 6.4 GB, 10.1 with all warps the same).  Each SM uses its
+// own part of the scratch, for groups and for pairs per thread one after the other:
+// given out over the whole chip, or apart from the groups', the same work took up
+// to a tenth longer (80,000 extend_hint pairs of 50 to 300 bases 3.5 ms, apart 3.8).
 __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob job, GotohConst K) {
     static_assert(GROUP_BLOCK == PAIR_BLOCK, "one shared array serves both sections");
     __shared__ uint32_t s_lut[10];
@@ -2595,23 +2608,33 @@ __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob jo
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const uint64_t warp_slot = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t total = *job.list_count;
     const uint64_t split = job.group_plan[0];
     stagger((split << job.group_plan[1]) / 64 + (total - split + 63) / 64, job.sms);
+    uint64_t tb, rb;      // the warp's words
+    bool threads = true;  // it owns what pairs per thread take
+    if (job.thread_warps) {
+        uint32_t sm, k = 0;
+        asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+        const uint32_t unit = (sm % (uint32_t)job.sms) * 4 + (threadIdx.x >> 5);
+        if (lane == 0) k = atomicAdd(job.unit_warps + unit, 1u);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (k >= job.max_warps) return;  // more blocks here than the SM holds at a time
+        threads = k < job.thread_warps;
+        const uint64_t early = min(k, job.thread_warps), late = k - early;
+        tb = unit * job.unit_tb_words + early * job.warp_tb_words + late * 64 * job.group_tb_words;
+        rb = unit * job.unit_rb_words + early * job.warp_rb_words + late * job.group_warp_rb;
+    } else {
+        const uint64_t warp_slot = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+        tb = warp_slot * job.warp_tb_words;
+        rb = warp_slot * job.warp_rb_words;
+    }
     group_section(job, K, s_lut, s_lut25, split / 2, (int)job.group_plan[1],
-                  reinterpret_cast<uint2 *>(job.tb + warp_slot * job.group_warp_tb),
-                  reinterpret_cast<uint2 *>(job.rb + warp_slot * job.group_warp_rb), lane,
+                  reinterpret_cast<uint2 *>(job.tb + tb), reinterpret_cast<uint2 *>(job.rb + rb), lane,
                   s_words + threadIdx.x, s_words + STRIP * GROUP_BLOCK + threadIdx.x);
-    if (split >= total) return;
-    uint32_t slot = 0;
-    if (lane == 0) slot = atomicAdd(job.thread_slot, 1u);
-    slot = __shfl_sync(0xffffffffu, slot, 0);
-    if (slot < job.thread_slots)
-        paired_section(job, K, s_lut, s_lut25, split, total,
-                       job.thread_tb + (uint64_t)slot * 64 * job.tb_words + 2 * lane,
-                       job.thread_rb + (uint64_t)slot * 64 * job.rb_words + 2 * lane, lane,
-                       s_words + threadIdx.x);
+    if (threads)
+        paired_section(job, K, s_lut, s_lut25, split, total, job.tb + tb + 2 * lane,
+                       job.rb + rb + 2 * lane, lane, s_words + threadIdx.x);
 }
 
 cudaError_t launch_gotoh_mixed(const GotohJob &job, const GotohConst &k, int warps,

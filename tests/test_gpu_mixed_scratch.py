@@ -1,13 +1,14 @@
-"""The mixed kernel's scratch: a warp's own for groups, and slots for pairs per
-thread that warps take as they come.  Batches that use both, under budgets
-that leave one block, a few warps and slots, or all; every record and
+"""The mixed kernel's scratch: warps that run pairs per thread own more of it
+than those that run groups only.  Batches that use both kinds, under budgets
+that leave one block, a few warps, or all of either kind; every record and
 CIGAR equals that of the same pairs by the one-pair kernel."""
 import numpy as np
 import pytest
-import torch
 
 from esperanto_gb300 import batch as B
+from esperanto_gb300 import serve as SV
 from esperanto_gb300.extend import ExtendBuffer, ExtendParams
+from esperanto_gb300.split import Genome
 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -31,14 +32,20 @@ def test_budgets(budget, mode, monkeypatch):
     assert (got[0] == want[0]).all() and (got[1] == want[1]).all()
 
 
-def test_scratch_of_a_middling_batch():
-    """65,536 extend_hint pairs of 150 x 214: 1.04 MB a warp with two pairs a
-    lane (19 strips x 214 columns x 64 words), 0.28 MB with groups of 4.  1,152
-    slots of the first kind (32 items a warp, an eighth more for lone pairs)
-    and groups in all 2,432 resident warps: 1.9 GB; 2.5 GB if every warp had the
-    first."""
-    arena, pairs = W.synth_gotoh(1, 65536, 0)
-    buf = ExtendBuffer()
-    free = torch.cuda.mem_get_info()[0]
-    _run(pairs, arena, B.MODE_HINT, buf)
-    assert free - torch.cuda.mem_get_info()[0] < 2 << 30
+def test_serving_launch_takes_half_the_pool():
+    """65,536 reads of at most 300 bases in windows of 428: 4.2 MB a warp with
+    two pairs a lane (38 strips x 428 columns x 64 words), 10.1 GB if all 2,432
+    resident warps had that.  The 1,152 that have such work (32 items each, an
+    eighth more for lone pairs) are two of the four on every scheduler."""
+    garena, contigs = W.synth_genome(5, 2_000_000, 2)
+    g = Genome(garena, contigs)
+    arena, reads = W.synth_request(5, 3, garena, contigs, 65536)
+    reads = reads.copy()
+    reads["read_len"][0] = 300
+    reads["win_len"][0] = 428
+    srv = SV.Server(g, n_streams=1, max_reads=65536, mem_budget=16 << 30)
+    t = srv.submit(arena, reads)
+    assert srv.wait(t)[0] == 0
+    st = srv.stats()
+    srv.destroy()
+    assert st["launches"] == 1 and st["pool_peak_bytes"] < 8 << 30, st
