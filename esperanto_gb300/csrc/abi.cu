@@ -112,6 +112,36 @@ void settle_kernel_choices(esp_handle *h) {
     for (int v = 0; v < esp::kGotohVariants; v++) gotoh_blocks(h, v);
 }
 
+// What the widest pairs of an attempt tell about groups for a batch of them alone:
+// lanes_lg: log2 of the lanes that have work.  The strips of a whole matrix run
+// one column behind each other, so all do; a strip of a band of w columns begins
+// 9 columns after the one above it and ends after w + 7, so that about (w + 8) / 9
+// do.  9,000 pairs of 150 in 65 columns 0.31 ms with 16 lanes, 0.22 with 8; of
+// 50 in 33 columns 0.156 with 16, 0.107 with 4; 30,000 whole windows of 64 rows
+// 0.39 with 4, 0.33 with 8.
+// single_line: up to how far above the mean finish (bin_plan) such pairs run
+// one per thread, which the lanes' empty ends at the first and the last strips
+// make the faster way.  In groups and one per thread, in ms: 6,500 pairs of 50 in 33
+// columns 0.109 / 0.098, 13,000 0.123 / 0.098; 13,000 of 100 in 129 0.32 / 0.37, 18,000
+// 0.40 / 0.37; 24,000 of 150 in 65 0.41 / 0.44, 30,000 0.49 / 0.44; 30,000 of 250 in
+// 129 1.26 / 1.22.  Whole windows stay with groups (36,000 of 64 rows 0.36 / 0.38).
+struct GroupShape {
+    int lanes_lg = 5;
+    float single_line = 0.0f;
+};
+
+static GroupShape group_shape(const Limits &L) {
+    GroupShape g;
+    const uint64_t strips = (L.max_m + 7ull) / 8;
+    const bool flat = L.rb_words >= L.max_n;  // rb_words: w + 7 for a band
+    const uint64_t busy = flat ? strips : std::min(strips, (L.rb_words + 1) / 9);
+    if (flat) g.lanes_lg = busy <= 4 ? 2 : (busy <= 8 ? 3 : (busy <= 16 ? 4 : 5));
+    else g.lanes_lg = busy < 6 ? 2 : (busy < 12 ? 3 : (busy < 23 ? 4 : 5));
+    if (strips <= 4) g.single_line = 1e9f;  // 9,000 pairs of 30 rows 0.088 / 0.078
+    else if (!flat) g.single_line = strips > 16 ? 1.75f : (g.lanes_lg == 2 ? 8.0f : 2.6f);
+    return g;
+}
+
 // How one batch of n_pairs uses DP scratch: which kernel runs, with how
 // many warps, and the traceback / row-buffer bytes they need (the choices
 // enqueue_batch makes; the serve loop charges launches with it).
@@ -121,13 +151,16 @@ struct DpPlan {
     bool per_class = false;  // one launch per length class of the binned list
     bool paired = false;     // a two-pairs-per-thread variant is among the launches
     bool mixed = false;      // the mixed kernel
-    bool all_groups = false; // ... with every item in groups of at least 1 << min_lg lanes
-    int min_lg = 2;
+    bool all_groups = false; // ... with every item in groups, unless all run per thread
+    int min_lg[2] = {2, 2};  // least log2 of a group's lanes, per attempt
+    GroupShape shape[2];
     uint64_t gtw = 0, grw = 0;    // its groups' word pairs per lane / per group
     uint64_t gwt = 0, gwr = 0;    // its words per warp for groups
     uint64_t wtb = 0, wrb = 0;    // ... for pairs per thread too
     uint32_t thread_warps = 0;    // warps of a unit with the latter (0: all warps of the launch)
     uint32_t max_warps = 0;       // warps of a unit
+    bool pairs_ok = false;        // some warps own words for pairs per thread
+    uint64_t single_warps = 0;    // warps of a launch of one pair per thread in its place, if planned
     float threads = 0;            // threads of its full grid
     uint64_t warps = 0;
     uint64_t tbw = 0, rbw = 0;  // words per thread (warp kernel: per warp)
@@ -156,30 +189,38 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
         P.mixed = P.paired = true;
         P.threads = (float)(resident * 32);
         // bin_plan's x for pairs of one cost, the least it can be: below its
-        // line all items are the costliest, and all go to groups
+        // line all items are the costliest, and all go to groups or run one per
+        // thread (scratch for two per thread from a little above that line on)
         const double x = P.threads * 0.305 / (0.4 * (double)items);
         P.all_groups = x * 0.4 > 1.1;
-        if (P.all_groups) P.min_lg = x < 5 ? 2 : (x < 11 ? 3 : (x < 60 ? 4 : 5));
-        auto size = [&](int lg) {
-            P.min_lg = lg;
+        const bool pairs_ok = x * 0.4 <= 1.25;
+        const int least = !P.all_groups || x < 5 ? 2 : (x < 11 ? 3 : (x < 60 ? 4 : 5));
+        uint64_t want = 0;
+        auto size = [&](int lg) {  // lg: a lower bound of the lanes
             P.gtw = P.grw = 0;
-            for (const Limits *L : {&L1, &L2}) {
-                if (L == &L2 && mode != ESP_MODE_HINT) continue;
-                P.gtw = std::max(P.gtw, esp::group_steps(L->max_m, L->max_n, L->rb_words, lg));
-                P.grw = std::max<uint64_t>(P.grw, L->max_n + 1ull);
+            uint32_t row_buffers = 0;  // of a warp
+            // (a launch that leaves schedulers idle may take more lanes an item)
+            want = std::min(P.all_groups ? resident / 4 : resident, items);
+            for (int a = 0; a < (mode == ESP_MODE_HINT ? 2 : 1); a++) {
+                const Limits &L = a ? L2 : L1;
+                P.shape[a] = group_shape(L);
+                P.min_lg[a] = std::max(lg, std::min(least, P.shape[a].lanes_lg));
+                const uint32_t groups = 32u >> P.min_lg[a];
+                P.gtw = std::max(P.gtw, esp::group_steps(L.max_m, L.max_n, L.rb_words, P.min_lg[a]));
+                P.grw = std::max<uint64_t>(P.grw, L.max_n + 1ull);
+                row_buffers = std::max(row_buffers, groups);
+                want = std::max(want, std::min(resident, (items + groups - 1) / groups));
             }
             P.gwt = 64 * P.gtw;
-            P.gwr = 2 * P.grw * (32u >> lg);
-            P.wtb = P.all_groups ? P.gwt : std::max(P.gwt, 64 * P.tbw);
-            P.wrb = P.all_groups ? P.gwr : std::max(P.gwr, 64 * P.rbw);
-            const uint64_t groups = 32u >> lg;
-            const uint64_t want = std::min(resident, P.all_groups ? (items + groups - 1) / groups : items);
+            P.gwr = 2 * P.grw * row_buffers;
+            P.wtb = pairs_ok ? std::max(P.gwt, 64 * P.tbw) : P.gwt;
+            P.wrb = pairs_ok ? std::max(P.gwr, 64 * P.rbw) : P.gwr;
             P.warps = std::min(want, std::max<uint64_t>(1, h->scratch_budget / ((P.wtb + P.wrb) * 4)));
             P.warps = (P.warps + 3) / 4 * 4;  // whole blocks: every launched warp owns its scratch
             return P.warps >= want;
         };
         // more lanes an item need less scratch for as many items in flight
-        int lg = P.min_lg;
+        int lg = 2;
         while (!size(lg) && P.all_groups && lg < 5) lg++;
         P.tb_bytes = P.warps * P.wtb * 4;
         P.rb_bytes = P.warps * P.wrb * 4;
@@ -195,7 +236,7 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
         const uint64_t tb = units * (busy * P.wtb + (most - busy) * P.gwt) * 4;
         const uint64_t rb = units * (busy * P.wrb + (most - busy) * P.gwr) * 4;
         const uint64_t ample = h->scratch_external ? h->scratch_budget / 2 : h->scratch_budget;
-        if (!P.all_groups && busy < most && resident * (P.wtb + P.wrb) * 4 > ample &&
+        if (pairs_ok && busy < most && want >= resident && resident * (P.wtb + P.wrb) * 4 > ample &&
             tb + rb <= h->scratch_budget) {
             P.thread_warps = (uint32_t)busy;
             P.max_warps = (uint32_t)most;
@@ -203,6 +244,15 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
             P.tb_bytes = tb;
             P.rb_bytes = rb;
         }
+        P.pairs_ok = pairs_ok;
+        // a launch of one pair per thread for the plans that may ask for it,
+        // in the same scratch if that holds them all
+        bool may = false;
+        for (int a = 0; a < (mode == ESP_MODE_HINT ? 2 : 1); a++) may |= x * 0.4 <= P.shape[a].single_line;
+        const uint64_t singles = (n_pairs + 127) / 128 * 4;
+        if (may && 2 * n_pairs <= resident * 32 && singles * 128 * P.tbw <= P.tb_bytes &&
+            singles * 128 * P.rbw <= P.rb_bytes)
+            P.single_warps = singles;
         return P;
     }
     // scratch slots: one warp per 32 pairs up to the resident limit, bounded
@@ -371,12 +421,22 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
     const uint32_t *order = nullptr;
     const uint32_t *list_len = nullptr;  // device word: length of a padded list
     auto plan_for = [&](int attempt) {
-        return esp::BinPlan{h->d_ctr + 40 + 4 * attempt, h->d_ctr + 36 + 2 * attempt, P.min_lg,
-                            P.all_groups, P.threads};
+        return esp::BinPlan{h->d_ctr + 40 + 4 * attempt, h->d_ctr + 48 + 4 * attempt,
+                            P.min_lg[attempt], P.shape[attempt].lanes_lg, P.all_groups, P.pairs_ok,
+                            P.single_warps ? P.shape[attempt].single_line : 0.0f, P.threads};
     };
     auto launch_dp = [&](esp::GotohJob &j, int attempt) {
         if (!P.mixed) return esp::launch_gotoh(j, K, (int)warps, 128, st, var);
-        j.group_plan = h->d_ctr + 36 + 2 * attempt;
+        if (P.single_warps) {  // by the plan, one of the two launches finds work
+            esp::GotohJob one = j;
+            one.list_count = h->d_ctr + 51 + 4 * attempt;
+            one.queue = h->d_ctr + 8 + 2 * attempt;
+            const cudaError_t e = esp::launch_gotoh(one, K, (int)P.single_warps, 128, st, 1);
+            if (e != cudaSuccess) return e;
+            h->launches++;
+        }
+        j.list_count = h->d_ctr + 50 + 4 * attempt;
+        j.group_plan = h->d_ctr + 48 + 4 * attempt;
         j.group_queue = h->d_ctr + 32 + 2 * attempt;
         j.group_tb_words = P.gtw;
         j.group_rb_words = P.grw;

@@ -270,40 +270,70 @@ __global__ void class_bounds(const uint32_t *__restrict__ hist, const uint32_t *
     }
 }
 
-// The mixed kernel's plan from the batch's costs (in cells; an item is two
-// pairs): {list entries its groups run, log2 of a group's lanes}.
+// First list position of bin b, after the scatter: the end of the bin before,
+// rounded up to even.
+__device__ __forceinline__ uint32_t bin_start(const uint32_t *__restrict__ cursor, uint32_t b) {
+    const uint32_t end = b ? cursor[b - 1] : 0u;
+    return end + (end & 1u);
+}
+
+// The plan of a batch that the mixed kernel may run, from the batch's costs (in
+// cells; an item is two pairs): {list entries its groups run, log2 of a group's
+// lanes, its list's length, the list's length for one pair per thread} -- one of the
+// two lengths is 0.
 //
 // A thread takes ~25 ns a row of 8 x 2 cells when its warp has the scheduler
 // to itself (52 cycles, measured), the full chip 1.9 T cells/s: an item
 // finishes with the rest of the batch when its cost is the mean cost times
 // items / 23,700 (0.305 x the 77,824 resident threads).  Batches whose costliest
 // item takes more than 1.1 times that give the items above half of it to
-// groups: 45,000 pairs of 150 x 214 (1.05 of it) take 0.56 ms by threads and 0.75
-// in groups of 4; 65,536 mixed pairs (3.3 times it) 2.98 ms by threads, 1.43 split.
-// A line at 1.5 or 2 costs 200,000 mixed pairs 4.0 ms, not 2.76.
-// Lanes of a group from how far the costliest item is above it (the fastest of
-// 4, 8, 16 and 32 lanes at 4,096 to 200,000 pairs of one shape and mixed).
-__global__ void bin_plan(const uint32_t *__restrict__ hist, const uint32_t *__restrict__ total,
-                         const BinStats *__restrict__ stats, int mode, int min_lg, bool all,
-                         float threads, uint32_t *__restrict__ plan) {
+// groups: 65,536 mixed pairs (3.3 times it) 2.98 ms by threads, 1.43 split; a line
+// at 1.5 or 2 costs 200,000 mixed pairs 4.0 ms, not 2.76.
+// Lanes of a group from how far the costliest item is above the mean finish
+// (the fastest of 4, 8, 16 and 32 lanes at 4,096 to 200,000 pairs of one shape
+// and mixed).  Where nearly all pairs are among the costliest, groups wait for
+// their empty lanes, not for the rest of the batch: then no more lanes than have
+// work, unless the batch leaves schedulers without a warp, and one pair per
+// thread where that is faster (group_shape, abi.cu), up to two warps a
+// scheduler; above that two per thread: 36,000 pairs of 100 in 129 columns 0.52 ms
+// one per thread, 0.61 two; 45,000 0.70 / 0.62; 45,000 of 100 to 150 in 65 0.64 in
+// groups, 0.49 two per thread.
+__global__ void bin_plan(const uint32_t *__restrict__ cursor, const uint32_t *__restrict__ total,
+                         const BinStats *__restrict__ stats, int mode, BinPlan b) {
     if (threadIdx.x != 0) return;
-    const float even = (float)stats->cost / (threads * 0.305f);  // of one pair of the item
+    const uint32_t n = *total;
+    const float even = (float)stats->cost / (b.threads * 0.305f);  // of one pair of the item
     const float top = 2.0f * (float)stats->max_cost;
-    const float x = even > 0.0f ? top / (0.4f * even) : 0.0f;
-    const int lg = x < 5.0f ? 2 : (x < 11.0f ? 3 : (x < 60.0f ? 4 : 5));
+    const float above = even > 0.0f ? top / even : 0.0f;
+    const float x = above / 0.4f;
+    int lg = x < 5.0f ? 2 : (x < 11.0f ? 3 : (x < 60.0f ? 4 : 5));
+    const bool alike = (float)stats->cost > 0.6f * (float)stats->max_cost * (float)n;
+    const bool filled = 2.0f * (float)n > b.threads;  // one per thread: over two warps a scheduler
     uint32_t split = 0;
-    if (all) {
-        split = *total;
-    } else if (top > 1.1f * even) {
+    if (alike && filled && b.pairs_ok) {
+        split = 0;
+    } else if (b.all) {
+        split = n;
+    } else if (above > 1.1f) {
         // items of w columns a row and more: the list's order.  extend_hint's
         // first attempt has one width, its list goes by window length.
         const uint32_t cap = (1u << KEY_BITS) - 1;
         const float w = 0.55f * even / (float)max(stats->max_m, 1u);
-        if (mode == 1) split = *total;
-        else split = w < 1.0f ? *total : hist[NBINS - 1 - ((min((uint32_t)w, cap - 1u) << KEY_BITS) | cap)];
+        if (mode == 1) split = n;
+        else split = w < 1.0f ? n : bin_start(cursor, NBINS - 1 - ((min((uint32_t)w, cap - 1u) << KEY_BITS) | cap));
     }
-    plan[0] = split;
-    plan[1] = (uint32_t)max(lg, min_lg);
+    if (alike) {
+        // lanes that give each scheduler one warp: threads / 128 warps, 64 / lanes
+        // entries a warp
+        int idle = 2;
+        while (idle < 5 && (float)n * (float)(4 << idle) <= b.threads) idle++;
+        lg = min(lg, max(b.lanes_lg, idle));
+    }
+    const bool single = alike && !filled && above <= b.single_line;
+    b.plan[0] = single ? 0u : split;
+    b.plan[1] = (uint32_t)max(lg, b.min_lg);
+    b.plan[2] = single ? 0u : n;
+    b.plan[3] = single ? n : 0u;
 }
 
 cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t *hist,
@@ -326,10 +356,8 @@ cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t
     if (pad) bin_scan_down<true><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     else bin_scan_down<false><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     if (bounds) class_bounds<<<1, 32, 0, st>>>(hist, total, bounds);
-    if (plan)
-        bin_plan<<<1, 32, 0, st>>>(hist, total, stats, mode, plan->min_lg, plan->all, plan->threads,
-                                   plan->plan);
     bin_scatter<<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, order);
+    if (plan) bin_plan<<<1, 32, 0, st>>>(hist, total, stats, mode, *plan);
     return cudaGetLastError();
 }
 

@@ -194,9 +194,12 @@ cudaError_t launch_count_cells(const esp_pair *pairs, const esp_extension *out, 
 // more).
 struct BinPlan {
     uint32_t *stats;  // 4 zeroed device words, 8-byte aligned
-    uint32_t *plan;   // 2 device words: GotohJob::group_plan
-    int min_lg;       // fewest lanes (log2) the scratch was sized for
-    bool all;         // the whole list goes to groups
+    uint32_t *plan;   // 4 device words: GotohJob::group_plan and the two lists' lengths
+    int min_lg;         // fewest lanes (log2) the scratch was sized for
+    int lanes_lg;       // lanes (log2) that have work in pairs like the costliest
+    bool all;           // groups take the whole list or nothing
+    bool pairs_ok;      // there is scratch for two pairs per thread
+    float single_line;  // batches of like pairs run one per thread up to this (0: never)
     float threads;    // resident threads of the launch's full grid
 };
 cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t *hist,
