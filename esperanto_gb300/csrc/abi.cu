@@ -245,13 +245,14 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
             P.rb_bytes = rb;
         }
         P.pairs_ok = pairs_ok;
-        // a launch of one pair per thread for the plans that may ask for it,
-        // in the same scratch if that holds them all
-        bool may = false;
+        // a launch of one pair per thread for the plans that may ask for it (the
+        // pairs' shape or their offsets, bin_plan), in the same scratch if that
+        // holds enough of them
+        bool may = x * 0.4 <= 3.1;
         for (int a = 0; a < (mode == ESP_MODE_HINT ? 2 : 1); a++) may |= x * 0.4 <= P.shape[a].single_line;
-        const uint64_t singles = (n_pairs + 127) / 128 * 4;
-        if (may && 2 * n_pairs <= resident * 32 && singles * 128 * P.tbw <= P.tb_bytes &&
-            singles * 128 * P.rbw <= P.rb_bytes)
+        const uint64_t singles =
+            std::min<uint64_t>((n_pairs + 127) / 128 * 4, (uint64_t)h->num_sms * gotoh_blocks(h, 1) * 4);
+        if (may && singles * 128 * P.tbw <= P.tb_bytes && singles * 128 * P.rbw <= P.rb_bytes)
             P.single_warps = singles;
         return P;
     }
@@ -293,6 +294,11 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
     P.warps = (warps + 3) / 4 * 4;  // whole 128-thread blocks: every launched warp owns a slot
     P.tb_bytes = P.warps * slot_pairs * P.tbw * 32 * 4;
     P.rb_bytes = P.warps * slot_pairs * P.rbw * 32 * 4;
+    // the size chose the paired kernel: pairs of unlike geometry take the
+    // one-pair kernel instead (bin_plan)
+    const bool by_size = mode == ESP_MODE_HINT ? h->hint_variant < 0 : h->variant_by_size && !h->tuned;
+    if (P.paired && !P.per_class && by_size)
+        P.single_warps = std::min<uint64_t>({2 * P.warps, need_warps, (uint64_t)h->num_sms * gotoh_blocks(h, 1) * 4}) / 4 * 4;
     return P;
 }
 
@@ -421,12 +427,12 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
     const uint32_t *order = nullptr;
     const uint32_t *list_len = nullptr;  // device word: length of a padded list
     auto plan_for = [&](int attempt) {
-        return esp::BinPlan{h->d_ctr + 40 + 4 * attempt, h->d_ctr + 48 + 4 * attempt,
-                            P.min_lg[attempt], P.shape[attempt].lanes_lg, P.all_groups, P.pairs_ok,
-                            P.single_warps ? P.shape[attempt].single_line : 0.0f, P.threads};
+        return esp::BinPlan{P.mixed ? h->d_ctr + 40 + 4 * attempt : nullptr, h->d_ctr + 48 + 4 * attempt,
+                            h->d_ctr + 36 + attempt, P.single_warps != 0, P.min_lg[attempt],
+                            P.shape[attempt].lanes_lg, P.all_groups, P.pairs_ok,
+                            P.shape[attempt].single_line, P.threads};
     };
     auto launch_dp = [&](esp::GotohJob &j, int attempt) {
-        if (!P.mixed) return esp::launch_gotoh(j, K, (int)warps, 128, st, var);
         if (P.single_warps) {  // by the plan, one of the two launches finds work
             esp::GotohJob one = j;
             one.list_count = h->d_ctr + 51 + 4 * attempt;
@@ -435,7 +441,8 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
             if (e != cudaSuccess) return e;
             h->launches++;
         }
-        j.list_count = h->d_ctr + 50 + 4 * attempt;
+        if (P.mixed || P.single_warps) j.list_count = h->d_ctr + 50 + 4 * attempt;
+        if (!P.mixed) return esp::launch_gotoh(j, K, (int)warps, 128, st, var);
         j.group_plan = h->d_ctr + 48 + 4 * attempt;
         j.group_queue = h->d_ctr + 32 + 2 * attempt;
         j.group_tb_words = P.gtw;
@@ -461,8 +468,8 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
         CK(h, esp::launch_binning(d_pairs, n_pairs, mode == ESP_MODE_HINT ? 1 : 0, h->d_hist,
                                   h->d_order, h->num_sms, st, h->d_ctr + 29,
                                   per_class ? h->d_ctr + 24 : nullptr, paired, nullptr, nullptr,
-                                  P.mixed ? &bp : nullptr));
-        h->launches += 5 + (per_class || P.mixed ? 1 : 0);  // kernels; the memsets are not counted
+                                  P.mixed || P.single_warps ? &bp : nullptr));
+        h->launches += 5 + (per_class || P.mixed || P.single_warps ? 1 : 0);  // kernels; the memsets are not counted
         order = h->d_order;
         if (paired) list_len = h->d_ctr + 29;
     }
@@ -548,8 +555,8 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
             const esp::BinPlan bp = plan_for(1);
             CK(h, esp::launch_binning(d_pairs, n_pairs, 2, h->d_hist, h->d_order, h->num_sms, st,
                                       h->d_ctr + 31, nullptr, paired, h->d_esc, h->d_ctr + 4,
-                                      P.mixed ? &bp : nullptr));
-            h->launches += 5 + (P.mixed ? 1 : 0);
+                                      P.mixed || P.single_warps ? &bp : nullptr));
+            h->launches += 5 + (P.mixed || P.single_warps ? 1 : 0);
             j2.list = h->d_order;
             j2.list_count = paired ? h->d_ctr + 31 : h->d_ctr + 4;
         }

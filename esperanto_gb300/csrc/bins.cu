@@ -192,17 +192,47 @@ __global__ void __launch_bounds__(256) bin_scan_down(uint32_t *__restrict__ hist
     tile[threadIdx.x] = r;
 }
 
+// Whether two pairs have one band geometry, as two pairs of an item must to share
+// its cells (process_item2 and group_section, gotoh.cu).
+__device__ __forceinline__ bool same_band(const esp_pair &a, const esp_pair &b, int mode) {
+    if (a.read_len != b.read_len || a.win_len != b.win_len) return false;
+    if (mode == 2) return true;
+    if (mode == 1) return a.win_len <= 30 || a.band_offset == b.band_offset;
+    if (a.band_half < 0 || b.band_half < 0) return a.band_half < 0 && b.band_half < 0;
+    return a.band_half == b.band_half && a.band_offset == b.band_offset;
+}
+
+// ITEMS: also counts the items, list positions 2k and 2k + 1 (the list pre-filled
+// with NO_PAIR), whose pairs do not have one geometry: an item's word takes each
+// of them in one atomic, and the second finds the first there.
+template <bool ITEMS>
 __global__ void bin_scatter(const esp_pair *__restrict__ pairs, uint64_t n, BinInput in, int mode,
-                            uint32_t *__restrict__ cursor, uint32_t *__restrict__ order) {
+                            uint32_t *__restrict__ cursor, uint32_t *__restrict__ order,
+                            uint32_t *__restrict__ unlike) {
     const uint64_t cnt = in.size(n);
+    uint32_t found = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t pi = in.at(i);
         if (pi >= n) continue;
-        uint32_t key = geometry_key(pairs[pi], mode);
+        const esp_pair P = pairs[pi];
         uint32_t slot;
-        agg_add(cursor, NBINS - 1 - key, &slot);
-        order[slot] = pi;
+        agg_add(cursor, NBINS - 1 - geometry_key(P, mode), &slot);
+        if (ITEMS) {
+            const unsigned long long none = 0xffffffffull;
+            const bool second = slot & 1u;
+            const unsigned long long old =
+                atomicAnd(reinterpret_cast<unsigned long long *>(order) + (slot >> 1),
+                          second ? ((unsigned long long)pi << 32) | none : (none << 32) | pi);
+            const uint32_t other = (uint32_t)(second ? old : old >> 32);
+            if (other != (uint32_t)none && !same_band(P, pairs[other], mode)) found++;
+        } else {
+            order[slot] = pi;
+        }
+    }
+    if (ITEMS) {
+        found = __reduce_add_sync(0xffffffffu, found);
+        if ((threadIdx.x & 31) == 0 && found) atomicAdd(unlike, found);
     }
 }
 
@@ -280,7 +310,7 @@ __device__ __forceinline__ uint32_t bin_start(const uint32_t *__restrict__ curso
 // The plan of a batch that the mixed kernel may run, from the batch's costs (in
 // cells; an item is two pairs): {list entries its groups run, log2 of a group's
 // lanes, its list's length, the list's length for one pair per thread} -- one of the
-// two lengths is 0.
+// two lengths is 0.  For the paired kernel (no stats) the two lengths alone.
 //
 // A thread takes ~25 ns a row of 8 x 2 cells when its warp has the scheduler
 // to itself (52 cycles, measured), the full chip 1.9 T cells/s: an item
@@ -298,10 +328,28 @@ __device__ __forceinline__ uint32_t bin_start(const uint32_t *__restrict__ curso
 // scheduler; above that two per thread: 36,000 pairs of 100 in 129 columns 0.52 ms
 // one per thread, 0.61 two; 45,000 0.70 / 0.62; 45,000 of 100 to 150 in 65 0.64 in
 // groups, 0.49 two per thread.
+//
+// Items whose two pairs differ in geometry (the bins know width and rows, not the
+// band's offset) take both kernels of pairs twice the time, and with them every
+// item of their warp.  So beyond one such item in UNLIKE the list goes to the
+// one-pair kernel, unless its costliest pair alone takes a thread as long as the
+// batch takes groups at half their rate (3.1 times the mean finish): 65,536 pairs of
+// 150 x 214 at offsets of 12 to 52 1.68 -> 0.77 ms, 200,000 mixed pairs 7.1 -> 4.8;
+// 4,096 mixed pairs stay with groups (0.83, one per thread 1.84), 65,536 too (3.5 /
+// 3.6).  In large batches one warp's second pass weighs less: 600,000 pairs of which
+// 0.5 % are at other offsets take 4.4 ms in pairs, 2 % 5.9, one per thread 5.2.
+constexpr uint32_t UNLIKE = 256, UNLIKE_LARGE = 48;
+
 __global__ void bin_plan(const uint32_t *__restrict__ cursor, const uint32_t *__restrict__ total,
                          const BinStats *__restrict__ stats, int mode, BinPlan b) {
     if (threadIdx.x != 0) return;
     const uint32_t n = *total;
+    if (!stats) {  // a list for the paired kernel
+        const bool single = (uint64_t)*b.unlike * UNLIKE_LARGE > n / 2;
+        b.plan[2] = single ? 0u : n;
+        b.plan[3] = single ? n : 0u;
+        return;
+    }
     const float even = (float)stats->cost / (b.threads * 0.305f);  // of one pair of the item
     const float top = 2.0f * (float)stats->max_cost;
     const float above = even > 0.0f ? top / even : 0.0f;
@@ -329,7 +377,8 @@ __global__ void bin_plan(const uint32_t *__restrict__ cursor, const uint32_t *__
         while (idle < 5 && (float)n * (float)(4 << idle) <= b.threads) idle++;
         lg = min(lg, max(b.lanes_lg, idle));
     }
-    const bool single = alike && !filled && above <= b.single_line;
+    const bool apart = (uint64_t)*b.unlike * UNLIKE > n / 2 && above <= 3.1f;
+    const bool single = b.single_ok && (apart || (alike && !filled && above <= b.single_line));
     b.plan[0] = single ? 0u : split;
     b.plan[1] = (uint32_t)max(lg, b.min_lg);
     b.plan[2] = single ? 0u : n;
@@ -348,7 +397,7 @@ cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t
     int grid = num_sms * 4;
     uint64_t need = (n + 255) / 256;
     if ((uint64_t)grid > need) grid = (int)(need ? need : 1);
-    BinStats *stats = plan ? reinterpret_cast<BinStats *>(plan->stats) : nullptr;
+    BinStats *stats = plan && plan->stats ? reinterpret_cast<BinStats *>(plan->stats) : nullptr;
     bin_hist<<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, stats);
     if (pad) bin_scan_up<true><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     else bin_scan_up<false><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
@@ -356,7 +405,10 @@ cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t
     if (pad) bin_scan_down<true><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     else bin_scan_down<false><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     if (bounds) class_bounds<<<1, 32, 0, st>>>(hist, total, bounds);
-    bin_scatter<<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, order);
+    if (plan)
+        bin_scatter<true><<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, order, plan->unlike);
+    else
+        bin_scatter<false><<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, order, nullptr);
     if (plan) bin_plan<<<1, 32, 0, st>>>(hist, total, stats, mode, *plan);
     return cudaGetLastError();
 }

@@ -190,17 +190,19 @@ cudaError_t launch_count_cells(const esp_pair *pairs, const esp_extension *out, 
 // mode: 0 band, 1 extend_hint's first attempt, 2 its full-matrix attempt.
 // list / list_count (device, optional): bin only the pairs list[0 ..
 // *list_count), n bounding the count (extend_hint's escalations).
-// plan (optional): also weigh the pairs and plan the mixed kernel (one launch
-// more).
+// plan (optional, with pad): also weigh the pairs and plan the mixed kernel, or
+// choose between the paired and the one-pair kernel (one launch more).
 struct BinPlan {
-    uint32_t *stats;  // 4 zeroed device words, 8-byte aligned
+    uint32_t *stats;  // 4 zeroed device words, 8-byte aligned (null: a list for the paired kernel)
     uint32_t *plan;   // 4 device words: GotohJob::group_plan and the two lists' lengths
+    uint32_t *unlike; // zeroed device word: items of two geometries
+    bool single_ok;   // the list may go to one pair per thread
     int min_lg;         // fewest lanes (log2) the scratch was sized for
     int lanes_lg;       // lanes (log2) that have work in pairs like the costliest
     bool all;           // groups take the whole list or nothing
     bool pairs_ok;      // there is scratch for two pairs per thread
-    float single_line;  // batches of like pairs run one per thread up to this (0: never)
-    float threads;    // resident threads of the launch's full grid
+    float single_line;  // batches of like pairs run one per thread up to this
+    float threads;      // resident threads of the launch's full grid
 };
 cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t *hist,
                            uint32_t *order, int num_sms, cudaStream_t st, uint32_t *total,

@@ -989,6 +989,7 @@ __device__ void process_pair(const GotohJob &job, const GotohConst &K,
 
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB) gotoh_kernel(GotohJob job, GotohConst K) {
+    if (job.list_count && *job.list_count == 0) return;  // the plan gave the list to another kernel
     __shared__ uint32_t s_lut[10];
     __shared__ int8_t s_lut25[32];
     if (threadIdx.x == 0) {  // static indices keep the parameter block out of local memory
