@@ -467,7 +467,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
         const esp::BinPlan bp = plan_for(0);
         CK(h, esp::launch_binning(d_pairs, n_pairs, mode == ESP_MODE_HINT ? 1 : 0, h->d_hist,
                                   h->d_order, h->num_sms, st, h->d_ctr + 29,
-                                  per_class ? h->d_ctr + 24 : nullptr, paired, nullptr, nullptr,
+                                  per_class ? h->d_ctr + 24 : nullptr, paired, h->d_ctr + 38, nullptr, nullptr,
                                   P.mixed || P.single_warps ? &bp : nullptr));
         h->launches += 5 + (per_class || P.mixed || P.single_warps ? 1 : 0);  // kernels; the memsets are not counted
         order = h->d_order;
@@ -476,6 +476,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
     esp::GotohJob job{};
     job.list = order;
     job.list_count = list_len;
+    job.window_n = order ? h->d_ctr + 38 : nullptr;
     job.pairs = d_pairs;
     job.n_pairs = n_pairs;
     job.arena = d_arena;
@@ -554,7 +555,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
         if (order) {
             const esp::BinPlan bp = plan_for(1);
             CK(h, esp::launch_binning(d_pairs, n_pairs, 2, h->d_hist, h->d_order, h->num_sms, st,
-                                      h->d_ctr + 31, nullptr, paired, h->d_esc, h->d_ctr + 4,
+                                      h->d_ctr + 31, nullptr, paired, h->d_ctr + 38, h->d_esc, h->d_ctr + 4,
                                       P.mixed || P.single_warps ? &bp : nullptr));
             h->launches += 5 + (P.mixed || P.single_warps ? 1 : 0);
             j2.list = h->d_order;

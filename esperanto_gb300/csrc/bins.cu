@@ -81,8 +81,10 @@ struct BinStats {
 };
 
 __global__ void bin_hist(const esp_pair *__restrict__ pairs, uint64_t n, BinInput in, int mode,
-                         uint32_t *__restrict__ hist, BinStats *__restrict__ stats) {
+                         uint32_t *__restrict__ hist, BinStats *__restrict__ stats,
+                         uint32_t *__restrict__ window_n) {
     const uint64_t cnt = in.size(n);
+    uint32_t with_n = 0;
     unsigned long long cost = 0;
     uint32_t max_cost = 0, max_m = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
@@ -91,6 +93,7 @@ __global__ void bin_hist(const esp_pair *__restrict__ pairs, uint64_t n, BinInpu
         if (pi >= n) continue;  // never index past the batch
         const esp_pair P = pairs[pi];
         agg_add(hist, NBINS - 1 - geometry_key(P, mode), nullptr);  // descending cost order
+        with_n |= P.n_win;
         if (stats) {
             const uint32_t c = cost_of(P, mode);
             cost += c;
@@ -98,6 +101,7 @@ __global__ void bin_hist(const esp_pair *__restrict__ pairs, uint64_t n, BinInpu
             max_m = max(max_m, P.read_len);
         }
     }
+    if (__any_sync(0xffffffffu, with_n != 0) && (threadIdx.x & 31) == 0) *window_n = 1u;
     if (stats) {
         for (int o = 16; o; o >>= 1) cost += __shfl_down_sync(0xffffffffu, cost, o);
         max_cost = __reduce_max_sync(0xffffffffu, max_cost);
@@ -387,7 +391,7 @@ __global__ void bin_plan(const uint32_t *__restrict__ cursor, const uint32_t *__
 
 cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t *hist,
                            uint32_t *order, int num_sms, cudaStream_t st, uint32_t *total,
-                           uint32_t *bounds, bool pad, const uint32_t *list,
+                           uint32_t *bounds, bool pad, uint32_t *window_n, const uint32_t *list,
                            const uint32_t *list_count, const BinPlan *plan) {
     const BinInput in{list, list_count};
     cudaError_t e = cudaMemsetAsync(hist, 0, bin_scratch_bytes(), st);
@@ -398,7 +402,7 @@ cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t
     uint64_t need = (n + 255) / 256;
     if ((uint64_t)grid > need) grid = (int)(need ? need : 1);
     BinStats *stats = plan && plan->stats ? reinterpret_cast<BinStats *>(plan->stats) : nullptr;
-    bin_hist<<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, stats);
+    bin_hist<<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, stats, window_n);
     if (pad) bin_scan_up<true><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     else bin_scan_up<false><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     bin_scan_top<<<1, 1024, 0, st>>>(hist + NBINS, total);

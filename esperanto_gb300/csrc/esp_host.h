@@ -56,15 +56,15 @@ struct esp_handle {
     size_t d_esc_cap = 0;       // bytes
     uint32_t *d_wide = nullptr; // pairs outside the int16 domain (the wide kernel's list)
     size_t d_wide_cap = 0;      // bytes
-    // d_ctr: u64 queues at [0..1] (attempt 1), [2..3] (attempt 2),
-    // u32 esc count at [4], u64 class queues (or those of one pair per
-    // thread in place of two, [8..9] and [10..11]) at [8..15], class bounds at
-    // [24..28], binned list length at [29], wide-list count at [30], binned
-    // escalation list length at [31]; the mixed kernel's group queues at
-    // [32..33] and [34..35] (second attempt), items of two geometries at [36]
-    // and [37], batch costs at [40..43] and
-    // [44..47], plans at [48..51] and [52..55], its units' counts from kCounters
-    // on, 4 * num_sms an attempt
+    // d_ctr: u64 queues at [0..1] (attempt 1), [2..3] (attempt 2), u32 esc count
+    // at [4], u64 class queues (or those of one pair per thread in place of
+    // two, [8..9] and [10..11]) at [8..15], class bounds at [24..28], binned
+    // list length at [29], wide-list count at [30], binned escalation list
+    // length at [31]; the mixed kernel's group queues at [32..33] and [34..35]
+    // (second attempt), items of two geometries at [36] and [37], whether a
+    // window holds N at [38], batch costs at [40..43] and [44..47], plans at
+    // [48..51] and [52..55], its units' counts from kCounters on, 4 * num_sms
+    // an attempt
     uint32_t *d_ctr = nullptr;
     int tune[esp::kLengthClasses] = {-1, -1, -1, -1};  // DP variant per length class (autotuned)
     bool tuned = false;

@@ -57,6 +57,7 @@ struct GotohJob {
     uint64_t rb_words;
     uint32_t *queue;            // device work counter (zeroed before launch)
     int sms;                    // SMs of the device (0: unknown)
+    const uint32_t *window_n;   // device: whether a window may hold N (null: by n_iv_count)
     // Pairs outside the int16 domain (read longer than GotohConst::max_m):
     // the int16 kernels append them to wide_list (count in *wide_count) and
     // leave them to the wide kernel, which sets `wide` and runs them in
@@ -204,9 +205,11 @@ struct BinPlan {
     float single_line;  // batches of like pairs run one per thread up to this
     float threads;      // resident threads of the launch's full grid
 };
+// window_n (a device word): set when a pair's window holds N.
 cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t *hist,
                            uint32_t *order, int num_sms, cudaStream_t st, uint32_t *total,
-                           uint32_t *bounds, bool pad, const uint32_t *list = nullptr,
+                           uint32_t *bounds, bool pad, uint32_t *window_n,
+                           const uint32_t *list = nullptr,
                            const uint32_t *list_count = nullptr, const BinPlan *plan = nullptr);
 // Spare slots a padded list may add to n pairs (the list holds n + this).
 uint64_t bin_pad_slots(uint64_t n);

@@ -2025,12 +2025,17 @@ __device__ __noinline__ bool setup_call(const GotohJob &job, const GotohConst &K
 // fills both halves, in the same pass over the lanes (lanes that took turns
 // doubled a warp's time), and a second pass takes the other pair of a
 // mismatched item.  N in a window costs one more instruction a row; a batch
-// that has N runs at all runs that fill for all its pairs, as the two fills do
+// that has a window with N runs that fill for all its pairs, as the two fills do
 // not fit the instruction cache together (1,000,003 mixed pairs, N in 0.5 % of
-// the windows: 12.3 ms with the fill chosen per warp, 10.1 so).  The
-// descriptors are resolved again for the finish rather than kept live across
-// the fill.
+// the windows: 12.3 ms with the fill chosen per warp, 9.9 so; N in reads alone, which
+// a row's score word takes care of, 7.8).  The descriptors are resolved again for
+// the finish rather than kept live across the fill.
 constexpr uint32_t NO_PAIR = 0xffffffffu;
+
+// Whether a window of the batch may hold N (counted with the bins).
+__device__ __forceinline__ bool windows_n(const GotohJob &job) {
+    return job.window_n ? *job.window_n != 0 : job.n_iv_count != 0;
+}
 
 __device__ void process_item2(const GotohJob &job, const GotohConst &K,
                               const uint32_t *__restrict__ s_lut, const int8_t *__restrict__ lut,
@@ -2060,7 +2065,7 @@ __device__ void process_item2(const GotohJob &job, const GotohConst &K,
                 }
             }
             if (now) {
-                if (job.n_iv_count) fill2_call<true>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
+                if (windows_n(job)) fill2_call<true>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
                 else fill2_call<false>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
             }
         }
@@ -2576,7 +2581,7 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
             if (need == 4 && fits) setup_group(job, K, p[1], false, B);
             const int all_steps = __reduce_max_sync(0xffffffffu, steps);
             FillResult FA, FB;
-            if (job.n_iv_count)  // as in process_item2
+            if (windows_n(job))  // as in process_item2
                 group_fill<true>(K, s_lut, A, B, nstrips, R, all_steps, tb, rb, lane, lg, first, track, FA,
                                   FB);
             else
