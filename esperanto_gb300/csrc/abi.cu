@@ -119,7 +119,7 @@ void settle_kernel_choices(esp_handle *h) {
 // do.  9,000 pairs of 150 in 65 columns 0.31 ms with 16 lanes, 0.22 with 8; of
 // 50 in 33 columns 0.156 with 16, 0.107 with 4; 30,000 whole windows of 64 rows
 // 0.39 with 4, 0.33 with 8.
-// single_line: up to how far above the mean finish (bin_plan) such pairs run
+// single_line: up to how far above the mean finish (make_plan) such pairs run
 // one per thread, which the lanes' empty ends at the first and the last strips
 // make the faster way.  In groups and one per thread, in ms: 6,500 pairs of 50 in 33
 // columns 0.109 / 0.098, 13,000 0.123 / 0.098; 13,000 of 100 in 129 0.32 / 0.37, 18,000
@@ -188,7 +188,7 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
         const uint64_t items = (n_pairs + 1) / 2;
         P.mixed = P.paired = true;
         P.threads = (float)(resident * 32);
-        // bin_plan's x for pairs of one cost, the least it can be: below its
+        // make_plan's x for pairs of one cost, the least it can be: below its
         // line all items are the costliest, and all go to groups or run one per
         // thread (scratch for two per thread from a little above that line on)
         const double x = P.threads * 0.305 / (0.4 * (double)items);
@@ -246,7 +246,7 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
         }
         P.pairs_ok = pairs_ok;
         // a launch of one pair per thread for the plans that may ask for it (the
-        // pairs' shape or their offsets, bin_plan), in the same scratch if that
+        // pairs' shape or their offsets, make_plan), in the same scratch if that
         // holds enough of them
         bool may = x * 0.4 <= 3.1;
         for (int a = 0; a < (mode == ESP_MODE_HINT ? 2 : 1); a++) may |= x * 0.4 <= P.shape[a].single_line;
@@ -295,7 +295,7 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
     P.tb_bytes = P.warps * slot_pairs * P.tbw * 32 * 4;
     P.rb_bytes = P.warps * slot_pairs * P.rbw * 32 * 4;
     // the size chose the paired kernel: pairs of unlike geometry take the
-    // one-pair kernel instead (bin_plan)
+    // one-pair kernel instead (make_plan)
     const bool by_size = mode == ESP_MODE_HINT ? h->hint_variant < 0 : h->variant_by_size && !h->tuned;
     if (P.paired && !P.per_class && by_size)
         P.single_warps = std::min<uint64_t>({2 * P.warps, need_warps, (uint64_t)h->num_sms * gotoh_blocks(h, 1) * 4}) / 4 * 4;
@@ -423,12 +423,12 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
     if (mode == ESP_MODE_HINT &&
         (rc = grow_device(h, (void **)&h->d_esc, &h->d_esc_cap, n_pairs * sizeof(uint32_t))) != ESP_OK)
         return rc;
-    CK(h, cudaMemsetAsync(h->d_ctr, 0, 4 * (esp::kCounters + (P.mixed ? 8 * h->num_sms : 0)), st));
+    CK(h, cudaMemsetAsync(h->d_ctr, 0, sizeof(uint32_t) * (esp::kCounters + (P.paired ? 4 * h->num_sms : 0)), st));
     const uint32_t *order = nullptr;
     const uint32_t *list_len = nullptr;  // device word: length of a padded list
     auto plan_for = [&](int attempt) {
         return esp::BinPlan{P.mixed ? h->d_ctr + 40 + 4 * attempt : nullptr, h->d_ctr + 48 + 4 * attempt,
-                            h->d_ctr + 36 + attempt, P.single_warps != 0, P.min_lg[attempt],
+                            h->d_ctr + 36 + attempt, h->d_ctr + 56 + attempt, P.single_warps != 0, P.min_lg[attempt],
                             P.shape[attempt].lanes_lg, P.all_groups, P.pairs_ok,
                             P.shape[attempt].single_line, P.threads};
     };
@@ -441,6 +441,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
             if (e != cudaSuccess) return e;
             h->launches++;
         }
+        j.sm_blocks = h->d_ctr + esp::kCounters + attempt * h->num_sms;
         if (P.mixed || P.single_warps) j.list_count = h->d_ctr + 50 + 4 * attempt;
         if (!P.mixed) return esp::launch_gotoh(j, K, (int)warps, 128, st, var);
         j.group_plan = h->d_ctr + 48 + 4 * attempt;
@@ -454,7 +455,6 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
         j.group_warp_rb = P.gwr;
         j.unit_tb_words = P.tb_bytes / (16 * h->num_sms);
         j.unit_rb_words = P.rb_bytes / (16 * h->num_sms);
-        j.unit_warps = h->d_ctr + esp::kCounters + attempt * 4 * h->num_sms;
         return esp::launch_gotoh_mixed(j, K, (int)warps, st);
     };
     if (h->binning && n_pairs > 32) {
@@ -469,7 +469,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
                                   h->d_order, h->num_sms, st, h->d_ctr + 29,
                                   per_class ? h->d_ctr + 24 : nullptr, paired, h->d_ctr + 38, nullptr, nullptr,
                                   P.mixed || P.single_warps ? &bp : nullptr));
-        h->launches += 5 + (per_class || P.mixed || P.single_warps ? 1 : 0);  // kernels; the memsets are not counted
+        h->launches += 5 + (per_class ? 1 : 0);  // kernels; the memsets are not counted
         order = h->d_order;
         if (paired) list_len = h->d_ctr + 29;
     }
@@ -494,6 +494,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
     job.rb_words = rbw;
     job.sms = h->num_sms;
     job.queue = h->d_ctr;
+    job.sm_blocks = h->d_ctr + esp::kCounters;
     job.esc_list = h->d_esc;
     job.esc_count = h->d_ctr + 4;
     job.mode = mode == ESP_MODE_HINT ? 1 : 0;
@@ -516,6 +517,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
                         js.queue = h->d_ctr + 8 + 2 * s;
                     }
                     CK(h, cudaMemsetAsync(js.queue, 0, 8, st));
+                    CK(h, cudaMemsetAsync(js.sm_blocks, 0, h->num_sms * sizeof(uint32_t), st));
                     // every timed run lists the wide pairs anew
                     CK(h, cudaMemsetAsync(h->d_ctr + 30, 0, 4, st));
                     CK(h, cudaEventRecord(ev[0], st));
@@ -535,6 +537,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
             esp::GotohJob js = job;
             js.range = h->d_ctr + 24 + s;
             js.queue = h->d_ctr + 8 + 2 * s;
+            js.sm_blocks += s * h->num_sms;
             CK(h, esp::launch_gotoh(js, K, (int)warps, 128, st, h->tune[s] >= 0 ? h->tune[s] : var));
             h->launches++;
         }
@@ -557,7 +560,7 @@ int enqueue_batch(esp_handle *h, int mode, const esp_pair *d_pairs, uint64_t n_p
             CK(h, esp::launch_binning(d_pairs, n_pairs, 2, h->d_hist, h->d_order, h->num_sms, st,
                                       h->d_ctr + 31, nullptr, paired, h->d_ctr + 38, h->d_esc, h->d_ctr + 4,
                                       P.mixed || P.single_warps ? &bp : nullptr));
-            h->launches += 5 + (P.mixed || P.single_warps ? 1 : 0);
+            h->launches += 5;
             j2.list = h->d_order;
             j2.list_count = paired ? h->d_ctr + 31 : h->d_ctr + 4;
         }
@@ -596,7 +599,7 @@ int esp_create(esp_handle **out, int device) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess)
-        e = cudaMalloc((void **)&h->d_ctr, 4 * (esp::kCounters + 8 * (size_t)h->num_sms));
+        e = cudaMalloc((void **)&h->d_ctr, sizeof(uint32_t) * (esp::kCounters + 4 * (size_t)h->num_sms));
     if (e != cudaSuccess) {
         delete h;
         return ESP_ECUDA;

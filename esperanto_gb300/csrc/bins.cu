@@ -196,6 +196,90 @@ __global__ void __launch_bounds__(256) bin_scan_down(uint32_t *__restrict__ hist
     tile[threadIdx.x] = r;
 }
 
+// First list position of bin b, after the scatter: the end of the bin before,
+// rounded up to even.
+__device__ __forceinline__ uint32_t bin_start(const uint32_t *cursor, uint32_t b) {
+    const uint32_t end = b ? __ldcg(cursor + b - 1) : 0u;
+    return end + (end & 1u);
+}
+
+// The plan of a batch that the mixed kernel may run, from the batch's costs (in
+// cells; an item is two pairs): {list entries its groups run, log2 of a group's
+// lanes, its list's length, the list's length for one pair per thread} -- one of the
+// two lengths is 0.  For the paired kernel (no stats) the two lengths alone.
+//
+// A thread takes ~25 ns a row of 8 x 2 cells when its warp has the scheduler
+// to itself (52 cycles, measured), the full chip 1.9 T cells/s: an item
+// finishes with the rest of the batch when its cost is the mean cost times
+// items / 23,700 (0.305 x the 77,824 resident threads).  Batches whose costliest
+// item takes more than 1.1 times that give the items above half of it to
+// groups: 65,536 mixed pairs (3.3 times it) 2.98 ms by threads, 1.43 split; a line
+// at 1.5 or 2 costs 200,000 mixed pairs 4.0 ms, not 2.76.
+// Lanes of a group from how far the costliest item is above the mean finish
+// (the fastest of 4, 8, 16 and 32 lanes at 4,096 to 200,000 pairs of one shape
+// and mixed).  Where nearly all pairs are among the costliest, groups wait for
+// their empty lanes, not for the rest of the batch: then no more lanes than have
+// work, unless the batch leaves schedulers without a warp, and one pair per
+// thread where that is faster (group_shape, abi.cu), up to two warps a
+// scheduler; above that two per thread: 36,000 pairs of 100 in 129 columns 0.52 ms
+// one per thread, 0.61 two; 45,000 0.70 / 0.62; 45,000 of 100 to 150 in 65 0.64 in
+// groups, 0.49 two per thread.
+//
+// Items whose two pairs differ in geometry (the bins know width and rows, not the
+// band's offset) take both kernels of pairs twice the time, and with them every
+// item of their warp.  So beyond one such item in UNLIKE the list goes to the
+// one-pair kernel, unless its costliest pair alone takes a thread as long as the
+// batch takes groups at half their rate (3.1 times the mean finish): 65,536 pairs of
+// 150 x 214 at offsets of 12 to 52 1.68 -> 0.77 ms, 200,000 mixed pairs 7.1 -> 4.8;
+// 4,096 mixed pairs stay with groups (0.83, one per thread 1.84; 65,536 3.5 /
+// 3.6, about even).  In large batches one warp's second pass weighs less: 600,000 pairs of which
+// 0.5 % are at other offsets take 4.4 ms in pairs, 2 % 5.9, one per thread 5.2.
+constexpr uint32_t UNLIKE = 256, UNLIKE_LARGE = 48, SAMPLE = 16;
+
+__device__ void make_plan(const uint32_t *cursor, uint32_t n, const BinStats *stats, int mode,
+                          const BinPlan &b) {
+    const uint32_t unlike = __ldcg(b.unlike);
+    if (!stats) {  // a list for the paired kernel
+        const bool single = (uint64_t)unlike * SAMPLE * UNLIKE_LARGE > n / 2;
+        b.plan[2] = single ? 0u : n;
+        b.plan[3] = single ? n : 0u;
+        return;
+    }
+    const float even = (float)stats->cost / (b.threads * 0.305f);  // of one pair of the item
+    const float top = 2.0f * (float)stats->max_cost;
+    const float above = even > 0.0f ? top / even : 0.0f;
+    const float x = above / 0.4f;
+    int lg = x < 5.0f ? 2 : (x < 11.0f ? 3 : (x < 60.0f ? 4 : 5));
+    const bool alike = (float)stats->cost > 0.6f * (float)stats->max_cost * (float)n;
+    const bool filled = 2.0f * (float)n > b.threads;  // one per thread: over two warps a scheduler
+    uint32_t split = 0;
+    if (alike && filled && b.pairs_ok) {
+        split = 0;
+    } else if (b.all) {
+        split = n;
+    } else if (above > 1.1f) {
+        // items of w columns a row and more: the list's order.  extend_hint's
+        // first attempt has one width, its list goes by window length.
+        const uint32_t cap = (1u << KEY_BITS) - 1;
+        const float w = 0.55f * even / (float)max(stats->max_m, 1u);
+        if (mode == 1) split = n;
+        else split = w < 1.0f ? n : bin_start(cursor, NBINS - 1 - ((min((uint32_t)w, cap - 1u) << KEY_BITS) | cap));
+    }
+    if (alike) {
+        // lanes that give each scheduler one warp: threads / 128 warps, 64 / lanes
+        // entries a warp
+        int idle = 2;
+        while (idle < 5 && (float)n * (float)(4 << idle) <= b.threads) idle++;
+        lg = min(lg, max(b.lanes_lg, idle));
+    }
+    const bool apart = (uint64_t)unlike * UNLIKE > n / 2 && above <= 3.1f;
+    const bool single = b.single_ok && (apart || (alike && !filled && above <= b.single_line));
+    b.plan[0] = single ? 0u : split;
+    b.plan[1] = (uint32_t)max(lg, b.min_lg);
+    b.plan[2] = single ? 0u : n;
+    b.plan[3] = single ? n : 0u;
+}
+
 // Whether two pairs have one band geometry, as two pairs of an item must to share
 // its cells (process_item2 and group_section, gotoh.cu).
 __device__ __forceinline__ bool same_band(const esp_pair &a, const esp_pair &b, int mode) {
@@ -206,13 +290,16 @@ __device__ __forceinline__ bool same_band(const esp_pair &a, const esp_pair &b, 
     return a.band_half == b.band_half && a.band_offset == b.band_offset;
 }
 
-// ITEMS: also counts the items, list positions 2k and 2k + 1 (the list pre-filled
+// PLAN: also counts the items, list positions 2k and 2k + 1 (the list pre-filled
 // with NO_PAIR), whose pairs do not have one geometry: an item's word takes each
-// of them in one atomic, and the second finds the first there.
-template <bool ITEMS>
+// of them in one atomic, and the second finds the first there.  Large lists, which
+// the paired kernel runs, count one item in SAMPLE (all of them: 4,194,304 mixed
+// pairs 0.3 % longer).  The last block to end makes the plan (a launch of its
+// own took 4 us).
+template <bool PLAN>
 __global__ void bin_scatter(const esp_pair *__restrict__ pairs, uint64_t n, BinInput in, int mode,
-                            uint32_t *__restrict__ cursor, uint32_t *__restrict__ order,
-                            uint32_t *__restrict__ unlike) {
+                            uint32_t *cursor, uint32_t *order, const uint32_t *total,
+                            const BinStats *stats, BinPlan plan) {
     const uint64_t cnt = in.size(n);
     uint32_t found = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
@@ -222,7 +309,7 @@ __global__ void bin_scatter(const esp_pair *__restrict__ pairs, uint64_t n, BinI
         const esp_pair P = pairs[pi];
         uint32_t slot;
         agg_add(cursor, NBINS - 1 - geometry_key(P, mode), &slot);
-        if (ITEMS) {
+        if (PLAN && (stats || (slot >> 1) % SAMPLE == 0)) {
             const unsigned long long none = 0xffffffffull;
             const bool second = slot & 1u;
             const unsigned long long old =
@@ -234,9 +321,15 @@ __global__ void bin_scatter(const esp_pair *__restrict__ pairs, uint64_t n, BinI
             order[slot] = pi;
         }
     }
-    if (ITEMS) {
+    if (PLAN) {
         found = __reduce_add_sync(0xffffffffu, found);
-        if ((threadIdx.x & 31) == 0 && found) atomicAdd(unlike, found);
+        if ((threadIdx.x & 31) == 0 && found) atomicAdd(plan.unlike, found);
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0 && atomicAdd(plan.done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            make_plan(cursor, *total, stats, mode, plan);
+        }
     }
 }
 
@@ -304,91 +397,6 @@ __global__ void class_bounds(const uint32_t *__restrict__ hist, const uint32_t *
     }
 }
 
-// First list position of bin b, after the scatter: the end of the bin before,
-// rounded up to even.
-__device__ __forceinline__ uint32_t bin_start(const uint32_t *__restrict__ cursor, uint32_t b) {
-    const uint32_t end = b ? cursor[b - 1] : 0u;
-    return end + (end & 1u);
-}
-
-// The plan of a batch that the mixed kernel may run, from the batch's costs (in
-// cells; an item is two pairs): {list entries its groups run, log2 of a group's
-// lanes, its list's length, the list's length for one pair per thread} -- one of the
-// two lengths is 0.  For the paired kernel (no stats) the two lengths alone.
-//
-// A thread takes ~25 ns a row of 8 x 2 cells when its warp has the scheduler
-// to itself (52 cycles, measured), the full chip 1.9 T cells/s: an item
-// finishes with the rest of the batch when its cost is the mean cost times
-// items / 23,700 (0.305 x the 77,824 resident threads).  Batches whose costliest
-// item takes more than 1.1 times that give the items above half of it to
-// groups: 65,536 mixed pairs (3.3 times it) 2.98 ms by threads, 1.43 split; a line
-// at 1.5 or 2 costs 200,000 mixed pairs 4.0 ms, not 2.76.
-// Lanes of a group from how far the costliest item is above the mean finish
-// (the fastest of 4, 8, 16 and 32 lanes at 4,096 to 200,000 pairs of one shape
-// and mixed).  Where nearly all pairs are among the costliest, groups wait for
-// their empty lanes, not for the rest of the batch: then no more lanes than have
-// work, unless the batch leaves schedulers without a warp, and one pair per
-// thread where that is faster (group_shape, abi.cu), up to two warps a
-// scheduler; above that two per thread: 36,000 pairs of 100 in 129 columns 0.52 ms
-// one per thread, 0.61 two; 45,000 0.70 / 0.62; 45,000 of 100 to 150 in 65 0.64 in
-// groups, 0.49 two per thread.
-//
-// Items whose two pairs differ in geometry (the bins know width and rows, not the
-// band's offset) take both kernels of pairs twice the time, and with them every
-// item of their warp.  So beyond one such item in UNLIKE the list goes to the
-// one-pair kernel, unless its costliest pair alone takes a thread as long as the
-// batch takes groups at half their rate (3.1 times the mean finish): 65,536 pairs of
-// 150 x 214 at offsets of 12 to 52 1.68 -> 0.77 ms, 200,000 mixed pairs 7.1 -> 4.8;
-// 4,096 mixed pairs stay with groups (0.83, one per thread 1.84), 65,536 too (3.5 /
-// 3.6).  In large batches one warp's second pass weighs less: 600,000 pairs of which
-// 0.5 % are at other offsets take 4.4 ms in pairs, 2 % 5.9, one per thread 5.2.
-constexpr uint32_t UNLIKE = 256, UNLIKE_LARGE = 48;
-
-__global__ void bin_plan(const uint32_t *__restrict__ cursor, const uint32_t *__restrict__ total,
-                         const BinStats *__restrict__ stats, int mode, BinPlan b) {
-    if (threadIdx.x != 0) return;
-    const uint32_t n = *total;
-    if (!stats) {  // a list for the paired kernel
-        const bool single = (uint64_t)*b.unlike * UNLIKE_LARGE > n / 2;
-        b.plan[2] = single ? 0u : n;
-        b.plan[3] = single ? n : 0u;
-        return;
-    }
-    const float even = (float)stats->cost / (b.threads * 0.305f);  // of one pair of the item
-    const float top = 2.0f * (float)stats->max_cost;
-    const float above = even > 0.0f ? top / even : 0.0f;
-    const float x = above / 0.4f;
-    int lg = x < 5.0f ? 2 : (x < 11.0f ? 3 : (x < 60.0f ? 4 : 5));
-    const bool alike = (float)stats->cost > 0.6f * (float)stats->max_cost * (float)n;
-    const bool filled = 2.0f * (float)n > b.threads;  // one per thread: over two warps a scheduler
-    uint32_t split = 0;
-    if (alike && filled && b.pairs_ok) {
-        split = 0;
-    } else if (b.all) {
-        split = n;
-    } else if (above > 1.1f) {
-        // items of w columns a row and more: the list's order.  extend_hint's
-        // first attempt has one width, its list goes by window length.
-        const uint32_t cap = (1u << KEY_BITS) - 1;
-        const float w = 0.55f * even / (float)max(stats->max_m, 1u);
-        if (mode == 1) split = n;
-        else split = w < 1.0f ? n : bin_start(cursor, NBINS - 1 - ((min((uint32_t)w, cap - 1u) << KEY_BITS) | cap));
-    }
-    if (alike) {
-        // lanes that give each scheduler one warp: threads / 128 warps, 64 / lanes
-        // entries a warp
-        int idle = 2;
-        while (idle < 5 && (float)n * (float)(4 << idle) <= b.threads) idle++;
-        lg = min(lg, max(b.lanes_lg, idle));
-    }
-    const bool apart = (uint64_t)*b.unlike * UNLIKE > n / 2 && above <= 3.1f;
-    const bool single = b.single_ok && (apart || (alike && !filled && above <= b.single_line));
-    b.plan[0] = single ? 0u : split;
-    b.plan[1] = (uint32_t)max(lg, b.min_lg);
-    b.plan[2] = single ? 0u : n;
-    b.plan[3] = single ? n : 0u;
-}
-
 cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t *hist,
                            uint32_t *order, int num_sms, cudaStream_t st, uint32_t *total,
                            uint32_t *bounds, bool pad, uint32_t *window_n, const uint32_t *list,
@@ -410,10 +418,9 @@ cudaError_t launch_binning(const esp_pair *pairs, uint64_t n, int mode, uint32_t
     else bin_scan_down<false><<<SCAN_BLOCKS, 256, 0, st>>>(hist, hist + NBINS);
     if (bounds) class_bounds<<<1, 32, 0, st>>>(hist, total, bounds);
     if (plan)
-        bin_scatter<true><<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, order, plan->unlike);
+        bin_scatter<true><<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, order, total, stats, *plan);
     else
-        bin_scatter<false><<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, order, nullptr);
-    if (plan) bin_plan<<<1, 32, 0, st>>>(hist, total, stats, mode, *plan);
+        bin_scatter<false><<<grid, 256, 0, st>>>(pairs, n, in, mode, hist, order, nullptr, nullptr, BinPlan{});
     return cudaGetLastError();
 }
 

@@ -63,8 +63,8 @@ struct esp_handle {
     // length at [31]; the mixed kernel's group queues at [32..33] and [34..35]
     // (second attempt), items of two geometries at [36] and [37], whether a
     // window holds N at [38], batch costs at [40..43] and [44..47], plans at
-    // [48..51] and [52..55], its units' counts from kCounters on, 4 * num_sms
-    // an attempt
+    // [48..51] and [52..55], the scatters' ended blocks at [56] and [57],
+    // the blocks begun on each SM from kCounters on, num_sms an attempt or class
     uint32_t *d_ctr = nullptr;
     int tune[esp::kLengthClasses] = {-1, -1, -1, -1};  // DP variant per length class (autotuned)
     bool tuned = false;

@@ -56,7 +56,8 @@ struct GotohJob {
     uint32_t *rb;               // row-buffer scratch: slots * rb_words * 32 words
     uint64_t rb_words;
     uint32_t *queue;            // device work counter (zeroed before launch)
-    int sms;                    // SMs of the device (0: unknown)
+    int sms;                    // SMs of the device
+    uint32_t *sm_blocks;        // paired and mixed kernels: sms zeroed device counts
     const uint32_t *window_n;   // device: whether a window may hold N (null: by n_iv_count)
     // Pairs outside the int16 domain (read longer than GotohConst::max_m):
     // the int16 kernels append them to wide_list (count in *wide_count) and
@@ -76,10 +77,9 @@ struct GotohJob {
     // them, 64 * group_tb_words and group_warp_rb for the others up to max_warps
     uint32_t thread_warps, max_warps;
     uint64_t unit_tb_words, unit_rb_words, group_warp_rb;
-    uint32_t *unit_warps;  // 4 * sms device counts (zeroed)
 };
 
-constexpr int kCounters = 64;  // words of a handle's counters (esp_handle::d_ctr) before the units'
+constexpr int kCounters = 64;  // words of a handle's counters (esp_handle::d_ctr) before those by SM
 
 // Launch the persistent DP kernel with `warps` warps total.
 // variant 0: one pair per thread, 3 resident 128-thread blocks per SM (168
@@ -192,11 +192,11 @@ cudaError_t launch_count_cells(const esp_pair *pairs, const esp_extension *out, 
 // list / list_count (device, optional): bin only the pairs list[0 ..
 // *list_count), n bounding the count (extend_hint's escalations).
 // plan (optional, with pad): also weigh the pairs and plan the mixed kernel, or
-// choose between the paired and the one-pair kernel (one launch more).
+// choose between the paired and the one-pair kernel.
 struct BinPlan {
     uint32_t *stats;  // 4 zeroed device words, 8-byte aligned (null: a list for the paired kernel)
     uint32_t *plan;   // 4 device words: GotohJob::group_plan and the two lists' lengths
-    uint32_t *unlike; // zeroed device word: items of two geometries
+    uint32_t *unlike, *done;  // zeroed device words: items of two geometries; blocks done
     bool single_ok;   // the list may go to one pair per thread
     int min_lg;         // fewest lanes (log2) the scratch was sized for
     int lanes_lg;       // lanes (log2) that have work in pairs like the costliest

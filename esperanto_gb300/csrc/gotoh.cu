@@ -2104,24 +2104,30 @@ __device__ __forceinline__ void paired_section(const GotohJob &job, const GotohC
     }
 }
 
+// How many of the launch's blocks began on this SM before this one.
+__device__ __forceinline__ uint32_t sm_turn(const GotohJob &job) {
+    __shared__ uint32_t s_turn;
+    if (threadIdx.x == 0) {
+        uint32_t sm;
+        asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+        s_turn = atomicAdd(job.sm_blocks + sm % (uint32_t)job.sms, 1u);
+    }
+    __syncthreads();
+    return s_turn;
+}
+
 // The warps of a launch take chunks of work from one queue.  With fewer chunks
-// than warps those that ask first get them, and they crowd: an SM with four
-// busy warps a scheduler takes twice the time of one with two while others
-// idle.  So each SM's second, third and fourth blocks (by the order blocks are
-// placed) wait 12,000 cycles (6 us) each for those before them; blocks that
-// find a chunk for every warp of those before them leave at once (false).
-// 65,536 pairs of 150 x 214 (1,024 chunks on 608 schedulers) 0.86 -> 0.53 ms;
-// at 2 us an SM's blocks still overtake each other in some runs.  extend_hint over
-// 20,000 pairs that all keep their first attempt 0.127 ms, 0.143 when the blocks of
-// the empty second one waited.
-__device__ __forceinline__ bool stagger(uint64_t chunks, int sms) {
-    const uint32_t warps = blockDim.x / 32;
-    if (sms <= 0 || chunks >= (uint64_t)gridDim.x * warps) return true;
-    const uint32_t turn = min(blockIdx.x / (uint32_t)sms, 3u);
-    if (chunks <= (uint64_t)turn * (uint32_t)sms * warps) return false;
-    const long long t0 = clock64(), wait = 12000ll * turn;
-    while (clock64() - t0 < wait) __nanosleep(200);
-    return true;
+// than warps those that ask first get them, and they crowd: a scheduler with three
+// busy warps takes 0.61 ms for pairs of 150 x 214, one with two 0.49, while others
+// idle.  So only as many of an SM's blocks as the chunks need of every SM stay, by
+// the order in which they begin there (block numbers do not tell: the first 152
+// blocks lie on 148 SMs, on which ones depends on the kernels before).  65,536 pairs
+// (1,024 chunks on 608 schedulers) 0.86 ms when all ask, 0.54 so; with waits of 6 us
+// by block number 0.53 or 0.65.  20,000 extend_hint pairs that all keep their first
+// attempt 0.127 ms, 0.143 when the blocks of the empty second one waited.
+__device__ __forceinline__ bool block_needed(const GotohJob &job, uint64_t chunks, uint32_t turn) {
+    const uint64_t warps = blockDim.x / 32;
+    return chunks >= gridDim.x * warps || chunks > turn * warps * (uint32_t)job.sms;
 }
 
 // Persistent paired kernel over the (class range of the) list.  Scratch per
@@ -2147,7 +2153,7 @@ __global__ void __launch_bounds__(PAIR_BLOCK, MINB) gotoh2_kernel(GotohJob job, 
         b0 = job.range[0];
         b1 = job.range[1] > job.range[0] ? job.range[1] : b0;
     }
-    if (!stagger((b1 - b0 + 63) / 64, job.sms)) return;
+    if (!block_needed(job, (b1 - b0 + 63) / 64, sm_turn(job))) return;
     paired_section(job, K, s_lut, s_lut25, b0, b1, tb, rb, lane, s_first + threadIdx.x);
 }
 
@@ -2167,7 +2173,7 @@ __global__ void __launch_bounds__(PAIR_BLOCK, MINB) gotoh2_kernel(GotohJob job, 
 // thread the chip holds 155,648 pairs before it is full.  A group of G lanes
 // takes 1/G of that time and holds 1/G of the pairs, so small and middling
 // batches fill the chip; small groups waste fewer steps at a pair's ends,
-// large ones finish it sooner (plan_dp in abi.cu and bin_plan in bins.cu choose).
+// large ones finish it sooner (plan_dp in abi.cu and make_plan in bins.cu choose).
 //
 // Cells, keys and packing are the paired kernel's.  A row is computed only
 // inside its window by predicates: `act` has a bit per row whose window holds
@@ -2603,7 +2609,7 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
 // (job.group_plan: list entries, log2 of a group's lanes), the rest two pairs
 // per thread.  A thread's pair takes as long as it takes, so the items that
 // would outlast the rest of the batch are the ones given to groups, and the
-// others keep the paired kernel's higher throughput (bin_plan, bins.cu).
+// others keep the paired kernel's higher throughput (make_plan, bins.cu).
 //
 // Two pairs a lane take several times a group's scratch.  With job.thread_warps
 // set only that many of the warps an SM starts in one of a block's four places
@@ -2627,18 +2633,17 @@ __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob jo
     const int lane = threadIdx.x & 31;
     const uint32_t total = *job.list_count;
     const uint64_t split = job.group_plan[0];
-    if (!stagger((split << job.group_plan[1]) / 64 + (total - split + 63) / 64, job.sms)) return;
+    const uint32_t turn = sm_turn(job);
+    if (!block_needed(job, (split << job.group_plan[1]) / 64 + (total - split + 63) / 64, turn)) return;
     uint64_t tb, rb;      // the warp's words
     bool threads = true;  // it owns what pairs per thread take
     if (job.thread_warps) {
-        uint32_t sm, k = 0;
+        uint32_t sm;
         asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
-        const uint32_t unit = (sm % (uint32_t)job.sms) * 4 + (threadIdx.x >> 5);
-        if (lane == 0) k = atomicAdd(job.unit_warps + unit, 1u);
-        k = __shfl_sync(0xffffffffu, k, 0);
-        if (k >= job.max_warps) return;  // more blocks here than the SM holds at a time
-        threads = k < job.thread_warps;
-        const uint64_t early = min(k, job.thread_warps), late = k - early;
+        if (sm >= (uint32_t)job.sms || turn >= job.max_warps) return;  // no words for such a block
+        const uint64_t unit = sm * 4ull + (threadIdx.x >> 5);
+        threads = turn < job.thread_warps;
+        const uint64_t early = min(turn, job.thread_warps), late = turn - early;
         tb = unit * job.unit_tb_words + early * job.warp_tb_words + late * 64 * job.group_tb_words;
         rb = unit * job.unit_rb_words + early * job.warp_rb_words + late * job.group_warp_rb;
     } else {
