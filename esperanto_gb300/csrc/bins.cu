@@ -205,7 +205,7 @@ __device__ __forceinline__ uint32_t bin_start(const uint32_t *cursor, uint32_t b
 
 // The plan of a batch that the mixed kernel may run, from the batch's costs (in
 // cells; an item is two pairs): {list entries its groups run, log2 of a group's
-// lanes, its list's length, the list's length for one pair per thread} -- one of the
+// lanes (and 8 for pairs of about one cost), its list's length, the list's length for one pair per thread} -- one of the
 // two lengths is 0.  For the paired kernel (no stats) the two lengths alone.
 //
 // A thread takes ~25 ns a row of 8 x 2 cells when its warp has the scheduler
@@ -275,7 +275,8 @@ __device__ void make_plan(const uint32_t *cursor, uint32_t n, const BinStats *st
     const bool apart = (uint64_t)unlike * UNLIKE > n / 2 && above <= 3.1f;
     const bool single = b.single_ok && (apart || (alike && !filled && above <= b.single_line));
     b.plan[0] = single ? 0u : split;
-    b.plan[1] = (uint32_t)max(lg, b.min_lg);
+    const bool same = (float)stats->cost > 0.9f * (float)stats->max_cost * (float)n;
+    b.plan[1] = (uint32_t)max(lg, b.min_lg) | (same ? 8u : 0u);
     b.plan[2] = single ? 0u : n;
     b.plan[3] = single ? n : 0u;
 }

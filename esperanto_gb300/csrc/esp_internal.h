@@ -67,7 +67,7 @@ struct GotohJob {
     uint32_t *wide_count;
     int wide;
     // mixed kernel: device {list entries run by groups, log2 of a group's
-    // lanes}, the groups' queue, and a warp's scratch, which both sections use
+    // lanes | 8 for pairs of about one cost}, the groups' queue, and a warp's scratch, which both sections use
     const uint32_t *group_plan;
     uint32_t *group_queue;
     uint64_t group_tb_words, group_rb_words;  // word pairs per lane / per group

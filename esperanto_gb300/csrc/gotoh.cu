@@ -976,13 +976,19 @@ __device__ __forceinline__ bool finish_pair(const GotohJob &job, const GotohCons
     return esc;
 }
 
+// Whether a window of the batch may hold N (counted with the bins).
+__device__ __forceinline__ bool windows_n(const GotohJob &job) {
+    return job.window_n ? *job.window_n != 0 : job.n_iv_count != 0;
+}
+
 __device__ void process_pair(const GotohJob &job, const GotohConst &K,
                              const uint32_t *__restrict__ s_lut, const int8_t *__restrict__ lut,
                              uint32_t pi, uint32_t *tb, uint32_t *rb) {
     PairSetup S;
     if (!setup_pair(job, K, pi, job.tb_words, job.rb_words, true, S)) return;
+    // one fill for the batch: lanes with N and lanes without would take turns
     FillResult F =
-        S.win.cnt ? dp_fill<true>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb)
+        windows_n(job) ? dp_fill<true>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb)
                   : dp_fill<false>(K, s_lut, S.m, S.n, S.g, S.read, S.win, tb, S.sw, rb);
     finish_pair(job, K, lut, pi, S, F, StripTb<32>{tb, S.sw});
 }
@@ -2032,11 +2038,7 @@ __device__ __noinline__ bool setup_call(const GotohJob &job, const GotohConst &K
 // the finish rather than kept live across the fill.
 constexpr uint32_t NO_PAIR = 0xffffffffu;
 
-// Whether a window of the batch may hold N (counted with the bins).
-__device__ __forceinline__ bool windows_n(const GotohJob &job) {
-    return job.window_n ? *job.window_n != 0 : job.n_iv_count != 0;
-}
-
+template <bool MAYN>
 __device__ void process_item2(const GotohJob &job, const GotohConst &K,
                               const uint32_t *__restrict__ s_lut, const int8_t *__restrict__ lut,
                               const uint32_t (&p)[2], uint32_t *tb, uint32_t *rb, uint32_t *hf) {
@@ -2065,7 +2067,7 @@ __device__ void process_item2(const GotohJob &job, const GotohConst &K,
                 }
             }
             if (now) {
-                if (windows_n(job)) fill2_call<true>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
+                if (MAYN && windows_n(job)) fill2_call<true>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
                 else fill2_call<false>(K, s_lut, A, B, tb, rb, hf, F[0], F[1]);
             }
         }
@@ -2082,6 +2084,7 @@ __device__ void process_item2(const GotohJob &job, const GotohConst &K,
 
 // Work items of two list entries each, positions b0 + 2k and b0 + 2k + 1 below
 // b1; neighbours in the binned list share their geometry key.
+template <bool MAYN>
 __device__ __forceinline__ void paired_section(const GotohJob &job, const GotohConst &K,
                                                const uint32_t *__restrict__ s_lut,
                                                const int8_t *__restrict__ lut, uint64_t b0,
@@ -2100,7 +2103,7 @@ __device__ __forceinline__ void paired_section(const GotohJob &job, const GotohC
             p[0] = job.list ? job.list[x] : (uint32_t)x;
             if (y < b1) p[1] = job.list ? job.list[y] : (uint32_t)y;
         }
-        process_item2(job, K, s_lut, lut, p, tb, rb, hf);
+        process_item2<MAYN>(job, K, s_lut, lut, p, tb, rb, hf);
     }
 }
 
@@ -2119,15 +2122,23 @@ __device__ __forceinline__ uint32_t sm_turn(const GotohJob &job) {
 // The warps of a launch take chunks of work from one queue.  With fewer chunks
 // than warps those that ask first get them, and they crowd: a scheduler with three
 // busy warps takes 0.61 ms for pairs of 150 x 214, one with two 0.49, while others
-// idle.  So only as many of an SM's blocks as the chunks need of every SM stay, by
-// the order in which they begin there (block numbers do not tell: the first 152
-// blocks lie on 148 SMs, on which ones depends on the kernels before).  65,536 pairs
-// (1,024 chunks on 608 schedulers) 0.86 ms when all ask, 0.54 so; with waits of 6 us
-// by block number 0.53 or 0.65.  20,000 extend_hint pairs that all keep their first
-// attempt 0.127 ms, 0.143 when the blocks of the empty second one waited.
-__device__ __forceinline__ bool block_needed(const GotohJob &job, uint64_t chunks, uint32_t turn) {
-    const uint64_t warps = blockDim.x / 32;
-    return chunks >= gridDim.x * warps || chunks > turn * warps * (uint32_t)job.sms;
+// idle; and of a batch of unlike pairs the costliest chunks, the list's first, crowd
+// too.  So an SM's second to fourth block (`turn` 1 to 3) wait 12,000 cycles (6 us)
+// each for those before them, and blocks that find a chunk for every warp of those
+// leave (false).  65,536 pairs (1,024 chunks on 608 schedulers) 0.86 ms when all ask
+// at once, 0.54 so.  At 2 us an SM's blocks still overtake each other in some runs.
+//
+// The turn of a block in a batch of like pairs is its order on its SM: the first
+// 152 blocks lie on 148 SMs, on which ones depends on the kernels before, and by
+// block number 65,536 pairs take 0.53 or 0.65 ms.  For unlike pairs it is by block
+// number: an SM then has chunks of all costs in each turn, not one warp a scheduler
+// left with the costliest at the end (138,000 pairs of 129 to 244 bases with N 2.25
+// ms, 2.4 by order on the SM).
+__device__ __forceinline__ bool stagger(const GotohJob &job, uint64_t chunks, uint32_t turn) {
+    if (chunks <= turn * (blockDim.x / 32ull) * (uint32_t)job.sms) return false;
+    const long long t0 = clock64(), wait = 12000ll * min(turn, 3u);
+    while (clock64() - t0 < wait) __nanosleep(200);
+    return true;
 }
 
 // Persistent paired kernel over the (class range of the) list.  Scratch per
@@ -2153,8 +2164,9 @@ __global__ void __launch_bounds__(PAIR_BLOCK, MINB) gotoh2_kernel(GotohJob job, 
         b0 = job.range[0];
         b1 = job.range[1] > job.range[0] ? job.range[1] : b0;
     }
-    if (!block_needed(job, (b1 - b0 + 63) / 64, sm_turn(job))) return;
-    paired_section(job, K, s_lut, s_lut25, b0, b1, tb, rb, lane, s_first + threadIdx.x);
+    const uint64_t chunks = (b1 - b0 + 63) / 64;
+    if (chunks < gridDim.x * (PAIR_BLOCK / 32ull) && !stagger(job, chunks, sm_turn(job))) return;
+    paired_section<true>(job, K, s_lut, s_lut25, b0, b1, tb, rb, lane, s_first + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -2507,10 +2519,11 @@ __device__ __noinline__ bool setup_group(const GotohJob &job, const GotohConst &
     return setup_pair(job, K, pi, ~0ull, ~0ull, write, S);
 }
 
-// Out of line as in the paired kernel: inlined, the walk shared registers with all
-// that the kernel keeps, and any change there moved extend_hint over 60,000 pairs
-// between 1.58 and 1.72 ms (so 1.47), over 45,000 of 50 to 150 bases between 1.14 and
-// 1.24 (1.11).
+// Out of line for batches without intervals: inlined, the walk shares registers with
+// all that the kernel keeps, and any change there moved extend_hint over 60,000
+// pairs between 1.58 and 1.72 ms (so 1.47), over 45,000 of 50 to 150 bases between
+// 1.14 and 1.24 (1.11).  Not so beside the N-taking fill, which loses more than the
+// walk gains (9,718 whole windows with N 0.31 ms, 0.35 with the walk out of line).
 __device__ __noinline__ void finish_group(const GotohJob &job, const GotohConst &K,
                                           const int8_t *__restrict__ lut, uint32_t pi, PairSetup &S,
                                           const FillResult &F, const GroupTb &tb) {
@@ -2521,6 +2534,7 @@ __device__ __noinline__ void finish_group(const GotohJob &job, const GotohConst 
 // lanes; item k is positions 2k and 2k + 1.  A warp takes 32 >> lg items at a
 // time.  Scratch: the warp's traceback region (group_tb_words word pairs per
 // lane) and row buffers (group_rb_words word pairs per group).
+template <bool MAYN>
 __device__ void group_section(const GotohJob &job, const GotohConst &K,
                               const uint32_t *__restrict__ s_lut, const int8_t *__restrict__ lut,
                               uint64_t items, int lg, uint2 *tb, uint2 *rb0, int lane,
@@ -2587,7 +2601,7 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
             if (need == 4 && fits) setup_group(job, K, p[1], false, B);
             const int all_steps = __reduce_max_sync(0xffffffffu, steps);
             FillResult FA, FB;
-            if (windows_n(job))  // as in process_item2
+            if (MAYN && windows_n(job))  // as in process_item2
                 group_fill<true>(K, s_lut, A, B, nstrips, R, all_steps, tb, rb, lane, lg, first, track, FA,
                                   FB);
             else
@@ -2598,7 +2612,8 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
                 const int gfirst = lane & ~(G - 1);
                 PairSetup &S = gl ? B : A;
                 const GroupTb view{reinterpret_cast<const uint32_t *>(tb) + gl, lg, gfirst, R, A.g.lo(1)};
-                finish_group(job, K, lut, p[gl ? 1 : q], S, gl ? FB : FA, view);
+                if (MAYN) finish_pair(job, K, lut, p[gl ? 1 : q], S, gl ? FB : FA, view);
+                else finish_group(job, K, lut, p[gl ? 1 : q], S, gl ? FB : FA, view);
             }
             __syncwarp();
         }
@@ -2618,6 +2633,8 @@ __device__ void group_section(const GotohJob &job, const GotohConst &K,
 // own part of the scratch, for groups and for pairs per thread one after the other:
 // given out over the whole chip, or apart from the groups', the same work took up
 // to a tenth longer (80,000 extend_hint pairs of 50 to 300 bases 3.5 ms, apart 3.8).
+// MAYN: the batch has N intervals, in reads or windows.
+template <bool MAYN>
 __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob job, GotohConst K) {
     static_assert(GROUP_BLOCK == PAIR_BLOCK, "one shared array serves both sections");
     __shared__ uint32_t s_lut[10];
@@ -2633,8 +2650,12 @@ __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob jo
     const int lane = threadIdx.x & 31;
     const uint32_t total = *job.list_count;
     const uint64_t split = job.group_plan[0];
-    const uint32_t turn = sm_turn(job);
-    if (!block_needed(job, (split << job.group_plan[1]) / 64 + (total - split + 63) / 64, turn)) return;
+    const uint32_t lg = job.group_plan[1] & 7u;
+    const uint64_t chunks = (split << lg) / 64 + (total - split + 63) / 64;
+    const bool few = chunks < gridDim.x * (GROUP_BLOCK / 32ull), alike = job.group_plan[1] >> 3;
+    // (a count that nothing needs would only change the order of the first chunks)
+    const uint32_t turn = (few && alike) || job.thread_warps ? sm_turn(job) : 0u;
+    if (few && !stagger(job, chunks, alike ? turn : blockIdx.x / (uint32_t)job.sms)) return;
     uint64_t tb, rb;      // the warp's words
     bool threads = true;  // it owns what pairs per thread take
     if (job.thread_warps) {
@@ -2651,17 +2672,18 @@ __global__ void __launch_bounds__(GROUP_BLOCK, 4) gotoh_mixed_kernel(GotohJob jo
         tb = warp_slot * job.warp_tb_words;
         rb = warp_slot * job.warp_rb_words;
     }
-    group_section(job, K, s_lut, s_lut25, split / 2, (int)job.group_plan[1],
+    group_section<MAYN>(job, K, s_lut, s_lut25, split / 2, (int)lg,
                   reinterpret_cast<uint2 *>(job.tb + tb), reinterpret_cast<uint2 *>(job.rb + rb), lane,
                   s_words + threadIdx.x, s_words + STRIP * GROUP_BLOCK + threadIdx.x);
     if (threads)
-        paired_section(job, K, s_lut, s_lut25, split, total, job.tb + tb + 2 * lane,
+        paired_section<MAYN>(job, K, s_lut, s_lut25, split, total, job.tb + tb + 2 * lane,
                        job.rb + rb + 2 * lane, lane, s_words + threadIdx.x);
 }
 
 cudaError_t launch_gotoh_mixed(const GotohJob &job, const GotohConst &k, int warps,
                                cudaStream_t st) {
-    gotoh_mixed_kernel<<<(warps + 3) / 4, GROUP_BLOCK, 0, st>>>(job, k);
+    if (job.n_iv_count) gotoh_mixed_kernel<true><<<(warps + 3) / 4, GROUP_BLOCK, 0, st>>>(job, k);
+    else gotoh_mixed_kernel<false><<<(warps + 3) / 4, GROUP_BLOCK, 0, st>>>(job, k);
     return cudaGetLastError();
 }
 
@@ -2745,7 +2767,7 @@ int gotoh_blocks_per_sm(int block, int variant) {
 
 int gotoh_mixed_blocks_per_sm() {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, gotoh_mixed_kernel, GROUP_BLOCK, 0) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, gotoh_mixed_kernel<true>, GROUP_BLOCK, 0) != cudaSuccess)
         return 1;
     return nb > 0 ? nb : 1;
 }
