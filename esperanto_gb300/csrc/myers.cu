@@ -282,14 +282,11 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, bool whole, uint32_t
     const char *rows = reinterpret_cast<const char *>(col);
     constexpr uint32_t ROW = MY_BLOCK * 4;  // bytes, a power of two
     uint32_t done = 0;
-    // Columns of the next chunk, 17 for 16 that go one by one beside other lanes'.
-    // The texts of global alignments are about as long as their reads, and begin
-    // with n % 16 columns (319,000 of 64 in 64 to 72 0.042 ms, the other way 0.047).
-    uint32_t cols = GLOB ? n & 15 : (whole ? 16u : ((n - 1) & 15) + 1);
-    if (!GLOB && !whole && cols == 16) cols = 17;
-    for (; done < n; done += GLOB ? cols : min(cols, 16u), cols = 16) {
-        if (GLOB && cols == 0) continue;
-        const uint32_t cnt = GLOB ? cols : min(cols, 16u);
+    // columns of the next chunk, 17 for 16 that go one by one beside other lanes'
+    uint32_t cols = whole ? 16u : ((n - 1) & 15) + 1;
+    if (!whole && cols == 16) cols = 17;
+    for (; done < n; done += min(cols, 16u), cols = 16) {
+        const uint32_t cnt = min(cols, 16u);
         CodeWin win = text_codes(job, P, tiv, rev, rev ? n - done - cnt : done, (int)cnt);
         int least = INT_MAX;
         if (cols == 16 && win.n >> 16 == 0) {
@@ -428,7 +425,7 @@ __global__ void __launch_bounds__(MY_BLOCK)
         limbs = have ? limbs_of<NW>(job.pairs[k].read_len) : 0;
     }
     limbs = max(1, __reduce_max_sync(0xffffffffu, limbs));
-    const bool whole = !GLOB && whole_texts(job, k, have);
+    const bool whole = whole_texts(job, k, have);
     if (have) myers_limbs<NW, GLOB>(job, (uint32_t)k, whole, smem, limbs);
 }
 
@@ -437,7 +434,7 @@ template <int NW, bool GLOB>
 __global__ void __launch_bounds__(MY_BLOCK) myers_kernel(const __grid_constant__ MyersJob job) {
     extern __shared__ uint32_t smem[];
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool have = k < job.n_pairs, whole = !GLOB && whole_texts(job, k, have);
+    const bool have = k < job.n_pairs, whole = whole_texts(job, k, have);
     if (have) myers_pair<NW, GLOB>(job, (uint32_t)k, whole, smem);
 }
 
