@@ -230,19 +230,16 @@ __device__ __forceinline__ uint32_t virtual_bits(int off, int w) {
 //
 // The loop is bound by the ALU (92 % busy): 10 operations a limb and column (the
 // add with carry, seven three-input logic operations, two shifts), the rest
-// counts a column.  Columns go 16 a chunk, after the text's first 1 to 16 (all
-// lanes take that part together, in as many steps as the last of them; `whole`: it
-// has 16 columns in every lane), so that a full chunk has constant shifts and no N
-// test, and its best column is the least of score * 16 + column, one operation
-// each; a column's Peq row is read a column ahead.  (A part of 0 to 15 columns
-// cost a warp 15 steps beside a full chunk wherever the longest text has a
-// multiple of 16: 300,000 reads of 30 to 60 bases 0.058 ms, so 0.051.)
+// counts a column.  Columns go 16 a chunk, after the text's first n % 16 (all
+// lanes take that partial chunk together), so that a full chunk has constant
+// shifts and no N test, and its best column is the least of score * 16 +
+// column, one operation each; a column's Peq row is read a column ahead.
 // 1,048,576 reads of 150 bases in texts of 200: 0.747 -> 0.687 ms; 12,000 of 200
 // in 260 (few warps, latency) 37.6 -> 33.5 us.  Shifts as products with 2 (the
 // multiply pipe) took fewer ALU operations and as long: their high halves
 // stall the dispatch.
 template <int NW, bool GLOB>
-__device__ void myers_pair(const MyersJob &job, uint32_t k, bool whole, uint32_t *__restrict__ peq) {
+__device__ void myers_pair(const MyersJob &job, uint32_t k, uint32_t *__restrict__ peq) {
     const esp_myers_pair P = job.pairs[k];
     const int m = (int)P.read_len;
     const uint32_t n = P.text_len;
@@ -282,14 +279,11 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, bool whole, uint32_t
     const char *rows = reinterpret_cast<const char *>(col);
     constexpr uint32_t ROW = MY_BLOCK * 4;  // bytes, a power of two
     uint32_t done = 0;
-    // columns of the next chunk, 17 for 16 that go one by one beside other lanes'
-    uint32_t cols = whole ? 16u : ((n - 1) & 15) + 1;
-    if (!whole && cols == 16) cols = 17;
-    for (; done < n; done += min(cols, 16u), cols = 16) {
-        const uint32_t cnt = min(cols, 16u);
+    for (uint32_t cnt = n & 15; done < n; done += cnt, cnt = 16) {
+        if (cnt == 0) continue;
         CodeWin win = text_codes(job, P, tiv, rev, rev ? n - done - cnt : done, (int)cnt);
         int least = INT_MAX;
-        if (cols == 16 && win.n >> 16 == 0) {
+        if (cnt == 16 && win.n >> 16 == 0) {
             constexpr int STEP = 2;  // columns unrolled
             uint32_t next[NW];  // the next column's Peq row, read a column ahead
             const uint32_t *pe = reinterpret_cast<const uint32_t *>(rows + (win.c >> 30) * ROW);
@@ -351,21 +345,15 @@ __device__ void myers_pair(const MyersJob &job, uint32_t k, bool whole, uint32_t
 }
 
 template <int NW, bool GLOB>
-__device__ __noinline__ void myers_call(const MyersJob &job, uint32_t k, bool whole, uint32_t *peq) {
-    myers_pair<NW, GLOB>(job, k, whole, peq);
-}
-
-// Whether the texts of all the warp's pairs have a multiple of 16 columns.
-__device__ __forceinline__ bool whole_texts(const MyersJob &job, uint64_t k, bool have) {
-    return __all_sync(0xffffffffu, !have || job.pairs[k].text_len % 16 == 0);
+__device__ __noinline__ void myers_call(const MyersJob &job, uint32_t k, uint32_t *peq) {
+    myers_pair<NW, GLOB>(job, k, peq);
 }
 
 // The limbs of the warp's longest read, 1..NW, choose its pairs' code.
 template <int NW, bool GLOB>
-__device__ __forceinline__ void myers_limbs(const MyersJob &job, uint32_t k, bool whole, uint32_t *peq,
-                                            int limbs) {
-    if (limbs == NW) myers_call<NW, GLOB>(job, k, whole, peq);
-    else if constexpr (NW > 1) myers_limbs<NW - 1, GLOB>(job, k, whole, peq, limbs);
+__device__ __forceinline__ void myers_limbs(const MyersJob &job, uint32_t k, uint32_t *peq, int limbs) {
+    if (limbs == NW) myers_call<NW, GLOB>(job, k, peq);
+    else if constexpr (NW > 1) myers_limbs<NW - 1, GLOB>(job, k, peq, limbs);
 }
 
 template <int NW>
@@ -425,8 +413,7 @@ __global__ void __launch_bounds__(MY_BLOCK)
         limbs = have ? limbs_of<NW>(job.pairs[k].read_len) : 0;
     }
     limbs = max(1, __reduce_max_sync(0xffffffffu, limbs));
-    const bool whole = whole_texts(job, k, have);
-    if (have) myers_limbs<NW, GLOB>(job, (uint32_t)k, whole, smem, limbs);
+    if (have) myers_limbs<NW, GLOB>(job, (uint32_t)k, smem, limbs);
 }
 
 // A thread a pair, in the batch's order.
@@ -434,8 +421,7 @@ template <int NW, bool GLOB>
 __global__ void __launch_bounds__(MY_BLOCK) myers_kernel(const __grid_constant__ MyersJob job) {
     extern __shared__ uint32_t smem[];
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool have = k < job.n_pairs, whole = whole_texts(job, k, have);
-    if (have) myers_pair<NW, GLOB>(job, (uint32_t)k, whole, smem);
+    if (k < job.n_pairs) myers_pair<NW, GLOB>(job, (uint32_t)k, smem);
 }
 
 template <int NW, bool GLOB>
