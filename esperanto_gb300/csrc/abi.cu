@@ -118,7 +118,9 @@ void settle_kernel_choices(esp_handle *h) {
 // 9 columns after the one above it and ends after w + 7, so that about (w + 8) / 9
 // do.  9,000 pairs of 150 in 65 columns 0.31 ms with 16 lanes, 0.22 with 8; of
 // 50 in 33 columns 0.156 with 16, 0.107 with 4; 30,000 whole windows of 64 rows
-// 0.39 with 4, 0.33 with 8.
+// 0.39 with 4, 0.33 with 8.  Where that is all of a short read's strips they are
+// rounded up, as those of whole windows: 5,541 pairs of 86 in 257 columns 0.42 with 8,
+// 0.345 with 16.
 // single_line: up to how far above the mean finish (make_plan) such pairs run
 // one per thread, which the lanes' empty ends at the first and the last strips
 // make the faster way.  In groups and one per thread, in ms: 6,500 pairs of 50 in 33
@@ -135,7 +137,7 @@ static GroupShape group_shape(const Limits &L) {
     const uint64_t strips = (L.max_m + 7ull) / 8;
     const bool flat = L.rb_words >= L.max_n;  // rb_words: w + 7 for a band
     const uint64_t busy = flat ? strips : std::min(strips, (L.rb_words + 1) / 9);
-    if (flat) g.lanes_lg = busy <= 4 ? 2 : (busy <= 8 ? 3 : (busy <= 16 ? 4 : 5));
+    if (busy == strips) g.lanes_lg = busy <= 4 ? 2 : (busy <= 8 ? 3 : (busy <= 16 ? 4 : 5));
     else g.lanes_lg = busy < 6 ? 2 : (busy < 12 ? 3 : (busy < 23 ? 4 : 5));
     if (strips <= 4) g.single_line = 1e9f;  // 9,000 pairs of 30 rows 0.088 / 0.078
     else if (!flat) g.single_line = strips > 16 ? 1.75f : (g.lanes_lg == 2 ? 8.0f : 2.6f);
@@ -195,12 +197,16 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
         P.all_groups = x * 0.4 > 1.1;
         const bool pairs_ok = x * 0.4 <= 1.25;
         const int least = !P.all_groups || x < 5 ? 2 : (x < 11 ? 3 : (x < 60 ? 4 : 5));
-        uint64_t want = 0;
+        uint64_t want = 0;  // as many warps as groups of the fewest lanes fill
         auto size = [&](int lg) {  // lg: a lower bound of the lanes
             P.gtw = P.grw = 0;
             uint32_t row_buffers = 0;  // of a warp
-            // (a launch that leaves schedulers idle may take more lanes an item)
+            // (a launch that leaves schedulers idle may take more lanes an item, and
+            // one of unlike pairs as many as the costliest ask for: 7,441 of 52 to 253
+            // in 33 columns 0.50 ms with the warps of the fewest lanes, 0.37 so)
             want = std::min(P.all_groups ? resident / 4 : resident, items);
+            const uint32_t wide = 32u >> std::max(lg, least);
+            const uint64_t most = std::max(want, std::min(resident, (items + wide - 1) / wide));
             for (int a = 0; a < (mode == ESP_MODE_HINT ? 2 : 1); a++) {
                 const Limits &L = a ? L2 : L1;
                 P.shape[a] = group_shape(L);
@@ -215,7 +221,7 @@ static DpPlan plan_dp(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L
             P.gwr = 2 * P.grw * row_buffers;
             P.wtb = pairs_ok ? std::max(P.gwt, 64 * P.tbw) : P.gwt;
             P.wrb = pairs_ok ? std::max(P.gwr, 64 * P.rbw) : P.gwr;
-            P.warps = std::min(want, std::max<uint64_t>(1, h->scratch_budget / ((P.wtb + P.wrb) * 4)));
+            P.warps = std::min(std::max(want, most), std::max<uint64_t>(1, h->scratch_budget / ((P.wtb + P.wrb) * 4)));
             P.warps = (P.warps + 3) / 4 * 4;  // whole blocks: every launched warp owns its scratch
             return P.warps >= want;
         };
