@@ -50,7 +50,7 @@ MYERS_OPS_PER_CELL = 10.0 / 32.0
 # and the Myers batch (1,048,576 pairs, one launch); the mixed-length batch
 # per DP cell, captured on a
 # 524,288-pair case of the same distribution and scaled by cells.
-TRAFFIC_BYTES = {0: 29.8e6 + 358.9e6, 1: 125.4e6 + 8.4e6}
+TRAFFIC_BYTES = {0: 29.5e6 + 353.1e6, 1: 125.4e6 + 5.4e6}
 # keyed by (workload, SIMD lanes): one pair per thread, two pairs per thread
 TRAFFIC_PER_CELL = {(2, 1): (2713001472 + 6431804160) / 7716062109,
                     (2, 2): (3486293760 + 7249786624) / 7716062109}

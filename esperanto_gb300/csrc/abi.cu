@@ -32,7 +32,9 @@ static void resolve_variant(esp_handle *h) {
 // handle left at the default runs batches of 2^18 pairs and more on the paired
 // kernel (262,144 pairs of 150 x 214 in 1.51 ms against 2.44 with one pair per
 // thread, mixed 3.52 / 4.63; 600,000 mixed 4.94 / 8.16).  esp_batch_autotune
-// measures instead of assuming.
+// measures instead of assuming.  (Where the band offsets of one size's pairs differ
+// in more than a few items, the list goes to the one-pair kernel all the same:
+// make_plan, bins.cu.)
 static int band_variant(esp_handle *h, uint64_t n) {
     resolve_variant(h);
     if (h->variant_by_size && h->binning && n >= (1u << 18)) return 3;

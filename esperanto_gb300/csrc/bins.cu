@@ -232,8 +232,9 @@ __device__ __forceinline__ uint32_t bin_start(const uint32_t *cursor, uint32_t b
 // batch takes groups at half their rate (3.1 times the mean finish): 65,536 pairs of
 // 150 x 214 at offsets of 12 to 52 1.68 -> 0.77 ms, 200,000 mixed pairs 7.1 -> 4.8;
 // 4,096 mixed pairs stay with groups (0.83, one per thread 1.84; 65,536 3.5 /
-// 3.6, about even).  In large batches one warp's second pass weighs less: 600,000 pairs of which
-// 0.5 % are at other offsets take 4.4 ms in pairs, 2 % 5.9, one per thread 5.2.
+// 3.6, about even).  In large batches one warp's second pass weighs less: 600,000
+// pairs of which 0.5 % are at other offsets take 4.4 ms in pairs, 2 % 5.9, one per
+// thread 5.2.
 constexpr uint32_t UNLIKE = 256, UNLIKE_LARGE = 48, SAMPLE = 16;
 
 __device__ void make_plan(const uint32_t *cursor, uint32_t n, const BinStats *stats, int mode,
@@ -250,8 +251,8 @@ __device__ void make_plan(const uint32_t *cursor, uint32_t n, const BinStats *st
     const float above = even > 0.0f ? top / even : 0.0f;
     const float x = above / 0.4f;
     int lg = x < 5.0f ? 2 : (x < 11.0f ? 3 : (x < 60.0f ? 4 : 5));
-    // (42,555 whole windows of 112 to 155 bases, 0.69 of their costliest:
-    // 1.51 ms as alike, 1.34 not; 93,996 extend_hint pairs of 133 to 270 5.8, 4.36)
+    // (42,555 whole windows of 112 to 155 bases, 0.69 of their costliest, 1.51 ms
+    // as alike, 1.34 not; 93,996 extend_hint pairs of 133 to 270 5.8, 4.36)
     const bool alike = (float)stats->cost > 0.8f * (float)stats->max_cost * (float)n;
     const bool filled = 2.0f * (float)n > b.threads;  // one per thread: over two warps a scheduler
     uint32_t split = 0;

@@ -258,9 +258,9 @@ void settle_kernel_choices(esp_handle *h);
 void dp_scratch_bytes(esp_handle *h, int mode, uint64_t n_pairs, const Limits &L1,
                       const Limits &L2, uint64_t &tb_bytes, uint64_t &rb_bytes);
 
-// Grow a handle's escalation and binning lists once for one-pair-kernel
-// batches of up to max_pairs pairs (abi.cu), so later batches of that size
-// allocate nothing but their DP scratch.
+// Grow a handle's escalation and binning lists once for batches of up to
+// max_pairs pairs, whatever kernel they run (abi.cu), so later batches of that
+// size allocate nothing but their DP scratch.
 int reserve_lists(esp_handle *h, uint64_t max_pairs);
 
 // The spliced pseudo-reference DP over exon slices (spliced.cu): gather the

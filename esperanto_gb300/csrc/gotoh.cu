@@ -1049,7 +1049,7 @@ __global__ void __launch_bounds__(128, MINB) gotoh_kernel(GotohJob job, GotohCon
 // are applied by selects (a branch a row ends the overlap), and a third pass of
 // strips no longer waits for the second.  Measured against one column a step,
 // a pass at a time: one extend_hint call of 150 x 214 111 -> 104 us, with its
-// second attempt 197 -> 172; 1,000 mixed pairs in bands 0.38 -> 0.295 ms, 2,000
+// second attempt 197 -> 172; 1,000 mixed pairs in bands 0.38 -> 0.277 ms, 2,000
 // 0.54 ms.  Strips of 2 or 4 rows (more lanes at work in a band) were slower:
 // 122 and 257 us, since a step's shuffles, windows and vote cost as before.
 // ---------------------------------------------------------------------------
